@@ -2404,11 +2404,19 @@ __global__ void __launch_bounds__(256) rerank_kernel(ArenaLayout L, const float*
 // Device-side fallback: gather / scatter of the overflowed queries.
 __global__ void fb_gather_kernel(const int32_t* __restrict__ ovf, const float* __restrict__ q,
                                  const int64_t* __restrict__ probes, int nprobe, int d, int cap, float* __restrict__ fq,
-                                 int64_t* __restrict__ fprobes, int32_t* __restrict__ fcount) {
+                                 int64_t* __restrict__ fprobes, int32_t* __restrict__ fcount,
+                                 const float* __restrict__ thr, const uint32_t* __restrict__ kthr,
+                                 uint32_t* __restrict__ gthr) {
     const int cnt = min(ovf[0], cap);
     if (blockIdx.x == 0 && threadIdx.x == 0) *fcount = cnt;
     for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
         const int qi = ovf[1 + i];
+        // The query's threshold so far bounds its k-th distance from above
+        // (none unless it is a number below FLT_MAX).
+        if (threadIdx.x == 0) {
+            const float t = thr ? thr[qi] : o2f(kthr[qi]);
+            gthr[i] = t < FLT_MAX ? f2o(t) : 0xffffffffu;
+        }
         for (int j = threadIdx.x; j < d; j += blockDim.x) fq[static_cast<size_t>(i) * d + j] = q[static_cast<size_t>(qi) * d + j];
         for (int j = threadIdx.x; j < nprobe; j += blockDim.x)
             fprobes[static_cast<size_t>(i) * nprobe + j] = probes[static_cast<size_t>(qi) * nprobe + j];
@@ -2490,8 +2498,9 @@ cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qa
 }
 
 cudaError_t launch_fb_gather(const int32_t* ovf, const float* q, const int64_t* probes, int nprobe, int d, int cap,
-                             float* fq, int64_t* fprobes, int32_t* fcount, cudaStream_t s) {
-    fb_gather_kernel<<<64, 128, 0, s>>>(ovf, q, probes, nprobe, d, cap, fq, fprobes, fcount);
+                             float* fq, int64_t* fprobes, int32_t* fcount, const float* thr, const uint32_t* kthr,
+                             uint32_t* gthr, cudaStream_t s) {
+    fb_gather_kernel<<<64, 128, 0, s>>>(ovf, q, probes, nprobe, d, cap, fq, fprobes, fcount, thr, kthr, gthr);
     return cudaGetLastError();
 }
 

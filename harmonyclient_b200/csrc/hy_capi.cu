@@ -479,25 +479,37 @@ int check_search_args(hy_index* h, size_t n, size_t k) {
 // Search n device queries with device probe lists (nprobe per query) into
 // device D/I.  Runs on stream s; does not synchronise.
 // nq_dev (optional): a device count of the queries to search (the first
-// *nq_dev of the n); the scan's CTAs then loop over them, one wave of
-// query slots per SM.
+// *nq_dev of the n): one CTA per SM loops over their work units, whose
+// splits follow from the count, and the shared thresholds (w_gthr) hold each
+// query's starting bound (launch_fb_gather).
 int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t nprobe, const int64_t* dprobes,
                    const uint32_t* init_thr, float* dD, int64_t* dI, cudaStream_t s, bool timed,
                    int64_t* drows = nullptr, const int32_t* nq_dev = nullptr) {
     const int kp = k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 256;
-    int nsplit = 1;
-    const size_t target_ctas = 2 * 148;
-    if (n < target_ctas) nsplit = (int)std::min<size_t>((target_ctas + n - 1) / n, std::max<size_t>(nprobe, 1));
-    while ((nprobe + nsplit - 1) / nsplit > 2048) ++nsplit;
-    HY_RET(h->w_parts.ensure(n * nsplit * kp * sizeof(uint64_t)));
+    if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
+    const int pparts = hy::scan_probe_parts(h->L, (int)k, (int)nprobe);
+    // Tile splits: SCAN_WAVES work units per SM (one CTA fills an SM), so the
+    // last wave is short, but no more than leaves every warp of a unit a tile
+    // of an average probe list (16 warps).  A single wave for up to a few
+    // queries: their units are as even as the tiles.
+    constexpr size_t SCAN_WAVES = 4;
+    const size_t nsm = (size_t)h->nsm;
+    const size_t tiles = std::max<size_t>(1, h->arena_rows / 32 / std::max<size_t>(h->nlist, 1) * nprobe);
+    size_t tsplit = n * 4 <= nsm ? nsm / std::max<size_t>(n, 1) : (SCAN_WAVES * nsm + n - 1) / n;
+    tsplit = std::max<size_t>(1, std::min(tsplit, (tiles + 7) / 8));
+    const size_t all = n * (size_t)pparts;
+    HY_RET(h->w_parts.ensure((nq_dev ? std::max(all, nsm) : all * tsplit) * kp * sizeof(uint64_t)));
     uint32_t* gthr = nullptr;
-    if (nsplit > 1) {
+    if (nq_dev) {
+        gthr = h->w_gthr.as<uint32_t>();  // set by the gather of the counted queries
+    } else if (pparts * tsplit > 1) {
         HY_RET(h->w_gthr.ensure(n * sizeof(uint32_t)));
         gthr = h->w_gthr.as<uint32_t>();
         if (init_thr)
             HY_CUDA(cudaMemcpyAsync(gthr, init_thr, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
         else
             HY_CUDA(cudaMemsetAsync(gthr, 0xff, n * sizeof(uint32_t), s));
+        h->launches += 1;
     }
     hy::ScanParams p;
     p.L = h->L;
@@ -513,24 +525,21 @@ int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t npro
     p.err = h->w_err.as<int>();
     p.nq = (int)n;
     p.nprobe = (int)nprobe;
-    p.nsplit = nsplit;
+    p.pparts = pparts;
+    p.tsplit = (int)tsplit;
     p.k = (int)k;
     p.metric = h->metric;
     p.prune = 1;
     p.nq_dev = nq_dev;
-    if (nq_dev) {
-        if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
-        p.qgrid = h->nsm;
-    }
+    p.units = h->nsm;
     if (timed) HY_CUDA(ev_record(h->ev[2], s));
-    h->launches += 2 + (nsplit > 1 ? 1 : 0);
+    h->launches += 2;
     int smem = 0;
     cudaError_t e = hy::launch_scan_plain(p, &smem, s);
     if (e != cudaSuccess)
         return fail(HY_ERR_CUDA, std::string("scan launch (") + std::to_string(smem) + " B shared): " + cudaGetErrorString(e));
     if (timed) HY_CUDA(ev_record(h->ev[3], s));
-    HY_CUDA(hy::launch_merge(h->w_parts.as<uint64_t>(), (int)n, nsplit, kp, (int)k, h->metric, h->ids.as<int64_t>(),
-                             dD, dI, s, drows, nq_dev));
+    HY_CUDA(hy::launch_merge(p, h->ids.as<int64_t>(), dD, dI, s, drows));
     if (timed) HY_CUDA(ev_record(h->ev[4], s));
     return HY_OK;
 }
@@ -667,8 +676,10 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
     HY_CUDA(hy::launch_list_topk(p.cand, p.cand_cnt, (int)m, (int)capq, (int)k, h->metric, 1, thr,
                                  h->ids.as<int64_t>(), dD, dI, ovf, s));
     // Overflowed queries: the query-major scan over the same probe lists.
+    HY_RET(h->w_gthr.ensure(m * sizeof(uint32_t)));
     HY_CUDA(hy::launch_fb_gather(ovf, qq, probes, (int)nprobe, (int)h->d, (int)m, h->b_fq.as<float>(),
-                                 h->b_fpr.as<int64_t>(), h->b_fcnt.as<int32_t>(), s));
+                                 h->b_fpr.as<int64_t>(), h->b_fcnt.as<int32_t>(), nullptr, thr,
+                                 h->w_gthr.as<uint32_t>(), s));
     HY_RET(scan_and_merge(h, m, h->b_fq.as<float>(), k, nprobe, h->b_fpr.as<int64_t>(), nullptr, h->b_fD.as<float>(),
                           h->b_fI.as<int64_t>(), s, false, nullptr, h->b_fcnt.as<int32_t>()));
     HY_CUDA(hy::launch_fb_scatter(ovf, h->b_fD.as<float>(), h->b_fI.as<int64_t>(), (int)k, (int)m, dD, dI,
@@ -995,6 +1006,7 @@ int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD
     // Exact fallback on the device: every overflowed query of a chunk is
     // searched again by the plain scan over the same probe lists.
     const size_t fbcap = qc;
+    HY_RET(h->w_gthr.ensure(fbcap * sizeof(uint32_t)));
     HY_RET(h->b_fq.ensure(fbcap * h->d * sizeof(float)));
     HY_RET(h->b_fpr.ensure(fbcap * nprobe * sizeof(int64_t)));
     HY_RET(h->b_fD.ensure(fbcap * k * sizeof(float)));
@@ -1154,7 +1166,8 @@ int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[4], s));
         const int fb = (int)std::min<size_t>(m, fbcap);
         HY_CUDA(hy::launch_fb_gather(w.overflow, qq, h->w_probes.as<int64_t>(), (int)nprobe, (int)h->d, fb,
-                                     h->b_fq.as<float>(), h->b_fpr.as<int64_t>(), h->b_fcnt.as<int32_t>(), s));
+                                     h->b_fq.as<float>(), h->b_fpr.as<int64_t>(), h->b_fcnt.as<int32_t>(),
+                                     h->b_thr.as<float>(), nullptr, h->w_gthr.as<uint32_t>(), s));
         HY_RET(scan_and_merge(h, (size_t)fb, h->b_fq.as<float>(), k, nprobe, h->b_fpr.as<int64_t>(), nullptr,
                               h->b_fD.as<float>(), h->b_fI.as<int64_t>(), s, false, nullptr, h->b_fcnt.as<int32_t>()));
         HY_CUDA(hy::launch_fb_scatter(w.overflow, h->b_fD.as<float>(), h->b_fI.as<int64_t>(), (int)k, fb, dD + q0 * k,

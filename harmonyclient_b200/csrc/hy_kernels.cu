@@ -347,22 +347,30 @@ __global__ void __launch_bounds__(256) warmup_warp_kernel(const __grid_constant_
 // ---------------------------------------------------------------------------
 // The plain FP32 list scan.
 //
-// Grid: one CTA per (query, split); split s handles probes j = s, s+nsplit, ...
-// (the reference's vector partition across teams becomes a partition of the
-// probe list across CTAs).  Each CTA enumerates the 32-row tiles of its lists
-// and its warps take tiles from a shared counter.  A warp runs S independent
+// Grid: one CTA per (query, split): a query's probe list in pparts parts (one
+// unless the probe table outgrows shared memory), a part's 32-row tiles dealt
+// round robin to tsplit CTAs (the reference's vector partition across teams
+// becomes a partition of the rows across CTAs), so a few queries still fill
+// the chip however uneven their lists are (whole lists per CTA left one query
+// of nprobe 64 on 64 CTAs that waited for the longest list).  With a device count of queries the
+// splits follow from it and the CTAs loop over the work units.  Each CTA's
+// warps take its tiles from a shared counter.  A warp runs S independent
 // tile slots: each slot loads one dimension block of its tile with a bulk
 // copy, accumulates the block into every lane's partial distance (lane = row),
 // prunes rows whose partial exceeds the query's running threshold, and loads
 // the next block only if some row of the tile is still alive — so pruned
 // tiles stop costing HBM bytes (the reference's DIVIDE_DIM / in-rank 4-chunk
 // prune, src/node.cpp:634-657 and 1055-1114, moved inside one kernel).
-// Survivors enter a per-warp candidate buffer.  The CTA keeps one sorted
-// top-K' (K' = 32*KR >= k) in shared memory; a warp whose buffer fills takes
-// the CTA's merge lock, merges its candidates into that list with register
-// bitonic networks and lowers the CTA threshold to the list's k-th key, so
-// the threshold reflects every row the CTA has seen.  At the end the list
-// holds the CTA's K' best keys.
+// Survivors enter a per-warp candidate buffer; 32 of them are folded into the
+// warp's own sorted top-K' (K' = 32*KR >= k, register bitonic networks), which
+// the warp publishes into the CTA's shared top-K' whenever no other warp is
+// doing so, lowering the thresholds to that list's k-th key.  No warp waits
+// for the shared list; what was not published is folded in at the end.  Bound
+// by HBM latency and bandwidth for few queries.  Measured, 1M x 128, nprobe
+// 64: one query 252 -> 20 us (93 MB of tiles: 4.7 TB/s), where tiles without
+// the waitless fold took 258 us (85 % of the warps' time went to the merge
+// lock); 33 queries on 200k x 97, nprobe 20: 566 -> 64 us; 1 to 14 overflowed
+// queries of a tensor-core search: 0.99-3.3 ms -> 0.07 ms and less.
 //
 // Threshold = min(warm-up threshold, the CTA list's k-th key, the k-th key
 // published by other splits of the query).  Each is an upper bound
@@ -376,15 +384,12 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
     const ArenaLayout& L = p.L;
     const int W = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = blockIdx.x % p.nsplit;
-    // Queries of this CTA: blockIdx.x / nsplit, then every (grid / nsplit)-th
-    // after it, below the device count when one is given (a grid of nq *
-    // nsplit CTAs takes one query each).
     const int nq_eff = p.nq_dev ? min(*p.nq_dev, p.nq) : p.nq;
-    const int qstride = gridDim.x / p.nsplit;
-    if (static_cast<int>(blockIdx.x / p.nsplit) >= nq_eff) return;  // whole CTA, before any barrier
-    const int npc = (p.nprobe - split + p.nsplit - 1) / p.nsplit;  // probes of this CTA
-    const int npa = ((p.nprobe + p.nsplit - 1) / p.nsplit + 3) & ~3;  // table entries, padded for alignment
+    const int tsplit = p.nq_dev ? scan_tile_splits(p.units, nq_eff, p.pparts) : p.tsplit;
+    const int nsplit = p.pparts * tsplit;
+    const long long nunits = static_cast<long long>(nq_eff) * nsplit;
+    if (blockIdx.x >= nunits) return;  // whole CTA, before any barrier
+    const int npa = ((p.nprobe + p.pparts - 1) / p.pparts + 3) & ~3;  // table entries, padded for alignment
     const size_t slot_floats = static_cast<size_t>(32) * L.max_pitch;
 
     float* bufs = reinterpret_cast<float*>(smem);
@@ -408,30 +413,26 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
 #pragma unroll
     for (int s = 0; s < S; ++s) sphase[s] = 0;
 
-    for (int qi = blockIdx.x / p.nsplit; qi < nq_eff; qi += qstride) {
-    // The previous query's result has been copied out (and, first time, the
+    for (long long unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
+    const int qi = static_cast<int>(unit / nsplit), split = static_cast<int>(unit % nsplit);
+    const int part = split / tsplit, tofs = split % tsplit;
+    const int npc = (p.nprobe - part + p.pparts - 1) / p.pparts;  // probes of this part
+    // The previous unit's result has been copied out (and, first time, the
     // barriers are initialised) before the shared state is set up again.
     __syncthreads();
     // --- CTA setup: query, probe table (tile prefix), threshold.
     stage_query(L, p.q + static_cast<size_t>(qi) * L.d, qs);
+    for (int m = threadIdx.x; m < npc; m += blockDim.x) {
+        const int64_t l = p.probes[static_cast<size_t>(qi) * p.nprobe + part + static_cast<size_t>(m) * p.pparts];
+        s_size[m] = l >= 0 ? p.list_size[l] : 0;
+        s_row0[m] = l >= 0 ? p.list_off[l] : 0;
+    }
+    __syncthreads();
     if (warp == 0) {
         int carry = 0;
         for (int base = 0; base < npc; base += 32) {
             const int m = base + lane;
-            int tiles = 0;
-            if (m < npc) {
-                const int64_t l = p.probes[static_cast<size_t>(qi) * p.nprobe + split + static_cast<size_t>(m) * p.nsplit];
-                int sz = 0;
-                int64_t r0 = 0;
-                if (l >= 0) {
-                    sz = p.list_size[l];
-                    r0 = p.list_off[l];
-                }
-                s_size[m] = sz;
-                s_row0[m] = r0;
-                tiles = (sz + 31) >> 5;
-            }
-            int incl = tiles;
+            int incl = m < npc ? (s_size[m] + 31) >> 5 : 0;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int t = __shfl_up_sync(FULL, incl, o);
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
         }
         if (lane == 0) {
             s_ntiles = carry;
-            s_next = 0;
+            s_next = tofs;
             s_lock = 0;
             s_thr = p.init_thr ? p.init_thr[qi] : 0xffffffffu;
         }
@@ -458,6 +459,9 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
     const bool prune = p.prune && l2;
 
     int ccount = 0;
+    uint64_t own[KR];  // this warp's sorted best keys not yet in the CTA's list
+#pragma unroll
+    for (int r = 0; r < KR; ++r) own[r] = KEY_MAX;
     unsigned long long loaded = 0, possible = 0;
     uint32_t gcache = p.g_thr ? p.g_thr[qi] : 0xffffffffu;
 
@@ -495,7 +499,7 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
 
     auto grab = [&](int s) -> bool {
         int g = 0;
-        if (lane == 0) g = atomicAdd(&s_next, 1);
+        if (lane == 0) g = atomicAdd(&s_next, tsplit);
         g = __shfl_sync(FULL, g, 0);
         if (g >= ntiles) return false;
         int lo = 0, hi = npc - 1;
@@ -519,52 +523,61 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
         return true;
     };
 
-    // Merge this warp's candidates into the CTA list under the merge lock
-    // (bounded spin; on timeout the device status word is raised).
+    // Publish this warp's list into the CTA's if no other warp is doing so
+    // (the warp never waits: what is not published now is later, or in the
+    // final fold) and lower the thresholds to the merged list's k-th key.
+    auto publish = [&]() {
+        int got = 0;
+        if (lane == 0) got = atomicCAS(&s_lock, 0, 1) == 0;
+        got = __shfl_sync(FULL, got, 0);
+        if (!got) return;
+        __threadfence_block();
+        volatile uint64_t* vt = ctop;
+        uint64_t t[KR];
+#pragma unroll
+        for (int r = 0; r < KR; ++r) t[r] = vt[r * 32 + lane];
+        warp_merge<KR>(t, own, lane);
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+            vt[r * 32 + lane] = t[r];
+            own[r] = KEY_MAX;
+        }
+        const uint64_t kth = warp_get<KR>(t, p.k - 1);
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) {
+            atomicExch(&s_lock, 0);
+            if (kth != KEY_MAX) {
+                const uint32_t key = static_cast<uint32_t>(kth >> 32);
+                if (key < atomicMin(&s_thr, key) && p.g_thr) atomicMin(&p.g_thr[qi], key);
+            }
+        }
+    };
+
+    // Fold this warp's buffered candidates that still reach the threshold
+    // into its own sorted list, then try to publish it.
     auto flush = [&]() {
         __syncwarp();
-        int got = 0;
-        if (lane == 0) {
-            for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-                if (atomicCAS(&s_lock, 0, 1) == 0) {
-                    got = 1;
-                    break;
-                }
-                __nanosleep(32);
-            }
-            if (!got) atomicCAS(p.err, 0, DEV_ERR_TIMEOUT);
-        }
-        got = __shfl_sync(FULL, got, 0);
-        if (got) {
-            __threadfence_block();
-            volatile uint64_t* vt = ctop;
-            uint64_t t[KR];
+        const uint32_t now = min(*reinterpret_cast<volatile unsigned int*>(&s_thr), gcache);
+        bool any = false;
+        for (int base = 0; base < ccount; base += KP) {
+            uint64_t c[KR];
+            bool have = false;
 #pragma unroll
-            for (int r = 0; r < KR; ++r) t[r] = vt[r * 32 + lane];
-            for (int base = 0; base < ccount; base += KP) {
-                uint64_t c[KR];
-#pragma unroll
-                for (int r = 0; r < KR; ++r) {
-                    const int idx = base + r * 32 + lane;
-                    c[r] = idx < ccount ? wc[idx] : KEY_MAX;
-                }
-                warp_sort<KR>(c, lane);
-                warp_merge<KR>(t, c, lane);
+            for (int r = 0; r < KR; ++r) {
+                const int idx = base + r * 32 + lane;
+                c[r] = idx < ccount ? wc[idx] : KEY_MAX;
+                if (static_cast<uint32_t>(c[r] >> 32) > now) c[r] = KEY_MAX;
+                have |= c[r] != KEY_MAX;
             }
-#pragma unroll
-            for (int r = 0; r < KR; ++r) vt[r * 32 + lane] = t[r];
-            const uint64_t kth = warp_get<KR>(t, p.k - 1);
-            if (kth != KEY_MAX && lane == 0) {
-                const uint32_t key = static_cast<uint32_t>(kth >> 32);
-                atomicMin(&s_thr, key);
-                if (p.g_thr) atomicMin(&p.g_thr[qi], key);
-            }
-            __threadfence_block();
-            __syncwarp();
-            if (lane == 0) atomicExch(&s_lock, 0);
+            if (!__any_sync(FULL, have)) continue;
+            any = true;
+            warp_sort<KR>(c, lane);
+            warp_merge<KR>(own, c, lane);
         }
         __syncwarp();
         ccount = 0;
+        if (any) publish();
     };
 
 #pragma unroll
@@ -661,14 +674,14 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
             const unsigned bal = __ballot_sync(FULL, isc);
             if (bal) {
                 const int nc = __popc(bal);
-                // Merge once 32 candidates are buffered (or the buffer would
-                // overflow), so the CTA threshold follows the scan closely.
-                if (ccount + nc > CAP || ccount >= 32) flush();
                 if (isc) {
                     const int pos = ccount + __popc(bal & ((1u << lane) - 1u));
                     wc[pos] = (static_cast<uint64_t>(f2o(score)) << 32) | static_cast<uint32_t>(srow[s] + lane);
                 }
                 ccount += nc;
+                // Fold once 32 candidates are buffered (room for the next
+                // tile's 32 remains), so the thresholds follow the scan.
+                if (ccount >= 32) flush();
             }
         }
         sact[s] = grab(s);
@@ -714,51 +727,108 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
         atomicAdd(&p.counters[0], loaded);
         atomicAdd(&p.counters[1], possible);
     }
+    // The warps' unpublished lists, folded pairwise through the candidate
+    // buffers (each as large as two lists), and then into the CTA's list.
+    for (int h = W >> 1; h > 0; h >>= 1) {
+        __syncthreads();
+        if (warp >= h && warp < 2 * h) {
+#pragma unroll
+            for (int r = 0; r < KR; ++r) cand[(warp - h) * CAP + r * 32 + lane] = own[r];
+        }
+        __syncthreads();
+        if (warp < h) {
+            uint64_t c[KR];
+#pragma unroll
+            for (int r = 0; r < KR; ++r) c[r] = cand[warp * CAP + r * 32 + lane];
+            if (__shfl_sync(FULL, c[0], 0) != KEY_MAX) warp_merge<KR>(own, c, lane);
+        }
+    }
+    if (warp == 0) {
+        uint64_t c[KR];
+#pragma unroll
+        for (int r = 0; r < KR; ++r) c[r] = ctop[r * 32 + lane];
+        warp_merge<KR>(c, own, lane);
+#pragma unroll
+        for (int r = 0; r < KR; ++r) ctop[r * 32 + lane] = c[r];
+    }
     __syncthreads();
-    uint64_t* dst = p.out + (static_cast<size_t>(qi) * p.nsplit + split) * KP;
+    uint64_t* dst = p.out + static_cast<size_t>(unit) * KP;
     for (int i = threadIdx.x; i < KP; i += blockDim.x) dst[i] = ctop[i];
-    }  // queries of this CTA
+    }  // work units of this CTA
 }
 
-// Final merge: per query, the k best of nparts sorted lists of kp keys, then
-// keys -> (distance, id).  Unfilled entries get the reference's heap_init
+// Final merge: per query (one CTA), the k best of its splits' sorted lists of
+// KP keys, then keys -> (distance, id).  Each warp folds every W-th list into
+// a sorted register list by bitonic merges (a list whose smallest key is at
+// or above the warp's k-th is skipped), then the warps' lists are folded
+// pairwise through shared memory: a full sort of 148 lists cost more than
+// the scan of one query.  Unfilled entries get the reference's heap_init
 // values (FLT_MAX / -FLT_MAX, id -1; src/heap.hpp:13-25).
-__global__ void __launch_bounds__(256) merge_kernel(const uint64_t* __restrict__ parts, int nq, int nparts, int kp, int k,
-                                                    int metric, const int64_t* __restrict__ ids,
+template <int KR>
+__global__ void __launch_bounds__(512) merge_kernel(const uint64_t* __restrict__ parts, int nq, int pparts, int tsplit,
+                                                    int units, int k, int metric, const int64_t* __restrict__ ids,
                                                     float* __restrict__ D, int64_t* __restrict__ I,
                                                     int64_t* __restrict__ rows, const int32_t* __restrict__ nq_dev) {
+    constexpr int KP = KR * 32;
     extern __shared__ __align__(16) unsigned char sm[];
-    uint64_t* a = reinterpret_cast<uint64_t*>(sm);
+    uint64_t* fold = reinterpret_cast<uint64_t*>(sm);  // [W / 2][KP]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
     // Query blockIdx.x, then every gridDim.x-th after it, below the device
     // count when one is given.
     const int nq_eff = nq_dev ? min(*nq_dev, nq) : nq;
+    const int nparts = pparts * (nq_dev ? scan_tile_splits(units, nq_eff, pparts) : tsplit);
     for (size_t qi = blockIdx.x; qi < static_cast<size_t>(nq_eff); qi += gridDim.x) {
-    const int n = nparts * kp;
-    const uint64_t* src = parts + qi * n;
-    const uint64_t* best = src;
-    if (nparts > 1) {
-        const int P = next_pow2(n);
-        __syncthreads();  // the previous query's keys have been read
-        for (int i = threadIdx.x; i < P; i += blockDim.x) a[i] = i < n ? src[i] : KEY_MAX;
-        __syncthreads();
-        cta_bitonic_sort(a, P);
-        best = a;
+    const uint64_t* src = parts + qi * nparts * KP;
+    uint64_t t[KR];
+#pragma unroll
+    for (int r = 0; r < KR; ++r) t[r] = warp < nparts ? src[static_cast<size_t>(warp) * KP + r * 32 + lane] : KEY_MAX;
+    uint64_t c[KR];
+#pragma unroll
+    for (int r = 0; r < KR; ++r)
+        c[r] = warp + W < nparts ? src[static_cast<size_t>(warp + W) * KP + r * 32 + lane] : KEY_MAX;
+    for (int j = warp + W; j < nparts; j += W) {
+        uint64_t nx[KR];  // the next list, in flight while this one is folded
+#pragma unroll
+        for (int r = 0; r < KR; ++r)
+            nx[r] = j + W < nparts ? src[static_cast<size_t>(j + W) * KP + r * 32 + lane] : KEY_MAX;
+        if (__shfl_sync(FULL, c[0], 0) < warp_get<KR>(t, k - 1)) warp_merge<KR>(t, c, lane);
+#pragma unroll
+        for (int r = 0; r < KR; ++r) c[r] = nx[r];
     }
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        const uint64_t key = i < n ? best[i] : KEY_MAX;
-        float dv;
-        int64_t iv;
-        if (key == KEY_MAX) {
-            dv = metric == METRIC_L2 ? FLT_MAX : -FLT_MAX;
-            iv = -1;
-        } else {
-            const float sc = o2f(static_cast<uint32_t>(key >> 32));
-            dv = metric == METRIC_L2 ? sc : -sc;
-            iv = ids[key & 0xffffffffu];
+    for (int h = W >> 1; h > 0; h >>= 1) {
+        __syncthreads();  // the round before (or the previous query) has been read
+        if (warp >= h && warp < 2 * h) {
+#pragma unroll
+            for (int r = 0; r < KR; ++r) fold[static_cast<size_t>(warp - h) * KP + r * 32 + lane] = t[r];
         }
-        D[qi * k + i] = dv;
-        I[qi * k + i] = iv;
-        if (rows) rows[qi * k + i] = key == KEY_MAX ? -1 : static_cast<int64_t>(key & 0xffffffffu);
+        __syncthreads();
+        if (warp < h) {
+#pragma unroll
+            for (int r = 0; r < KR; ++r) c[r] = fold[static_cast<size_t>(warp) * KP + r * 32 + lane];
+            warp_merge<KR>(t, c, lane);
+        }
+    }
+    if (warp == 0) {
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+            const int i = r * 32 + lane;
+            if (i < k) {
+                const uint64_t key = t[r];
+                float dv;
+                int64_t iv;
+                if (key == KEY_MAX) {
+                    dv = metric == METRIC_L2 ? FLT_MAX : -FLT_MAX;
+                    iv = -1;
+                } else {
+                    const float sc = o2f(static_cast<uint32_t>(key >> 32));
+                    dv = metric == METRIC_L2 ? sc : -sc;
+                    iv = ids[key & 0xffffffffu];
+                }
+                D[qi * k + i] = dv;
+                I[qi * k + i] = iv;
+                if (rows) rows[qi * k + i] = key == KEY_MAX ? -1 : static_cast<int64_t>(key & 0xffffffffu);
+            }
+        }
     }
     }  // queries of this CTA
 }
@@ -992,32 +1062,47 @@ cudaError_t launch_warmup(const ArenaLayout& L, const float* codes, const int64_
     return cudaGetLastError();
 }
 
+// Warps, slots and K' are chosen so that one CTA's shared memory fits: 16
+// warps with 2 slots each for pitches up to 32 floats per block (d <= 128
+// with 4 blocks), 8 warps for wider blocks.  Slots are processed in pairs.
+static int scan_warps(const ArenaLayout& L) {
+    const int slot_kb = L.max_pitch / 8;  // 32 rows x pitch floats, in KiB
+    return slot_kb * 2 * 16 <= 128 ? 16 : slot_kb * 2 * 8 <= 160 ? 8 : 4;
+}
+static int scan_kr(int k) { return k <= 32 ? 1 : k <= 64 ? 2 : k <= 128 ? 4 : 8; }
+static size_t scan_smem(const ArenaLayout& L, int k, int nprobe, int pparts) {
+    const size_t W = scan_warps(L), S = 2, kp = scan_kr(k) * 32;
+    const size_t npa = ((nprobe + pparts - 1) / pparts + 3) & ~3;
+    return W * S * 32 * L.max_pitch * 4 + W * S * 8 + W * 2 * kp * 8 + kp * 8 + npa * 8 +
+           static_cast<size_t>(L.row_pitch) * 4 + npa * 8;
+}
+
+int scan_probe_parts(const ArenaLayout& L, int k, int nprobe) {
+    int pp = (nprobe + 2047) / 2048;
+    if (pp < 1) pp = 1;
+    while (pp < nprobe && scan_smem(L, k, nprobe, pp) > 227 * 1024) ++pp;
+    return pp;
+}
+
 template <int KR, int S>
 static cudaError_t launch_scan_t(const ScanParams& p, int W, int* smem_out, cudaStream_t s) {
-    const int npa = ((p.nprobe + p.nsplit - 1) / p.nsplit + 3) & ~3;
-    const size_t smem = static_cast<size_t>(W) * S * 32 * p.L.max_pitch * 4 + static_cast<size_t>(W) * S * 8 +
-                        static_cast<size_t>(W) * 2 * KR * 32 * 8 + static_cast<size_t>(KR) * 32 * 8 +
-                        static_cast<size_t>(npa) * 8 +
-                        static_cast<size_t>(p.L.row_pitch) * 4 + static_cast<size_t>(npa) * 8;
+    const size_t smem = scan_smem(p.L, p.k, p.nprobe, p.pparts);
     if (smem_out) *smem_out = static_cast<int>(smem);
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(scan_plain_kernel<KR, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    // With a device count and a query grid, the CTAs loop over the queries.
-    const int gq = (p.nq_dev && p.qgrid > 0) ? std::min(p.nq, p.qgrid) : p.nq;
-    if (gq < 1) return cudaSuccess;
-    scan_plain_kernel<KR, S><<<gq * p.nsplit, W * 32, smem, s>>>(p);
+    // With a device count, the CTAs loop over the work units.
+    const int64_t all = static_cast<int64_t>(p.nq) * p.pparts;
+    const int64_t grid = p.nq_dev ? std::min<int64_t>(std::max<int64_t>(all, p.units), p.units) : all * p.tsplit;
+    if (p.nq < 1 || grid < 1) return cudaSuccess;
+    scan_plain_kernel<KR, S><<<static_cast<unsigned>(grid), W * 32, smem, s>>>(p);
     return cudaGetLastError();
 }
 
-// Warps, slots and K' are chosen so that one CTA's shared memory fits: 16
-// warps with 2 slots each for pitches up to 32 floats per block (d <= 128
-// with 4 blocks), 8 warps for wider blocks.  Slots are processed in pairs.
 cudaError_t launch_scan_plain(const ScanParams& p, int* smem_out, cudaStream_t s) {
-    const int kr = p.k <= 32 ? 1 : p.k <= 64 ? 2 : p.k <= 128 ? 4 : 8;
-    const int slot_kb = p.L.max_pitch / 8;  // 32 rows x pitch floats, in KiB
-    const int W = slot_kb * 2 * 16 <= 128 ? 16 : slot_kb * 2 * 8 <= 160 ? 8 : 4;
+    const int kr = scan_kr(p.k);
+    const int W = scan_warps(p.L);
 #define HY_SCAN_CASE(KR) \
     case KR:             \
         return launch_scan_t<KR, 2>(p, W, smem_out, s);
@@ -1032,15 +1117,30 @@ cudaError_t launch_scan_plain(const ScanParams& p, int* smem_out, cudaStream_t s
 #undef HY_SCAN_CASE
 }
 
-cudaError_t launch_merge(const uint64_t* parts, int nq, int nparts, int kp, int k, int metric, const int64_t* ids,
-                         float* D, int64_t* I, cudaStream_t s, int64_t* rows, const int32_t* nq_dev) {
-    const size_t smem = nparts > 1 ? static_cast<size_t>(next_pow2(nparts * kp)) * 8 : 0;
-    cudaError_t e = cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
+cudaError_t launch_merge(const ScanParams& p, const int64_t* ids, float* D, int64_t* I, cudaStream_t s,
+                         int64_t* rows) {
     // With a device count the grid is capped and the CTAs loop over queries.
-    const int grid = nq_dev ? std::min(nq, 1024) : nq;
+    const int grid = p.nq_dev ? std::min(p.nq, 1024) : p.nq;
     if (grid < 1) return cudaSuccess;
-    merge_kernel<<<grid, 256, smem, s>>>(parts, nq, nparts, kp, k, metric, ids, D, I, rows, nq_dev);
+    // Warps: up to 16, one per list (a power of two for the pairwise folds).
+    int W = 1;
+    while (W < 16 && (p.nq_dev || W < p.pparts * p.tsplit)) W <<= 1;
+    const int kr = scan_kr(p.k);
+    const size_t smem = static_cast<size_t>(W / 2) * kr * 32 * 8;
+#define HY_MERGE_CASE(KR)                                                                                          \
+    case KR:                                                                                                       \
+        merge_kernel<KR><<<grid, 32 * W, smem, s>>>(p.out, p.nq, p.pparts, p.tsplit, p.units, p.k, p.metric, ids, D, \
+                                                    I, rows, p.nq_dev);                                            \
+        break;
+    switch (kr) {
+        HY_MERGE_CASE(1)
+        HY_MERGE_CASE(2)
+        HY_MERGE_CASE(4)
+        HY_MERGE_CASE(8)
+        default:
+            return cudaErrorInvalidValue;
+    }
+#undef HY_MERGE_CASE
     return cudaGetLastError();
 }
 

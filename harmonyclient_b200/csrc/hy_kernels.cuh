@@ -45,15 +45,28 @@ struct ScanParams {
     const int64_t* probes;     // [nq][nprobe], -1 = skip
     const uint32_t* init_thr;  // [nq] ordered-key thresholds or nullptr
     uint32_t* g_thr;           // [nq] shared threshold across splits or nullptr
-    uint64_t* out;             // [nq][nsplit][KR*32] sorted keys
+    uint64_t* out;             // [nq][pparts * tsplit][KR*32] sorted keys
     unsigned long long* counters;  // [2]: tile blocks loaded, tile blocks possible
     int* err;
-    int nq, nprobe, nsplit, k, metric, prune;
-    const int32_t* nq_dev = nullptr;  // optional device count: queries at or past it are skipped
-    // With nq_dev: the launch has min(nq, qgrid) query slots (qgrid > 0) whose
-    // CTAs loop over the queries below the device count.
-    int qgrid = 0;
+    int nq, nprobe, k, metric, prune;
+    // Work units of a query: its probe list in pparts parts (probe j belongs
+    // to part j % pparts), each part's 32-row tiles dealt to tsplit units.
+    int pparts = 1, tsplit = 1;
+    // Optional device count: queries at or past it are skipped, and the tile
+    // splits follow from it (scan_tile_splits over `units` work units).
+    const int32_t* nq_dev = nullptr;
+    int units = 0;
 };
+
+// Tile splits per probe part when nq queries of pparts parts share `units`
+// work units (at least one each).
+__host__ __device__ inline int scan_tile_splits(int units, int nq, int pparts) {
+    const int per = nq > 0 ? units / (nq * pparts) : 1;
+    return per > 1 ? per : 1;
+}
+// Probe parts of a plain scan: the fewest whose probe tables fit a CTA's
+// shared memory beside the staging for layout L and k.
+int scan_probe_parts(const ArenaLayout& L, int k, int nprobe);
 
 cudaError_t launch_coarse_scores(const float* q, int nq, const float* cent, int nlist, int d, int metric, float* out,
                                  cudaStream_t s);
@@ -70,10 +83,9 @@ cudaError_t launch_warmup(const ArenaLayout& L, const float* codes, const int64_
                           int skip_lo = 0, int skip_hi = -1);
 cudaError_t launch_scan_plain(const ScanParams& p, int* smem_bytes_out, cudaStream_t s);
 // rows (optional): the arena row of every result (-1 when unfilled).
-// nq_dev (optional): device count; queries at or past it are skipped.
-cudaError_t launch_merge(const uint64_t* parts, int nq, int nparts, int kp, int k, int metric, const int64_t* ids,
-                         float* D, int64_t* I, cudaStream_t s, int64_t* rows = nullptr,
-                         const int32_t* nq_dev = nullptr);
+// p: the scan whose parts are merged (its device count and splits).
+cudaError_t launch_merge(const ScanParams& p, const int64_t* ids, float* D, int64_t* I, cudaStream_t s,
+                         int64_t* rows = nullptr);
 
 // Per-query nprobe: probes at or beyond np[q] (clamped to [1, P]) become -1.
 cudaError_t launch_cut_probes(int64_t* probes, int n, int P, const int32_t* np, cudaStream_t s);

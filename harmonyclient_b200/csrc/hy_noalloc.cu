@@ -17,6 +17,7 @@
 // be serialised by the caller.  A call holds the index's call lock from its
 // first read of the index until its work has completed on the device, so
 // add / load / reset on the same index from another thread wait for it.
+#include <algorithm>
 #include <mutex>
 
 #include "../../include/hy.h"
@@ -104,12 +105,16 @@ extern "C" int hy_index_search_preassigned_noalloc(hy_index* h, size_t n, const 
     rc = scratch_for_device(v.device, &base);
     if (rc != HY_OK) return rc;
 
-    // Same split of the probe lists over CTAs as the allocating entry points.
+    // Work units per query: as many as the scratch formula counts, dealt by
+    // tiles (one part of the probe list unless its table needs more).
     const int kp = k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 256;
     int nsplit = 1;
     const size_t target_ctas = 2 * 148;
     if (n < target_ctas) nsplit = (int)std::min<size_t>((target_ctas + n - 1) / n, nprobe);
     while ((nprobe + nsplit - 1) / nsplit > 2048) ++nsplit;
+    const int pparts = std::min(nsplit, hy::scan_probe_parts(v.L, (int)k, (int)nprobe));
+    const int tsplit = nsplit / pparts;
+    nsplit = pparts * tsplit;
 
     // Scratch layout: status word, counters, thresholds, probes, parts.
     const size_t off_err = 0, off_cnt = 256, off_thr = 512;
@@ -148,14 +153,15 @@ extern "C" int hy_index_search_preassigned_noalloc(hy_index* h, size_t n, const 
     p.err = err;
     p.nq = (int)n;
     p.nprobe = (int)nprobe;
-    p.nsplit = nsplit;
+    p.pparts = pparts;
+    p.tsplit = tsplit;
     p.k = (int)k;
     p.metric = v.metric;
     p.prune = 1;
     int smem = 0;
     if (hy::launch_scan_plain(p, &smem, s) != cudaSuccess)
         return hy::set_error(HY_ERR_CUDA, "search_preassigned_noalloc: scan launch failed");
-    if (hy::launch_merge(parts, (int)n, nsplit, kp, (int)k, v.metric, v.ids, dD, dI, s) != cudaSuccess)
+    if (hy::launch_merge(p, v.ids, dD, dI, s) != cudaSuccess)
         return hy::set_error(HY_ERR_CUDA, "search_preassigned_noalloc: merge launch failed");
     int herr = 0;
     if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
