@@ -18,8 +18,8 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhy.so")
 SERVER = os.path.join(HERE, "harmony_serve")
-SOURCES = ["hy_kernels.cu", "hy_batched.cu", "hy_capi.cu", "hy_selftest.cu", "hy_noalloc.cu", "hy_mlp.cu", "hy_lists.cu"]
-HEADERS = ["hy_device.cuh", "hy_kernels.cuh", "hy_tc.cuh", "hy_common.cuh", "hy_batched.cuh", "hy_mlp.cuh", "hy_lists.cuh"]
+SOURCES = ["hy_kernels.cu", "hy_batched.cu", "hy_capi.cu", "hy_selftest.cu", "hy_noalloc.cu", "hy_mlp.cu", "hy_lists.cu", "hy_assign.cu"]
+HEADERS = ["hy_device.cuh", "hy_kernels.cuh", "hy_tc.cuh", "hy_common.cuh", "hy_batched.cuh", "hy_mlp.cuh", "hy_lists.cuh", "hy_assign.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -1631,49 +1631,70 @@ __global__ void __launch_bounds__(256) tighten_warp2_kernel(const float* __restr
 // (|c - hi - lo| <= 2^-16 |c|, against 2^-8 |c| for one bf16).  Bound terms
 // {|(|hi| + |lo|)|, |c - hi - lo|}: the first covers |hi + lo| and the
 // magnitudes the accumulation adds.
-__global__ void rowmajor_image_kernel(const float* __restrict__ x, int64_t n, int d, int nkb, int64_t rows,
-                                      unsigned char* __restrict__ out) {
-    const int w = nkb * 64;
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i >= rows * w) return;
-    const int64_t r = i / w;
-    const int j = static_cast<int>(i % w);
-    const float v = (r < n && j < d) ? x[r * d + j] : 0.0f;
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-    const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-    const uint32_t off = tc::kblock_offset(static_cast<uint32_t>(r & 127), j & 63);
-    unsigned char* tile = out + (r >> 7) * (2 * nkb) * KB_BYTES;
-    *reinterpret_cast<__nv_bfloat16*>(tile + (2 * (j >> 6)) * KB_BYTES + off) = hi;
-    *reinterpret_cast<__nv_bfloat16*>(tile + (2 * (j >> 6) + 1) * KB_BYTES + off) = lo;
-}
-
-__global__ void rowmajor_aux_kernel(const float* __restrict__ x, int64_t n, int d, int64_t rows,
-                                    float2* __restrict__ aux, float* __restrict__ xn) {
+//
+// One warp per image row (rows past n are zero), everything in one launch: a
+// k-means step builds the image anew.  tile_aux and cmax (the maxima over all
+// centroids of |c|, |lo|, |c - hi - lo| and |(|hi| + |lo|)|) are maxima of
+// non-negative floats as ordered bits, zeroed before; a NaN stays on top.
+__global__ void __launch_bounds__(256) centroid_image_kernel(const float* __restrict__ x, int64_t n, int d, int nkb,
+                                                             int64_t rows, unsigned char* __restrict__ out,
+                                                             float2* __restrict__ aux, unsigned int* __restrict__ taux,
+                                                             float* __restrict__ xn, unsigned int* __restrict__ cmax) {
     const int lane = threadIdx.x & 31;
     const int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (r >= rows) return;
-    float nn = 0.0f, ee = 0.0f;
-    if (r < n)
-        for (int j = lane; j < d; j += 32) {
-            const float v = x[r * d + j];
-            const float hi = __bfloat162float(__float2bfloat16_rn(v));
-            const float lo = __bfloat162float(__float2bfloat16_rn(v - hi));
-            const float m = fabsf(hi) + fabsf(lo);
-            const float e = (v - hi) - lo;  // exact: both differences are of nearby values
+    const bool in = r < n;
+    unsigned char* tile = out + (r >> 7) * (2 * nkb) * KB_BYTES;
+    float vv = 0.0f, ll = 0.0f, nn = 0.0f, ee = 0.0f;
+    for (int j = 2 * lane; j < nkb * 64; j += 64) {
+        __nv_bfloat162 h, l;
+        float v[2], hf[2], lf[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            v[i] = in && j + i < d ? x[r * d + j + i] : 0.0f;
+            const __nv_bfloat16 hb = __float2bfloat16_rn(v[i]);
+            hf[i] = __bfloat162float(hb);
+            const __nv_bfloat16 lb = __float2bfloat16_rn(v[i] - hf[i]);
+            lf[i] = __bfloat162float(lb);
+            if (i == 0) {
+                h.x = hb;
+                l.x = lb;
+            } else {
+                h.y = hb;
+                l.y = lb;
+            }
+            const float m = fabsf(hf[i]) + fabsf(lf[i]);
+            const float e = (v[i] - hf[i]) - lf[i];  // exact: both differences are of nearby values
+            vv = fmaf(v[i], v[i], vv);
+            ll = fmaf(lf[i], lf[i], ll);
             nn = fmaf(m, m, nn);
             ee = fmaf(e, e, ee);
         }
+        unsigned char* dst = tile + (2 * (j >> 6)) * KB_BYTES + tc::kblock_offset(static_cast<uint32_t>(r & 127), j & 63);
+        *reinterpret_cast<__nv_bfloat162*>(dst) = h;
+        *reinterpret_cast<__nv_bfloat162*>(dst + KB_BYTES) = l;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
+        vv += __shfl_xor_sync(FULL, vv, o);
+        ll += __shfl_xor_sync(FULL, ll, o);
         nn += __shfl_xor_sync(FULL, nn, o);
         ee += __shfl_xor_sync(FULL, ee, o);
     }
     if (lane == 0) {
         float sq = 0.0f;
-        if (r < n)
+        if (in)
+#pragma unroll 8
             for (int j = 0; j < d; ++j) sq = __fadd_rn(sq, __fmul_rn(x[r * d + j], x[r * d + j]));
-        aux[r] = make_float2(sqrtf(nn), sqrtf(ee));
+        const float2 a = make_float2(sqrtf(nn), sqrtf(ee));
+        aux[r] = a;
         xn[r] = sq;
+        atomicMax(&taux[2 * (r >> 7)], __float_as_uint(fabsf(a.x)));
+        atomicMax(&taux[2 * (r >> 7) + 1], __float_as_uint(fabsf(a.y)));
+        atomicMax(&cmax[0], __float_as_uint(fabsf(sqrtf(vv))));
+        atomicMax(&cmax[1], __float_as_uint(fabsf(sqrtf(ll))));
+        atomicMax(&cmax[2], __float_as_uint(fabsf(a.y)));
+        atomicMax(&cmax[3], __float_as_uint(fabsf(a.x)));
     }
 }
 
@@ -2511,13 +2532,15 @@ cudaError_t launch_fb_scatter(const int32_t* ovf, const float* fD, const int64_t
 }
 
 cudaError_t launch_centroid_image(const float* cent, int nlist, int d, void* img, float2* aux, float2* tile_aux,
-                                  float* xn, cudaStream_t s) {
+                                  float* xn, float* cmax, cudaStream_t s) {
     const int64_t rows = (static_cast<int64_t>(nlist) + TM - 1) / TM * TM;
     const int nkb = (d + 63) / 64;  // 64-dimension blocks (two k-blocks each in the image)
-    rowmajor_image_kernel<<<grid_for(rows * nkb * 64, 256), 256, 0, s>>>(cent, nlist, d, nkb, rows,
-                                                                         static_cast<unsigned char*>(img));
-    rowmajor_aux_kernel<<<grid_for(rows * 32, 256), 256, 0, s>>>(cent, nlist, d, rows, aux, xn);
-    tile_aux_kernel<<<grid_for(rows / TM * 32, 256), 256, 0, s>>>(aux, rows / TM, tile_aux);
+    // tile_aux and the maxima lie in one run: one clear.
+    cudaError_t e = cudaMemsetAsync(tile_aux, 0, rows / TM * sizeof(float2) + 4 * sizeof(float), s);
+    if (e != cudaSuccess) return e;
+    centroid_image_kernel<<<grid_for(rows * 32, 256), 256, 0, s>>>(
+        cent, nlist, d, nkb, rows, static_cast<unsigned char*>(img), aux, reinterpret_cast<unsigned int*>(tile_aux), xn,
+        reinterpret_cast<unsigned int*>(cmax));
     return cudaGetLastError();
 }
 

@@ -108,8 +108,10 @@ cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qa
 // with BatchedLaunch::ksplit), per-row {|(|hi| + |lo|)|, |c - hi - lo|},
 // per-tile maxima and squared norms, rows padded to whole 128-row tiles
 // (img: bf16_split_image_bytes(rows), aux/xn: rows, tile_aux: rows/128).
+// tile_aux's tiles are followed by the four floats of cmax, the maxima over
+// the centroids of |c|, |lo|, |c - hi - lo| and |(|hi| + |lo|)|.
 cudaError_t launch_centroid_image(const float* cent, int nlist, int d, void* img, float2* aux, float2* tile_aux,
-                                  float* xn, cudaStream_t s);
+                                  float* xn, float* cmax, cudaStream_t s);
 // Work of one coarse launch over nq queries: list_off[2], list_size[1] of the
 // centroid index; w.pairs [nq], w.items [ngroups*nslices], w.pair_cnt [1],
 // w.pair_off [2], w.item_off [2].

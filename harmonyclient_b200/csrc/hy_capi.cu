@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/hy.h"
+#include "hy_assign.cuh"
 #include "hy_batched.cuh"
 #include "hy_lists.cuh"
 #include "hy_kernels.cuh"
@@ -151,6 +152,7 @@ struct hy_index {
     DevBuf cent, list_off, list_size, ids, codes, norms;
     // workspace
     DevBuf w_q, w_scores, w_probes, w_thr, w_gthr, w_parts, w_D, w_I, w_f, w_counters, w_err;
+    DevBuf w_second, w_hard;  // tensor-core assignment: second candidates, undecided rows (count, ids)
     DevBuf w_x, w_lab, w_dist, w_keys, w_keys2, w_vals, w_vals2, w_sort, w_start, w_sums, w_cnt, w_rows, w_xn;
 
     cudaStream_t stream = nullptr;
@@ -261,6 +263,12 @@ int set_device(hy_index* h) {
     return HY_OK;
 }
 
+// Rows x centroids x dimensions from which assignment runs on the tensor
+// cores: there the exact kernels take about 60 us, the tensor-core steps'
+// six launches 40 us (20,000 x 300 x 40, half of it: 1.92 ms exact, 2.00 ms
+// here for a whole train, add and search).
+constexpr size_t ASSIGN_TENSOR_MIN = size_t(1) << 29;
+
 // Bytes of the coarse score scratch per query chunk.
 constexpr size_t SCORE_BUDGET = size_t(512) << 20;
 
@@ -271,16 +279,66 @@ size_t query_chunk(size_t nlist, size_t n) {
     return std::min(qc, n);
 }
 
-// Nearest centroid of each of n device rows (x), chunked: labels, scores.
+// The centroids' split tensor-core image and its bound terms, built on first
+// use of a centroid set.
+float* centroid_maxima(const hy_index* h) {
+    return h->c_taux.as<float>() + (h->nlist + hy::BATCH_ROW_ALIGN - 1) / hy::BATCH_ROW_ALIGN * 2;
+}
+
+int ensure_centroid_image(hy_index* h, cudaStream_t s) {
+    if (h->cimg_valid) return HY_OK;
+    const size_t rows = (h->nlist + hy::BATCH_ROW_ALIGN - 1) / hy::BATCH_ROW_ALIGN * hy::BATCH_ROW_ALIGN;
+    HY_RET(h->c_img.ensure(hy::bf16_split_image_bytes((int64_t)rows, (int)h->d)));
+    HY_RET(h->c_aux.ensure(rows * sizeof(float2)));
+    HY_RET(h->c_taux.ensure(rows / hy::BATCH_ROW_ALIGN * sizeof(float2) + 4 * sizeof(float)));  // tiles, maxima
+    HY_RET(h->c_norm.ensure(rows * sizeof(float)));
+    HY_RET(h->c_off.ensure(2 * sizeof(int64_t)));
+    HY_RET(h->c_size.ensure(sizeof(int32_t)));
+    HY_CUDA(hy::launch_centroid_image(h->cent.as<float>(), (int)h->nlist, (int)h->d, h->c_img.p, h->c_aux.as<float2>(),
+                                      h->c_taux.as<float2>(), h->c_norm.as<float>(), centroid_maxima(h), s));
+    h->cimg_valid = true;
+    return HY_OK;
+}
+
+// Whether n rows are assigned to their centroids on the tensor cores.
+bool assign_on_tensor(const hy_index* h, size_t n) {
+    return h->d <= hy::ASSIGN_DMAX && n * h->nlist * h->d >= ASSIGN_TENSOR_MIN;
+}
+
+// Nearest centroid of each of n device rows (x): labels, scores (score may be
+// null).  On the tensor cores, rows the bound leaves undecided (usually none)
+// go through the exact scores of every centroid, in chunks up to their device
+// count; else every row does.
 int assign_rows(hy_index* h, const float* x, size_t n, int64_t* labels, float* score, cudaStream_t s) {
     const size_t rc = query_chunk(h->nlist, n);
+    hy::RowPick pick;
     HY_RET(h->w_scores.ensure(rc * h->nlist * sizeof(float)));
+    if (assign_on_tensor(h, n)) {
+        if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
+        HY_RET(ensure_centroid_image(h, s));
+        HY_RET(h->w_second.ensure(n * sizeof(int32_t)));
+        HY_RET(h->w_hard.ensure((n + 1) * sizeof(int32_t)));
+        hy::AssignWork w;
+        w.cimg = h->c_img.p;
+        w.cxn = h->c_norm.as<float>();
+        w.cmax = centroid_maxima(h);
+        w.second = h->w_second.as<int32_t>();
+        w.hard_count = h->w_hard.as<int32_t>();
+        w.hard = h->w_hard.as<int32_t>() + 1;
+        w.err = h->w_err.as<int>();
+        HY_CUDA(hy::launch_assign(x, (int)n, (int)h->d, (int)h->nlist, h->metric, w, h->nsm, labels, s));
+        HY_CUDA(hy::launch_assign_exact(x, (int)n, (int)h->d, h->cent.as<float>(), h->metric, w, labels, score, s));
+        pick.rows = w.hard;
+        pick.count = w.hard_count;
+    }
     for (size_t r0 = 0; r0 < n; r0 += rc) {
         const size_t m = std::min(rc, n - r0);
-        HY_CUDA(hy::launch_coarse_scores(x + r0 * h->d, (int)m, h->cent.as<float>(), (int)h->nlist, (int)h->d,
-                                         h->metric, h->w_scores.as<float>(), s));
-        HY_CUDA(hy::launch_argmin(h->w_scores.as<float>(), (int)m, (int)h->nlist, labels + r0, score ? score + r0 : nullptr,
-                                  s));
+        const size_t at = pick.rows ? 0 : r0;  // a picked row's place comes from the list
+        pick.ofs = (int)r0;
+        HY_CUDA(hy::launch_coarse_scores(x + at * h->d, (int)m, h->cent.as<float>(), (int)h->nlist, (int)h->d,
+                                         h->metric, h->w_scores.as<float>(), s, pick));
+        HY_CUDA(hy::launch_argmin(h->w_scores.as<float>(), (int)m, (int)h->nlist, labels + at,
+                                  score ? score + at : nullptr, s, pick));
     }
     return HY_OK;
 }
@@ -305,6 +363,7 @@ int kmeans_device(hy_index* h, const float* xs, size_t ns, const std::vector<int
     HY_RET(h->w_sums.ensure(nlist * d * sizeof(double)));
     HY_RET(h->w_cnt.ensure(nlist * sizeof(unsigned long long)));
     for (int it = 0; it < niter; ++it) {
+        h->cimg_valid = false;
         HY_RET(assign_rows(h, assign_src, ns, h->w_lab.as<int64_t>(), nullptr, s));
         HY_CUDA(cudaMemsetAsync(h->w_sums.p, 0, nlist * d * sizeof(double), s));
         HY_CUDA(cudaMemsetAsync(h->w_cnt.p, 0, nlist * sizeof(unsigned long long), s));
@@ -844,21 +903,6 @@ int ensure_bf16_image(hy_index* h, cudaStream_t s) {
 bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
     return h->coarse_mode == HY_COARSE_TENSOR && h->form == HY_FORM_BF16 && nprobe <= 256 && h->d <= 256 &&
            hy::batched_group_size((int)h->d, false) > 0;
-}
-
-int ensure_centroid_image(hy_index* h, cudaStream_t s) {
-    if (h->cimg_valid) return HY_OK;
-    const size_t rows = (h->nlist + hy::BATCH_ROW_ALIGN - 1) / hy::BATCH_ROW_ALIGN * hy::BATCH_ROW_ALIGN;
-    HY_RET(h->c_img.ensure(hy::bf16_split_image_bytes((int64_t)rows, (int)h->d)));
-    HY_RET(h->c_aux.ensure(rows * sizeof(float2)));
-    HY_RET(h->c_taux.ensure(rows / hy::BATCH_ROW_ALIGN * sizeof(float2)));
-    HY_RET(h->c_norm.ensure(rows * sizeof(float)));
-    HY_RET(h->c_off.ensure(2 * sizeof(int64_t)));
-    HY_RET(h->c_size.ensure(sizeof(int32_t)));
-    HY_CUDA(hy::launch_centroid_image(h->cent.as<float>(), (int)h->nlist, (int)h->d, h->c_img.p, h->c_aux.as<float2>(),
-                                      h->c_taux.as<float2>(), h->c_norm.as<float>(), s));
-    h->cimg_valid = true;
-    return HY_OK;
 }
 
 // Coarse step on the tensor cores for m queries whose bf16 image and

@@ -29,14 +29,18 @@ constexpr int METRIC_L2 = 1;
 // 4 x 4 outputs per thread, dimensions staged 32 at a time in shared memory.
 // (The reference computes these with IVFScan::lite_scan_codes over all
 // centroids, src/IVFScan.hpp:108-138, src/Index.cpp:985-990.)
-template <int METRIC>
+// pick (optional): score the rows pick.rows[pick.ofs ...] of q, at most nq of
+// them, up to the device count *pick.count.
+template <int METRIC, bool PICK>
 __global__ void __launch_bounds__(256) coarse_scores_kernel(const float* __restrict__ q, int nq,
                                                             const float* __restrict__ c, int nlist, int d,
-                                                            float* __restrict__ out) {
+                                                            float* __restrict__ out, RowPick pick) {
     __shared__ __align__(16) float Qs[32][68];
     __shared__ __align__(16) float Cs[32][68];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int q0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+    const int c0 = blockIdx.x * 64;
+    if (PICK) nq = min(nq, *pick.count - pick.ofs);
+    for (int q0 = blockIdx.y * 64; q0 < nq; q0 += gridDim.y * 64) {
     float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -48,7 +52,8 @@ __global__ void __launch_bounds__(256) coarse_scores_kernel(const float* __restr
             const int r = i >> 5, j = i & 31;
             const int gj = d0 + j;
             const int gq = q0 + r, gc = c0 + r;
-            Qs[j][r] = (gq < nq && gj < d) ? q[static_cast<size_t>(gq) * d + gj] : 0.0f;
+            const size_t qr = PICK && gq < nq ? pick.rows[pick.ofs + gq] : gq;
+            Qs[j][r] = (gq < nq && gj < d) ? q[qr * d + gj] : 0.0f;
             Cs[j][r] = (gc < nlist && gj < d) ? c[static_cast<size_t>(gc) * d + gj] : 0.0f;
         }
         __syncthreads();
@@ -76,6 +81,7 @@ __global__ void __launch_bounds__(256) coarse_scores_kernel(const float* __restr
             if (gc < nlist) out[static_cast<size_t>(gq) * nlist + gc] = METRIC == METRIC_L2 ? acc[u][v] : -acc[u][v];
         }
     }
+    }  // query tiles of this CTA
 }
 
 // Per row of `scores` (n values, smaller is better): the m best, best first,
@@ -169,10 +175,11 @@ __global__ void __launch_bounds__(256) select_warp_kernel(const float* __restric
 // row — the reference's nearest-centroid rule (strict < in column order,
 // src/IVFScan.hpp:131, src/Clustering.cpp:107).
 __global__ void argmin_kernel(const float* __restrict__ scores, int nrows, int n, int64_t* __restrict__ out_idx,
-                              float* __restrict__ out_score) {
+                              float* __restrict__ out_score, RowPick pick) {
     const int lane = threadIdx.x & 31;
-    const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (row >= nrows) return;
+    if (pick.rows) nrows = min(nrows, *pick.count - pick.ofs);
+    for (int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < nrows;
+         row += (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5) {
     const float* src = scores + row * n;
     float best = INFINITY;
     int bi = n;
@@ -193,9 +200,11 @@ __global__ void argmin_kernel(const float* __restrict__ scores, int nrows, int n
         }
     }
     if (lane == 0) {
-        out_idx[row] = bi < n ? bi : 0;
-        if (out_score) out_score[row] = best;
+        const int64_t at = pick.rows ? pick.rows[pick.ofs + row] : row;
+        out_idx[at] = bi < n ? bi : 0;
+        if (out_score) out_score[at] = best;
     }
+    }  // rows of this warp
 }
 
 // Warm-up thresholds (Index::warmUpSearch, src/Index.cpp:999-1051, and the
@@ -1003,12 +1012,15 @@ inline int grid_for(int64_t n, int threads) {
 }  // namespace
 
 cudaError_t launch_coarse_scores(const float* q, int nq, const float* cent, int nlist, int d, int metric, float* out,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, const RowPick& pick) {
     dim3 grid((nlist + 63) / 64, (nq + 63) / 64);
+    // A counted pick is usually a few rows: a grid of a few waves loops.
+    if (pick.rows) grid.y = std::min(grid.y, std::max(1u, 1184u / grid.x));
+    auto run = [&](auto kern) { kern<<<grid, 256, 0, s>>>(q, nq, cent, nlist, d, out, pick); };
     if (metric == METRIC_L2)
-        coarse_scores_kernel<METRIC_L2><<<grid, 256, 0, s>>>(q, nq, cent, nlist, d, out);
+        pick.rows ? run(coarse_scores_kernel<METRIC_L2, true>) : run(coarse_scores_kernel<METRIC_L2, false>);
     else
-        coarse_scores_kernel<METRIC_IP><<<grid, 256, 0, s>>>(q, nq, cent, nlist, d, out);
+        pick.rows ? run(coarse_scores_kernel<METRIC_IP, true>) : run(coarse_scores_kernel<METRIC_IP, false>);
     return cudaGetLastError();
 }
 
@@ -1030,9 +1042,10 @@ cudaError_t launch_select(const float* scores, int nq, int n, int m, int64_t* ou
 }
 
 cudaError_t launch_argmin(const float* scores, int nrows, int n, int64_t* out_idx, float* out_score,
-                          cudaStream_t s) {
-    argmin_kernel<<<grid_for(static_cast<int64_t>(nrows) * 32, 256), 256, 0, s>>>(scores, nrows, n, out_idx,
-                                                                                  out_score);
+                          cudaStream_t s, const RowPick& pick) {
+    int grid = grid_for(static_cast<int64_t>(nrows) * 32, 256);
+    if (pick.rows) grid = std::min(grid, 1184);
+    argmin_kernel<<<grid, 256, 0, s>>>(scores, nrows, n, out_idx, out_score, pick);
     return cudaGetLastError();
 }
 

@@ -68,12 +68,21 @@ __host__ __device__ inline int scan_tile_splits(int units, int nq, int pparts) {
 // shared memory beside the staging for layout L and k.
 int scan_probe_parts(const ArenaLayout& L, int k, int nprobe);
 
+// Rows picked by a device list: entries [ofs, ofs + n) of rows, below the
+// device count.  rows = nullptr: every row.
+struct RowPick {
+    const int32_t* rows = nullptr;
+    const int32_t* count = nullptr;
+    int ofs = 0;
+};
+
 cudaError_t launch_coarse_scores(const float* q, int nq, const float* cent, int nlist, int d, int metric, float* out,
-                                 cudaStream_t s);
+                                 cudaStream_t s, const RowPick& pick = RowPick());
 cudaError_t launch_select(const float* scores, int nq, int n, int m, int64_t* out_idx, float* out_score,
                           cudaStream_t s);
+// With a pick, results go to the picked rows' places.
 cudaError_t launch_argmin(const float* scores, int nrows, int n, int64_t* out_idx, float* out_score,
-                          cudaStream_t s);
+                          cudaStream_t s, const RowPick& pick = RowPick());
 // skip_lo <= skip_hi: a query whose nearest list has between skip_lo and
 // skip_hi rows gets no warm-up (threshold FLT_MAX); the batched search's dense
 // first pass bounds it instead.
