@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstddef>
+#include <type_traits>
 
 #include "hy_batched.cuh"
 #include "hy_common.cuh"
@@ -149,6 +150,56 @@ __global__ void row_aux_kernel(ArenaLayout L, const float* __restrict__ codes, i
     if (lane == 0) aux[r] = make_float2(sqrtf(nn), sqrtf(ee));
 }
 
+// The same for TF32 operands, read from the FP32 rows as they are: the tensor
+// cores ignore a value's low 13 bits, so x~ is x with them cleared (an x~
+// rounded to nearest would be at least as near), and {norm of |x| + |x - x~|,
+// norm of x - x~} covers either.  Also, for the rule that sends a plain batch
+// to the tensor cores: stat[0] sums |x - x~| + 2^-11 |x| over the rows and
+// stat[1] the rows' distance to their list's centroid.
+__global__ void row_aux_tf32_kernel(ArenaLayout L, const float* __restrict__ codes, int64_t rows,
+                                    const int64_t* __restrict__ list_off, const int32_t* __restrict__ list_size,
+                                    int nlist, const float* __restrict__ cent, float2* __restrict__ aux,
+                                    double* __restrict__ stat) {
+    const int lane = threadIdx.x & 31;
+    const int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (r >= rows) return;
+    int lo = 0, hi = nlist - 1;  // the last list that starts at or before r
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (list_off[mid] <= r)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const float* c = cent + static_cast<size_t>(lo) * L.d;
+    float vv = 0.0f, nn = 0.0f, ee = 0.0f, dd = 0.0f;
+    for (int b = 0; b < L.nb; ++b)
+        for (int j = lane; j < L.bstart[b + 1] - L.bstart[b]; j += 32) {
+            const float v = codes[arena_offset(L, r, b, j)];
+            const float e = fabsf(v - __uint_as_float(__float_as_uint(v) & ~0x1fffu));
+            const float m = fabsf(v) + e, dc = v - c[L.bstart[b] + j];
+            vv = fmaf(v, v, vv);
+            nn = fmaf(m, m, nn);
+            ee = fmaf(e, e, ee);
+            dd = fmaf(dc, dc, dd);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        vv += __shfl_xor_sync(FULL, vv, o);
+        nn += __shfl_xor_sync(FULL, nn, o);
+        ee += __shfl_xor_sync(FULL, ee, o);
+        dd += __shfl_xor_sync(FULL, dd, o);
+    }
+    const bool valid = r - list_off[lo] < list_size[lo];
+    if (lane == 0) aux[r] = make_float2(sqrtf(nn), sqrtf(ee));
+    // One pair of adds per CTA (its first warp's row stands for its eight:
+    // a sample of the rows).
+    if (threadIdx.x == 0 && valid) {
+        atomicAdd(&stat[0], static_cast<double>(sqrtf(ee) + 0.00048828125f * sqrtf(vv)));
+        atomicAdd(&stat[1], static_cast<double>(sqrtf(dd)));
+    }
+}
+
 // Per 128-row tile: the largest |x~| and |x - x~| of its rows (the batched
 // kernel's per-tile relaxation of the error bound).
 __global__ void tile_aux_kernel(const float2* __restrict__ row_aux, int64_t tiles, float2* __restrict__ out) {
@@ -238,6 +289,12 @@ __global__ void prep_queries_f8_kernel(const float* __restrict__ q, int nq, int 
     }
 }
 
+// The exactness certificate of one query (launch_prep_queries): cert = the
+// arena's {integral flag, bits of its largest squared norm}.
+__device__ inline int32_t certified(const int* cert, bool integral, float qn) {
+    return cert && cert[0] && integral && qn + __int_as_float(cert[1]) < 8388608.0f ? 1 : 0;
+}
+
 // Queries: bf16 rows padded to nkb*64, and per query {|q|^2 (sequential f32,
 // the exact arithmetic's value), |q|, |q~|, |q - q~|}.  One warp per query
 // (PREP_WARPS per CTA): the lanes convert and reduce, and lane 0 takes the
@@ -246,7 +303,8 @@ constexpr int PREP_WARPS = 8;
 constexpr int PREP_DMAX = 768;  // the bf16 forms' largest d
 __global__ void __launch_bounds__(32 * PREP_WARPS) prep_queries_kernel(const float* __restrict__ q, int nq, int d,
                                                                        int nkb, __nv_bfloat16* __restrict__ qb,
-                                                                       float4* __restrict__ qaux, float amax,
+                                                                       float4* __restrict__ qaux,
+                                                                       const int* __restrict__ cert,
                                                                        int32_t* __restrict__ qexact) {
     __shared__ float rowbuf[PREP_WARPS][PREP_DMAX];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -278,7 +336,49 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) prep_queries_kernel(const flo
 #pragma unroll 8
         for (int j = 0; j < d; ++j) s = __fadd_rn(s, __fmul_rn(row[j], row[j]));
         qaux[i] = make_float4(s, sqrtf(s), sqrtf(nn), sqrtf(ee));
-        if (qexact) qexact[i] = (amax >= 0.0f && all_integral && s + amax < 8388608.0f) ? 1 : 0;
+        if (qexact) qexact[i] = certified(cert, all_integral, s);
+    }
+}
+
+// Queries as TF32 operands: the FP32 values in the arena's block-padded order
+// (row_pitch floats), and {|q|^2 (sequential f32), |q|, norm of |q| + |q - q~|,
+// |q - q~|} with q~ = q without its low 13 bits.  One warp per query.
+__global__ void __launch_bounds__(32 * PREP_WARPS) prep_queries_tf32_kernel(
+    const float* __restrict__ q, int nq, const __grid_constant__ ArenaLayout L, float* __restrict__ qb,
+    float4* __restrict__ qaux, const int* __restrict__ cert, int32_t* __restrict__ qexact) {
+    __shared__ float rowbuf[PREP_WARPS][PREP_DMAX];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * PREP_WARPS + warp;
+    if (i >= nq) return;  // whole warp
+    const float* src = q + static_cast<size_t>(i) * L.d;
+    float* row = rowbuf[warp];
+    float nn = 0.0f, ee = 0.0f;
+    bool integral = true;
+    for (int b = 0; b < L.nb; ++b)
+        for (int j = lane; j < L.pitch[b]; j += 32) {
+            const bool in = j < L.bstart[b + 1] - L.bstart[b];
+            const float v = in ? src[L.bstart[b] + j] : 0.0f;
+            if (in) row[L.bstart[b] + j] = v;
+            integral = integral && v == rintf(v) && fabsf(v) <= 256.0f;
+            qb[static_cast<size_t>(i) * L.row_pitch + L.boff[b] + j] = v;
+            const float e = fabsf(v - __uint_as_float(__float_as_uint(v) & ~0x1fffu));
+            const float m = fabsf(v) + e;
+            nn = fmaf(m, m, nn);
+            ee = fmaf(e, e, ee);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        nn += __shfl_xor_sync(FULL, nn, o);
+        ee += __shfl_xor_sync(FULL, ee, o);
+    }
+    const bool all_integral = __all_sync(FULL, integral);
+    __syncwarp();
+    if (lane == 0) {
+        float s = 0.0f;
+#pragma unroll 8
+        for (int j = 0; j < L.d; ++j) s = __fadd_rn(s, __fmul_rn(row[j], row[j]));
+        qaux[i] = make_float4(s, sqrtf(s), sqrtf(nn), sqrtf(ee));
+        if (qexact) qexact[i] = certified(cert, all_integral, s);
     }
 }
 
@@ -725,12 +825,14 @@ __device__ inline void named_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// QG: queries per group (MMA N: 128, 64 or 32); F8: e4m3 operands
-// (kind::f8f6f4, K = 32 per instruction) instead of bf16 (kind::f16, K = 16).
+// QG: queries per group (MMA N: 128, 64 or 32); OP: bf16 operands (kind::f16,
+// K = 16 per instruction), e4m3 (kind::f8f6f4, K = 32) or tf32 (kind::tf32, K =
+// 8; the list rows are the FP32 arena itself, whose layout is the operand's).
 // Either way a k-block row is 128 bytes and one instruction covers 32 bytes
 // of it, so the descriptors and the stage ring are the same.
-template <int QG, bool F8>
+template <int QG, Operand OP>
 __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __grid_constant__ BatchedParams p) {
+    constexpr bool F8 = OP == Operand::e4m3;
     constexpr int CW = QG / 2;            // accumulator columns per epilogue warp
     constexpr int CC = CW < 32 ? CW : 32;  // columns per candidate-test chunk
     constexpr int TMEM_COLS = 2 * QG;      // two accumulators
@@ -924,9 +1026,19 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                             break;
                         }
                         mbar_expect_tx(&full[s], KB_BYTES);
-                        bulk_g2s(sA + static_cast<size_t>(s) * KB_BYTES,
-                                 p.abf + ((tile0 + t) * nkb + kb) * static_cast<int64_t>(KB_BYTES), KB_BYTES,
-                                 &full[s]);
+                        if constexpr (OP == Operand::tf32) {
+                            // 32 dimensions of 128 arena rows: one 4 KB group
+                            // of each of their four 32-row tiles.
+                            const int64_t tile_bytes = static_cast<int64_t>(nkb) * 4096;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                bulk_g2s(sA + static_cast<size_t>(s) * KB_BYTES + i * 4096,
+                                         p.abf + ((tile0 + t) * 4 + i) * tile_bytes + kb * 4096, 4096, &full[s]);
+                        } else {
+                            bulk_g2s(sA + static_cast<size_t>(s) * KB_BYTES,
+                                     p.abf + ((tile0 + t) * nkb + kb) * static_cast<int64_t>(KB_BYTES), KB_BYTES,
+                                     &full[s]);
+                        }
                     }
                 }
                 if (!ok) break;
@@ -935,7 +1047,9 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
     } else if (warp == W_MMA) {
         // ---------------- MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = F8 ? tc::idesc_e4m3_f32(TM, QG) : tc::idesc_bf16_f32(TM, QG);
+            const uint32_t idesc = F8                      ? tc::idesc_e4m3_f32(TM, QG)
+                                   : OP == Operand::tf32 ? tc::idesc_tf32_f32(TM, QG)
+                                                         : tc::idesc_bf16_f32(TM, QG);
             int ms = 0;        // stage of the next k-block
             uint32_t mph = 0;  // its ring round's parity
             uint32_t tile_it = 0;
@@ -974,6 +1088,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                             const uint64_t bd = tc::sdesc_sw128(b0 + (kb >> p.ksplit) * BKB + kk * 32);
                             if constexpr (F8)
                                 tc::mma_e4m3(dcol, ad, bd, idesc, (kb | kk) != 0 ? 1u : 0u);
+                            else if constexpr (OP == Operand::tf32)
+                                tc::mma_tf32(dcol, ad, bd, idesc, (kb | kk) != 0 ? 1u : 0u);
                             else
                                 tc::mma_bf16(dcol, ad, bd, idesc, (kb | kk) != 0 ? 1u : 0u);
                         }
@@ -2021,7 +2137,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
 #pragma unroll
     for (int r = 0; r < PER; ++r) {
         const int e = entry(r);
-        const bool keep = e < nlist && lo[r] <= U;
+        const bool keep = e < nlist && !(lo[r] > U);  // (what is not a number has no bound: kept)
         const unsigned bal = __ballot_sync(FULL, keep);
         if (keep) {
             const int at = c + __popc(bal & ((1u << lane) - 1u));
@@ -2292,7 +2408,10 @@ __global__ void __launch_bounds__(256) rerank_warp_kernel(const __grid_constant_
     if (qi >= nq) return;  // whole warp
     const int cnt = w.cand_cnt[qi];
     const int n = min(cnt, capq);
-    if (cnt > capq || n > 256 || k > 256) {
+    const float4 qa = qaux[qi];
+    // (A query whose norm is not a number below 1e37 has no bounds: the CTA
+    // kernel reports it for the exact scan.)
+    if (cnt > capq || n > 256 || k > 256 || !(qa.x < 1e37f)) {
         if (lane == 0) w.big[1 + atomicAdd(&w.big[0], 1)] = qi;
         return;
     }
@@ -2305,7 +2424,7 @@ __global__ void __launch_bounds__(256) rerank_warp_kernel(const __grid_constant_
     }
     __syncwarp();
     const bool l2 = metric == 1;
-    const ErrCoef ec = err_coef(qaux[qi], l2, cK, cN);
+    const ErrCoef ec = err_coef(qa, l2, cK, cN);
     const uint64_t* cq = w.cand + static_cast<int64_t>(qi) * capq;
     float* Dq = D + static_cast<size_t>(qi) * k;
     int64_t* Iq = I + static_cast<size_t>(qi) * k;
@@ -2345,7 +2464,7 @@ __global__ void __launch_bounds__(256) rerank_kernel(ArenaLayout L, const float*
     const ErrCoef ec = err_coef(qa, l2, cK, cN);
     if (threadIdx.x == 0) {
         s_nsel = 0;
-        s_over = cnt > capq ? 1 : 0;
+        s_over = cnt > capq || !(qa.x < 1e37f) ? 1 : 0;
     }
     stage_query(L, q + static_cast<size_t>(qi) * L.d, qs);
     // Certified exact tensor-core distances need no bounds (e = 0).
@@ -2481,22 +2600,20 @@ cudaError_t launch_to_bf16_arena(const ArenaLayout& L, const float* codes, int64
     return cudaGetLastError();
 }
 
-// Error-bound constants for dimension d (see err_coef).
-// ksplit: every dimension accumulates two products (the split centroid
-// image's hi and lo parts).
-static void err_consts(int d, bool f8, float* cK, float* cN, bool ksplit = false) {
-    const int K = (f8 ? (d + 127) / 128 * 128 : (d + 63) / 64 * 64) * (ksplit ? 2 : 1);
+// Error-bound constants for dimension d and K accumulated products (see
+// err_coef).
+static void err_consts(int d, int K, float* cK, float* cN) {
     const double u = 1.0 / 16777216.0, inflate = 1.0 + 1.0 / 128.0;
     *cK = static_cast<float>((K + 8) * u * inflate);
     *cN = static_cast<float>((3.0 * d + 16) * u * inflate);
 }
 
 cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qaux, int nq, const BatchWork& w,
-                           int capq, int k, int metric, int d, bool f8, int nsm, float* thr, cudaStream_t s,
+                           int capq, int k, int metric, int d, int K, int nsm, float* thr, cudaStream_t s,
                            DenseFirst df) {
     df.dense_max = std::min(df.dense_max, capq);
     float cK, cN;
-    err_consts(d, f8, &cK, &cN);
+    err_consts(d, K, &cK, &cN);
     cudaError_t e = cudaMemsetAsync(w.big, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(w.big2, 0, sizeof(int32_t), s)) != cudaSuccess) return e;
@@ -2562,7 +2679,7 @@ cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q
                                  const float* cxn, const float2* caux, const float4* qaux, int d, int metric, int m,
                                  int64_t* out_idx, float* out_score, int* err, cudaStream_t s) {
     float cK, cN;
-    err_consts(d, false, &cK, &cN, true);  // the split centroid image
+    err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
     int warps = 4;
     while (warps > 1 && coarse_refine_smem(nlist, d, warps) > 200 * 1024) warps >>= 1;
     const size_t smem = coarse_refine_smem(nlist, d, warps);
@@ -2585,7 +2702,7 @@ cudaError_t launch_coarse_thr(const float2* cand, int nq, int S, int m, const fl
                               const float4* qaux, int d, int metric, float* thr, cudaStream_t s) {
     if (S > 1024 || m > S) return cudaErrorInvalidValue;
     float cK, cN;
-    err_consts(d, false, &cK, &cN, true);  // the split centroid image
+    err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
     coarse_thr_kernel<<<(nq + 7) / 8, 256, 0, s>>>(cand, nq, S, m, cxn, caux, qaux, metric, cK, cN, thr);
     return cudaGetLastError();
 }
@@ -2599,7 +2716,7 @@ cudaError_t launch_coarse_refine_keys(uint64_t* cand, const int32_t* ccnt, int n
     const size_t smem = coarse_refine_smem(0, d, warps);
     if (smem > 200 * 1024 || m > 256) return cudaErrorInvalidValue;
     float cK, cN;
-    err_consts(d, false, &cK, &cN, true);  // the split centroid image
+    err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
     const dim3 grid((nq + warps - 1) / warps);
     auto run = [&](auto kern) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -2617,15 +2734,23 @@ cudaError_t launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s) {
 }
 
 cudaError_t launch_prep_queries(const float* q, int nq, int d, void* qb, float4* qaux, float* qscale, cudaStream_t s,
-                                float amax, int32_t* qexact) {
+                                const int* cert, int32_t* qexact) {
     if (qscale) {
         prep_queries_f8_kernel<<<nq, 128, 0, s>>>(q, nq, d, (d + 127) / 128, static_cast<unsigned char*>(qb), qaux,
                                                   qscale);
     } else {
         if (d > PREP_DMAX) return cudaErrorInvalidValue;
         prep_queries_kernel<<<(nq + PREP_WARPS - 1) / PREP_WARPS, 32 * PREP_WARPS, 0, s>>>(
-            q, nq, d, (d + 63) / 64, static_cast<__nv_bfloat16*>(qb), qaux, amax, qexact);
+            q, nq, d, (d + 63) / 64, static_cast<__nv_bfloat16*>(qb), qaux, cert, qexact);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_prep_queries_tf32(const float* q, int nq, const ArenaLayout& L, float* qb, float4* qaux,
+                                     const int* cert, int32_t* qexact, cudaStream_t s) {
+    if (L.d > PREP_DMAX) return cudaErrorInvalidValue;
+    prep_queries_tf32_kernel<<<(nq + PREP_WARPS - 1) / PREP_WARPS, 32 * PREP_WARPS, 0, s>>>(q, nq, L, qb, qaux, cert,
+                                                                                           qexact);
     return cudaGetLastError();
 }
 
@@ -2652,6 +2777,18 @@ cudaError_t launch_to_f8_arena(const ArenaLayout& L, const float* codes, int64_t
 cudaError_t launch_row_aux(const ArenaLayout& L, const float* codes, int64_t rows, const float* tscale, float2* aux,
                            float2* tile_aux, cudaStream_t s) {
     row_aux_kernel<<<grid_for(rows * 32, 256), 256, 0, s>>>(L, codes, rows, tscale, aux);
+    const int64_t tiles = rows / TM;
+    tile_aux_kernel<<<grid_for(tiles * 32, 256), 256, 0, s>>>(aux, tiles, tile_aux);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_row_aux_tf32(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,
+                                const int32_t* list_size, int nlist, const float* cent, float2* aux, float2* tile_aux,
+                                double* stat, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(stat, 0, 2 * sizeof(double), s);
+    if (e != cudaSuccess) return e;
+    row_aux_tf32_kernel<<<grid_for(rows * 32, 256), 256, 0, s>>>(L, codes, rows, list_off, list_size, nlist, cent, aux,
+                                                                 stat);
     const int64_t tiles = rows / TM;
     tile_aux_kernel<<<grid_for(tiles * 32, 256), 256, 0, s>>>(aux, tiles, tile_aux);
     return cudaGetLastError();
@@ -2705,15 +2842,14 @@ cudaError_t launch_invert_probes(const int64_t* probes, int nq, int nprobe, int 
     return cudaGetLastError();
 }
 
-int batched_group_size(int d, bool f8) {
-    const int nkb = f8 ? (d + 127) / 128 : (d + 63) / 64;
+int batched_group_size(int nkb) {
     if (batched_stages<128>(nkb)) return 128;
     if (batched_stages<64>(nkb)) return 64;
     if (batched_stages<32>(nkb)) return 32;
     return 0;
 }
 
-template <int QG, bool F8>
+template <int QG, Operand OP>
 static cudaError_t launch_batched_t(BatchedParams p, int nsm, cudaStream_t s) {
     p.nslot = SLOT_MAX;
     p.ns = batched_stages<QG>(p.nkb >> p.ksplit, SLOT_MAX);
@@ -2723,10 +2859,10 @@ static cudaError_t launch_batched_t(BatchedParams p, int nsm, cudaStream_t s) {
     }
     if (p.ns == 0) return cudaErrorInvalidValue;
     const size_t smem = batched_smem<QG>(p.nkb >> p.ksplit, p.ns, p.nslot);
-    cudaError_t e = cudaFuncSetAttribute(batched_scan_kernel<QG, F8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(batched_scan_kernel<QG, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    batched_scan_kernel<QG, F8><<<nsm, BATCH_THREADS, smem, s>>>(p);
+    batched_scan_kernel<QG, OP><<<nsm, BATCH_THREADS, smem, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -2754,32 +2890,38 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
     p.err = err;
     p.nlist = b.nlist;
     p.ksplit = b.ksplit ? 1 : 0;
-    p.nkb = (b.f8 ? (b.d + 127) / 128 : (b.d + 63) / 64) << p.ksplit;
+    p.nkb = b.nkb << p.ksplit;
     p.rs = b.rs;
     p.capq = b.capq;
     p.metric = b.metric;
     p.dense_max = std::min(b.dense_max, b.capq);
     p.xaux = b.xaux;
-    err_consts(b.d, b.f8, &p.cK, &p.cN, b.ksplit);
+    err_consts(b.d, operand_k(b.op, p.nkb), &p.cK, &p.cN);
     cudaError_t e;
     if ((e = cudaMemsetAsync(w.work, 0, sizeof(unsigned int), s)) != cudaSuccess) return e;
-    switch (b.qg * 2 + (b.f8 ? 1 : 0)) {
-        case 256: return launch_batched_t<128, false>(p, b.nsm, s);
-        case 257: return launch_batched_t<128, true>(p, b.nsm, s);
-        case 128: return launch_batched_t<64, false>(p, b.nsm, s);
-        case 129: return launch_batched_t<64, true>(p, b.nsm, s);
-        case 64: return launch_batched_t<32, false>(p, b.nsm, s);
-        case 65: return launch_batched_t<32, true>(p, b.nsm, s);
+    auto run = [&](auto qg) -> cudaError_t {
+        constexpr int QG = decltype(qg)::value;
+        switch (b.op) {
+            case Operand::bf16: return launch_batched_t<QG, Operand::bf16>(p, b.nsm, s);
+            case Operand::e4m3: return launch_batched_t<QG, Operand::e4m3>(p, b.nsm, s);
+            case Operand::tf32: return launch_batched_t<QG, Operand::tf32>(p, b.nsm, s);
+        }
+        return cudaErrorInvalidValue;
+    };
+    switch (b.qg) {
+        case 128: return run(std::integral_constant<int, 128>());
+        case 64: return run(std::integral_constant<int, 64>());
+        case 32: return run(std::integral_constant<int, 32>());
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_rerank(const ArenaLayout& L, const float* codes, const int64_t* ids, const float* xn,
                           const float2* xaux, const float4* qaux, const float* q, int nq, const BatchWork& w, int qbase,
-                          int capq, int k, int rmax, int metric, bool f8, int nsm, float* D, int64_t* I,
+                          int capq, int k, int rmax, int metric, int K, int nsm, float* D, int64_t* I,
                           cudaStream_t s, const int32_t* qexact) {
     float cK, cN;
-    err_consts(L.d, f8, &cK, &cN);
+    err_consts(L.d, K, &cK, &cN);
     cudaError_t e = cudaMemsetAsync(w.big, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return e;
     const size_t wsmem = static_cast<size_t>(8) * (256 * sizeof(uint64_t) + L.row_pitch * sizeof(float));

@@ -25,9 +25,18 @@ inline size_t f8_image_bytes(int64_t rows, int d) {
     return static_cast<size_t>(rows / BATCH_ROW_ALIGN) * nkb * BATCH_KB_BYTES;
 }
 
-// Queries per group of the batched kernel for dimension d (128, 64 or 32:
-// the largest whose shared-memory footprint fits), 0 if none fits.
-int batched_group_size(int d, bool f8);
+// Operand type of a batched launch: the bf16 image, the e4m3 image or the FP32
+// arena itself read as TF32.
+enum class Operand { bf16, e4m3, tf32 };
+// 128-byte k-blocks of a row, and the products nkb of them accumulate.
+inline int operand_kblocks(Operand op, const ArenaLayout& L) {
+    return op == Operand::bf16 ? (L.d + 63) / 64 : op == Operand::e4m3 ? (L.d + 127) / 128 : L.row_pitch / 32;
+}
+inline int operand_k(Operand op, int nkb) { return nkb * (op == Operand::bf16 ? 64 : op == Operand::e4m3 ? 128 : 32); }
+
+// Queries per group of the batched kernel for rows of nkb k-blocks (128, 64 or
+// 32: the largest whose shared-memory footprint fits), 0 if none fits.
+int batched_group_size(int nkb);
 
 cudaError_t launch_to_bf16_arena(const ArenaLayout& L, const float* codes, int64_t rows, void* out, cudaStream_t s);
 // e4m3 image with per-list scales: tile_max [rows/128] scratch, lscale
@@ -37,14 +46,17 @@ cudaError_t launch_to_f8_arena(const ArenaLayout& L, const float* codes, int64_t
                                void* out, cudaStream_t s);
 // qscale == nullptr: bf16 queries; else e4m3 queries with per-query scales.
 // bf16 queries with qexact: qexact[i] = 1 when query i and the arena admit
-// exact tensor-core distances: amax >= 0 (the arena's certificate, see
-// launch_arena_integral: every value an integer of magnitude <= 256 and the
-// largest row squared norm amax), the query's values integers of magnitude
-// <= 256 and |q|^2 + amax < 2^23.  Then every product and partial sum of the
-// bf16 distance is an integer below 2^24, exact in f32, and the distance
+// exact tensor-core distances: cert (the arena's certificate on the device,
+// see launch_arena_integral) says that every value is an integer of magnitude
+// <= 256, the query's values are too, and |q|^2 + the largest row squared norm
+// < 2^23.  Then every product and partial sum of the
+// bf16 (or TF32) distance is an integer below 2^24, exact in f32, and the distance
 // equals the plain scan's bit for bit.
 cudaError_t launch_prep_queries(const float* q, int nq, int d, void* qb, float4* qaux, float* qscale, cudaStream_t s,
-                                float amax = -1.0f, int32_t* qexact = nullptr);
+                                const int* cert = nullptr, int32_t* qexact = nullptr);
+// Queries as TF32 operands (nq x row_pitch floats), with the same certificate.
+cudaError_t launch_prep_queries_tf32(const float* q, int nq, const ArenaLayout& L, float* qb, float4* qaux,
+                                     const int* cert, int32_t* qexact, cudaStream_t s);
 // flag (int, preset to 1) := 0 unless every one of the n values of codes is
 // an integer of magnitude <= 256; maxxn (preset to 0) := bit pattern of the
 // largest of xn[0..rows).
@@ -58,6 +70,12 @@ cudaError_t launch_arena_integral(const float* codes, int64_t n, const float* xn
 cudaError_t launch_tile_max(const float* xn, int64_t rows, float* tile_max, cudaStream_t s);
 cudaError_t launch_row_aux(const ArenaLayout& L, const float* codes, int64_t rows, const float* tscale, float2* aux,
                            float2* tile_aux, cudaStream_t s);
+
+// The bound terms of the arena rows read as TF32, and two sums over a sample of
+// the rows (see row_aux_tf32_kernel).
+cudaError_t launch_row_aux_tf32(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,
+                                const int32_t* list_size, int nlist, const float* cent, float2* aux, float2* tile_aux,
+                                double* stat, cudaStream_t s);
 
 // Work buffers of one batched search.
 struct BatchWork {
@@ -99,7 +117,7 @@ struct DenseFirst {
 // thr := min(thr, k-th smallest upper bound over each query's candidates),
 // and the candidates that can still reach the top-k are compacted as keys.
 cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qaux, int nq, const BatchWork& w,
-                           int capq, int k, int metric, int d, bool f8, int nsm, float* thr, cudaStream_t s,
+                           int capq, int k, int metric, int d, int K, int nsm, float* thr, cudaStream_t s,
                            DenseFirst df);
 
 // The coarse quantiser on the tensor cores (bf16 form).  The centroids
@@ -148,7 +166,7 @@ cudaError_t launch_coarse_refine_keys(uint64_t* cand, const int32_t* ccnt, int n
 constexpr size_t DENSE_MAX = 16384;
 
 struct BatchedLaunch {
-    const void* abf;
+    const void* abf;  // the operand type's image (tf32: the FP32 arena)
     const int64_t* list_off;
     const int32_t* list_size;
     const float* xn;
@@ -161,7 +179,8 @@ struct BatchedLaunch {
     const float* qscale = nullptr;  // e4m3 form: per-query scales
     int nlist, d, rs, capq, metric, nsm;
     int qg = 128;     // queries per group (batched_group_size)
-    bool f8 = false;  // e4m3 operands
+    Operand op = Operand::bf16;
+    int nkb = 0;      // 128-byte k-blocks of a query (operand_kblocks)
     bool ksplit = false;  // abf is a split image (launch_centroid_image): two k-blocks per query k-block
     // Lists of at most dense_max rows (capped at capq) are scanned densely:
     // every row's f32 score lands at the row's offset in the list within the
@@ -181,7 +200,7 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
 // whose tensor-core distances are exact keep them instead of recomputing.
 cudaError_t launch_rerank(const ArenaLayout& L, const float* codes, const int64_t* ids, const float* xn,
                           const float2* xaux, const float4* qaux, const float* q, int nq, const BatchWork& w, int qbase,
-                          int capq, int k, int rmax, int metric, bool f8, int nsm, float* D, int64_t* I,
+                          int capq, int k, int rmax, int metric, int K, int nsm, float* D, int64_t* I,
                           cudaStream_t s, const int32_t* qexact = nullptr);
 cudaError_t launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s);
 

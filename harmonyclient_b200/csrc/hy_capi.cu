@@ -198,7 +198,7 @@ struct hy_index {
 
     // plain form: query-major or list-major scan (hy_index_set_plain_scan)
     int plain_scan = HY_PLAIN_AUTO;
-    bool lm_last = false;  // the last plain search ran the list-major scan
+    bool fb_last = false;  // the last plain search ran a scan with an overflow fallback
     // batched tensor-core forms (bf16, e4m3)
     int form = HY_FORM_PLAIN;
     size_t capq = 8192;       // candidate slots per query
@@ -213,7 +213,10 @@ struct hy_index {
     DevBuf txn;               // per 128-row tile, the largest squared norm
     bool abf_valid = false;
     DevBuf b_cert;            // the bf16 image's exactness certificate {integral, max row norm}
-    float arena_maxxn = -1.0f;  // its largest row squared norm when integral (<= 256), else -1
+    bool cert_valid = false;
+    DevBuf x32aux, t32aux, a32stat;  // the arena read as TF32: bound terms, sums of launch_row_aux_tf32
+    bool a32_valid = false, a32_fits = false;  // built; the plain form's batches may run on it
+    DevBuf b_cqb, b_cqn;  // bf16 queries of the coarse step when the scan's operands are others
     DevBuf b_qx;              // per-query exact-distance flags
     DevBuf a8, x8aux, t8aux;  // the same for the e4m3 image
     DevBuf lscale, tscale, tmax;  // e4m3 per-list and per-tile scales, tile maxima
@@ -262,6 +265,12 @@ int set_device(hy_index* h) {
     HY_CUDA(cudaSetDevice(h->device));
     return HY_OK;
 }
+
+// (query, probed list) pairs from which a plain batch runs on the tensor
+// cores, and the largest mean TF32 error of a row against its distance to its
+// centroid at which it does (plain_on_tensor, ensure_operands).
+constexpr size_t TF32_MIN_PAIRS = 16384;
+constexpr double TF32_SPREAD_MAX = 0.03;
 
 // Rows x centroids x dimensions from which assignment runs on the tensor
 // cores: there the exact kernels take about 60 us, the tensor-core steps'
@@ -462,6 +471,8 @@ int build_arena(hy_index* h, const float* x, size_t n, const int32_t* order, con
     h->arena_rows = (size_t)h->h_list_off[nlist];
     const size_t rows_alloc = std::max<size_t>(h->arena_rows, hy::BATCH_ROW_ALIGN);
     h->abf_valid = false;
+    h->cert_valid = false;
+    h->a32_valid = false;
     h->a8_valid = false;
     h->c2c_valid = false;
     HY_RET(h->codes.ensure(rows_alloc * h->L.row_pitch * sizeof(float)));
@@ -754,8 +765,9 @@ int ensure_common(hy_index* h) {
     return HY_OK;
 }
 
-int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD, int64_t* dI, cudaStream_t s,
-                     bool timed);
+int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, size_t k, float* dD, int64_t* dI,
+                       cudaStream_t s, bool timed);
+bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s);
 
 bool learned_on(const hy_index* h) { return h->learned && h->model_ready; }
 bool batched_form(const hy_index* h) { return h->form == HY_FORM_BF16 || h->form == HY_FORM_FP8; }
@@ -783,18 +795,23 @@ int search_device_impl(hy_index* h, size_t n, const float* dq, size_t k, float* 
                        bool timed) {
     HY_RET(ensure_common(h));
     HY_CUDA(cudaMemsetAsync(h->w_counters.p, 0, 4 * sizeof(unsigned long long), s));
-    h->lm_last = false;
+    h->fb_last = false;
     h->stats.list_major = 0;
-    if (batched_form(h) && h->arena_rows > 0) return search_bf16_impl(h, n, dq, k, dD, dI, s, timed);
+    if (batched_form(h) && h->arena_rows > 0)
+        return search_tensor_impl(h, h->form == HY_FORM_FP8 ? hy::Operand::e4m3 : hy::Operand::bf16, n, dq, k, dD, dI,
+                                  s, timed);
     const size_t nprobe = std::min(h->nprobe, h->nlist);
     HY_CHECK(nprobe >= 1, HY_ERR_ARG, "search: nprobe must be >= 1");
     HY_CHECK(h->nlist <= 40000, HY_ERR_ARG, "search: nlist above 40000 is not supported by the coarse selector");
     HY_RET(ensure_common(h));
     size_t qc = query_chunk(h->nlist, n);
+    h->fb_last = plain_on_tensor(h, std::min(qc, std::max<size_t>(1, (size_t(2) << 30) / (h->capq * 8))), nprobe, s);
+    if (h->fb_last)
+        return search_tensor_impl(h, hy::Operand::tf32, n, dq, k, dD, dI, s, timed);
     // List-major scan: chunks sized so the candidate buffers stay within 2 GiB.
     const bool lm = use_list_major(h, qc, nprobe);
     if (lm) qc = std::min(qc, std::max<size_t>(1, (size_t(2) << 30) / (h->capq * 8)));
-    h->lm_last = lm;
+    h->fb_last = lm;
     h->stats.list_major = lm ? 1 : 0;
     HY_RET(h->w_scores.ensure(qc * h->nlist * sizeof(float)));
     HY_RET(h->w_probes.ensure(qc * nprobe * sizeof(int64_t)));
@@ -849,12 +866,34 @@ int search_device_impl(hy_index* h, size_t n, const float* dq, size_t k, float* 
     return HY_OK;
 }
 
-// The bf16 tensor-core image of the arena, built on first use after add/load.
-int ensure_bf16_image(hy_index* h, cudaStream_t s) {
-    if (h->form == HY_FORM_FP8) {
+// Largest squared norm per 128-row tile, for the tightening's bound.
+int ensure_tile_norms(hy_index* h, size_t rows, cudaStream_t s) {
+    HY_RET(h->txn.ensure(rows / hy::BATCH_ROW_ALIGN * sizeof(float)));
+    HY_CUDA(hy::launch_tile_max(h->norms.as<float>(), (int64_t)rows, h->txn.as<float>(), s));
+    return HY_OK;
+}
+
+// Exactness certificate of the arena (see launch_prep_queries), on the device.
+int ensure_certificate(hy_index* h, size_t rows, cudaStream_t s) {
+    if (h->cert_valid) return HY_OK;
+    HY_RET(h->b_cert.ensure(2 * sizeof(int32_t)));
+    HY_CUDA(cudaMemsetAsync(h->b_cert.as<int32_t>() + 1, 0, sizeof(int32_t), s));
+    HY_CUDA(cudaMemsetAsync(h->b_cert.p, 1, sizeof(int32_t), s));  // any nonzero value
+    HY_CUDA(hy::launch_arena_integral(h->codes.as<float>(), (int64_t)(rows * h->L.row_pitch), h->norms.as<float>(),
+                                      (int64_t)rows, h->b_cert.as<int>(),
+                                      reinterpret_cast<unsigned int*>(h->b_cert.as<int>() + 1), s));
+    h->cert_valid = true;
+    return HY_OK;
+}
+
+// What a batched search with these operands reads besides the arena, built on
+// first use after add/load: the bf16 or e4m3 image, the rows' bound terms, the
+// certificate.
+int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
+    const size_t rows = std::max<size_t>(h->arena_rows, hy::BATCH_ROW_ALIGN);
+    const size_t tiles = rows / hy::BATCH_ROW_ALIGN;
+    if (op == hy::Operand::e4m3) {
         if (h->a8_valid) return HY_OK;
-        const size_t rows = std::max<size_t>(h->arena_rows, hy::BATCH_ROW_ALIGN);
-        const size_t tiles = rows / hy::BATCH_ROW_ALIGN;
         HY_RET(h->a8.ensure(hy::f8_image_bytes((int64_t)rows, (int)h->d)));
         HY_RET(h->x8aux.ensure(rows * sizeof(float2)));
         HY_RET(h->t8aux.ensure(tiles * sizeof(float2)));
@@ -866,53 +905,88 @@ int ensure_bf16_image(hy_index* h, cudaStream_t s) {
                                        h->lscale.as<float>(), h->tscale.as<float>(), h->a8.p, s));
         HY_CUDA(hy::launch_row_aux(h->L, h->codes.as<float>(), (int64_t)rows, h->tscale.as<float>(),
                                    h->x8aux.as<float2>(), h->t8aux.as<float2>(), s));
-        HY_RET(h->txn.ensure(tiles * sizeof(float)));
-        HY_CUDA(hy::launch_tile_max(h->norms.as<float>(), (int64_t)rows, h->txn.as<float>(), s));
+        HY_RET(ensure_tile_norms(h, rows, s));
         h->a8_valid = true;
         return HY_OK;
     }
+    if (op == hy::Operand::tf32) {
+        if (h->a32_valid) return HY_OK;
+        HY_RET(h->x32aux.ensure(rows * sizeof(float2)));
+        HY_RET(h->t32aux.ensure(tiles * sizeof(float2)));
+        HY_RET(h->a32stat.ensure(2 * sizeof(double)));
+        HY_CUDA(hy::launch_row_aux_tf32(h->L, h->codes.as<float>(), (int64_t)rows, h->list_off.as<int64_t>(),
+                                        h->list_size.as<int32_t>(), (int)h->nlist, h->cent.as<float>(),
+                                        h->x32aux.as<float2>(), h->t32aux.as<float2>(), h->a32stat.as<double>(), s));
+        HY_RET(ensure_tile_norms(h, rows, s));
+        HY_RET(ensure_certificate(h, rows, s));
+        double stat[2] = {0, 0};
+        int32_t cert[2] = {0, 0};
+        HY_CUDA(cudaMemcpyAsync(stat, h->a32stat.p, sizeof(stat), cudaMemcpyDeviceToHost, s));
+        HY_CUDA(cudaMemcpyAsync(cert, h->b_cert.p, sizeof(cert), cudaMemcpyDeviceToHost, s));
+        HY_CUDA(cudaStreamSynchronize(s));
+        float maxxn;
+        std::memcpy(&maxxn, &cert[1], sizeof(float));
+        // Rows' TF32 error against their spread around the centroids: score
+        // differences between a query's rows are about 2 |q| |x - x'| and the
+        // bound about 2 |q| (|x - x~| + 2^-11 |x|), so above a few percent
+        // (values far from the origin next to their spread) the scores
+        // separate too few rows.  Infinities, NaN and huge rows: never.
+        h->a32_fits = maxxn < 1e37f && stat[0] < TF32_SPREAD_MAX * stat[1];
+        h->a32_valid = true;
+        return HY_OK;
+    }
     if (h->abf_valid) return HY_OK;
-    const size_t rows = std::max<size_t>(h->arena_rows, hy::BATCH_ROW_ALIGN);
     HY_RET(h->abf.ensure(hy::bf16_image_bytes((int64_t)rows, (int)h->d)));
     HY_RET(h->xaux.ensure(rows * sizeof(float2)));
-    HY_RET(h->taux.ensure(rows / hy::BATCH_ROW_ALIGN * sizeof(float2)));
+    HY_RET(h->taux.ensure(tiles * sizeof(float2)));
     HY_CUDA(hy::launch_to_bf16_arena(h->L, h->codes.as<float>(), (int64_t)rows, h->abf.p, s));
     HY_CUDA(hy::launch_row_aux(h->L, h->codes.as<float>(), (int64_t)rows, nullptr, h->xaux.as<float2>(), h->taux.as<float2>(),
                                s));
-    HY_RET(h->txn.ensure(rows / hy::BATCH_ROW_ALIGN * sizeof(float)));
-    HY_CUDA(hy::launch_tile_max(h->norms.as<float>(), (int64_t)rows, h->txn.as<float>(), s));
-    // Exactness certificate of the image (see launch_prep_queries).
-    HY_RET(h->b_cert.ensure(2 * sizeof(int32_t)));
-    const int32_t init[2] = {1, 0};
-    HY_CUDA(cudaMemcpyAsync(h->b_cert.p, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    HY_CUDA(hy::launch_arena_integral(h->codes.as<float>(), (int64_t)(rows * h->L.row_pitch), h->norms.as<float>(),
-                                      (int64_t)rows, h->b_cert.as<int>(), reinterpret_cast<unsigned int*>(h->b_cert.as<int>() + 1),
-                                      s));
-    int32_t cert[2] = {0, 0};
-    HY_CUDA(cudaMemcpyAsync(cert, h->b_cert.p, sizeof(cert), cudaMemcpyDeviceToHost, s));
-    HY_CUDA(cudaStreamSynchronize(s));
-    float mx;
-    std::memcpy(&mx, &cert[1], sizeof(float));
-    h->arena_maxxn = cert[0] ? mx : -1.0f;
+    HY_RET(ensure_tile_norms(h, rows, s));
+    HY_RET(ensure_certificate(h, rows, s));
     h->abf_valid = true;
     return HY_OK;
 }
 
-// Whether the bf16 form's coarse step runs on the tensor cores (the
+// Whether a plain search of m queries (per chunk) at nprobe that would run the
+// list-major scan runs on the tensor cores instead (the FP32 arena as TF32
+// operands, exact FP32 re-rank: the same answer).  From TF32_MIN_PAIRS (query,
+// probed list) pairs: below, its 20 launches cost more than the scan.  Not
+// with the inner-product window of OPT_TRIANGLE, whose answer off the unit
+// sphere depends on the scan's own thresholds.  The bound terms are built on
+// first use; while the stream is being captured, or without the memory for
+// them, the list-major scan runs.
+bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s) {
+    if (h->form != HY_FORM_PLAIN || h->plain_scan != HY_PLAIN_AUTO || !use_list_major(h, m, nprobe)) return false;
+    if (m * nprobe < TF32_MIN_PAIRS || (h->metric == HY_METRIC_IP && (h->opt_level & 1))) return false;
+    if (hy::batched_group_size(hy::operand_kblocks(hy::Operand::tf32, h->L)) == 0) return false;
+    if (!h->a32_valid) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return false;
+        if (ensure_operands(h, hy::Operand::tf32, s) != HY_OK) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    return h->a32_fits;
+}
+
+// Whether a batched search's coarse step runs on the tensor cores (the
 // conditions launch_coarse_refine's shared memory and select width need).
 bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
-    return h->coarse_mode == HY_COARSE_TENSOR && h->form == HY_FORM_BF16 && nprobe <= 256 && h->d <= 256 &&
-           hy::batched_group_size((int)h->d, false) > 0;
+    return h->coarse_mode == HY_COARSE_TENSOR && nprobe <= 256 && h->d <= 256 &&
+           (h->form == HY_FORM_BF16 || h->nlist <= 2048) && hy::batched_group_size((int)(h->d + 63) / 64) > 0;
 }
 
 // Coarse step on the tensor cores for m queries whose bf16 image and
-// {|q|^2, |q|, |q~|, |q - q~|} are in b_qb / b_qn: one dense batched launch
+// {|q|^2, |q|, |q~|, |q - q~|} are in qb / qn: one dense batched launch
 // over the centroid index, then the exact m best per query.
-int coarse_tensor(hy_index* h, size_t m, const float* qq, size_t nprobe, int64_t* probes, float* pscore,
-                  cudaStream_t s) {
+int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const float4* qn, size_t nprobe,
+                  int64_t* probes, float* pscore, cudaStream_t s) {
     HY_RET(ensure_centroid_image(h, s));
     const int nlist = (int)h->nlist;
-    const int qg = hy::batched_group_size((int)h->d, false);
+    const int nkb = (int)(h->d + 63) / 64;
+    const int qg = hy::batched_group_size(nkb);
     const int ngroups = (int)((m + qg - 1) / qg);
     // Row slices of a launch over the first `rows` centroids: enough to give
     // every SM an item, each at most 2048 rows.
@@ -950,15 +1024,15 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, size_t nprobe, int64_t
     b.xn = h->c_norm.as<float>();
     b.tile_aux = h->c_taux.as<float2>();
     b.xaux = h->c_aux.as<float2>();
-    b.qb = h->b_qb.p;
-    b.qaux = h->b_qn.as<float4>();
+    b.qb = qb;
+    b.qaux = qn;
+    b.nkb = nkb;
     b.thr = h->b_thr.as<float>();
     b.nlist = 1;
     b.d = (int)h->d;
     b.metric = h->metric;
     b.nsm = h->nsm;
     b.qg = qg;
-    b.f8 = false;
     b.ksplit = true;
     if (nlist <= 2048) {
         // Every (query, centroid) score, then the exact best.
@@ -971,7 +1045,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, size_t nprobe, int64_t
         HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
         HY_CUDA(hy::launch_coarse_refine(reinterpret_cast<float2*>(h->c_cand.p), (int)m, nlist, qq,
                                          h->cent.as<float>(), h->c_norm.as<float>(), h->c_aux.as<float2>(),
-                                         h->b_qn.as<float4>(), (int)h->d, h->metric, (int)nprobe, probes, pscore,
+                                         qn, (int)h->d, h->metric, (int)nprobe, probes, pscore,
                                          h->w_err.as<int>(), s));
         h->launches += 3;
         return HY_OK;
@@ -990,7 +1064,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, size_t nprobe, int64_t
     b.dense_max = S;
     HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
     HY_CUDA(hy::launch_coarse_thr(reinterpret_cast<const float2*>(h->c_cand.p), (int)m, S, (int)nprobe,
-                                  h->c_norm.as<float>(), h->c_aux.as<float2>(), h->b_qn.as<float4>(), (int)h->d,
+                                  h->c_norm.as<float>(), h->c_aux.as<float2>(), qn, (int)h->d,
                                   h->metric, h->b_thr.as<float>(), s));
     w.item_cap = (int64_t)ngroups * ns_full;
     HY_CUDA(hy::launch_coarse_items((int)m, nlist, ngroups, ns_full, h->c_off.as<int64_t>(), h->c_size.as<int32_t>(),
@@ -1001,29 +1075,34 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, size_t nprobe, int64_t
     b.dense_max = 0;
     HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
     HY_CUDA(hy::launch_coarse_refine_keys(h->c_cand.as<uint64_t>(), w.cand_cnt, (int)m, nlist, qq, h->cent.as<float>(),
-                                          h->c_norm.as<float>(), h->c_aux.as<float2>(), h->b_qn.as<float4>(),
+                                          h->c_norm.as<float>(), h->c_aux.as<float2>(), qn,
                                           (int)h->d, h->metric, (int)nprobe, probes, pscore, h->w_err.as<int>(), s));
     h->launches += 6;
     return HY_OK;
 }
 
-// Batched bf16 search of n device queries: coarse quantisation, warm-up
+// Batched search of n device queries on tensor-core operands op (the bf16 and
+// e4m3 forms, and large plain batches in TF32): coarse quantisation, warm-up
 // thresholds, probe inversion, the persistent tensor-core scan and the exact
 // re-rank, in query chunks sized so the candidate buffers stay within 2 GiB.
-int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD, int64_t* dI, cudaStream_t s,
-                     bool timed) {
+int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, size_t k, float* dD, int64_t* dI,
+                       cudaStream_t s, bool timed) {
     const size_t nprobe = std::min(h->nprobe, h->nlist);
     HY_CHECK(nprobe >= 1, HY_ERR_ARG, "search: nprobe must be >= 1");
     HY_CHECK(h->nlist <= 40000, HY_ERR_ARG, "search: nlist above 40000 is not supported by the coarse selector");
     HY_RET(ensure_common(h));
-    HY_RET(ensure_bf16_image(h, s));
+    HY_RET(ensure_operands(h, op, s));
     if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
     const size_t capq = h->capq;
     size_t qc = std::min(query_chunk(h->nlist, n), std::max<size_t>(1, (size_t(2) << 30) / (capq * 8)));
     qc = std::min(qc, n);
-    const bool f8 = h->form == HY_FORM_FP8;
-    const size_t nkb = f8 ? (h->d + 127) / 128 : (h->d + 63) / 64;  // 128-byte k-blocks per row
-    const int qg = hy::batched_group_size((int)h->d, f8);
+    const bool f8 = op == hy::Operand::e4m3, tf32 = op == hy::Operand::tf32;
+    const size_t nkb = (size_t)hy::operand_kblocks(op, h->L);  // 128-byte k-blocks per row
+    const int K = hy::operand_k(op, (int)nkb);
+    const float2* xaux = (f8 ? h->x8aux : tf32 ? h->x32aux : h->xaux).as<float2>();
+    const float2* taux = (f8 ? h->t8aux : tf32 ? h->t32aux : h->taux).as<float2>();
+    const int qg = hy::batched_group_size((int)nkb);
+    const bool coarse_tc = coarse_on_tensor(h, nprobe);
     HY_CHECK(qg > 0, HY_ERR_ARG, "search: d too large for the tensor-core form");
     const size_t nlist = h->nlist;
     HY_RET(h->w_scores.ensure(qc * nlist * sizeof(float)));
@@ -1032,6 +1111,10 @@ int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD
     HY_RET(h->w_thr.ensure(qc * sizeof(uint32_t)));
     HY_RET(h->b_thr.ensure(qc * sizeof(float)));
     HY_RET(h->b_qb.ensure(qc * nkb * 128));
+    if (coarse_tc && op != hy::Operand::bf16) {
+        HY_RET(h->b_cqb.ensure(qc * ((h->d + 63) / 64) * 128));
+        HY_RET(h->b_cqn.ensure(qc * sizeof(float4)));
+    }
     if (f8) HY_RET(h->b_qs.ensure(qc * sizeof(float)));
     HY_RET(h->b_qn.ensure(qc * sizeof(float4)));
     HY_RET(h->b_qx.ensure(qc * sizeof(int32_t)));
@@ -1116,11 +1199,23 @@ int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD
         w.overflow = h->b_ovf.as<int32_t>();  // [0] = count, then chunk-local query ids
         HY_CUDA(cudaMemsetAsync(w.overflow, 0, sizeof(int32_t), s));
         if (timed && q0 == 0) HY_CUDA(ev_record(h->ev[0], s));
-        HY_CUDA(hy::launch_prep_queries(qq, (int)m, (int)h->d, h->b_qb.p, h->b_qn.as<float4>(),
-                                        f8 ? h->b_qs.as<float>() : nullptr, s, f8 ? -1.0f : h->arena_maxxn,
-                                        f8 ? nullptr : h->b_qx.as<int32_t>()));
-        if (coarse_on_tensor(h, nprobe)) {
-            HY_RET(coarse_tensor(h, m, qq, nprobe, h->w_probes.as<int64_t>(),
+        if (tf32)
+            HY_CUDA(hy::launch_prep_queries_tf32(qq, (int)m, h->L, h->b_qb.as<float>(), h->b_qn.as<float4>(),
+                                                 h->b_cert.as<int>(), h->b_qx.as<int32_t>(), s));
+        else
+            HY_CUDA(hy::launch_prep_queries(qq, (int)m, (int)h->d, h->b_qb.p, h->b_qn.as<float4>(),
+                                            f8 ? h->b_qs.as<float>() : nullptr, s, f8 ? nullptr : h->b_cert.as<int>(),
+                                            f8 ? nullptr : h->b_qx.as<int32_t>()));
+        if (coarse_tc) {
+            const void* cqb = h->b_qb.p;
+            const float4* cqn = h->b_qn.as<float4>();
+            if (op != hy::Operand::bf16) {
+                HY_CUDA(hy::launch_prep_queries(qq, (int)m, (int)h->d, h->b_cqb.p, h->b_cqn.as<float4>(), nullptr, s));
+                cqb = h->b_cqb.p;
+                cqn = h->b_cqn.as<float4>();
+                h->launches += 1;
+            }
+            HY_RET(coarse_tensor(h, m, qq, cqb, cqn, nprobe, h->w_probes.as<int64_t>(),
                                  learned_on(h) ? h->m_pscore.as<float>() : nullptr, s));
         } else {
             HY_CUDA(hy::launch_coarse_scores(qq, (int)m, h->cent.as<float>(), (int)nlist, (int)h->d, h->metric,
@@ -1149,15 +1244,16 @@ int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD
         HY_CUDA(cudaMemsetAsync(w.cand_cnt, 0, m * sizeof(int32_t), s));
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[2], s));
         hy::BatchedLaunch b;
-        b.abf = f8 ? h->a8.p : h->abf.p;
+        b.abf = f8 ? h->a8.p : tf32 ? h->codes.p : h->abf.p;
         b.list_off = h->list_off.as<int64_t>();
         b.list_size = h->list_size.as<int32_t>();
         b.xn = h->norms.as<float>();
-        b.tile_aux = f8 ? h->t8aux.as<float2>() : h->taux.as<float2>();
-        b.xaux = f8 ? h->x8aux.as<float2>() : h->xaux.as<float2>();
+        b.tile_aux = taux;
+        b.xaux = xaux;
         b.lscale = f8 ? h->lscale.as<float>() : nullptr;
         b.qscale = f8 ? h->b_qs.as<float>() : nullptr;
-        b.f8 = f8;
+        b.op = op;
+        b.nkb = (int)nkb;
         b.qg = qg1;
         b.qb = h->b_qb.p;
         b.qaux = h->b_qn.as<float4>();
@@ -1187,11 +1283,10 @@ int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD
         df.list_size = h->list_size.as<int32_t>();
         df.list_off = h->list_off.as<int64_t>();
         df.dense_max = dense_max;
-        df.tile_aux = f8 ? h->t8aux.as<float2>() : h->taux.as<float2>();
+        df.tile_aux = taux;
         df.tile_xn = h->txn.as<float>();
-        HY_CUDA(hy::launch_tighten(h->norms.as<float>(), f8 ? h->x8aux.as<float2>() : h->xaux.as<float2>(),
-                                   h->b_qn.as<float4>(), (int)m, w, (int)capq, (int)k, h->metric, (int)h->d, f8,
-                                   h->nsm, h->b_thr.as<float>(), s, df));
+        HY_CUDA(hy::launch_tighten(h->norms.as<float>(), xaux, h->b_qn.as<float4>(), (int)m, w, (int)capq, (int)k,
+                                   h->metric, (int)h->d, K, h->nsm, h->b_thr.as<float>(), s, df));
         if (nprobe > 1) {
             HY_CUDA(hy::launch_invert_probes(h->w_probes.as<int64_t>(), (int)m, (int)nprobe, 1, (int)nprobe,
                                              (int)nlist, h->list_size.as<int32_t>(), (int)h->row_slice, qg2, w, s));
@@ -1203,10 +1298,9 @@ int search_bf16_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD
         }
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[3], s));
         const int rmax = f8 ? (int)std::min<size_t>(h->oversample * k, 4096) : 0;
-        HY_CUDA(hy::launch_rerank(h->L, h->codes.as<float>(), h->ids.as<int64_t>(), h->norms.as<float>(),
-                                  f8 ? h->x8aux.as<float2>() : h->xaux.as<float2>(), h->b_qn.as<float4>(), qq, (int)m,
-                                  w, 0, (int)capq, (int)k, rmax, h->metric, f8, h->nsm, dD + q0 * k, dI + q0 * k, s,
-                                  f8 ? nullptr : h->b_qx.as<int32_t>()));
+        HY_CUDA(hy::launch_rerank(h->L, h->codes.as<float>(), h->ids.as<int64_t>(), h->norms.as<float>(), xaux,
+                                  h->b_qn.as<float4>(), qq, (int)m, w, 0, (int)capq, (int)k, rmax, h->metric, K,
+                                  h->nsm, dD + q0 * k, dI + q0 * k, s, f8 ? nullptr : h->b_qx.as<int32_t>()));
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[4], s));
         const int fb = (int)std::min<size_t>(m, fbcap);
         HY_CUDA(hy::launch_fb_gather(w.overflow, qq, h->w_probes.as<int64_t>(), (int)nprobe, (int)h->d, fb,
@@ -1536,7 +1630,8 @@ int hy_index_set_form(hy_index* h, int form) {
     h->epoch++;  // a captured search graph no longer matches
     HY_CHECK(form == HY_FORM_PLAIN || form == HY_FORM_BF16 || form == HY_FORM_FP8, HY_ERR_ARG,
              "set_form: unknown form");
-    HY_CHECK(form == HY_FORM_PLAIN || hy::batched_group_size((int)h->d, form == HY_FORM_FP8) > 0, HY_ERR_ARG,
+    const hy::Operand op = form == HY_FORM_FP8 ? hy::Operand::e4m3 : hy::Operand::bf16;
+    HY_CHECK(form == HY_FORM_PLAIN || hy::batched_group_size(hy::operand_kblocks(op, h->L)) > 0, HY_ERR_ARG,
              "set_form: d too large for the tensor-core forms (bf16: d <= 768, e4m3: d <= 1536)");
     h->form = form;
     return HY_OK;
@@ -1758,7 +1853,7 @@ int search_host(hy_index* h, size_t n, const float* q, size_t k, float* D, int64
     h->stats.fallback_queries = 0;
     h->stats.mean_nprobe = (double)std::min(h->nprobe, h->nlist);
     if (learned_on(h)) h->stats.mean_nprobe = (double)h->hstat->learned_total / (double)n;
-    if ((batched_form(h) || h->lm_last) && h->arena_rows > 0) HY_RET(bf16_fallback(h));
+    if ((batched_form(h) || h->fb_last) && h->arena_rows > 0) HY_RET(bf16_fallback(h));
     return HY_OK;
 }
 
@@ -2175,7 +2270,8 @@ int hy_index_probes(hy_index* h, size_t n, const float* q, int64_t* probes) {
         const float* qq = h->w_q.as<float>() + q0 * h->d;
         if (tensor) {
             HY_CUDA(hy::launch_prep_queries(qq, (int)m, (int)h->d, h->b_qb.p, h->b_qn.as<float4>(), nullptr, s));
-            HY_RET(coarse_tensor(h, m, qq, nprobe, h->w_probes.as<int64_t>() + q0 * nprobe,
+            HY_RET(coarse_tensor(h, m, qq, h->b_qb.p, h->b_qn.as<float4>(), nprobe,
+                                 h->w_probes.as<int64_t>() + q0 * nprobe,
                                  learned_on(h) ? h->m_pscore.as<float>() : nullptr, s));
         } else {
             HY_CUDA(hy::launch_coarse_scores(qq, (int)m, h->cent.as<float>(), (int)h->nlist, (int)h->d, h->metric,
@@ -2237,7 +2333,7 @@ int hy_index_last_stats(const hy_index* hc, hy_search_stats_t* out) {
         HY_RET(set_device(h));
         HY_CUDA(cudaEventSynchronize(h->ev[4]));
         collect_times(h);
-        if ((batched_form(h) || h->lm_last) && h->b_fbtot.p) {
+        if ((batched_form(h) || h->fb_last) && h->b_fbtot.p) {
             unsigned long long c = 0;
             HY_CUDA(cudaMemcpy(&c, h->b_fbtot.p, sizeof(c), cudaMemcpyDeviceToHost));
             h->stats.fallback_queries = c;

@@ -597,13 +597,13 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
     auto block_sum = [&](int s) -> float {
         const int b = sblk[s];
         const int P = L.pitch[b];
-        const float* rowp = wb + static_cast<size_t>(s) * slot_floats + lane * P;
+        const float* rowp = wb + static_cast<size_t>(s) * slot_floats + lane * 32;
         const float* qb = qs + L.boff[b];
         float acc = 0.0f;
         for (int c8 = 0; c8 < (P >> 2); c8 += 8) {
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const float4 x = *reinterpret_cast<const float4*>(rowp + 4 * (c8 + (u ^ (lane & 7))));
+                const float4 x = *reinterpret_cast<const float4*>(rowp + 128 * c8 + 4 * (u ^ (lane & 7)));
                 const float4 y = *reinterpret_cast<const float4*>(qb + 4 * (c8 + u));
                 if (l2) {
                     acc = sq_add(acc, y.x, x.x);
@@ -626,15 +626,15 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
     auto block_sum2 = [&](int s0, int s1, float& a0, float& a1) {
         const int b0 = sblk[s0], b1 = sblk[s1];
         const int P = L.pitch[b0];
-        const float* r0 = wb + static_cast<size_t>(s0) * slot_floats + lane * P;
-        const float* r1 = wb + static_cast<size_t>(s1) * slot_floats + lane * P;
+        const float* r0 = wb + static_cast<size_t>(s0) * slot_floats + lane * 32;
+        const float* r1 = wb + static_cast<size_t>(s1) * slot_floats + lane * 32;
         const float* q0 = qs + L.boff[b0];
         const float* q1 = qs + L.boff[b1];
         float acc0 = 0.0f, acc1 = 0.0f;
         for (int c8 = 0; c8 < (P >> 2); c8 += 8) {
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const int pc = 4 * (c8 + (u ^ (lane & 7)));
+                const int pc = 128 * c8 + 4 * (u ^ (lane & 7));
                 const float4 x0 = *reinterpret_cast<const float4*>(r0 + pc);
                 const float4 x1 = *reinterpret_cast<const float4*>(r1 + pc);
                 const float4 y0 = *reinterpret_cast<const float4*>(q0 + 4 * (c8 + u));

@@ -13,9 +13,13 @@ namespace hy {
 // id is -1.  Inside a tile, the dimensions are split into `nb` blocks; block b
 // of all 32 rows is one contiguous run of 32 * pitch[b] floats, so the rows'
 // block b is a single bulk copy and a tile whose rows are all pruned after
-// block b never loads blocks b+1...  Within a row's block, 16-byte chunk c is
-// stored at chunk (c & ~7) | ((c ^ row) & 7), which lets 32 lanes reading the
-// same logical chunk of 32 rows hit 32 different shared-memory banks.
+// block b never loads blocks b+1...  A block is stored as pitch / 32 groups of
+// 32 floats (128 bytes) of the 32 rows, 4 KB each, row after row; within a
+// row's group, 16-byte chunk c is stored at chunk (c ^ row) & 7, which lets 32
+// lanes reading the same logical chunk of 32 rows hit 32 different
+// shared-memory banks.  That is the tensor cores' 128-byte-swizzled K-major
+// layout: a group of four consecutive tiles (128 rows) is a TF32 operand as it
+// lies.
 struct ArenaLayout {
     int d = 0;
     int nb = 0;                        // dimension blocks
@@ -31,9 +35,8 @@ __host__ __device__ inline size_t arena_offset(const ArenaLayout& L, int64_t r, 
     const int64_t tile = r >> 5;
     const int lr = static_cast<int>(r & 31);
     const int c = j >> 2;
-    const int pc = (c & ~7) | ((c ^ lr) & 7);
     return static_cast<size_t>(tile) * 32 * L.row_pitch + static_cast<size_t>(L.boff[b]) * 32 +
-           static_cast<size_t>(lr) * L.pitch[b] + static_cast<size_t>(pc) * 4 + (j & 3);
+           static_cast<size_t>(c >> 3) * 1024 + static_cast<size_t>(lr) * 32 + ((c ^ lr) & 7) * 4 + (j & 3);
 }
 
 struct ScanParams {

@@ -67,7 +67,8 @@ __device__ inline int4 decode_item(const ListScanParams& p, int64_t g) {
 }
 
 // One dimension block of one 32-row tile against the group's live queries.
-// `rowp`: this lane's row of the staged block (pitch P floats); `qb(qi)`:
+// `rowp`: this lane's row of the staged block's first group (pitch P floats in
+// all, groups 1024 floats apart); `qb(qi)`:
 // query qi's block.  sp[qi] accumulates the block sums in order.
 // MULTI = false: the block is one 32-float chunk group (pitch 32).
 template <int QG, bool MULTI>
@@ -108,7 +109,7 @@ __device__ __forceinline__ void block_compute(const float* rowp, const float* qs
             float4 xr[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c)
-                xr[c] = *reinterpret_cast<const float4*>(rowp + 4 * (s8 + (c ^ (lane & 7))));
+                xr[c] = *reinterpret_cast<const float4*>(rowp + 128 * s8 + 4 * (c ^ (lane & 7)));
 #pragma unroll
             for (int qi = 0; qi < QG; ++qi) {
                 if (live & (1u << qi)) {
@@ -525,7 +526,7 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
                 } else {
                     computed += static_cast<unsigned long long>(__popc(live)) * (L.pitch[b] >> 4);
                     const int P = L.pitch[b];
-                    const float* rowp = wb + static_cast<size_t>(slot) * slot_floats + lane * P;
+                    const float* rowp = wb + static_cast<size_t>(slot) * slot_floats + lane * 32;
                     block_compute<QG, MULTI>(rowp, qs, L.row_pitch, L.boff[b], P, b == 0, l2, live, sp, lane);
                     if (b + 1 < L.nb) {
                         if (prune) {

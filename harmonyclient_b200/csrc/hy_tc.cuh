@@ -53,6 +53,30 @@ __host__ __device__ constexpr uint32_t idesc_e4m3_f32(int M, int N) {
            | (static_cast<uint32_t>(M >> 4) << 24);    // M / 16
 }
 
+// Instruction descriptor of kind::tf32 (A and B formats 2 = TF32: 32-bit
+// values whose low 13 bits do not take part), f32 accumulator, both operands
+// K-major, shape M x N.
+__host__ __device__ constexpr uint32_t idesc_tf32_f32(int M, int N) {
+    return (1u << 4)                                   // D format: f32
+           | (2u << 7)                                 // A format: tf32
+           | (2u << 10)                                // B format: tf32
+           | (static_cast<uint32_t>(N >> 3) << 17)     // N / 8
+           | (static_cast<uint32_t>(M >> 4) << 24);    // M / 16
+}
+
+// D[tmem] (+)= A * B^T on tf32 operands (K = 8 per instruction), one thread.
+__device__ inline void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    const uint32_t z = 0;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t"
+        "}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z)
+        : "memory");
+}
+
 // D[tmem] (+)= A * B^T on e4m3 operands (K = 32 per instruction), one thread.
 __device__ inline void mma_e4m3(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     const uint32_t z = 0;
