@@ -41,9 +41,14 @@ namespace {
 
 constexpr int METRIC_IP = 0, METRIC_L2 = 1;  // include/hy.h's HY_METRIC_*
 constexpr int TM = 128;      // rows per tile (MMA M)
-constexpr int NS_MIN = 4;    // A stages (one 16 KiB k-block each): at least this many,
-constexpr int NS_MAX = 8;    // and as many more as shared memory holds
+constexpr int NS_MAX = 8;    // stages of the list k-block ring: at most
+constexpr int RING_MIN = 4;  // k-blocks the ring holds: at least (64 KiB in flight)
 constexpr int KB_BYTES = 16384;
+constexpr int NKB_MAX = 12;  // k-blocks of a row: at most (bf16 d <= 768, e4m3 d <= 1536)
+// k-blocks per stage: two where rows have two or more.  A stage costs its
+// issuers a barrier wait, a commit and their loops (about 350 cycles) beside
+// the copies (130 each) and MMAs, which one 16 KiB k-block does not cover.
+__host__ __device__ constexpr int stage_kblocks(int nkb) { return nkb >= 2 ? 2 : 1; }
 
 // ---------------------------------------------------------------------------
 // Conversion of the FP32 arena into the bf16 tensor-core image.
@@ -719,7 +724,7 @@ __global__ void __launch_bounds__(512) invert_fill_kernel(const int64_t* __restr
 
 // ---------------------------------------------------------------------------
 struct BatchedParams {
-    const unsigned char* abf;       // tensor-core image of the arena (bf16 or e4m3)
+    const unsigned char* abf;       // tensor-core image of the arena (tf32: the arena)
     const int64_t* list_off;        // [nlist+1]
     const int32_t* list_size;       // [nlist]
     const int64_t* item_off;        // [nlist+1]
@@ -742,7 +747,7 @@ struct BatchedParams {
     int* err;
     int nlist, nkb, rs, capq, metric;
     int ksplit;                     // 1: A k-blocks 2j, 2j+1 (hi, lo) both take query k-block j
-    int ns;                         // stages in the list k-block ring (NS_MIN..NS_MAX)
+    int ns;                         // stages in the list k-block ring (at most NS_MAX)
     int nslot;                      // item slots (2 or SLOT_MAX)
     int dense_max;                  // lists of at most this many rows: dense items (0 = none)
     float cK, cN;                   // error-bound constants (see err_coef)
@@ -756,15 +761,24 @@ constexpr int N_GATHER = 2;
 constexpr int W_EPI0 = 4;       // warps 4-11: epilogue (two per TMEM lane quadrant)
 constexpr int N_EPI = 8;
 constexpr int BATCH_THREADS = 32 * (W_EPI0 + N_EPI);
-constexpr int CB = 256;         // per-epilogue-warp candidate staging
+constexpr int CB = 128;         // per-epilogue-warp candidate staging
 
 // Item metadata of one query slot.  Two slots hold the item being scanned and
 // the next one being gathered; a third lets the gather run a further item
 // ahead, since a slot only frees when the epilogue has finished its item.
 constexpr int SLOT_MAX = 3;
-constexpr int NS_SLOT3 = 5;   // three slots only when they leave this many stages
-constexpr int RS_MAX = 2048;  // largest row slice (rows staged per slot)
-template <int QG>
+constexpr int RING_SLOT3 = 5;  // three slots only when they leave this many k-blocks in the ring
+// WIDE: rows of many k-blocks, whose query operands take most of the shared
+// memory: shorter row slices and candidate-test chunks make room for groups
+// of 64 where only 32 fit otherwise (an MMA of N = 32 costs 40 cycles, of 64
+// 48).
+template <int QG, bool WIDE>
+struct Shape {
+    static constexpr int CW = QG / 2;                                   // accumulator columns per epilogue warp
+    static constexpr int CC = WIDE ? 8 : CW < 16 ? CW : 16;             // columns per candidate-test chunk
+    static constexpr int RS_MAX = WIDE ? 512 : 2048;                    // largest row slice (rows staged per slot)
+};
+template <int QG, int RS_MAX>
 struct ItemSlot {
     int ntiles;  // -1 = no more items
     int nqv;
@@ -773,34 +787,32 @@ struct ItemSlot {
     int dense;   // 1: every row's score at its offset in the list, no threshold test
     long long row0;
     alignas(16) float xn[RS_MAX];  // |x|^2 of the slice's rows (cp.async target: 16-byte aligned)
-    float2 taux[RS_MAX / TM];    // per tile {max |x~|, max |x - x~|}
     int qid[QG];
     float qn[QG];    // |q|^2
-    float V[QG];     // threshold + bound constant - |q|^2 (score units)
-    float aq[QG];    // bound coefficient of |x~|
-    float bq[QG];    // bound coefficient of |x - x~|
-    float cq[QG];    // bound constant
+    // -(threshold + the largest error bound over the slice's rows - |q|^2),
+    // score units: row x is a candidate when cf ip + this <= -(|x|^2 - cx)
+    alignas(16) float nr[QG];
     alignas(16) float sc[QG];    // accumulator -> inner product scale (1, or list scale x query scale)
 };
 
-// Dynamic shared memory of the batched kernel for query groups of QG, nkb
-// 128-byte k-blocks per row, ns stages and nslot item slots.
-template <int QG>
-constexpr size_t batched_smem(int nkb, int ns, int nslot) {
-    constexpr int CW = QG / 2, CC = CW < 32 ? CW : 32;
-    return 1024 + nslot * static_cast<size_t>(nkb) * QG * 128 + static_cast<size_t>(ns) * KB_BYTES +
-           nslot * sizeof(ItemSlot<QG>) + N_EPI * CW * sizeof(float) + N_EPI * CB * (sizeof(int) + sizeof(uint64_t)) +
-           N_EPI * 32 * CC * sizeof(float);
+// Dynamic shared memory of the batched kernel for rows (and queries) of nkb
+// 128-byte k-blocks, `ring` k-blocks in the stage ring and nslot item slots.
+template <int QG, bool WIDE>
+constexpr size_t batched_smem(int nkb, int ring, int nslot) {
+    using S = Shape<QG, WIDE>;
+    return 1024 + nslot * static_cast<size_t>(nkb) * QG * 128 + static_cast<size_t>(ring) * KB_BYTES +
+           nslot * sizeof(ItemSlot<QG, S::RS_MAX>) + N_EPI * CB * (sizeof(int) + sizeof(uint64_t)) + N_EPI * 32 * S::CC * sizeof(float);
 }
 // Dynamic shared memory per CTA: the 227 KiB opt-in limit less room for the
 // kernel's static shared variables (barriers, TMEM base, flags).
 constexpr size_t BATCHED_SMEM_CAP = 227 * 1024 - 256;
 
-// The deepest stage ring in [NS_MIN, NS_MAX] that fits (0: none fits).
-template <int QG>
+// Stages of the deepest ring that fits (0: fewer than RING_MIN k-blocks).
+template <int QG, bool WIDE>
 constexpr int batched_stages(int nkb, int nslot = 2) {
-    for (int ns = NS_MAX; ns >= NS_MIN; --ns)
-        if (batched_smem<QG>(nkb, ns, nslot) <= BATCHED_SMEM_CAP) return ns;
+    const int ks = stage_kblocks(nkb);
+    for (int ns = NS_MAX; ns * ks >= RING_MIN; --ns)
+        if (batched_smem<QG, WIDE>(nkb, ns * ks, nslot) <= BATCHED_SMEM_CAP) return ns;
     return 0;
 }
 
@@ -830,14 +842,13 @@ __device__ inline void named_sync(int id, int nthreads) {
 // 8; the list rows are the FP32 arena itself, whose layout is the operand's).
 // Either way a k-block row is 128 bytes and one instruction covers 32 bytes
 // of it, so the descriptors and the stage ring are the same.
-template <int QG, Operand OP>
+template <int QG, Operand OP, bool WIDE>
 __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __grid_constant__ BatchedParams p) {
     constexpr bool F8 = OP == Operand::e4m3;
-    constexpr int CW = QG / 2;            // accumulator columns per epilogue warp
-    constexpr int CC = CW < 32 ? CW : 32;  // columns per candidate-test chunk
+    constexpr int CW = Shape<QG, WIDE>::CW, CC = Shape<QG, WIDE>::CC;
     constexpr int TMEM_COLS = 2 * QG;      // two accumulators
     constexpr int BKB = QG * 128;          // bytes of one B (query) k-block
-    using Slot = ItemSlot<QG>;
+    using Slot = ItemSlot<QG, Shape<QG, WIDE>::RS_MAX>;
     extern __shared__ unsigned char sm_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~uintptr_t(1023));
     const int nkb = p.nkb;                  // list (A) k-blocks per row
@@ -845,12 +856,12 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
     const int nsl = p.nslot;                                         // item slots
     unsigned char* sB = base;                                        // nsl slots x nkb x BKB (queries)
     const int ns = p.ns;                                             // stages in the ring
-    unsigned char* sA = sB + static_cast<size_t>(nsl) * nkbq * BKB;  // ns x 16 KiB (list k-blocks)
-    Slot* slot = reinterpret_cast<Slot*>(sA + static_cast<size_t>(ns) * KB_BYTES);  // [nsl], 1024-aligned
+    const int ks = stage_kblocks(nkb);                               // list k-blocks per stage
+    unsigned char* sA = sB + static_cast<size_t>(nsl) * nkbq * BKB;  // ns x ks x 16 KiB (list k-blocks)
+    Slot* slot = reinterpret_cast<Slot*>(sA + static_cast<size_t>(ns * ks) * KB_BYTES);  // [nsl], 1024-aligned
     static_assert(offsetof(Slot, xn) % 16 == 0 && offsetof(Slot, sc) % 16 == 0 && sizeof(Slot) % 16 == 0,
                   "ItemSlot alignment");
-    float* sR = reinterpret_cast<float*>(slot + nsl);                // [N_EPI][CW] per-tile test bounds
-    int* s_cq = reinterpret_cast<int*>(sR + N_EPI * CW);             // [N_EPI][CB]
+    int* s_cq = reinterpret_cast<int*>(slot + nsl);                  // [N_EPI][CB]
     uint64_t* s_ck = reinterpret_cast<uint64_t*>(s_cq + N_EPI * CB);  // [N_EPI][CB]
     float* s_ip = reinterpret_cast<float*>(s_ck + N_EPI * CB);       // [N_EPI][32 lanes][CC] candidate chunks
 
@@ -948,7 +959,16 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             // copies (the arena is padded to whole tiles, so the rounded-up
             // ranges stay inside it).
             for (int c = gt; c < (nrows + 3) / 4; c += 32 * N_GATHER) cp_async16(&S.xn[4 * c], p.xn + row0 + 4 * c);
-            for (int c = gt; c < (nrows + TM - 1) / TM; c += 32 * N_GATHER) S.taux[c] = p.tile_aux[row0 / TM + c];
+            // The slice's largest |x~| and |x - x~| (at most 16 tiles).
+            float2 ta = make_float2(0.0f, 0.0f);
+            if (lane < (nrows + TM - 1) / TM) ta = p.tile_aux[row0 / TM + lane];
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                ta.x = fmaxf(ta.x, __shfl_xor_sync(FULL, ta.x, o));
+                ta.y = fmaxf(ta.y, __shfl_xor_sync(FULL, ta.y, o));
+            }
+            ta.x = __shfl_sync(FULL, ta.x, 0);
+            ta.y = __shfl_sync(FULL, ta.y, 0);
             // Query i of the group sits in accumulator column col(i): even
             // queries in the first half of the columns, odd ones in the
             // second, so a small group keeps both epilogue warps of every
@@ -961,17 +981,11 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                     const float4 qa = p.qaux[qid];
                     const ErrCoef ec = err_coef(qa, l2, p.cK, p.cN);
                     S.qn[col] = l2 ? qa.x : 0.0f;
-                    S.V[col] = p.thr[qid] + ec.cq - (l2 ? qa.x : 0.0f);
-                    S.aq[col] = ec.aq;
-                    S.bq[col] = ec.bq;
-                    S.cq[col] = ec.cq;
+                    S.nr[col] = -(p.thr[qid] + ec.cq - (l2 ? qa.x : 0.0f) + fmaf(ta.x, ec.aq, ta.y * ec.bq));
                     S.sc[col] = F8 ? ls * p.qscale[qid] : 1.0f;
                 } else {
                     S.qn[col] = 0.0f;
-                    S.V[col] = -INFINITY;
-                    S.aq[col] = 0.0f;
-                    S.bq[col] = 0.0f;
-                    S.cq[col] = 0.0f;
+                    S.nr[col] = INFINITY;
                     S.sc[col] = 0.0f;
                 }
             }
@@ -1002,102 +1016,92 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             mbar_arrive_cta(&sfull[b]);
         }
     } else if (warp == W_PRODUCER) {
-        // ---------------- producer: list k-blocks into the stage ring
-        if (lane == 0) {
-            int ls = 0;        // stage of the next copy
-            uint32_t lph = 0;  // its ring round's parity
-            for (uint32_t it = 0;; ++it) {
-                const int b = static_cast<int>(it % nsl);
-                if (!wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort)) break;
-                const int ntiles = slot[b].ntiles;
-                if (ntiles < 0) break;
-                const int64_t tile0 = slot[b].row0 / TM;
-                bool ok = true;
-                for (int t = 0; t < ntiles && ok; ++t) {
-                    for (int kb = 0; kb < nkb; ++kb) {
-                        const int s = ls;
-                        const uint32_t ph = lph;
-                        if (++ls == ns) {
-                            ls = 0;
-                            lph ^= 1u;
-                        }
-                        if (!wait_or_abort(&empty[s], ph ^ 1u, p.err, vabort)) {
-                            ok = false;
-                            break;
-                        }
-                        mbar_expect_tx(&full[s], KB_BYTES);
-                        if constexpr (OP == Operand::tf32) {
-                            // 32 dimensions of 128 arena rows: one 4 KB group
-                            // of each of their four 32-row tiles.
-                            const int64_t tile_bytes = static_cast<int64_t>(nkb) * 4096;
-#pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                bulk_g2s(sA + static_cast<size_t>(s) * KB_BYTES + i * 4096,
-                                         p.abf + ((tile0 + t) * 4 + i) * tile_bytes + kb * 4096, 4096, &full[s]);
-                        } else {
-                            bulk_g2s(sA + static_cast<size_t>(s) * KB_BYTES,
-                                     p.abf + ((tile0 + t) * nkb + kb) * static_cast<int64_t>(KB_BYTES), KB_BYTES,
-                                     &full[s]);
-                        }
+        // ---------------- producer: list k-blocks into the stage ring (the
+        // whole warp keeps the loop, an elected lane issues)
+        int ls = 0;        // stage of the next copy
+        uint32_t lph = 0;  // its ring round's parity
+        bool ok = true;
+        for (uint32_t it = 0; ok; ++it) {
+            const int b = static_cast<int>(it % nsl);
+            if (!__all_sync(FULL, wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort))) break;
+            const int ntiles = slot[b].ntiles;
+            if (ntiles < 0) break;
+            const int64_t tile0 = slot[b].row0 / TM;
+            const unsigned char* src = p.abf + tile0 * nkb * KB_BYTES;
+            for (int t = 0; t < ntiles && ok; ++t) {
+                for (int kb = 0; kb < nkb; kb += ks) {
+                    ok = __all_sync(FULL, wait_or_abort(&empty[ls], lph ^ 1u, p.err, vabort));
+                    if (!ok) break;
+                    const int n = min(ks, nkb - kb);
+                    unsigned char* dst = sA + static_cast<size_t>(ls * ks) * KB_BYTES;
+                    if (tc::elect_one()) {
+                        mbar_expect_tx(&full[ls], n * KB_BYTES);
+                        bulk_g2s(dst, src, n * KB_BYTES, &full[ls]);
+                    }
+                    __syncwarp();
+                    src += n * KB_BYTES;
+                    if (++ls == ns) {
+                        ls = 0;
+                        lph ^= 1u;
                     }
                 }
-                if (!ok) break;
             }
         }
     } else if (warp == W_MMA) {
-        // ---------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = F8                      ? tc::idesc_e4m3_f32(TM, QG)
-                                   : OP == Operand::tf32 ? tc::idesc_tf32_f32(TM, QG)
-                                                         : tc::idesc_bf16_f32(TM, QG);
-            int ms = 0;        // stage of the next k-block
-            uint32_t mph = 0;  // its ring round's parity
-            uint32_t tile_it = 0;
-            bool ok = true;
-            for (uint32_t it = 0; ok; ++it) {
-                const int b = static_cast<int>(it % nsl);
-                if (!wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort)) break;
-                const int ntiles = slot[b].ntiles;
-                if (ntiles < 0) break;
-                tc::fence_after_sync();
-                const uint32_t b0 = smem_u32(sB + static_cast<size_t>(b) * nkbq * BKB);
-                for (int t = 0; t < ntiles && ok; ++t, ++tile_it) {
-                    const int buf = tile_it & 1;
-                    if (!wait_or_abort(&acce[buf], ((tile_it >> 1) & 1u) ^ 1u, p.err, vabort)) {
-                        ok = false;
-                        break;
-                    }
+        // ---------------- MMA issuer (the whole warp keeps the loop, an
+        // elected lane issues; descriptors are one base plus offsets in
+        // 16-byte units)
+        const uint32_t idesc = F8                      ? tc::idesc_e4m3_f32(TM, QG)
+                               : OP == Operand::tf32 ? tc::idesc_tf32_f32(TM, QG)
+                                                     : tc::idesc_bf16_f32(TM, QG);
+        const uint64_t adesc = tc::sdesc_sw128(smem_u32(sA)), bdesc = tc::sdesc_sw128(smem_u32(sB));
+        int ms = 0;        // stage of the next k-block
+        uint32_t mph = 0;  // its ring round's parity
+        uint32_t tile_it = 0;
+        bool ok = true;
+        for (uint32_t it = 0; ok; ++it) {
+            const int b = static_cast<int>(it % nsl);
+            if (!__all_sync(FULL, wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort))) break;
+            const int ntiles = slot[b].ntiles;
+            if (ntiles < 0) break;
+            const uint64_t b0 = bdesc + static_cast<uint32_t>(b * nkbq) * (BKB >> 4);
+            for (int t = 0; t < ntiles && ok; ++t, ++tile_it) {
+                const int buf = tile_it & 1;
+                ok = __all_sync(FULL, wait_or_abort(&acce[buf], ((tile_it >> 1) & 1u) ^ 1u, p.err, vabort));
+                if (!ok) break;
+                const uint32_t dcol = tmem + static_cast<uint32_t>(buf * QG);
+                for (int kb0 = 0; kb0 < nkb; kb0 += ks) {
+                    ok = __all_sync(FULL, wait_or_abort(&full[ms], mph, p.err, vabort));
+                    if (!ok) break;
                     tc::fence_after_sync();
-                    const uint32_t dcol = tmem + static_cast<uint32_t>(buf * QG);
-                    for (int kb = 0; kb < nkb; ++kb) {
-                        const int s = ms;
-                        const uint32_t ph = mph;
-                        if (++ms == ns) {
-                            ms = 0;
-                            mph ^= 1u;
-                        }
-                        if (!wait_or_abort(&full[s], ph, p.err, vabort)) {
-                            ok = false;
-                            break;
-                        }
-                        tc::fence_after_sync();
-                        const uint32_t a0 = smem_u32(sA + static_cast<size_t>(s) * KB_BYTES);
+                    const uint64_t a0 = adesc + static_cast<uint32_t>(ms * ks) * (KB_BYTES >> 4);
+                    const int last = min(kb0 + ks, nkb);
+                    if (tc::elect_one()) {
+                        for (int kb = kb0; kb < last; ++kb) {
+                            const uint64_t a1 = a0 + static_cast<uint32_t>(kb - kb0) * (KB_BYTES >> 4);
+                            const uint64_t b1 = b0 + static_cast<uint32_t>(kb >> p.ksplit) * (BKB >> 4);
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            const uint64_t ad = tc::sdesc_sw128(a0 + kk * 32);
-                            const uint64_t bd = tc::sdesc_sw128(b0 + (kb >> p.ksplit) * BKB + kk * 32);
-                            if constexpr (F8)
-                                tc::mma_e4m3(dcol, ad, bd, idesc, (kb | kk) != 0 ? 1u : 0u);
-                            else if constexpr (OP == Operand::tf32)
-                                tc::mma_tf32(dcol, ad, bd, idesc, (kb | kk) != 0 ? 1u : 0u);
-                            else
-                                tc::mma_bf16(dcol, ad, bd, idesc, (kb | kk) != 0 ? 1u : 0u);
+                            for (int kk = 0; kk < 4; ++kk) {
+                                if constexpr (F8)
+                                    tc::mma_e4m3(dcol, a1 + 2 * kk, b1 + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+                                else if constexpr (OP == Operand::tf32)
+                                    tc::mma_tf32(dcol, a1 + 2 * kk, b1 + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+                                else
+                                    tc::mma_bf16(dcol, a1 + 2 * kk, b1 + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+                            }
                         }
-                        tc::mma_commit(&empty[s]);
+                        tc::mma_commit(&empty[ms]);
+                        if (last == nkb) {
+                            tc::mma_commit(&accf[buf]);
+                            if (t == ntiles - 1) tc::mma_commit(&sfree[b]);  // the slot's queries are no longer read
+                        }
                     }
-                    if (ok) tc::mma_commit(&accf[buf]);
+                    __syncwarp();
+                    if (++ms == ns) {
+                        ms = 0;
+                        mph ^= 1u;
+                    }
                 }
-                if (ok) tc::mma_commit(&sfree[b]);  // the slot's queries are no longer read
             }
         }
     } else if (warp >= W_EPI0) {
@@ -1118,6 +1122,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
         constexpr int NSEG = 4, SEG = CB / NSEG, SJ = SEG / 32;
         int wc = 0, npend = 0;
         int pos0[SJ], pos1[SJ], pos2[SJ];  // reserved slots, oldest .. newest
+#pragma unroll
+        for (int j = 0; j < SJ; ++j) pos0[j] = pos1[j] = pos2[j] = p.capq;  // none yet
         auto reserve = [&](int seg, int n, int (&pos)[SJ]) {
 #pragma unroll
             for (int j = 0; j < SJ; ++j) {
@@ -1145,18 +1151,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             const int nrows = S.nrows;
             const long long row0 = S.row0;
             bool ok = true;
-            float* R = sR + e * CW;  // this warp's CW columns
             for (int t = 0; t < ntiles; ++t, ++tile_it) {
                 const int buf = tile_it & 1;
-                // Per-tile test bound of this warp's queries:
-                // V + max|x~| aq + max|x - x~| bq over the tile's rows.
-                const float2 ta = S.taux[t];
-                __syncwarp();
-                for (int cc = lane; cc < CW; cc += 32) {
-                    const int q = half * CW + cc;
-                    R[cc] = S.V[q] + fmaf(ta.x, S.aq[q], ta.y * S.bq[q]);
-                }
-                __syncwarp();
                 if (!wait_or_abort(&accf[buf], (tile_it >> 1) & 1u, p.err, vabort)) {
                     ok = false;
                     break;
@@ -1167,21 +1163,23 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                 const long long arow = row0 + rs_row;
                 const float xnv = rvalid ? S.xn[rs_row] : 0.0f;
                 // Rows past the slice end compare as NaN: never candidates.
-                const float ax = rvalid ? (l2 ? xnv - err_row_const(xnv, l2, p.cN) : 0.0f) : __int_as_float(0x7fffffff);
+                const float nax =
+                    rvalid ? (l2 ? err_row_const(xnv, l2, p.cN) - xnv : 0.0f) : __int_as_float(0x7fffffff);
                 // This warp's occupied columns in one TMEM load (the first
                 // chunk alone when the rest are empty); the accumulator is
                 // released to the MMA warp right after it.
                 uint32_t u[CW];
                 const uint32_t taddr =
                     tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(buf * QG + half * CW);
-                if constexpr (CW > CC) {
-                    if (nact <= CC) {
-                        uint32_t u0[CC];
-                        tc::tmem_ld_cols<CC>(taddr, u0);
+                constexpr int C1 = CW < 32 ? CW : 32;
+                if constexpr (CW > C1) {
+                    if (nact <= C1) {
+                        uint32_t u0[C1];
+                        tc::tmem_ld_cols<C1>(taddr, u0);
 #pragma unroll
-                        for (int j = 0; j < CC; ++j) u[j] = u0[j];
+                        for (int j = 0; j < C1; ++j) u[j] = u0[j];
 #pragma unroll
-                        for (int j = CC; j < CW; ++j) u[j] = 0u;
+                        for (int j = C1; j < CW; ++j) u[j] = 0u;
                     } else {
                         tc::tmem_ld_cols<CW>(taddr, u);
                     }
@@ -1216,44 +1214,43 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                 for (int c = 0; c < CW / CC; ++c) {
                     const int col0 = half * CW + c * CC;
                     if (c * CC >= nact) continue;
-                    // The chunk's test bounds (and, for e4m3, the
-                    // accumulator scales) in registers.
-                    float r[CC], m[CC];
+                    // candidate test: cf ip + (|x|^2 - cx) <= R_q (see
+                    // err_coef), as one multiply-add per element and the
+                    // chunk's minimum (compares chained by their predicate
+                    // took 17 cycles per column); the per-column mask is
+                    // built only where some row of the warp has one.
+                    float v[CC];
 #pragma unroll
                     for (int j = 0; j < CC; j += 4) {
-                        const float4 t4 = *reinterpret_cast<const float4*>(R + c * CC + j);
-                        r[j] = t4.x;
-                        r[j + 1] = t4.y;
-                        r[j + 2] = t4.z;
-                        r[j + 3] = t4.w;
+                        const float4 t4 = *reinterpret_cast<const float4*>(S.nr + col0 + j);
+                        float m[4] = {cf, cf, cf, cf};
                         if constexpr (F8) {
                             const float4 m4 = *reinterpret_cast<const float4*>(S.sc + col0 + j);
-                            m[j] = cf * m4.x;
-                            m[j + 1] = cf * m4.y;
-                            m[j + 2] = cf * m4.z;
-                            m[j + 3] = cf * m4.w;
-                        } else {
-                            m[j] = m[j + 1] = m[j + 2] = m[j + 3] = cf;
+                            m[0] *= m4.x;
+                            m[1] *= m4.y;
+                            m[2] *= m4.z;
+                            m[3] *= m4.w;
                         }
+                        v[j] = fmaf(m[0], __uint_as_float(u[c * CC + j]), t4.x);
+                        v[j + 1] = fmaf(m[1], __uint_as_float(u[c * CC + j + 1]), t4.y);
+                        v[j + 2] = fmaf(m[2], __uint_as_float(u[c * CC + j + 2]), t4.z);
+                        v[j + 3] = fmaf(m[3], __uint_as_float(u[c * CC + j + 3]), t4.w);
                     }
-                    // candidate test: cf*ip + (|x|^2 - cx) <= R_q (see err_coef).
-                    // First only whether any row of the warp has one in the
-                    // chunk (two instructions per element); the per-column
-                    // mask is built for such chunks alone.
-                    bool hit = false;
+                    float mn[CC / 4];
 #pragma unroll
-                    for (int j = 0; j < CC; ++j) hit |= fmaf(m[j], __uint_as_float(u[c * CC + j]), ax) <= r[j];
-                    if (!__any_sync(FULL, hit)) continue;
+                    for (int j = 0; j < CC / 4; ++j)
+                        mn[j] = fminf(fminf(v[4 * j], v[4 * j + 1]), fminf(v[4 * j + 2], v[4 * j + 3]));
+#pragma unroll
+                    for (int j = 1; j < CC / 4; ++j) mn[0] = fminf(mn[0], mn[j]);
+                    if (!__any_sync(FULL, mn[0] <= nax)) continue;
                     uint32_t mask = 0;
 #pragma unroll
-                    for (int j = 0; j < CC; ++j)
-                        mask |= (fmaf(m[j], __uint_as_float(u[c * CC + j]), ax) <= r[j]) ? (1u << j) : 0u;
-                    const unsigned cols = __reduce_or_sync(FULL, mask);
-                    if (cols) {
-                        // Some rows of the warp have candidates in the chunk.
-                        // Their accumulators go to private shared-memory rows;
-                        // then, column by column (warp-uniform), the lanes with
-                        // a candidate there write it at their ballot rank.
+                    for (int j = 0; j < CC; ++j) mask |= v[j] <= nax ? (1u << j) : 0u;
+                    {
+                        // A row's accumulators go to its private shared-memory
+                        // row; then, a candidate of every lane that has one
+                        // left at a time, they are written at their ballot
+                        // rank.
                         float* sip = s_ip + (e * 32 + lane) * CC;
                         if (mask) {
 #pragma unroll
@@ -1262,12 +1259,12 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                                     make_float4(__uint_as_float(u[c * CC + j]), __uint_as_float(u[c * CC + j + 1]),
                                                 __uint_as_float(u[c * CC + j + 2]), __uint_as_float(u[c * CC + j + 3]));
                         }
-                        unsigned left = cols;
-                        while (left) {
-                            const int j = __ffs(left) - 1;
-                            left &= left - 1u;
-                            const bool mine = (mask >> j) & 1u;
+                        for (;;) {
+                            const bool mine = mask != 0u;
                             const unsigned bal = __ballot_sync(FULL, mine);
+                            if (!bal) break;
+                            const int j = __ffs(mask) - 1;
+                            mask &= mask - 1u;
                             const int cnt = __popc(bal);
                             const bool cross = (wc + cnt) / SEG != wc / SEG;  // warp-uniform
                             if (cross && npend == NSEG - 1) {
@@ -2842,32 +2839,47 @@ cudaError_t launch_invert_probes(const int64_t* probes, int nq, int nprobe, int 
     return cudaGetLastError();
 }
 
+// Whether groups of qg (64) take the WIDE shape at nkb k-blocks.
+static bool batched_wide(int nkb, int qg) { return qg == 64 && !batched_stages<64, false>(nkb); }
+
 int batched_group_size(int nkb) {
-    if (batched_stages<128>(nkb)) return 128;
-    if (batched_stages<64>(nkb)) return 64;
-    if (batched_stages<32>(nkb)) return 32;
+    if (nkb > NKB_MAX) return 0;
+    if (batched_stages<128, false>(nkb)) return 128;
+    if (batched_stages<64, false>(nkb) || batched_stages<64, true>(nkb)) return 64;
+    if (batched_stages<32, false>(nkb)) return 32;
     return 0;
 }
 
-template <int QG, Operand OP>
+int batched_row_slice(int nkb, int qg) {
+    return batched_wide(nkb, qg) ? Shape<64, true>::RS_MAX : Shape<64, false>::RS_MAX;
+}
+
+template <int QG, Operand OP, bool WIDE>
 static cudaError_t launch_batched_t(BatchedParams p, int nsm, cudaStream_t s) {
+    const int nkbq = p.nkb >> p.ksplit;  // a split image has two list k-blocks per query k-block
+    const int ks = stage_kblocks(p.nkb);
+    auto stages = [&](int nslot) {
+        for (int ns = NS_MAX; ns * ks >= RING_MIN; --ns)
+            if (batched_smem<QG, WIDE>(nkbq, ns * ks, nslot) <= BATCHED_SMEM_CAP) return ns;
+        return 0;
+    };
     p.nslot = SLOT_MAX;
-    p.ns = batched_stages<QG>(p.nkb >> p.ksplit, SLOT_MAX);
-    if (p.ns < NS_SLOT3) {
+    p.ns = stages(SLOT_MAX);
+    if (p.ns * ks < RING_SLOT3) {
         p.nslot = 2;
-        p.ns = batched_stages<QG>(p.nkb >> p.ksplit, 2);
+        p.ns = stages(2);
     }
-    if (p.ns == 0) return cudaErrorInvalidValue;
-    const size_t smem = batched_smem<QG>(p.nkb >> p.ksplit, p.ns, p.nslot);
-    cudaError_t e = cudaFuncSetAttribute(batched_scan_kernel<QG, OP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    if (p.ns == 0 || p.rs > Shape<QG, WIDE>::RS_MAX) return cudaErrorInvalidValue;
+    const size_t smem = batched_smem<QG, WIDE>(nkbq, p.ns * ks, p.nslot);
+    auto kern = batched_scan_kernel<QG, OP, WIDE>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    batched_scan_kernel<QG, OP><<<nsm, BATCH_THREADS, smem, s>>>(p);
+    kern<<<nsm, BATCH_THREADS, smem, s>>>(p);
     return cudaGetLastError();
 }
 
 cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int* err, cudaStream_t s) {
-    BatchedParams p;
+    BatchedParams p{};
     p.abf = static_cast<const unsigned char*>(b.abf);
     p.list_off = b.list_off;
     p.list_size = b.list_size;
@@ -2899,19 +2911,23 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
     err_consts(b.d, operand_k(b.op, p.nkb), &p.cK, &p.cN);
     cudaError_t e;
     if ((e = cudaMemsetAsync(w.work, 0, sizeof(unsigned int), s)) != cudaSuccess) return e;
-    auto run = [&](auto qg) -> cudaError_t {
+    auto run = [&](auto qg, auto wide) -> cudaError_t {
         constexpr int QG = decltype(qg)::value;
+        constexpr bool WIDE = decltype(wide)::value;
         switch (b.op) {
-            case Operand::bf16: return launch_batched_t<QG, Operand::bf16>(p, b.nsm, s);
-            case Operand::e4m3: return launch_batched_t<QG, Operand::e4m3>(p, b.nsm, s);
-            case Operand::tf32: return launch_batched_t<QG, Operand::tf32>(p, b.nsm, s);
+            case Operand::bf16: return launch_batched_t<QG, Operand::bf16, WIDE>(p, b.nsm, s);
+            case Operand::e4m3: return launch_batched_t<QG, Operand::e4m3, WIDE>(p, b.nsm, s);
+            case Operand::tf32: return launch_batched_t<QG, Operand::tf32, WIDE>(p, b.nsm, s);
         }
         return cudaErrorInvalidValue;
     };
+    constexpr std::false_type narrow;
     switch (b.qg) {
-        case 128: return run(std::integral_constant<int, 128>());
-        case 64: return run(std::integral_constant<int, 64>());
-        case 32: return run(std::integral_constant<int, 32>());
+        case 128: return run(std::integral_constant<int, 128>(), narrow);
+        case 64:
+            return batched_wide(b.nkb, 64) ? run(std::integral_constant<int, 64>(), std::true_type())
+                                           : run(std::integral_constant<int, 64>(), narrow);
+        case 32: return run(std::integral_constant<int, 32>(), narrow);
         default: return cudaErrorInvalidValue;
     }
 }

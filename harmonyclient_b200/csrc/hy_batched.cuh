@@ -37,6 +37,8 @@ inline int operand_k(Operand op, int nkb) { return nkb * (op == Operand::bf16 ? 
 // Queries per group of the batched kernel for rows of nkb k-blocks (128, 64 or
 // 32: the largest whose shared-memory footprint fits), 0 if none fits.
 int batched_group_size(int nkb);
+// Largest rows per work item of groups of qg at nkb k-blocks.
+int batched_row_slice(int nkb, int qg);
 
 cudaError_t launch_to_bf16_arena(const ArenaLayout& L, const float* codes, int64_t rows, void* out, cudaStream_t s);
 // e4m3 image with per-list scales: tile_max [rows/128] scratch, lscale

@@ -993,7 +993,8 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     auto slicing = [&](int rows, int* rs_out) {
         const int tiles = (rows + 127) / 128;
         int ns = std::min(tiles, std::max(1, (h->nsm + ngroups - 1) / ngroups));
-        ns = std::max(ns, (tiles + 15) / 16);
+        const int most = hy::batched_row_slice(nkb, qg) / 128;  // tiles per slice
+        ns = std::max(ns, (tiles + most - 1) / most);
         const int rs = (tiles + ns - 1) / ns * 128;
         *rs_out = rs;
         return (rows + rs - 1) / rs;
@@ -1153,9 +1154,6 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     // Item descriptors: an upper bound on the item count from host-known
     // sizes (groups <= pairs/128 + lists, slices per list <= the largest
     // list's), capped at 4M; items beyond the cap are decoded by search.
-    size_t max_slices = 1;
-    for (size_t l = 0; l < nlist; ++l)
-        max_slices = std::max(max_slices, ((size_t)h->h_list_size[l] + h->row_slice - 1) / h->row_slice);
     // Queries per group of each pass (hy_index_set_group_size): by default
     // the smallest of 64 / 128 holding four times the pass's expected
     // queries per list (measured on 1M x 128 at about 10 queries per list:
@@ -1173,6 +1171,12 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
         (learned_on(h) && h->learned_mean > 0) ? std::max(0.0, h->learned_mean - 1.0) : (double)(nprobe - 1);
     const int qg1 = pass_group((double)qc);
     const int qg2 = pass_group((double)qc * np_rest);
+    const size_t rs1 = std::min(h->row_slice, (size_t)hy::batched_row_slice((int)nkb, qg1));
+    const size_t rs2 = std::min(h->row_slice, (size_t)hy::batched_row_slice((int)nkb, qg2));
+    const size_t rs_min = std::min(rs1, rs2);
+    size_t max_slices = 1;
+    for (size_t l = 0; l < nlist; ++l)
+        max_slices = std::max(max_slices, ((size_t)h->h_list_size[l] + rs_min - 1) / rs_min);
     const size_t item_cap =
         std::min<size_t>((qc / qg1 + qc * nprobe / qg2 + 2 * nlist) * max_slices, size_t(4) << 20);
     HY_RET(h->b_items.ensure(item_cap * sizeof(int4)));
@@ -1260,7 +1264,7 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
         b.thr = h->b_thr.as<float>();
         b.nlist = (int)nlist;
         b.d = (int)h->d;
-        b.rs = (int)h->row_slice;
+        b.rs = (int)rs1;
         b.capq = (int)capq;
         b.metric = h->metric;
         b.nsm = h->nsm;
@@ -1270,7 +1274,7 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
         // bound; pass 2: the remaining probed lists under the tight threshold.
         const bool last = timed && q0 + qc >= n;
         HY_CUDA(hy::launch_invert_probes(h->w_probes.as<int64_t>(), (int)m, (int)nprobe, 0, 1, (int)nlist,
-                                         h->list_size.as<int32_t>(), (int)h->row_slice, qg1, w, s));
+                                         h->list_size.as<int32_t>(), (int)rs1, qg1, w, s));
         if (last) HY_CUDA(ev_record(h->ev[6], s));
         b.dense_max = dense_max;
         HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
@@ -1289,8 +1293,9 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
                                    h->metric, (int)h->d, K, h->nsm, h->b_thr.as<float>(), s, df));
         if (nprobe > 1) {
             HY_CUDA(hy::launch_invert_probes(h->w_probes.as<int64_t>(), (int)m, (int)nprobe, 1, (int)nprobe,
-                                             (int)nlist, h->list_size.as<int32_t>(), (int)h->row_slice, qg2, w, s));
+                                             (int)nlist, h->list_size.as<int32_t>(), (int)rs2, qg2, w, s));
             b.qg = qg2;
+            b.rs = (int)rs2;
             if (last) HY_CUDA(ev_record(h->ev[8], s));
             HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
             if (last) HY_CUDA(ev_record(h->ev[9], s));

@@ -307,14 +307,13 @@ __device__ inline float row_l2_global(const ArenaLayout& L, const float* __restr
                                       const float* qs, bool blockwise) {
     float total = 0.0f;
     const int lr = static_cast<int>(r & 31);
-    const float* tile = codes + static_cast<size_t>(r >> 5) * 32 * L.row_pitch;
     for (int b = 0; b < L.nb; ++b) {
-        const float* rowp = tile + static_cast<size_t>(L.boff[b]) * 32 + lr * 32;
+        const float* rowp = codes + arena_tile_offset(L, r >> 5, L.boff[b] >> 5) + lr * 32;
         const float* qb = qs + L.boff[b];
         const int w = L.bstart[b + 1] - L.bstart[b];
         float s = blockwise ? 0.0f : total;
         for (int c = 0; c * 4 < w; ++c) {
-            const int pc = (c >> 3) * 256 + ((c ^ lr) & 7);  // 16-byte chunk of the row's group
+            const int pc = (c >> 3) * 1024 + ((c ^ lr) & 7);  // 16-byte chunk within the row's groups
             const float4 x = __ldg(reinterpret_cast<const float4*>(rowp + pc * 4));
             const float4 y = *reinterpret_cast<const float4*>(qb + c * 4);
             const int j = c * 4;
@@ -335,15 +334,14 @@ __device__ inline float row_ip_global(const ArenaLayout& L, const float* __restr
                                       const float* qs) {
     float total = 0.0f;
     const int lr = static_cast<int>(r & 31);
-    const float* tile = codes + static_cast<size_t>(r >> 5) * 32 * L.row_pitch;
     for (int b = 0; b < L.nb; ++b) {
-        const float* rowp = tile + static_cast<size_t>(L.boff[b]) * 32 + lr * 32;
+        const float* rowp = codes + arena_tile_offset(L, r >> 5, L.boff[b] >> 5) + lr * 32;
         const float* qb = qs + L.boff[b];
         const int w = L.bstart[b + 1] - L.bstart[b];
         float s = 0.0f;
         for (int j = 0; j < w; ++j) {
             const int c = j >> 2;
-            const int pc = (c >> 3) * 256 + ((c ^ lr) & 7);  // 16-byte chunk of the row's group
+            const int pc = (c >> 3) * 1024 + ((c ^ lr) & 7);  // 16-byte chunk within the row's groups
             s = __fadd_rn(s, __fmul_rn(qb[j], __ldg(rowp + pc * 4 + (j & 3))));
         }
         total = b == 0 ? s : __fadd_rn(total, s);

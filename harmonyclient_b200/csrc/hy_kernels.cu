@@ -497,11 +497,12 @@ __global__ void __launch_bounds__(512, 1) scan_plain_kernel(const __grid_constan
     auto issue = [&](int s) {
         const int b = sblk[s];
         const uint32_t bytes = static_cast<uint32_t>(32 * L.pitch[b] * sizeof(float));
-        const float* src = p.codes + static_cast<size_t>(srow[s] >> 5) * 32 * L.row_pitch + static_cast<size_t>(L.boff[b]) * 32;
         if (lane == 0) {
             fence_proxy_async();
             mbar_expect_tx(&wbar[s], bytes);
-            bulk_g2s(wb + static_cast<size_t>(s) * slot_floats, src, bytes, &wbar[s]);
+            for (int g = 0; g < L.pitch[b] >> 5; ++g)
+                bulk_g2s(wb + static_cast<size_t>(s) * slot_floats + g * 1024,
+                         p.codes + arena_tile_offset(L, srow[s] >> 5, (L.boff[b] >> 5) + g), 4096, &wbar[s]);
         }
         ++loaded;
     };

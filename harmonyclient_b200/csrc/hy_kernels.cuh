@@ -8,17 +8,16 @@
 
 namespace hy {
 
-// Layout of the list arena (device).  Rows are grouped in tiles of 32; each
-// list starts on a tile boundary and its tail is padded with zero rows whose
-// id is -1.  Inside a tile, the dimensions are split into `nb` blocks; block b
-// of all 32 rows is one contiguous run of 32 * pitch[b] floats, so the rows'
-// block b is a single bulk copy and a tile whose rows are all pruned after
-// block b never loads blocks b+1...  A block is stored as pitch / 32 groups of
-// 32 floats (128 bytes) of the 32 rows, 4 KB each, row after row; within a
-// row's group, 16-byte chunk c is stored at chunk (c ^ row) & 7, which lets 32
-// lanes reading the same logical chunk of 32 rows hit 32 different
-// shared-memory banks.  That is the tensor cores' 128-byte-swizzled K-major
-// layout: a group of four consecutive tiles (128 rows) is a TF32 operand as it
+// Layout of the list arena (device).  Each list starts on a 128-row boundary
+// and its tail is padded with zero rows whose id is -1.  The dimensions are
+// split into `nb` blocks, block b padded to pitch[b] floats, a multiple of 32;
+// a row is thus row_pitch / 32 groups of 32 floats (128 bytes).  128 rows are
+// stored group by group: 16 KB of 128 bytes per row, row after row, with a
+// row's 16-byte chunk c at chunk (c ^ row) & 7.  So 32 rows' block b is pitch /
+// 32 runs of 4 KB, one bulk copy each, and a 32-row tile whose rows are all
+// pruned after block b never loads blocks b+1...; 32 lanes reading the same
+// logical chunk of 32 rows hit 32 different shared-memory banks; and a group of
+// 128 rows is a TF32 tensor-core operand (128-byte swizzle, K-major) as it
 // lies.
 struct ArenaLayout {
     int d = 0;
@@ -30,13 +29,16 @@ struct ArenaLayout {
     int max_pitch = 0;
 };
 
+// Float offset of 32 rows' (tile: arena row / 32) group g.
+__host__ __device__ inline size_t arena_tile_offset(const ArenaLayout& L, int64_t tile, int g) {
+    return static_cast<size_t>(tile >> 2) * 128 * L.row_pitch + static_cast<size_t>(g) * 4096 +
+           static_cast<size_t>(tile & 3) * 1024;
+}
+
 // Float offset of (arena row r, block b, dimension j within the block).
 __host__ __device__ inline size_t arena_offset(const ArenaLayout& L, int64_t r, int b, int j) {
-    const int64_t tile = r >> 5;
-    const int lr = static_cast<int>(r & 31);
-    const int c = j >> 2;
-    return static_cast<size_t>(tile) * 32 * L.row_pitch + static_cast<size_t>(L.boff[b]) * 32 +
-           static_cast<size_t>(c >> 3) * 1024 + static_cast<size_t>(lr) * 32 + ((c ^ lr) & 7) * 4 + (j & 3);
+    const int lr = static_cast<int>(r & 31), c = j >> 2;
+    return arena_tile_offset(L, r >> 5, (L.boff[b] >> 5) + (c >> 3)) + lr * 32 + ((c ^ lr) & 7) * 4 + (j & 3);
 }
 
 struct ScanParams {

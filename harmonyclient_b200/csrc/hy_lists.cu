@@ -389,14 +389,15 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
                 const int slot = static_cast<int>(iss % R);
                 const int b = it_b;
                 const uint32_t bytes = static_cast<uint32_t>(32 * L.pitch[b] * sizeof(float));
-                const float* src = p.codes + static_cast<size_t>((row0 >> 5) + it_tile) * 32 * L.row_pitch +
-                                   static_cast<size_t>(L.boff[b]) * 32;
                 if (lane == 0) {
                     s_tag_tile[warp][slot] = it_tile;
                     s_tag_b[warp][slot] = b;
                     fence_proxy_async();
                     mbar_expect_tx(&wbar[slot], bytes);
-                    bulk_g2s(wb + static_cast<size_t>(slot) * slot_floats, src, bytes, &wbar[slot]);
+                    for (int g = 0; g < L.pitch[b] >> 5; ++g)
+                        bulk_g2s(wb + static_cast<size_t>(slot) * slot_floats + g * 1024,
+                                 p.codes + arena_tile_offset(L, (row0 >> 5) + it_tile, (L.boff[b] >> 5) + g), 4096,
+                                 &wbar[slot]);
                 }
                 ++iss;
                 ++loaded;
