@@ -2385,7 +2385,7 @@ __device__ void rerank_warp_query(const ArenaLayout& L, const float* __restrict_
 }
 
 // One warp per query; a query with more than 256 candidates (or k > 256, or
-// an overflowed buffer) is listed in w.big for the CTA kernel.  (Capping the
+// an overflowed buffer) is listed in w.big3 for the CTA kernel.  (Capping the
 // register sorts at 256 keys keeps the kernel at 64 registers: four CTAs per
 // SM.)
 __global__ void __launch_bounds__(256) rerank_warp_kernel(const __grid_constant__ ArenaLayout L,
@@ -2409,7 +2409,7 @@ __global__ void __launch_bounds__(256) rerank_warp_kernel(const __grid_constant_
     // (A query whose norm is not a number below 1e37 has no bounds: the CTA
     // kernel reports it for the exact scan.)
     if (cnt > capq || n > 256 || k > 256 || !(qa.x < 1e37f)) {
-        if (lane == 0) w.big[1 + atomicAdd(&w.big[0], 1)] = qi;
+        if (lane == 0) w.big3[1 + atomicAdd(&w.big3[0], 1)] = qi;
         return;
     }
     const float* src = q + static_cast<size_t>(qi) * L.d;
@@ -2449,10 +2449,10 @@ __global__ void __launch_bounds__(256) rerank_kernel(ArenaLayout L, const float*
     __shared__ uint32_t sh[2];
     __shared__ int s_nsel, s_over;
     const bool l2 = metric == 1;
-    // Queries left by the warp re-rank (w.big: count, then ids), a CTA each.
-    const int nbig = w.big[0];
+    // Queries left by the warp re-rank (w.big3: count, then ids), a CTA each.
+    const int nbig = w.big3[0];
     for (int li = blockIdx.x; li < nbig; li += gridDim.x) {
-    const int qi = w.big[1 + li];
+    const int qi = w.big3[1 + li];
     __syncthreads();  // the previous query's shared state is no longer read
     const int cnt = w.cand_cnt[qi];
     const int n = min(cnt, capq);
@@ -2611,13 +2611,11 @@ cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qa
     df.dense_max = std::min(df.dense_max, capq);
     float cK, cN;
     err_consts(d, K, &cK, &cN);
-    cudaError_t e = cudaMemsetAsync(w.big, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(w.big2, 0, sizeof(int32_t), s)) != cudaSuccess) return e;
+    cudaError_t e;
     if (df.dense_max > 0) {
-        if ((e = cudaMemsetAsync(w.rest, 0, sizeof(int32_t), s)) != cudaSuccess) return e;
         tighten_dense_kernel<<<(nq + 7) / 8, 256, 0, s>>>(xn, xaux, qaux, nq, w, capq, k, metric, cK, cN, thr, df);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (df.max_list <= df.dense_max) return cudaSuccess;  // no thresholded first-pass list
     }
     tighten_warp_kernel<<<df.dense_max > 0 ? 2 * nsm : (nq + 7) / 8, 256, 0, s>>>(xn, xaux, qaux, nq, w, capq, k,
                                                                                   metric, cK, cN, thr, df);
@@ -2801,7 +2799,6 @@ cudaError_t launch_invert_probes(const int64_t* probes, int nq, int nprobe, int 
                                  const int32_t* list_size, int rs, int qg, const BatchWork& w, cudaStream_t s) {
     const int64_t n = static_cast<int64_t>(nq) * (j1 - j0);
     cudaError_t e;
-    if ((e = cudaMemsetAsync(w.pair_cnt, 0, nlist * sizeof(int32_t), s)) != cudaSuccess) return e;
     if (nlist <= INVERT_SMEM_LISTS && w.done) {
         // Up to about one CTA of 512 threads per SM (at least 1024 pairs each).
         const int64_t per = std::max<int64_t>(1024, (n + 147) / 148);
@@ -2909,8 +2906,6 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
     p.dense_max = std::min(b.dense_max, b.capq);
     p.xaux = b.xaux;
     err_consts(b.d, operand_k(b.op, p.nkb), &p.cK, &p.cN);
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(w.work, 0, sizeof(unsigned int), s)) != cudaSuccess) return e;
     auto run = [&](auto qg, auto wide) -> cudaError_t {
         constexpr int QG = decltype(qg)::value;
         constexpr bool WIDE = decltype(wide)::value;
@@ -2938,8 +2933,7 @@ cudaError_t launch_rerank(const ArenaLayout& L, const float* codes, const int64_
                           cudaStream_t s, const int32_t* qexact) {
     float cK, cN;
     err_consts(L.d, K, &cK, &cN);
-    cudaError_t e = cudaMemsetAsync(w.big, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
     const size_t wsmem = static_cast<size_t>(8) * (256 * sizeof(uint64_t) + L.row_pitch * sizeof(float));
     if ((e = cudaFuncSetAttribute(rerank_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(wsmem))) != cudaSuccess)

@@ -79,7 +79,10 @@ cudaError_t launch_row_aux_tf32(const ArenaLayout& L, const float* codes, int64_
                                 const int32_t* list_size, int nlist, const float* cent, float2* aux, float2* tile_aux,
                                 double* stat, cudaStream_t s);
 
-// Work buffers of one batched search.
+// Work buffers of one batched search.  The caller zeroes the counters: pair_cnt
+// before an inversion, work before a scan, cand_cnt and the counts at the head
+// of overflow, big, big2, big3 and rest before a search (one clear of one run
+// of memory: a clear of each took a launch, 13 in a search).
 struct BatchWork {
     int32_t* pair_cnt;   // [nlist]
     int32_t* pair_fill;  // [nlist]
@@ -93,8 +96,9 @@ struct BatchWork {
     uint64_t* cand;      // [nq*capq]
     int32_t* cand_cnt;   // [nq]
     int32_t* overflow;   // [1 + nq]: count, then query ids
-    int32_t* big;        // [1 + nq]: queries re-ranked by the CTA kernel (count, then ids)
+    int32_t* big;        // [1 + nq]: queries tightened by the second warp kernel (count, then ids)
     int32_t* big2;       // [1 + nq]: queries tightened by the CTA kernel (count, then ids)
+    int32_t* big3;       // [1 + nq]: queries re-ranked by the CTA kernel (count, then ids)
     int32_t* rest = nullptr;  // [1 + nq]: queries whose first-pass list was not dense (count, then ids)
     unsigned int* done = nullptr;  // [1], zero between launches: the inversion's ticket
 };
@@ -113,6 +117,7 @@ struct DenseFirst {
     const int32_t* list_size = nullptr;
     const int64_t* list_off = nullptr;
     int dense_max = 0;
+    int max_list = 1 << 30;  // the largest list
     const float2* tile_aux = nullptr;  // per arena tile {max |x~|, max |x - x~|}
     const float* tile_xn = nullptr;    // per arena tile, max |x|^2
 };

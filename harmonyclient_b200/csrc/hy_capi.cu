@@ -65,15 +65,15 @@ struct Status {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool owned = true;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     int ensure(size_t n) {
         if (n <= bytes) return HY_OK;
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
+        release();
+        owned = true;
         size_t want = std::max<size_t>(n, 256);
         cudaError_t e = cudaMalloc(&p, want);
         if (e != cudaSuccess) {
@@ -91,12 +91,18 @@ struct DevBuf {
             return fail(HY_ERR_CUDA, "cudaMemset of a new buffer failed");
         return rc;
     }
+    // A piece of another buffer (not freed here).
+    void alias(void* at, size_t n) {
+        p = at;
+        bytes = n;
+        owned = false;
+    }
     template <class T>
     T* as() const {
         return static_cast<T*>(p);
     }
     void release() {
-        if (p) cudaFree(p);
+        if (p && owned) cudaFree(p);
         p = nullptr;
         bytes = 0;
     }
@@ -123,12 +129,13 @@ ArenaLayout make_layout(int d, int nb) {
 
 }  // namespace
 
-// Device status of a host-pointer call, read back in one pinned block.
+// Device status of a call: one block on the device (w_err, w_counters, b_fbtot
+// and m_total point into it), read back in one copy.
 struct HostStatus {
     int err = 0;
     unsigned long long counters[4] = {0, 0, 0, 0};  // scan counters (block copies, blocks unpruned, block sums, sums unpruned)
+    unsigned long long fallback = 0;          // queries answered by the device fallback
     unsigned long long learned_total = 0;     // sum of the learned nprobes
-    unsigned long long fallback = 0;  // queries answered by the device fallback
 };
 
 struct hy_index {
@@ -151,8 +158,9 @@ struct hy_index {
 
     DevBuf cent, list_off, list_size, ids, codes, norms;
     // workspace
+    DevBuf w_status;  // HostStatus on the device: w_err, w_counters, b_fbtot, m_total
     DevBuf w_q, w_scores, w_probes, w_thr, w_gthr, w_parts, w_D, w_I, w_f, w_counters, w_err;
-    DevBuf w_second, w_hard;  // tensor-core assignment: second candidates, undecided rows (count, ids)
+    DevBuf w_undecided;  // tensor-core assignment: undecided rows (count, ids), second candidates
     DevBuf w_x, w_lab, w_dist, w_keys, w_keys2, w_vals, w_vals2, w_sort, w_start, w_sums, w_cnt, w_rows, w_xn;
 
     cudaStream_t stream = nullptr;
@@ -190,6 +198,7 @@ struct hy_index {
     int graph_kev = 0;
     cudaEvent_t gev[2] = {};
     bool times_pending = false;  // a device-API search recorded events not yet read
+    unsigned char* hout = nullptr;  // pinned results of small host-pointer calls
     HostStatus* hstat = nullptr;  // pinned status block of host-pointer calls (finish_host_call)
     int64_t* hjudge = nullptr;    // pinned results of the learned judge's rows
     size_t hjudge_cap = 0;
@@ -222,8 +231,8 @@ struct hy_index {
     DevBuf lscale, tscale, tmax;  // e4m3 per-list and per-tile scales, tile maxima
     bool a8_valid = false;
     DevBuf b_qs;              // e4m3 per-query scales
-    DevBuf b_big;             // queries re-ranked by the CTA kernel
-    DevBuf b_qb, b_qn, b_thr, b_pcnt, b_pfill, b_poff, b_pairs, b_icnt, b_ioff, b_work, b_cand, b_ccnt, b_ovf, b_items;
+    DevBuf b_qb, b_qn, b_thr, b_pfill, b_poff, b_pairs, b_icnt, b_ioff, b_cand, b_items;
+    DevBuf b_zero;            // the counters of a search, cleared together
     DevBuf b_done;            // the probe inversion's ticket (zero between launches)
     DevBuf b_fq, b_fpr, b_fD, b_fI, b_fcnt, b_fbtot;  // device-side exact fallback
     // coarse quantiser on the tensor cores (bf16 form): the centroids as a
@@ -235,8 +244,9 @@ struct hy_index {
     // its list's centroid and per 32-row tile {max, min} (built on first use).
     DevBuf c2c, c2c_tile;
     bool c2c_valid = false;
+    DevBuf c_all;  // pieces: the image, row and tile terms, norms, list offsets and size
     DevBuf c_img, c_aux, c_taux, c_norm, c_off, c_size;
-    DevBuf c_pcnt, c_poff, c_pairs, c_ioff, c_items, c_work, c_cand, c_ccnt;
+    DevBuf c_pcnt, c_poff, c_pairs, c_ioff, c_items, c_cand, c_ccnt;
 
     // learned probe predictor
     bool model_ready = false;
@@ -266,10 +276,16 @@ int set_device(hy_index* h) {
     return HY_OK;
 }
 
-// (query, probed list) pairs from which a plain batch runs on the tensor
-// cores, and the largest mean TF32 error of a row against its distance to its
-// centroid at which it does (plain_on_tensor, ensure_operands).
-constexpr size_t TF32_MIN_PAIRS = 16384;
+// FP32 bytes of (query, probed row) pairs from which a plain batch runs on the
+// tensor cores, and, where it cannot, from which the list-major scan serves
+// queries that share lists; below, the query-major scan's few launches win.
+// Measured (us, query-major / list-major / tensor): 1M x 128, nprobe 64: 512 MB
+// 187 / 344 / 283, 1 GB 412 / 383 / 289, 8 GB 1370 / 661 / 352; 200k x 200,
+// nprobe 16: 320 MB 249 / 456 / 253, 640 MB 352 / 525 / 265, 5 GB 1536 / 1241 /
+// 350; 10k x 128, nprobe 10: 524 MB 179 / 228 / 197.
+constexpr double TF32_MIN_BYTES = 600e6, LIST_MAJOR_MIN_BYTES = 1e9;
+// Largest mean TF32 error of a row against its distance to its centroid at
+// which a plain batch runs on the tensor cores (ensure_operands).
 constexpr double TF32_SPREAD_MAX = 0.03;
 
 // Rows x centroids x dimensions from which assignment runs on the tensor
@@ -297,12 +313,22 @@ float* centroid_maxima(const hy_index* h) {
 int ensure_centroid_image(hy_index* h, cudaStream_t s) {
     if (h->cimg_valid) return HY_OK;
     const size_t rows = (h->nlist + hy::BATCH_ROW_ALIGN - 1) / hy::BATCH_ROW_ALIGN * hy::BATCH_ROW_ALIGN;
-    HY_RET(h->c_img.ensure(hy::bf16_split_image_bytes((int64_t)rows, (int)h->d)));
-    HY_RET(h->c_aux.ensure(rows * sizeof(float2)));
-    HY_RET(h->c_taux.ensure(rows / hy::BATCH_ROW_ALIGN * sizeof(float2) + 4 * sizeof(float)));  // tiles, maxima
-    HY_RET(h->c_norm.ensure(rows * sizeof(float)));
-    HY_RET(h->c_off.ensure(2 * sizeof(int64_t)));
-    HY_RET(h->c_size.ensure(sizeof(int32_t)));
+    // One allocation in pieces.
+    const size_t bytes[6] = {hy::bf16_split_image_bytes((int64_t)rows, (int)h->d),
+                             rows * sizeof(float2),
+                             rows / hy::BATCH_ROW_ALIGN * sizeof(float2) + 4 * sizeof(float),  // tiles, maxima
+                             rows * sizeof(float),
+                             2 * sizeof(int64_t),
+                             sizeof(int32_t)};
+    DevBuf* const piece[6] = {&h->c_img, &h->c_aux, &h->c_taux, &h->c_norm, &h->c_off, &h->c_size};
+    size_t total = 0;
+    for (size_t b : bytes) total += (b + 255) & ~size_t(255);
+    HY_RET(h->c_all.ensure(total));
+    unsigned char* at = h->c_all.as<unsigned char>();
+    for (int i = 0; i < 6; ++i) {
+        piece[i]->alias(at, bytes[i]);
+        at += (bytes[i] + 255) & ~size_t(255);
+    }
     HY_CUDA(hy::launch_centroid_image(h->cent.as<float>(), (int)h->nlist, (int)h->d, h->c_img.p, h->c_aux.as<float2>(),
                                       h->c_taux.as<float2>(), h->c_norm.as<float>(), centroid_maxima(h), s));
     h->cimg_valid = true;
@@ -325,15 +351,14 @@ int assign_rows(hy_index* h, const float* x, size_t n, int64_t* labels, float* s
     if (assign_on_tensor(h, n)) {
         if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
         HY_RET(ensure_centroid_image(h, s));
-        HY_RET(h->w_second.ensure(n * sizeof(int32_t)));
-        HY_RET(h->w_hard.ensure((n + 1) * sizeof(int32_t)));
+        HY_RET(h->w_undecided.ensure((2 * n + 1) * sizeof(int32_t)));
         hy::AssignWork w;
         w.cimg = h->c_img.p;
         w.cxn = h->c_norm.as<float>();
         w.cmax = centroid_maxima(h);
-        w.second = h->w_second.as<int32_t>();
-        w.hard_count = h->w_hard.as<int32_t>();
-        w.hard = h->w_hard.as<int32_t>() + 1;
+        w.hard_count = h->w_undecided.as<int32_t>();
+        w.hard = w.hard_count + 1;
+        w.second = w.hard + n;
         w.err = h->w_err.as<int>();
         HY_CUDA(hy::launch_assign(x, (int)n, (int)h->d, (int)h->nlist, h->metric, w, h->nsm, labels, s));
         HY_CUDA(hy::launch_assign_exact(x, (int)n, (int)h->d, h->cent.as<float>(), h->metric, w, labels, score, s));
@@ -558,15 +583,23 @@ int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t npro
     const int kp = k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 256;
     if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
     const int pparts = hy::scan_probe_parts(h->L, (int)k, (int)nprobe);
-    // Tile splits: SCAN_WAVES work units per SM (one CTA fills an SM), so the
-    // last wave is short, but no more than leaves every warp of a unit a tile
-    // of an average probe list (16 warps).  A single wave for up to a few
-    // queries: their units are as even as the tiles.
-    constexpr size_t SCAN_WAVES = 4;
+    // Tile splits: the fewest rounds of the chip (one CTA fills an SM) by what
+    // a unit takes: its set-up and folds, and its tiles 32 at a time (16 warps
+    // of two slots), at the average list size.  100 queries of 35 tiles: whole
+    // 22 us, 5 splits 37; 33 queries of 417 tiles: 4 splits as 18, 68 us.
+    constexpr double UNIT_US = 6.0, ROUND_US = 4.0;
     const size_t nsm = (size_t)h->nsm;
     const size_t tiles = std::max<size_t>(1, h->arena_rows / 32 / std::max<size_t>(h->nlist, 1) * nprobe);
-    size_t tsplit = n * 4 <= nsm ? nsm / std::max<size_t>(n, 1) : (SCAN_WAVES * nsm + n - 1) / n;
-    tsplit = std::max<size_t>(1, std::min(tsplit, (tiles + 7) / 8));
+    size_t tsplit = 1;
+    double least = 1e30;
+    for (size_t t = 1; t <= nsm && t <= (tiles + 7) / 8; ++t) {
+        const double rounds = (double)((n * (size_t)pparts * t + nsm - 1) / nsm);
+        const double us = rounds * (UNIT_US + ROUND_US * std::max(1.0, (double)tiles / (double)(t * 32)));
+        if (us < least) {
+            least = us;
+            tsplit = t;
+        }
+    }
     const size_t all = n * (size_t)pparts;
     HY_RET(h->w_parts.ensure((nq_dev ? std::max(all, nsm) : all * tsplit) * kp * sizeof(uint64_t)));
     uint32_t* gthr = nullptr;
@@ -614,15 +647,36 @@ int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t npro
     return HY_OK;
 }
 
+// Places in a run of counters cleared together (32-bit words, 16-byte aligned).
+struct ZeroRun {
+    size_t words = 0;
+    size_t take(size_t n) {
+        const size_t at = words;
+        words += (n + 3) & ~size_t(3);
+        return at;
+    }
+};
+
 // Rows per work item of the list-major scan (32 tiles: four per warp).
 constexpr int LM_ROW_SLICE = 1024;
 
+// Inner product with OPT_TRIANGLE: the list-major scan's window.
+bool ip_window(const hy_index* h) { return h->metric == HY_METRIC_IP && (h->opt_level & 1); }
+
+// FP32 bytes of the (query, probed row) pairs of m queries at the mean list.
+double pair_bytes(const hy_index* h, size_t m, size_t nprobe) {
+    return (double)m * (double)nprobe * ((double)h->ntotal / (double)h->nlist) * (double)h->L.row_pitch * 4.0;
+}
+
 // Whether a plain search of m queries (per chunk) at nprobe runs the
-// list-major scan.
+// list-major scan when it does not run on the tensor cores: when its queries
+// share lists (four per list) and their pairs are worth its 17 launches (with
+// the inner-product window, whose answer off the unit sphere is the list-major
+// scan's own, always when they share lists).
 bool use_list_major(const hy_index* h, size_t m, size_t nprobe) {
     if (h->plain_scan == HY_PLAIN_QUERY_MAJOR || h->arena_rows == 0 || !hy::list_scan_fits(h->L)) return false;
     if (h->plain_scan == HY_PLAIN_LIST_MAJOR) return true;
-    return m * nprobe >= 4 * h->nlist;
+    return m * nprobe >= 4 * h->nlist && (ip_window(h) || pair_bytes(h, m, nprobe) >= LIST_MAJOR_MIN_BYTES);
 }
 
 // The list-major plain scan of m device queries whose probe lists (m x
@@ -638,17 +692,19 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
     const size_t nlist = h->nlist;
     const size_t capq = h->capq;
     const int rs = LM_ROW_SLICE;
-    HY_RET(h->b_pcnt.ensure(nlist * sizeof(int32_t)));
     HY_RET(h->b_pfill.ensure(nlist * sizeof(int32_t)));
     HY_RET(h->b_poff.ensure((nlist + 1) * sizeof(int64_t)));
     HY_RET(h->b_pairs.ensure(m * nprobe * sizeof(int32_t)));
     HY_RET(h->b_icnt.ensure(nlist * sizeof(int32_t)));
     HY_RET(h->b_ioff.ensure((nlist + 1) * sizeof(int64_t)));
-    HY_RET(h->b_work.ensure(sizeof(unsigned int)));
     HY_RET(h->b_done.ensure_zeroed(sizeof(unsigned int)));
     HY_RET(h->b_cand.ensure(m * capq * sizeof(uint64_t)));
-    HY_RET(h->b_ccnt.ensure(m * sizeof(int32_t)));
-    HY_RET(h->b_ovf.ensure((m + 1) * sizeof(int32_t)));
+    ZeroRun z;
+    const size_t z_work = z.take(2), z_pc1 = z.take(nlist), z_pc2 = z.take(nlist), z_cc = z.take(m),
+                 z_ovf = z.take(m + 1);
+    HY_RET(h->b_zero.ensure(z.words * sizeof(int32_t)));
+    int32_t* const zero = h->b_zero.as<int32_t>();
+    HY_CUDA(cudaMemsetAsync(zero, 0, z.words * sizeof(int32_t), s));
     size_t max_slices = 1;
     for (size_t l = 0; l < nlist; ++l)
         max_slices = std::max(max_slices, ((size_t)h->h_list_size[l] + rs - 1) / rs);
@@ -659,21 +715,18 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
     HY_RET(h->b_fD.ensure(m * k * sizeof(float)));
     HY_RET(h->b_fI.ensure(m * k * sizeof(int64_t)));
     HY_RET(h->b_fcnt.ensure(sizeof(int32_t)));
-    HY_RET(h->b_fbtot.ensure(sizeof(unsigned long long)));
     hy::BatchWork w{};
     w.items = h->b_items.as<int4>();
     w.item_cap = (int64_t)item_cap;
-    w.pair_cnt = h->b_pcnt.as<int32_t>();
+    w.pair_cnt = zero + z_pc1;
     w.pair_fill = h->b_pfill.as<int32_t>();
     w.pair_off = h->b_poff.as<int64_t>();
     w.pairs = h->b_pairs.as<int32_t>();
     w.item_cnt = h->b_icnt.as<int32_t>();
     w.item_off = h->b_ioff.as<int64_t>();
-    w.work = h->b_work.as<unsigned int>();
+    w.work = reinterpret_cast<unsigned int*>(zero + z_work);
     w.done = h->b_done.as<unsigned int>();
-    int32_t* ovf = h->b_ovf.as<int32_t>();
-    HY_CUDA(cudaMemsetAsync(h->b_ccnt.p, 0, m * sizeof(int32_t), s));
-    HY_CUDA(cudaMemsetAsync(ovf, 0, sizeof(int32_t), s));
+    int32_t* ovf = zero + z_ovf;
     hy::ListScanParams p;
     p.L = h->L;
     p.codes = h->codes.as<float>();
@@ -688,7 +741,7 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
     p.pair_cnt = w.pair_cnt;
     p.thr = thr;
     p.cand = h->b_cand.as<uint64_t>();
-    p.cand_cnt = h->b_ccnt.as<int32_t>();
+    p.cand_cnt = zero + z_cc;
     p.work = w.work;
     p.counters = h->w_counters.as<unsigned long long>();
     p.err = h->w_err.as<int>();
@@ -723,24 +776,26 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
     // Pass 1: each query's nearest list.
     HY_CUDA(hy::launch_invert_probes(probes, (int)m, (int)nprobe, 0, 1, (int)nlist, h->list_size.as<int32_t>(), rs,
                                      hy::LM_GROUP, w, s));
-    HY_CUDA(cudaMemsetAsync(w.work, 0, sizeof(unsigned int), s));
     if (timed) HY_CUDA(ev_record(h->ev[6], s));
     HY_CUDA(hy::launch_list_scan(p, h->nsm, s));
     if (timed) HY_CUDA(ev_record(h->ev[7], s));
     if (timed) h->kev = 1;
     HY_CUDA(hy::launch_list_topk(p.cand, p.cand_cnt, (int)m, (int)capq, (int)k, h->metric, 0, thr, nullptr, nullptr,
                                  nullptr, nullptr, s));
-    h->launches += 8;
+    h->launches += 5;
     if (nprobe > 1) {
         // Pass 2: the other probed lists under the lowered thresholds.
+        w.pair_cnt = zero + z_pc2;
+        w.work = w.work + 1;
+        p.pair_cnt = w.pair_cnt;
+        p.work = w.work;
         HY_CUDA(hy::launch_invert_probes(probes, (int)m, (int)nprobe, 1, (int)nprobe, (int)nlist,
                                          h->list_size.as<int32_t>(), rs, hy::LM_GROUP, w, s));
-        HY_CUDA(cudaMemsetAsync(w.work, 0, sizeof(unsigned int), s));
         if (timed) HY_CUDA(ev_record(h->ev[8], s));
         HY_CUDA(hy::launch_list_scan(p, h->nsm, s));
         if (timed) HY_CUDA(ev_record(h->ev[9], s));
         if (timed) h->kev = 2;
-        h->launches += 7;
+        h->launches += 3;
     }
     if (timed) HY_CUDA(ev_record(h->ev[3], s));
     HY_CUDA(hy::launch_list_topk(p.cand, p.cand_cnt, (int)m, (int)capq, (int)k, h->metric, 1, thr,
@@ -760,14 +815,26 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
 }
 
 int ensure_common(hy_index* h) {
-    HY_RET(h->w_counters.ensure(4 * sizeof(unsigned long long)));
-    HY_RET(h->w_err.ensure(sizeof(int)));
+    if (h->w_status.p) return HY_OK;
+    HY_RET(h->w_status.ensure(sizeof(HostStatus)));
+    HY_CUDA(cudaMemset(h->w_status.p, 0, sizeof(HostStatus)));
+    unsigned char* b = h->w_status.as<unsigned char>();
+    h->w_err.alias(b + offsetof(HostStatus, err), sizeof(int));
+    h->w_counters.alias(b + offsetof(HostStatus, counters), sizeof(HostStatus::counters));
+    h->b_fbtot.alias(b + offsetof(HostStatus, fallback), sizeof(HostStatus::fallback));
+    h->m_total.alias(b + offsetof(HostStatus, learned_total), sizeof(HostStatus::learned_total));
     return HY_OK;
 }
 
 int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, size_t k, float* dD, int64_t* dI,
                        cudaStream_t s, bool timed);
 bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s);
+
+// The scan counters and the fallback count (which follow one another) to zero.
+int clear_counters(hy_index* h, cudaStream_t s) {
+    HY_CUDA(cudaMemsetAsync(h->w_counters.p, 0, sizeof(HostStatus::counters) + sizeof(HostStatus::fallback), s));
+    return HY_OK;
+}
 
 bool learned_on(const hy_index* h) { return h->learned && h->model_ready; }
 bool batched_form(const hy_index* h) { return h->form == HY_FORM_BF16 || h->form == HY_FORM_FP8; }
@@ -794,7 +861,7 @@ int apply_learned_probes(hy_index* h, size_t m, size_t nprobe, cudaStream_t s, i
 int search_device_impl(hy_index* h, size_t n, const float* dq, size_t k, float* dD, int64_t* dI, cudaStream_t s,
                        bool timed) {
     HY_RET(ensure_common(h));
-    HY_CUDA(cudaMemsetAsync(h->w_counters.p, 0, 4 * sizeof(unsigned long long), s));
+    HY_RET(clear_counters(h, s));
     h->fb_last = false;
     h->stats.list_major = 0;
     if (batched_form(h) && h->arena_rows > 0)
@@ -818,10 +885,6 @@ int search_device_impl(hy_index* h, size_t n, const float* dq, size_t k, float* 
     if (learned_on(h)) HY_RET(h->m_pscore.ensure(qc * nprobe * sizeof(float)));
     const bool warm = h->warmup_list > 0 && h->metric == HY_METRIC_L2;
     if (warm || lm) HY_RET(h->w_thr.ensure(qc * sizeof(uint32_t)));
-    if (lm) {
-        HY_RET(h->b_fbtot.ensure(sizeof(unsigned long long)));
-        HY_CUDA(cudaMemsetAsync(h->b_fbtot.p, 0, sizeof(unsigned long long), s));
-    }
     for (size_t q0 = 0; q0 < n; q0 += qc) {
         const size_t m = std::min(qc, n - q0);
         h->stats.chunk_queries = m;  // the last chunk's count remains
@@ -948,17 +1011,15 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
     return HY_OK;
 }
 
-// Whether a plain search of m queries (per chunk) at nprobe that would run the
-// list-major scan runs on the tensor cores instead (the FP32 arena as TF32
-// operands, exact FP32 re-rank: the same answer).  From TF32_MIN_PAIRS (query,
-// probed list) pairs: below, its 20 launches cost more than the scan.  Not
-// with the inner-product window of OPT_TRIANGLE, whose answer off the unit
-// sphere depends on the scan's own thresholds.  The bound terms are built on
-// first use; while the stream is being captured, or without the memory for
-// them, the list-major scan runs.
+// Whether a plain search of m queries (per chunk) at nprobe runs on the tensor
+// cores (the FP32 arena as TF32 operands, exact FP32 re-rank: the other scans'
+// answer): from TF32_MIN_BYTES of pairs.  Not with the inner-product window of
+// OPT_TRIANGLE, whose answer off the unit sphere depends on the scan's own
+// thresholds.  The bound terms are built on first use; while the stream is
+// being captured, or without the memory for them, the other scans run.
 bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s) {
-    if (h->form != HY_FORM_PLAIN || h->plain_scan != HY_PLAIN_AUTO || !use_list_major(h, m, nprobe)) return false;
-    if (m * nprobe < TF32_MIN_PAIRS || (h->metric == HY_METRIC_IP && (h->opt_level & 1))) return false;
+    if (h->form != HY_FORM_PLAIN || h->plain_scan != HY_PLAIN_AUTO || h->arena_rows == 0 || ip_window(h)) return false;
+    if (pair_bytes(h, m, nprobe) < TF32_MIN_BYTES) return false;
     if (hy::batched_group_size(hy::operand_kblocks(hy::Operand::tf32, h->L)) == 0) return false;
     if (!h->a32_valid) {
         cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -980,9 +1041,10 @@ bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
 
 // Coarse step on the tensor cores for m queries whose bf16 image and
 // {|q|^2, |q|, |q~|, |q - q~|} are in qb / qn: one dense batched launch
-// over the centroid index, then the exact m best per query.
+// over the centroid index, then the exact m best per query.  work: two
+// counters at zero.
 int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const float4* qn, size_t nprobe,
-                  int64_t* probes, float* pscore, cudaStream_t s) {
+                  int64_t* probes, float* pscore, unsigned int* work, cudaStream_t s) {
     HY_RET(ensure_centroid_image(h, s));
     const int nlist = (int)h->nlist;
     const int nkb = (int)(h->d + 63) / 64;
@@ -1006,7 +1068,6 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     HY_RET(h->c_pairs.ensure(m * sizeof(int32_t)));
     HY_RET(h->c_ioff.ensure(2 * sizeof(int64_t)));
     HY_RET(h->c_items.ensure((size_t)ngroups * ns_full * sizeof(int4)));
-    HY_RET(h->c_work.ensure(sizeof(unsigned int)));
     HY_RET(h->c_cand.ensure(m * nlist * sizeof(float2)));
     HY_RET(h->c_ccnt.ensure(m * sizeof(int32_t)));
     hy::BatchWork w{};
@@ -1015,7 +1076,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     w.pair_off = h->c_poff.as<int64_t>();
     w.pairs = h->c_pairs.as<int32_t>();
     w.item_off = h->c_ioff.as<int64_t>();
-    w.work = h->c_work.as<unsigned int>();
+    w.work = work;
     w.cand = h->c_cand.as<uint64_t>();
     w.cand_cnt = h->c_ccnt.as<int32_t>();
     hy::BatchedLaunch b;
@@ -1071,6 +1132,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     HY_CUDA(hy::launch_coarse_items((int)m, nlist, ngroups, ns_full, h->c_off.as<int64_t>(), h->c_size.as<int32_t>(),
                                     w, s));
     HY_CUDA(cudaMemsetAsync(w.cand_cnt, 0, m * sizeof(int32_t), s));
+    w.work = work + 1;
     b.rs = rs_full;
     b.capq = nlist;
     b.dense_max = 0;
@@ -1078,7 +1140,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     HY_CUDA(hy::launch_coarse_refine_keys(h->c_cand.as<uint64_t>(), w.cand_cnt, (int)m, nlist, qq, h->cent.as<float>(),
                                           h->c_norm.as<float>(), h->c_aux.as<float2>(), qn,
                                           (int)h->d, h->metric, (int)nprobe, probes, pscore, h->w_err.as<int>(), s));
-    h->launches += 6;
+    h->launches += 7;
     return HY_OK;
 }
 
@@ -1119,18 +1181,20 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     if (f8) HY_RET(h->b_qs.ensure(qc * sizeof(float)));
     HY_RET(h->b_qn.ensure(qc * sizeof(float4)));
     HY_RET(h->b_qx.ensure(qc * sizeof(int32_t)));
-    HY_RET(h->b_pcnt.ensure(nlist * sizeof(int32_t)));
     HY_RET(h->b_pfill.ensure(nlist * sizeof(int32_t)));
     HY_RET(h->b_poff.ensure((nlist + 1) * sizeof(int64_t)));
     HY_RET(h->b_pairs.ensure(qc * nprobe * sizeof(int32_t)));
     HY_RET(h->b_icnt.ensure(nlist * sizeof(int32_t)));
     HY_RET(h->b_ioff.ensure((nlist + 1) * sizeof(int64_t)));
-    HY_RET(h->b_work.ensure(sizeof(unsigned int)));
     HY_RET(h->b_done.ensure_zeroed(sizeof(unsigned int)));
     HY_RET(h->b_cand.ensure(qc * capq * sizeof(uint64_t)));
-    HY_RET(h->b_ccnt.ensure(qc * sizeof(int32_t)));
-    HY_RET(h->b_ovf.ensure((qc + 1) * sizeof(int32_t)));
-    HY_RET(h->b_big.ensure(3 * (qc + 1) * sizeof(int32_t)));
+    ZeroRun z;
+    const size_t z_work = z.take(4), z_pc1 = z.take(nlist), z_pc2 = z.take(nlist), z_cc = z.take(qc),
+                 z_ovf = z.take(qc + 1), z_big = z.take(qc + 1), z_big2 = z.take(qc + 1), z_big3 = z.take(qc + 1),
+                 z_rest = z.take(qc + 1);
+    HY_RET(h->b_zero.ensure(z.words * sizeof(int32_t)));
+    int32_t* const zero = h->b_zero.as<int32_t>();
+    unsigned int* const work = reinterpret_cast<unsigned int*>(zero + z_work);
     // Exact fallback on the device: every overflowed query of a chunk is
     // searched again by the plain scan over the same probe lists.
     const size_t fbcap = qc;
@@ -1140,8 +1204,6 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     HY_RET(h->b_fD.ensure(fbcap * k * sizeof(float)));
     HY_RET(h->b_fI.ensure(fbcap * k * sizeof(int64_t)));
     HY_RET(h->b_fcnt.ensure(sizeof(int32_t)));
-    HY_RET(h->b_fbtot.ensure(sizeof(unsigned long long)));
-    HY_CUDA(cudaMemsetAsync(h->b_fbtot.p, 0, sizeof(unsigned long long), s));
     // Warm-up for the bf16 form: its threshold only bounds the first pass
     // (each query's nearest list), so three lists suffice by default.  A
     // query whose nearest list has between k and dense_max rows needs none:
@@ -1174,34 +1236,37 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     const size_t rs1 = std::min(h->row_slice, (size_t)hy::batched_row_slice((int)nkb, qg1));
     const size_t rs2 = std::min(h->row_slice, (size_t)hy::batched_row_slice((int)nkb, qg2));
     const size_t rs_min = std::min(rs1, rs2);
-    size_t max_slices = 1;
-    for (size_t l = 0; l < nlist; ++l)
-        max_slices = std::max(max_slices, ((size_t)h->h_list_size[l] + rs_min - 1) / rs_min);
+    int max_list = 0;
+    for (size_t l = 0; l < nlist; ++l) max_list = std::max(max_list, h->h_list_size[l]);
+    const size_t max_slices = std::max<size_t>(1, ((size_t)max_list + rs_min - 1) / rs_min);
     const size_t item_cap =
         std::min<size_t>((qc / qg1 + qc * nprobe / qg2 + 2 * nlist) * max_slices, size_t(4) << 20);
     HY_RET(h->b_items.ensure(item_cap * sizeof(int4)));
     hy::BatchWork w;
     w.items = h->b_items.as<int4>();
     w.item_cap = (int64_t)item_cap;
-    w.pair_cnt = h->b_pcnt.as<int32_t>();
+    w.pair_cnt = zero + z_pc1;
     w.pair_fill = h->b_pfill.as<int32_t>();
     w.pair_off = h->b_poff.as<int64_t>();
     w.pairs = h->b_pairs.as<int32_t>();
     w.item_cnt = h->b_icnt.as<int32_t>();
     w.item_off = h->b_ioff.as<int64_t>();
-    w.work = h->b_work.as<unsigned int>();
+    w.work = work;
     w.done = h->b_done.as<unsigned int>();
     w.cand = h->b_cand.as<uint64_t>();
-    w.cand_cnt = h->b_ccnt.as<int32_t>();
-    w.big = h->b_big.as<int32_t>();
-    w.big2 = w.big + (qc + 1);
-    w.rest = w.big2 + (qc + 1);
+    w.cand_cnt = zero + z_cc;
+    w.overflow = zero + z_ovf;  // [0] = count, then chunk-local query ids
+    w.big = zero + z_big;
+    w.big2 = zero + z_big2;
+    w.big3 = zero + z_big3;
+    w.rest = zero + z_rest;
     for (size_t q0 = 0; q0 < n; q0 += qc) {
         const size_t m = std::min(qc, n - q0);
         h->stats.chunk_queries = m;  // the last chunk's count remains
         const float* qq = dq + q0 * h->d;
-        w.overflow = h->b_ovf.as<int32_t>();  // [0] = count, then chunk-local query ids
-        HY_CUDA(cudaMemsetAsync(w.overflow, 0, sizeof(int32_t), s));
+        HY_CUDA(cudaMemsetAsync(zero, 0, z.words * sizeof(int32_t), s));
+        w.pair_cnt = zero + z_pc1;
+        w.work = work;
         if (timed && q0 == 0) HY_CUDA(ev_record(h->ev[0], s));
         if (tf32)
             HY_CUDA(hy::launch_prep_queries_tf32(qq, (int)m, h->L, h->b_qb.as<float>(), h->b_qn.as<float4>(),
@@ -1220,7 +1285,7 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
                 h->launches += 1;
             }
             HY_RET(coarse_tensor(h, m, qq, cqb, cqn, nprobe, h->w_probes.as<int64_t>(),
-                                 learned_on(h) ? h->m_pscore.as<float>() : nullptr, s));
+                                 learned_on(h) ? h->m_pscore.as<float>() : nullptr, work + 2, s));
         } else {
             HY_CUDA(hy::launch_coarse_scores(qq, (int)m, h->cent.as<float>(), (int)nlist, (int)h->d, h->metric,
                                              h->w_scores.as<float>(), s));
@@ -1245,7 +1310,6 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
             HY_CUDA(hy::launch_fill_f32(h->b_thr.as<float>(), (int64_t)m, INFINITY, s));
         }
         if (timed && q0 == 0) HY_CUDA(ev_record(h->ev[1], s));
-        HY_CUDA(cudaMemsetAsync(w.cand_cnt, 0, m * sizeof(int32_t), s));
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[2], s));
         hy::BatchedLaunch b;
         b.abf = f8 ? h->a8.p : tf32 ? h->codes.p : h->abf.p;
@@ -1287,11 +1351,14 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
         df.list_size = h->list_size.as<int32_t>();
         df.list_off = h->list_off.as<int64_t>();
         df.dense_max = dense_max;
+        df.max_list = max_list;
         df.tile_aux = taux;
         df.tile_xn = h->txn.as<float>();
         HY_CUDA(hy::launch_tighten(h->norms.as<float>(), xaux, h->b_qn.as<float4>(), (int)m, w, (int)capq, (int)k,
                                    h->metric, (int)h->d, K, h->nsm, h->b_thr.as<float>(), s, df));
         if (nprobe > 1) {
+            w.pair_cnt = zero + z_pc2;
+            w.work = work + 1;
             HY_CUDA(hy::launch_invert_probes(h->w_probes.as<int64_t>(), (int)m, (int)nprobe, 1, (int)nprobe,
                                              (int)nlist, h->list_size.as<int32_t>(), (int)rs2, qg2, w, s));
             b.qg = qg2;
@@ -1315,8 +1382,9 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
                               h->b_fD.as<float>(), h->b_fI.as<int64_t>(), s, false, nullptr, h->b_fcnt.as<int32_t>()));
         HY_CUDA(hy::launch_fb_scatter(w.overflow, h->b_fD.as<float>(), h->b_fI.as<int64_t>(), (int)k, fb, dD + q0 * k,
                                       dI + q0 * k, h->b_fbtot.as<unsigned long long>(), s));
-        h->launches += 3;
-        h->launches += nprobe > 1 ? 24 : 18;
+        // Clear, query preparation, warm-up, inversion, scan, tightening,
+        // re-rank, fallback.
+        h->launches += (nprobe > 1 ? 13 : 10) + (max_list > dense_max ? 3 : 0);
     }
     return HY_OK;
 }
@@ -1354,11 +1422,7 @@ int finish_host_call(hy_index* h, cudaStream_t s, bool timed, size_t n, size_t n
     if (!h->hstat) HY_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->hstat), sizeof(HostStatus), cudaHostAllocDefault));
     HostStatus* st = h->hstat;
     *st = HostStatus{};
-    HY_CUDA(cudaMemcpyAsync(&st->err, h->w_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    HY_CUDA(cudaMemcpyAsync(st->counters, h->w_counters.p, sizeof(st->counters), cudaMemcpyDeviceToHost, s));
-    if (h->m_total.p)
-        HY_CUDA(cudaMemcpyAsync(&st->learned_total, h->m_total.p, sizeof(st->learned_total), cudaMemcpyDeviceToHost, s));
-    if (h->b_fbtot.p) HY_CUDA(cudaMemcpyAsync(&st->fallback, h->b_fbtot.p, sizeof(st->fallback), cudaMemcpyDeviceToHost, s));
+    HY_CUDA(cudaMemcpyAsync(st, h->w_status.p, sizeof(HostStatus), cudaMemcpyDeviceToHost, s));
     HY_CUDA(cudaStreamSynchronize(s));
     if (st->err != 0) {
         const int err = st->err;
@@ -1381,10 +1445,8 @@ int finish_host_call(hy_index* h, cudaStream_t s, bool timed, size_t n, size_t n
 int reset_counters(hy_index* h, cudaStream_t s) {
     HY_RET(ensure_common(h));
     h->launches = 0;
-    HY_RET(h->m_total.ensure(sizeof(unsigned long long)));
-    HY_CUDA(cudaMemsetAsync(h->m_total.p, 0, sizeof(unsigned long long), s));
-    HY_CUDA(cudaMemsetAsync(h->w_counters.p, 0, 4 * sizeof(unsigned long long), s));
-    return HY_OK;
+    if (learned_on(h)) HY_CUDA(cudaMemsetAsync(h->m_total.p, 0, sizeof(unsigned long long), s));
+    return HY_OK;  // the search clears its own counters
 }
 
 void drop_graph(hy_index* h) {
@@ -1535,6 +1597,7 @@ int hy_index_destroy(hy_index* h) {
         if (ev) cudaEventDestroy(ev);
     if (h->hstat) cudaFreeHost(h->hstat);
     if (h->hjudge) cudaFreeHost(h->hjudge);
+    if (h->hout) cudaFreeHost(h->hout);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return HY_OK;
@@ -1816,6 +1879,9 @@ int hy_index_set_graph(hy_index* h, int enabled) {
 
 namespace {
 
+// Results up to this size come back through pinned memory.
+constexpr size_t SMALL_OUT = size_t(256) << 10;
+
 // The host-pointer search of one batch: upload, device search, download,
 // bf16 overflow fallback, statistics.
 int search_host(hy_index* h, size_t n, const float* q, size_t k, float* D, int64_t* I,
@@ -1828,8 +1894,15 @@ int search_host(hy_index* h, size_t n, const float* q, size_t k, float* D, int64
     const size_t m = judge_rows ? judge_rows->size() : 0;
     const size_t nt = n + m;
     HY_RET(h->w_q.ensure(nt * h->d * sizeof(float)));
-    HY_RET(h->w_D.ensure(nt * k * sizeof(float)));
-    HY_RET(h->w_I.ensure(nt * k * sizeof(int64_t)));
+    // Distances and, after them, ids: a small result comes back in one copy
+    // through pinned memory (each copy to pageable memory is a wait of its own).
+    const size_t i_off = (nt * k * sizeof(float) + 15) & ~size_t(15);
+    const size_t out_bytes = i_off + nt * k * sizeof(int64_t);
+    const bool small = out_bytes <= SMALL_OUT;
+    HY_RET(h->w_D.ensure(out_bytes));
+    int64_t* const outI = reinterpret_cast<int64_t*>(h->w_D.as<unsigned char>() + i_off);
+    if (small && !h->hout)
+        HY_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->hout), SMALL_OUT, cudaHostAllocDefault));
     HY_RET(reset_counters(h, s));
     const size_t d = h->d;
     HY_CUDA(cudaMemcpyAsync(h->w_q.p, q, n * d * sizeof(float), cudaMemcpyHostToDevice, s));
@@ -1843,17 +1916,27 @@ int search_host(hy_index* h, size_t n, const float* q, size_t k, float* D, int64
     // Graph mode replays the captured search (the workspace pointers and
     // the stream are the handle's own, so repeated calls of one shape match).
     const int rc = h->graph_on
-                       ? run_device_search(h, nt, h->w_q.as<float>(), k, h->w_D.as<float>(), h->w_I.as<int64_t>(), s)
-                       : search_device_impl(h, nt, h->w_q.as<float>(), k, h->w_D.as<float>(), h->w_I.as<int64_t>(), s,
+                       ? run_device_search(h, nt, h->w_q.as<float>(), k, h->w_D.as<float>(), outI, s)
+                       : search_device_impl(h, nt, h->w_q.as<float>(), k, h->w_D.as<float>(), outI, s,
                                             true);
     h->learned_rows = SIZE_MAX;
     HY_RET(rc);
     // The results go back before the status checks (one synchronisation for
     // both); a batch searched again below is copied again.
-    HY_CUDA(cudaMemcpyAsync(D, h->w_D.p, n * k * sizeof(float), cudaMemcpyDeviceToHost, s));
-    HY_CUDA(cudaMemcpyAsync(I, h->w_I.p, n * k * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    if (m) HY_CUDA(cudaMemcpyAsync(jI, h->w_I.as<int64_t>() + n * k, m * k * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    if (small) {
+        HY_CUDA(cudaMemcpyAsync(h->hout, h->w_D.p, out_bytes, cudaMemcpyDeviceToHost, s));
+    } else {
+        HY_CUDA(cudaMemcpyAsync(D, h->w_D.p, n * k * sizeof(float), cudaMemcpyDeviceToHost, s));
+        HY_CUDA(cudaMemcpyAsync(I, outI, n * k * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        if (m) HY_CUDA(cudaMemcpyAsync(jI, outI + n * k, m * k * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    }
     HY_RET(finish_host_call(h, s, true, nt, std::min(h->nprobe, h->nlist)));
+    if (small) {
+        const int64_t* hI = reinterpret_cast<const int64_t*>(h->hout + i_off);
+        std::memcpy(D, h->hout, n * k * sizeof(float));
+        std::memcpy(I, hI, n * k * sizeof(int64_t));
+        if (m) std::memcpy(jI, hI + n * k, m * k * sizeof(int64_t));
+    }
     h->stats.nq = n;
     h->stats.fallback_queries = 0;
     h->stats.mean_nprobe = (double)std::min(h->nprobe, h->nlist);
@@ -2220,6 +2303,7 @@ int hy_index_search_preassigned(hy_index* h, size_t n, const float* q, size_t k,
     HY_RET(h->w_D.ensure(n * k * sizeof(float)));
     HY_RET(h->w_I.ensure(n * k * sizeof(int64_t)));
     HY_RET(reset_counters(h, s));
+    HY_RET(clear_counters(h, s));
     HY_CUDA(cudaMemcpyAsync(h->w_q.p, q, n * h->d * sizeof(float), cudaMemcpyHostToDevice, s));
     HY_CUDA(cudaMemcpyAsync(h->w_probes.p, probes, n * nprobe * sizeof(int64_t), cudaMemcpyHostToDevice, s));
     const uint32_t* thr = nullptr;
@@ -2269,15 +2353,17 @@ int hy_index_probes(hy_index* h, size_t n, const float* q, int64_t* probes) {
         HY_RET(h->b_qb.ensure(qc * ((h->d + 63) / 64) * 128));
         HY_RET(h->b_qn.ensure(qc * sizeof(float4)));
         HY_RET(h->b_thr.ensure(qc * sizeof(float)));
+        HY_RET(h->b_zero.ensure(2 * sizeof(unsigned int)));
     }
     for (size_t q0 = 0; q0 < n; q0 += qc) {
         const size_t m = std::min(qc, n - q0);
         const float* qq = h->w_q.as<float>() + q0 * h->d;
         if (tensor) {
             HY_CUDA(hy::launch_prep_queries(qq, (int)m, (int)h->d, h->b_qb.p, h->b_qn.as<float4>(), nullptr, s));
+            HY_CUDA(cudaMemsetAsync(h->b_zero.p, 0, 2 * sizeof(unsigned int), s));
             HY_RET(coarse_tensor(h, m, qq, h->b_qb.p, h->b_qn.as<float4>(), nprobe,
                                  h->w_probes.as<int64_t>() + q0 * nprobe,
-                                 learned_on(h) ? h->m_pscore.as<float>() : nullptr, s));
+                                 learned_on(h) ? h->m_pscore.as<float>() : nullptr, h->b_zero.as<unsigned int>(), s));
         } else {
             HY_CUDA(hy::launch_coarse_scores(qq, (int)m, h->cent.as<float>(), (int)h->nlist, (int)h->d, h->metric,
                                              h->w_scores.as<float>(), s));

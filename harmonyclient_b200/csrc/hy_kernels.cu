@@ -84,6 +84,49 @@ __global__ void __launch_bounds__(256) coarse_scores_kernel(const float* __restr
     }  // query tiles of this CTA
 }
 
+// The same scores for a few queries: a warp per query, a lane per centroid (32
+// centroids and 8 queries per CTA), 128 dimensions staged at a time, each sum
+// in dimension order as above.  Bound by latency: the 64 x 64 tiles leave
+// one query 16 CTAs of mostly empty rows (1024 x 128: 18 us, this 3.3).
+constexpr int CS_DIMS = 128;
+template <int METRIC>
+__global__ void __launch_bounds__(256) coarse_small_kernel(const float* __restrict__ q, int nq,
+                                                           const float* __restrict__ c, int nlist, int d,
+                                                           float* __restrict__ out) {
+    __shared__ __align__(16) float Cs[32][CS_DIMS + 4];
+    __shared__ __align__(16) float Qs[8][CS_DIMS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = blockIdx.x * 32, q0 = blockIdx.y * 8;
+    float acc = 0.0f;
+    for (int d0 = 0; d0 < d; d0 += CS_DIMS) {
+        const int jn = min(CS_DIMS, d - d0);
+        for (int i = threadIdx.x; i < 32 * CS_DIMS; i += 256) {
+            const int r = i / CS_DIMS, j = i % CS_DIMS;
+            if (j < jn && c0 + r < nlist) cp_async4(&Cs[r][j], c + static_cast<size_t>(c0 + r) * d + d0 + j);
+        }
+        for (int i = threadIdx.x; i < 8 * CS_DIMS; i += 256) {
+            const int r = i / CS_DIMS, j = i % CS_DIMS;
+            if (j < jn && q0 + r < nq) cp_async4(&Qs[r][j], q + static_cast<size_t>(q0 + r) * d + d0 + j);
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        const float* a = Qs[warp];
+        const float* b = Cs[lane];
+        int j = 0;
+        for (; j + 4 <= jn; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(a + j), y = *reinterpret_cast<const float4*>(b + j);
+            acc = METRIC == METRIC_L2 ? sq_add(acc, x.x, y.x) : ip_add(acc, x.x, y.x);
+            acc = METRIC == METRIC_L2 ? sq_add(acc, x.y, y.y) : ip_add(acc, x.y, y.y);
+            acc = METRIC == METRIC_L2 ? sq_add(acc, x.z, y.z) : ip_add(acc, x.z, y.z);
+            acc = METRIC == METRIC_L2 ? sq_add(acc, x.w, y.w) : ip_add(acc, x.w, y.w);
+        }
+        for (; j < jn; ++j) acc = METRIC == METRIC_L2 ? sq_add(acc, a[j], b[j]) : ip_add(acc, a[j], b[j]);
+        __syncthreads();
+    }
+    if (q0 + warp < nq && c0 + lane < nlist)
+        out[static_cast<size_t>(q0 + warp) * nlist + c0 + lane] = METRIC == METRIC_L2 ? acc : -acc;
+}
+
 // Per row of `scores` (n values, smaller is better): the m best, best first,
 // ties broken by lower column.  One CTA per row.
 __global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ scores, int n, int m,
@@ -108,6 +151,63 @@ __global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ s
         const uint64_t key = sel[i];
         out_idx[row * m + i] = static_cast<int64_t>(key & 0xffffffffu);
         if (out_score) out_score[row * m + i] = o2f(static_cast<uint32_t>(key >> 32));
+    }
+}
+
+// The same for a few rows, m <= 32 KR: each warp of the row's CTA sorts runs of
+// 32 KR (ordered score, column) keys in registers and folds them into its
+// best, then the warps' lists are folded pairwise through shared memory; the
+// order is select_kernel's.  Bound by latency: a warp's radix passes over a
+// whole row of 1024 take 14 us however few rows there are, sorting the row in
+// shared memory 10, this 4.
+template <int KR>
+__global__ void __launch_bounds__(512) select_fold_kernel(const float* __restrict__ scores, int n, int m,
+                                                          int64_t* __restrict__ out_idx,
+                                                          float* __restrict__ out_score) {
+    constexpr int KP = KR * 32, W = 16;
+    __shared__ uint64_t fold[W / 2][KP];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t row = blockIdx.x;
+    const float* src = scores + row * n;
+    uint64_t t[KR];
+    auto load = [&](uint64_t (&v)[KR], int base) {
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+            const int i = base + r * 32 + lane;
+            v[r] = i < n ? (static_cast<uint64_t>(f2o(src[i])) << 32) | static_cast<uint32_t>(i) : KEY_MAX;
+        }
+    };
+    load(t, warp * KP);
+    warp_sort<KR>(t, lane);
+    for (int base = (warp + W) * KP; base < n; base += W * KP) {
+        uint64_t c[KR];
+        load(c, base);
+        warp_sort<KR>(c, lane);
+        warp_merge<KR>(t, c, lane);
+    }
+    for (int h = W / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if (warp >= h && warp < 2 * h) {
+#pragma unroll
+            for (int r = 0; r < KR; ++r) fold[warp - h][r * 32 + lane] = t[r];
+        }
+        __syncthreads();
+        if (warp < h) {
+            uint64_t c[KR];
+#pragma unroll
+            for (int r = 0; r < KR; ++r) c[r] = fold[warp][r * 32 + lane];
+            warp_merge<KR>(t, c, lane);
+        }
+    }
+    if (warp == 0) {
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+            const int i = r * 32 + lane;
+            if (i < m) {
+                out_idx[row * m + i] = static_cast<int64_t>(t[r] & 0xffffffffu);
+                if (out_score) out_score[row * m + i] = o2f(static_cast<uint32_t>(t[r] >> 32));
+            }
+        }
     }
 }
 
@@ -1012,8 +1112,20 @@ inline int grid_for(int64_t n, int threads) {
 
 }  // namespace
 
+// Queries up to which the small-batch coarse kernels run (one to two CTAs per
+// SM; beyond, the tiled scores and the warp selection have enough rows).
+constexpr int COARSE_SMALL = 128, SELECT_SMALL = 148;
+
 cudaError_t launch_coarse_scores(const float* q, int nq, const float* cent, int nlist, int d, int metric, float* out,
                                  cudaStream_t s, const RowPick& pick) {
+    if (nq <= COARSE_SMALL && !pick.rows) {
+        const dim3 g((nlist + 31) / 32, (nq + 7) / 8);
+        if (metric == METRIC_L2)
+            coarse_small_kernel<METRIC_L2><<<g, 256, 0, s>>>(q, nq, cent, nlist, d, out);
+        else
+            coarse_small_kernel<METRIC_IP><<<g, 256, 0, s>>>(q, nq, cent, nlist, d, out);
+        return cudaGetLastError();
+    }
     dim3 grid((nlist + 63) / 64, (nq + 63) / 64);
     // A counted pick is usually a few rows: a grid of a few waves loops.
     if (pick.rows) grid.y = std::min(grid.y, std::max(1u, 1184u / grid.x));
@@ -1027,6 +1139,14 @@ cudaError_t launch_coarse_scores(const float* q, int nq, const float* cent, int 
 
 cudaError_t launch_select(const float* scores, int nq, int n, int m, int64_t* out_idx, float* out_score,
                           cudaStream_t s) {
+    if (nq <= SELECT_SMALL && n <= 4096 && m <= 256 && m <= n) {
+        auto run = [&](auto kern) { kern<<<nq, 512, 0, s>>>(scores, n, m, out_idx, out_score); };
+        m <= 32    ? run(select_fold_kernel<1>)
+        : m <= 64  ? run(select_fold_kernel<2>)
+        : m <= 128 ? run(select_fold_kernel<4>)
+                   : run(select_fold_kernel<8>);
+        return cudaGetLastError();
+    }
     if (m <= 256 && n <= 1024) {
         select_warp_kernel<32><<<(nq + 7) / 8, 256, 0, s>>>(scores, nq, n, m, out_idx, out_score);
         return cudaGetLastError();

@@ -91,7 +91,7 @@ def test_candidate_overflow():
     assert _same(idx, q, 100)["fallback_queries"] > 0
 
 
-def test_far_offset_keeps_the_list_major_scan():
+def test_far_offset_keeps_the_exact_scans():
     x, q = _data(32, 9_000, 1_500, "float", 8)
     _same(_index(x + 30_000), q + 30_000, 10, tensor=False)
 
