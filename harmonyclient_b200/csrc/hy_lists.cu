@@ -41,7 +41,9 @@ namespace hy {
 namespace {
 
 constexpr int METRIC_L2 = 1;  // include/hy.h's HY_METRIC_L2
-constexpr int LM_WARPS = 8;
+// Warps of the scan's CTA: 16 for blocks of two groups (one ring slot each), the
+// occupancy that two CTAs of 8 give one group; else 8.
+__host__ __device__ constexpr int lm_warps(int NG) { return NG == 2 ? 16 : 8; }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
@@ -70,19 +72,22 @@ __device__ inline int4 decode_item(const ListScanParams& p, int64_t g) {
 // `rowp`: this lane's row of the staged block's first group (pitch P floats in
 // all, groups 1024 floats apart); `qb(qi)`:
 // query qi's block.  sp[qi] accumulates the block sums in order.
-// MULTI = false: the block is one 32-float chunk group (pitch 32).
-template <int QG, bool MULTI>
+template <int QG>
 __device__ __forceinline__ void block_compute(const float* rowp, const float* qs, int row_pitch, int boff, int P,
                                               bool first, bool l2, uint32_t live, float (&sp)[QG], int lane) {
-    if (!MULTI) {
+    float acc[QG];
+#pragma unroll
+    for (int qi = 0; qi < QG; ++qi) acc[qi] = 0.0f;
+    for (int s8 = 0; s8 < (P >> 2); s8 += 8) {
         float4 xr[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) xr[c] = *reinterpret_cast<const float4*>(rowp + 4 * (c ^ (lane & 7)));
+        for (int c = 0; c < 8; ++c)
+            xr[c] = *reinterpret_cast<const float4*>(rowp + 128 * s8 + 4 * (c ^ (lane & 7)));
 #pragma unroll
         for (int qi = 0; qi < QG; ++qi) {
             if (live & (1u << qi)) {
-                const float* qb = qs + qi * row_pitch + boff;
-                float a = 0.0f;
+                const float* qb = qs + qi * row_pitch + boff + 4 * s8;
+                float a = acc[qi];
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const float4 y = *reinterpret_cast<const float4*>(qb + 4 * c);
@@ -98,98 +103,74 @@ __device__ __forceinline__ void block_compute(const float* rowp, const float* qs
                         a = ip_add(a, y.w, xr[c].w);
                     }
                 }
-                sp[qi] = first ? a : __fadd_rn(sp[qi], a);
+                acc[qi] = a;
             }
         }
-    } else {
-        float acc[QG];
-#pragma unroll
-        for (int qi = 0; qi < QG; ++qi) acc[qi] = 0.0f;
-        for (int s8 = 0; s8 < (P >> 2); s8 += 8) {
-            float4 xr[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                xr[c] = *reinterpret_cast<const float4*>(rowp + 128 * s8 + 4 * (c ^ (lane & 7)));
-#pragma unroll
-            for (int qi = 0; qi < QG; ++qi) {
-                if (live & (1u << qi)) {
-                    const float* qb = qs + qi * row_pitch + boff + 4 * s8;
-                    float a = acc[qi];
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const float4 y = *reinterpret_cast<const float4*>(qb + 4 * c);
-                        if (l2) {
-                            a = sq_add(a, y.x, xr[c].x);
-                            a = sq_add(a, y.y, xr[c].y);
-                            a = sq_add(a, y.z, xr[c].z);
-                            a = sq_add(a, y.w, xr[c].w);
-                        } else {
-                            a = ip_add(a, y.x, xr[c].x);
-                            a = ip_add(a, y.y, xr[c].y);
-                            a = ip_add(a, y.z, xr[c].z);
-                            a = ip_add(a, y.w, xr[c].w);
-                        }
-                    }
-                    acc[qi] = a;
-                }
-            }
-        }
-#pragma unroll
-        for (int qi = 0; qi < QG; ++qi)
-            if (live & (1u << qi)) sp[qi] = first ? acc[qi] : __fadd_rn(sp[qi], acc[qi]);
     }
+#pragma unroll
+    for (int qi = 0; qi < QG; ++qi)
+        if (live & (1u << qi)) sp[qi] = first ? acc[qi] : __fadd_rn(sp[qi], acc[qi]);
 }
 
-// Chunks [C0, C1) (4 dimensions each) of one query's block sum (qb: its 32
-// block values) against this lane's row (xr), continuing from a, in
-// dimension order; and of two queries at once, as two independent
-// dependency chains.
-template <bool L2, int C0, int C1>
-__device__ __forceinline__ float chain1(const float* qb, const float4 (&xr)[8], float a) {
+// Chunks [C0, C1) (4 dimensions each) of one query's block sum (qb: its block
+// values) against this lane's row (xr: NG groups of 8 chunks, ng of them in
+// the block), continuing from a, in dimension order; and of two queries at
+// once, as two independent dependency chains.
+template <bool L2>
+__device__ __forceinline__ float sum4(float a, const float4 y, const float4 x) {
+    a = L2 ? sq_add(a, y.x, x.x) : ip_add(a, y.x, x.x);
+    a = L2 ? sq_add(a, y.y, x.y) : ip_add(a, y.y, x.y);
+    a = L2 ? sq_add(a, y.z, x.z) : ip_add(a, y.z, x.z);
+    return L2 ? sq_add(a, y.w, x.w) : ip_add(a, y.w, x.w);
+}
+template <bool L2, int NG, int C0, int C1>
+__device__ __forceinline__ float chain1(const float* qb, const float4 (&xr)[8 * NG], int ng, float a) {
 #pragma unroll
-    for (int c = C0; c < C1; ++c) {
-        const float4 y = *reinterpret_cast<const float4*>(qb + 4 * c);
-        if (L2) {
-            a = sq_add(a, y.x, xr[c].x);
-            a = sq_add(a, y.y, xr[c].y);
-            a = sq_add(a, y.z, xr[c].z);
-            a = sq_add(a, y.w, xr[c].w);
-        } else {
-            a = ip_add(a, y.x, xr[c].x);
-            a = ip_add(a, y.y, xr[c].y);
-            a = ip_add(a, y.z, xr[c].z);
-            a = ip_add(a, y.w, xr[c].w);
+    for (int g = C0 / 8; g < (C1 + 7) / 8; ++g) {
+        if (g > 0 && g >= ng) break;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = 8 * g + i;
+            if (c < C0 || c >= C1) continue;
+            a = sum4<L2>(a, *reinterpret_cast<const float4*>(qb + 4 * c), xr[c]);
         }
     }
     return a;
 }
 
-template <bool L2, int C0, int C1>
-__device__ __forceinline__ void chain2(const float* qa, const float* qb, const float4 (&xr)[8], float& a0,
+template <bool L2, int NG, int C0, int C1>
+__device__ __forceinline__ void chain2(const float* qa, const float* qb, const float4 (&xr)[8 * NG], int ng, float& a0,
                                        float& a1) {
     float s0 = a0, s1 = a1;
 #pragma unroll
-    for (int c = C0; c < C1; ++c) {
-        const float4 y0 = *reinterpret_cast<const float4*>(qa + 4 * c);
-        const float4 y1 = *reinterpret_cast<const float4*>(qb + 4 * c);
-        if (L2) {
-            s0 = sq_add(s0, y0.x, xr[c].x);
-            s1 = sq_add(s1, y1.x, xr[c].x);
-            s0 = sq_add(s0, y0.y, xr[c].y);
-            s1 = sq_add(s1, y1.y, xr[c].y);
-            s0 = sq_add(s0, y0.z, xr[c].z);
-            s1 = sq_add(s1, y1.z, xr[c].z);
-            s0 = sq_add(s0, y0.w, xr[c].w);
-            s1 = sq_add(s1, y1.w, xr[c].w);
-        } else {
-            s0 = ip_add(s0, y0.x, xr[c].x);
-            s1 = ip_add(s1, y1.x, xr[c].x);
-            s0 = ip_add(s0, y0.y, xr[c].y);
-            s1 = ip_add(s1, y1.y, xr[c].y);
-            s0 = ip_add(s0, y0.z, xr[c].z);
-            s1 = ip_add(s1, y1.z, xr[c].z);
-            s0 = ip_add(s0, y0.w, xr[c].w);
-            s1 = ip_add(s1, y1.w, xr[c].w);
+    for (int g = C0 / 8; g < (C1 + 7) / 8; ++g) {
+        if (g > 0 && g >= ng) break;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = 8 * g + i;
+            if (c < C0 || c >= C1) continue;
+            const float4 y0 = *reinterpret_cast<const float4*>(qa + 4 * c);
+            const float4 y1 = *reinterpret_cast<const float4*>(qb + 4 * c);
+            const float4 x = xr[c];
+            if (L2) {
+                s0 = sq_add(s0, y0.x, x.x);
+                s1 = sq_add(s1, y1.x, x.x);
+                s0 = sq_add(s0, y0.y, x.y);
+                s1 = sq_add(s1, y1.y, x.y);
+                s0 = sq_add(s0, y0.z, x.z);
+                s1 = sq_add(s1, y1.z, x.z);
+                s0 = sq_add(s0, y0.w, x.w);
+                s1 = sq_add(s1, y1.w, x.w);
+            } else {
+                s0 = ip_add(s0, y0.x, x.x);
+                s1 = ip_add(s1, y1.x, x.x);
+                s0 = ip_add(s0, y0.y, x.y);
+                s1 = ip_add(s1, y1.y, x.y);
+                s0 = ip_add(s0, y0.z, x.z);
+                s1 = ip_add(s1, y1.z, x.z);
+                s0 = ip_add(s0, y0.w, x.w);
+                s1 = ip_add(s1, y1.w, x.w);
+            }
         }
     }
     a0 = s0;
@@ -197,19 +178,28 @@ __device__ __forceinline__ void chain2(const float* qa, const float* qb, const f
 }
 
 // Persistent list-major scan.  QG queries per group (<= 32), R bulk-copy
-// slots per warp, LM_WARPS warps.  Blocks of pitch 32 (MULTI = false) keep
-// each (query, row) partial sum in shared memory and walk the live queries of
-// a tile two at a time; wider blocks keep them in registers.
-template <int QG, int R, bool MULTI, bool L2>
-__global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
+// slots per warp, lm_warps warps.  Blocks of up to NG groups of 32 floats (NG
+// 1 to 4) keep a lane's row in registers, each (query, row) partial sum in
+// shared memory, and walk the live queries of a tile two at a time; wider
+// blocks (NG 0) keep the partial sums in registers and take the row group by
+// group.  (With partial sums of 32 queries in registers, every query's code is
+// unrolled and predicated: 2,000 queries on 300k x 200 took 2.2 ms in blocks of
+// two groups, 1.3 ms so.)
+template <int QG, int R, int NG, bool L2>
+__global__ void __launch_bounds__(lm_warps(NG) * 32, NG == 1 ? 2 : 1)
     list_scan_kernel(const __grid_constant__ ListScanParams p) {
+    constexpr bool MULTI = NG == 0;
+    constexpr int LM_WARPS = lm_warps(NG);
+    // With 16 warps a list's tiles (about 20) end unevenly: units of half the
+    // group's queries.
+    constexpr int SPLIT = NG == 2 ? 2 : 1;
     extern __shared__ __align__(128) unsigned char smem[];
     const ArenaLayout& L = p.L;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t slot_floats = static_cast<size_t>(32) * L.max_pitch;
     float* bufs = reinterpret_cast<float*>(smem);
     float* qs = bufs + static_cast<size_t>(LM_WARPS) * R * slot_floats;
-    float* sps = qs + static_cast<size_t>(QG) * L.row_pitch;  // [warp][query][lane] partial sums (pitch 32)
+    float* sps = qs + static_cast<size_t>(QG) * L.row_pitch;  // [warp][query][lane] partial sums (NG > 0)
     uint64_t* bars = reinterpret_cast<uint64_t*>(sps + (MULTI ? 0 : static_cast<size_t>(LM_WARPS) * QG * 32));
     __shared__ float s_thr[QG];
     __shared__ float s_lo[QG], s_hi[QG];  // OPT_TRIANGLE: each query's candidate2centroid window
@@ -353,7 +343,10 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
         const int64_t row0 = s_row0;
         const uint32_t qmask = nqv >= 32 ? 0xffffffffu : ((1u << nqv) - 1u);
 
+        // The queries of a unit.
+        auto unit_mask = [&](int u) { return SPLIT == 1 ? 0xffffffffu : (u & 1) ? 0xffff0000u : 0x0000ffffu; };
         // Issuer state (warp-uniform): the tile being issued and its next block.
+        // (a unit: a tile, or with SPLIT 2 a tile with half of the queries)
         int it_tile = -1, it_b = 0;
         bool more = true;
         // Consumer state.
@@ -370,17 +363,19 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
                     int g = 0;
                     if (lane == 0) g = atomicAdd(&s_next, 1);
                     g = __shfl_sync(FULL, g, 0);
-                    if (g >= ntiles) {
+                    if (g >= ntiles * SPLIT) {
                         more = false;
                         return;
                     }
+                    const uint32_t qm = qmask & unit_mask(g);
+                    if (!qm) continue;
                     possible += L.nb;
-                    possible_sums += static_cast<unsigned long long>(L.row_pitch >> 4) * nqv;
+                    possible_sums += static_cast<unsigned long long>(L.row_pitch >> 4) * __popc(qm);
                     if (p.triangle) {
                         // A tile whose rows lie outside every query's window
                         // is not loaded.
-                        const float2 tr = p.c2c_tile[(row0 >> 5) + g];
-                        const bool hit = lane < nqv && !(tr.y > s_hi[lane]) && !(tr.x < s_lo[lane]);
+                        const float2 tr = p.c2c_tile[(row0 >> 5) + g / SPLIT];
+                        const bool hit = ((qm >> lane) & 1u) && !(tr.y > s_hi[lane]) && !(tr.x < s_lo[lane]);
                         if (!__any_sync(FULL, hit)) continue;
                     }
                     it_tile = g;
@@ -396,7 +391,7 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
                     mbar_expect_tx(&wbar[slot], bytes);
                     for (int g = 0; g < L.pitch[b] >> 5; ++g)
                         bulk_g2s(wb + static_cast<size_t>(slot) * slot_floats + g * 1024,
-                                 p.codes + arena_tile_offset(L, (row0 >> 5) + it_tile, (L.boff[b] >> 5) + g), 4096,
+                                 p.codes + arena_tile_offset(L, (row0 >> 5) + it_tile / SPLIT, (L.boff[b] >> 5) + g), 4096,
                                  &wbar[slot]);
                 }
                 ++iss;
@@ -419,12 +414,12 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
                 for (; con != iss; ++con) mbar_wait_bounded(&wbar[con % R], (con / R) & 1u, p.err);
                 break;
             }
-            const int tile = s_tag_tile[warp][slot];
+            const int unit = s_tag_tile[warp][slot], tile = unit / SPLIT;
             const int b = s_tag_b[warp][slot];
-            if (tile != cur_tile) {
-                cur_tile = tile;
+            if (unit != cur_tile) {
+                cur_tile = unit;
                 const int nv = min(32, nrows - 32 * tile);
-                alive = lane < nv ? qmask : 0u;
+                alive = lane < nv ? qmask & unit_mask(unit) : 0u;
                 if (p.triangle && lane < nv) {
                     const float cc = p.c2c[row0 + 32 * static_cast<int64_t>(tile) + lane];
 #pragma unroll
@@ -432,17 +427,23 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
                         if (cc > s_hi[qi] || cc < s_lo[qi]) alive &= ~(1u << qi);
                 }
             }
-            if (tile != dead_tile) {
+            if (unit != dead_tile) {
                 const uint32_t live = __reduce_or_sync(FULL, alive);
                 if (live == 0u) {
-                    dead_tile = tile;
-                    if (it_tile == tile) it_tile = -1;  // issue none of its further blocks
+                    dead_tile = unit;
+                    if (it_tile == unit) it_tile = -1;  // issue none of its further blocks
                 } else if (!MULTI) {
                     const float* rowp = wb + static_cast<size_t>(slot) * slot_floats + lane * 32;
-                    float4 xr[8];
+                    constexpr int XG = NG > 0 ? NG : 1;
+                    const int ng = NG > 1 ? L.pitch[b] >> 5 : 1;
+                    float4 xr[8 * XG];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        xr[c] = *reinterpret_cast<const float4*>(rowp + 4 * (c ^ (lane & 7)));
+                    for (int g = 0; g < XG; ++g)
+                        if (g == 0 || g < ng) {
+#pragma unroll
+                            for (int c = 0; c < 8; ++c)
+                                xr[8 * g + c] = *reinterpret_cast<const float4*>(rowp + 1024 * g + 4 * (c ^ (lane & 7)));
+                        }
                     const float* qbase = qs + L.boff[b];
                     const bool first = b == 0, last = b + 1 == L.nb;
                     const int64_t arow = row0 + 32 * static_cast<int64_t>(tile) + lane;
@@ -504,31 +505,31 @@ __global__ void __launch_bounds__(LM_WARPS * 32, MULTI ? 1 : 2)
                             todo &= todo - 1;
                             const float* yb = qbase + qb * L.row_pitch;
                             float a0 = 0.0f, a1 = 0.0f;
-                            chain2<L2, 0, 4>(ya, yb, xr, a0, a1);
+                            chain2<L2, XG, 0, 4>(ya, yb, xr, ng, a0, a1);
                             bool da, db;
                             half_dead2(qa, a0, qb, a1, da, db);
-                            computed += 4 - (da ? 1 : 0) - (db ? 1 : 0);
+                            computed += 2 + (da ? 0 : 2 * ng - 1) + (db ? 0 : 2 * ng - 1);
                             if (!da && !db) {
-                                chain2<L2, 4, 8>(ya, yb, xr, a0, a1);
+                                chain2<L2, XG, 4, 8 * XG>(ya, yb, xr, ng, a0, a1);
                                 finish(qa, a0);
                                 finish(qb, a1);
                             } else if (!da) {
-                                finish(qa, chain1<L2, 4, 8>(ya, xr, a0));
+                                finish(qa, chain1<L2, XG, 4, 8 * XG>(ya, xr, ng, a0));
                             } else if (!db) {
-                                finish(qb, chain1<L2, 4, 8>(yb, xr, a1));
+                                finish(qb, chain1<L2, XG, 4, 8 * XG>(yb, xr, ng, a1));
                             }
                         } else {
-                            const float a0 = chain1<L2, 0, 4>(ya, xr, 0.0f);
+                            const float a0 = chain1<L2, XG, 0, 4>(ya, xr, ng, 0.0f);
                             const bool da = half_dead(qa, a0);
-                            computed += da ? 1 : 2;
-                            if (!da) finish(qa, chain1<L2, 4, 8>(ya, xr, a0));
+                            computed += da ? 1 : 2 * ng;
+                            if (!da) finish(qa, chain1<L2, XG, 4, 8 * XG>(ya, xr, ng, a0));
                         }
                     }
                 } else {
                     computed += static_cast<unsigned long long>(__popc(live)) * (L.pitch[b] >> 4);
                     const int P = L.pitch[b];
                     const float* rowp = wb + static_cast<size_t>(slot) * slot_floats + lane * 32;
-                    block_compute<QG, MULTI>(rowp, qs, L.row_pitch, L.boff[b], P, b == 0, l2, live, sp, lane);
+                    block_compute<QG>(rowp, qs, L.row_pitch, L.boff[b], P, b == 0, l2, live, sp, lane);
                     if (b + 1 < L.nb) {
                         if (prune) {
 #pragma unroll
@@ -698,17 +699,19 @@ __global__ void row_centroid_kernel(ArenaLayout L, const float* __restrict__ cod
     if (lane == 0) c2c_tile[gw] = make_float2(mx, mn);
 }
 
-template <int QG, int R, bool MULTI>
+template <int QG, int R, int NG>
 size_t list_scan_smem(const ArenaLayout& L) {
+    constexpr int LM_WARPS = lm_warps(NG);
     return static_cast<size_t>(LM_WARPS) * R * 32 * L.max_pitch * 4 + static_cast<size_t>(QG) * L.row_pitch * 4 +
-           (MULTI ? 0 : static_cast<size_t>(LM_WARPS) * QG * 32 * 4) + static_cast<size_t>(LM_WARPS) * R * 8;
+           (NG > 0 ? static_cast<size_t>(LM_WARPS) * QG * 32 * 4 : 0) + static_cast<size_t>(LM_WARPS) * R * 8;
 }
 
-template <int QG, int R, bool MULTI, bool L2>
+template <int QG, int R, int NG, bool L2>
 cudaError_t launch_list_scan_m(const ListScanParams& p, int nsm, cudaStream_t s) {
-    const size_t smem = list_scan_smem<QG, R, MULTI>(p.L);
+    const size_t smem = list_scan_smem<QG, R, NG>(p.L);
+    constexpr int LM_WARPS = lm_warps(NG);
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
-    auto kern = list_scan_kernel<QG, R, MULTI, L2>;
+    auto kern = list_scan_kernel<QG, R, NG, L2>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -719,34 +722,35 @@ cudaError_t launch_list_scan_m(const ListScanParams& p, int nsm, cudaStream_t s)
     return cudaGetLastError();
 }
 
-template <int QG, int R, bool MULTI>
+template <int QG, int R, int NG>
 cudaError_t launch_list_scan_t(const ListScanParams& p, int nsm, cudaStream_t s) {
-    return p.metric == METRIC_L2 ? launch_list_scan_m<QG, R, MULTI, true>(p, nsm, s)
-                                 : launch_list_scan_m<QG, R, MULTI, false>(p, nsm, s);
+    return p.metric == METRIC_L2 ? launch_list_scan_m<QG, R, NG, true>(p, nsm, s)
+                                 : launch_list_scan_m<QG, R, NG, false>(p, nsm, s);
 }
+
+// Shared memory left for the kernel's static variables.
+constexpr size_t LM_SMEM_CAP = 227 * 1024 - 2048;
 
 }  // namespace
 
-bool list_scan_multi(const ArenaLayout& L) {
-    for (int b = 0; b < L.nb; ++b)
-        if (L.pitch[b] != 32) return true;
-    return false;
-}
-
 bool list_scan_fits(const ArenaLayout& L) {
-    if (!list_scan_multi(L)) return list_scan_smem<LM_GROUP, 2, false>(L) <= 227 * 1024;
-    if (L.max_pitch <= 64) return list_scan_smem<LM_GROUP, 2, true>(L) <= 227 * 1024;
-    return list_scan_smem<LM_GROUP, 1, true>(L) <= 227 * 1024;
+    if (L.max_pitch == 32) return list_scan_smem<LM_GROUP, 2, 1>(L) <= 227 * 1024;
+    if (L.max_pitch <= 64) return list_scan_smem<LM_GROUP, 2, 0>(L) <= 227 * 1024;
+    return list_scan_smem<LM_GROUP, 1, 0>(L) <= 227 * 1024;
 }
 
 cudaError_t launch_list_scan(const ListScanParams& p, int nsm, cudaStream_t s) {
     if (p.qg != LM_GROUP) return cudaErrorInvalidValue;
-    // Pitch-32 blocks: two ring slots per warp (with the shared-memory
-    // partial sums, two CTAs per SM); wider blocks: two slots while they fit
-    // (pitch <= 64 floats), else one.
-    if (!list_scan_multi(p.L)) return launch_list_scan_t<LM_GROUP, 2, false>(p, nsm, s);
-    if (p.L.max_pitch <= 64) return launch_list_scan_t<LM_GROUP, 2, true>(p, nsm, s);
-    return launch_list_scan_t<LM_GROUP, 1, true>(p, nsm, s);
+    // The widest block's groups choose the form; two ring slots per warp for
+    // one or two groups (with the shared-memory partial sums, two CTAs per SM
+    // for one), else one.
+    const int ng = p.L.max_pitch / 32;
+    if (ng == 1) return launch_list_scan_t<LM_GROUP, 2, 1>(p, nsm, s);
+    if (ng == 2 && list_scan_smem<LM_GROUP, 1, 2>(p.L) <= LM_SMEM_CAP) return launch_list_scan_t<LM_GROUP, 1, 2>(p, nsm, s);
+    if (ng == 3 && list_scan_smem<LM_GROUP, 1, 3>(p.L) <= LM_SMEM_CAP) return launch_list_scan_t<LM_GROUP, 1, 3>(p, nsm, s);
+    if (ng == 4 && list_scan_smem<LM_GROUP, 1, 4>(p.L) <= LM_SMEM_CAP) return launch_list_scan_t<LM_GROUP, 1, 4>(p, nsm, s);
+    if (ng <= 2) return launch_list_scan_t<LM_GROUP, 2, 0>(p, nsm, s);
+    return launch_list_scan_t<LM_GROUP, 1, 0>(p, nsm, s);
 }
 
 cudaError_t launch_row_centroid(const ArenaLayout& L, const float* codes, const int64_t* list_off,

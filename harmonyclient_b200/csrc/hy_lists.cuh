@@ -42,9 +42,6 @@ struct ListScanParams {
     const float* cent = nullptr;
 };
 
-// True when some dimension block is wider than 32 floats (the multi-chunk
-// kernel variant).
-bool list_scan_multi(const ArenaLayout& L);
 // True when the scan's shared memory (block-copy slots and the group's
 // queries) fits one CTA for this layout.
 bool list_scan_fits(const ArenaLayout& L);
