@@ -1831,14 +1831,18 @@ __global__ void coarse_items_kernel(int nq, int nlist, int64_t rows, int ngroups
     }
 }
 
-// Staging row pitch of coarse_refine_kernel (floats): d + 4 when d is a
-// multiple of 4 (16-byte rows), else d + 1 (conflict-free column reads).
-__host__ __device__ inline int refine_pitch(int d) { return (d & 3) == 0 ? d + 4 : d + 1; }
+// Dimensions of a centroid staged at a time by the refine kernels: whole rows
+// up to REFINE_DIMS (one bulk copy each), else runs of REFINE_CHUNK.
+constexpr int REFINE_DIMS = 256, REFINE_CHUNK = 128;
+__host__ __device__ inline int refine_dims(int d) { return d <= REFINE_DIMS ? d : REFINE_CHUNK; }
+// Staging row pitch (floats) for w staged dimensions of d: w + 4 when d is a
+// multiple of 4 (16-byte rows), else w + 1 (conflict-free column reads).
+__host__ __device__ inline int refine_pitch(int d) { return refine_dims(d) + ((d & 3) == 0 ? 4 : 1); }
 // Shared memory per warp of the refine kernels: the copy barrier (16 bytes
 // with padding), 256 histogram bins, the query and a 32-row staging block.
+__host__ __device__ inline size_t refine_query_floats(int d) { return (static_cast<size_t>(d) + 7) & ~size_t(3); }
 __host__ __device__ inline size_t refine_warp_bytes(int d) {
-    const size_t pitch = refine_pitch(d);
-    return (16 + 1024 + pitch * 4 + 32 * pitch * 4 + 15) & ~size_t(15);
+    return (16 + 1024 + refine_query_floats(d) * 4 + 32 * static_cast<size_t>(refine_pitch(d)) * 4 + 15) & ~size_t(15);
 }
 
 // Exact coarse selection from the tensor-core scores.  Per query (one warp):
@@ -1933,7 +1937,6 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
     auto cid_of = [&](int e) { return ids_smem ? sids[e] : static_cast<int>(keys[e]); };
     uint64_t kr[4] = {KEY_MAX, KEY_MAX, KEY_MAX, KEY_MAX};
     if (v4) {
-        const uint32_t rb = static_cast<uint32_t>(d) * 4u;  // bytes of one row
         uint64_t* bar = &bars[0];
         if (lane == 0) {
             mbar_init(bar, 1);
@@ -1941,31 +1944,39 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
         }
         __syncwarp();
         uint32_t issued = 0, used = 0;  // phases of the barrier issued and consumed
-        // nr rows: lane i's row (centroid cid_) by one bulk copy completing
-        // on the barrier.  A round's reads of the staging block have all
-        // returned (every lane's sum used them before the __syncwarp that
-        // precedes the next round's copies), as in a copy pipeline whose
-        // consumers release a stage by arriving on a barrier.
-        auto copy_rows = [&](int cid_, int nr) {
-            if (lane == 0) mbar_expect_tx(bar, static_cast<uint32_t>(nr) * rb);
+        // nr rows' dimensions [j, j + w): lane i's row (centroid cid_) by one
+        // bulk copy completing on the barrier.  A step's reads of the staging
+        // block have all returned (every lane's sum used them before the
+        // __syncwarp that precedes the next step's copies), as in a copy
+        // pipeline whose consumers release a stage by arriving on a barrier.
+        auto copy_rows = [&](int cid_, int nr, int j, int w) {
+            if (lane == 0) mbar_expect_tx(bar, static_cast<uint32_t>(nr * w) * 4u);
             __syncwarp();
-            if (lane < nr) bulk_g2s(stage + lane * pitch, cent + static_cast<size_t>(cid_) * d, rb, bar);
+            if (lane < nr) bulk_g2s(stage + lane * pitch, cent + static_cast<size_t>(cid_) * d + j, w * 4u, bar);
             ++issued;
         };
+        const int W = refine_dims(d);
         int cid = lane < min(32, c) ? cid_of(lane) : 0;
-        if (c > 0) copy_rows(cid, min(32, c));
+        if (c > 0) copy_rows(cid, min(32, c), 0, W);
         bool ok = true;
-        for (int c0 = 0, r = 0; c0 < c; c0 += 32, ++r) {
+        for (int c0 = 0, r = 0; c0 < c && ok; c0 += 32, ++r) {
             const int nr = min(32, c - c0);
             const int nn = max(0, min(32, c - c0 - 32));  // next round's rows
             const int cidn = lane < nn ? cid_of(c0 + 32 + lane) : 0;
             float acc = 0.0f;
-            ok = mbar_wait_bounded(bar, used & 1u, err);
+            for (int j = 0; j < d; j += W) {
+                const int w = min(W, d - j);
+                ok = __all_sync(FULL, mbar_wait_bounded(bar, used & 1u, err));
+                if (!ok) break;
+                ++used;
+                if (lane < nr) acc = coarse_dot<METRIC>(qs + j, stage + lane * pitch, 0, w, acc);
+                __syncwarp();
+                if (j + W < d)
+                    copy_rows(cid, nr, j + W, min(W, d - j - W));
+                else if (nn)
+                    copy_rows(cidn, nn, 0, W);
+            }
             if (!ok) break;
-            ++used;
-            if (lane < nr) acc = coarse_dot<METRIC>(qs, stage + lane * pitch, 0, d, acc);
-            __syncwarp();
-            if (nn) copy_rows(cidn, nn);
             if (lane < nr) {
                 const float score = METRIC == METRIC_L2 ? acc : -acc;
                 const uint64_t key = (static_cast<uint64_t>(f2o(score)) << 32) | static_cast<uint32_t>(cid);
@@ -1988,21 +1999,28 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
         }
         __syncwarp();
     } else {
+        const int W = refine_dims(d);
         for (int c0 = 0, r = 0; c0 < c; c0 += 32, ++r) {
             const int nr = min(32, c - c0);
             const int cidr = lane < nr ? cid_of(c0 + lane) : 0;
-            for (int rr = 0; rr < nr; ++rr) {
-                const float* src = cent + static_cast<size_t>(__shfl_sync(FULL, cidr, rr)) * d;
-                float* dst = stage + rr * pitch;
-                for (int j = lane; j < d; j += 32) cp_async4(dst + j, src + j);
+            float acc = 0.0f;
+            for (int j0 = 0; j0 < d; j0 += W) {
+                const int w = min(W, d - j0);
+                for (int rr = 0; rr < nr; ++rr) {
+                    const float* src = cent + static_cast<size_t>(__shfl_sync(FULL, cidr, rr)) * d + j0;
+                    float* dst = stage + rr * pitch;
+                    for (int j = lane; j < w; j += 32) cp_async4(dst + j, src + j);
+                }
+                cp_async_wait_all();
+                __syncwarp();
+                if (lane < nr) {
+                    const float* row = stage + lane * pitch;
+                    for (int jj = 0; jj < w; ++jj)
+                        acc = METRIC == METRIC_L2 ? sq_add(acc, qs[j0 + jj], row[jj]) : ip_add(acc, qs[j0 + jj], row[jj]);
+                }
+                __syncwarp();
             }
-            cp_async_wait_all();
-            __syncwarp();
             if (lane < nr) {
-                const float* row = stage + lane * pitch;
-                float acc = 0.0f;
-                for (int jj = 0; jj < d; ++jj)
-                    acc = METRIC == METRIC_L2 ? sq_add(acc, qs[jj], row[jj]) : ip_add(acc, qs[jj], row[jj]);
                 const float score = METRIC == METRIC_L2 ? acc : -acc;
                 const uint64_t key = (static_cast<uint64_t>(f2o(score)) << 32) | static_cast<uint32_t>(cidr);
                 if (in_regs) {
@@ -2080,7 +2098,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
     uint64_t* bars = reinterpret_cast<uint64_t*>(base);
     int* hist = reinterpret_cast<int*>(base + 16);
     float* qs = reinterpret_cast<float*>(hist + 256);
-    float* stage = qs + pitch;
+    float* stage = qs + refine_query_floats(d);
     const int qi = blockIdx.x * (blockDim.x >> 5) + warp;
     if (qi >= nq) return;  // whole warp
     const float* qrow = q + static_cast<size_t>(qi) * d;
@@ -2100,7 +2118,8 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
     float lo[PER];
     auto bound = [&](int r, float sc, float ax, float ay, float xn) {
         const float eb = fmaf(ax, ec.aq, fmaf(ay, ec.bq, err_row_const(xn, l2, cN) + ec.cq));
-        hi[r] = f2o(sc + eb);
+        // What is not a finite number bounds nothing from above.
+        hi[r] = fabsf(sc + eb) < INFINITY ? f2o(sc + eb) : 0xffffffffu;
         lo[r] = sc - eb;
     };
     if (vec) {
@@ -2211,7 +2230,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_keys_kernel(uint64_t* __
     uint64_t* bars = reinterpret_cast<uint64_t*>(base);
     int* hist = reinterpret_cast<int*>(base + 16);
     float* qs = reinterpret_cast<float*>(hist + 256);
-    float* stage = qs + pitch;
+    float* stage = qs + refine_query_floats(d);
     const int qi = blockIdx.x * (blockDim.x >> 5) + warp;
     if (qi >= nq) return;  // whole warp
     const float* qrow = q + static_cast<size_t>(qi) * d;

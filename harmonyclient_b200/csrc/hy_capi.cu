@@ -1035,7 +1035,7 @@ bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s) {
 // Whether a batched search's coarse step runs on the tensor cores (the
 // conditions launch_coarse_refine's shared memory and select width need).
 bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
-    return h->coarse_mode == HY_COARSE_TENSOR && nprobe <= 256 && h->d <= 256 &&
+    return h->coarse_mode == HY_COARSE_TENSOR && nprobe <= 256 && (h->d <= 256 || h->nlist <= 2048) &&
            (h->form == HY_FORM_BF16 || h->nlist <= 2048) && hy::batched_group_size((int)(h->d + 63) / 64) > 0;
 }
 
