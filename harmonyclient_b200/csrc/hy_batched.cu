@@ -749,6 +749,7 @@ struct BatchedParams {
     int ksplit;                     // 1: A k-blocks 2j, 2j+1 (hi, lo) both take query k-block j
     int ns;                         // stages in the list k-block ring (at most NS_MAX)
     int nslot;                      // item slots (2 or SLOT_MAX)
+    int nbuf;                       // query operand buffers: one per slot, or a single one
     int dense_max;                  // lists of at most this many rows: dense items (0 = none)
     float cK, cN;                   // error-bound constants (see err_coef)
 };
@@ -769,9 +770,8 @@ constexpr int CB = 128;         // per-epilogue-warp candidate staging
 constexpr int SLOT_MAX = 3;
 constexpr int RING_SLOT3 = 5;  // three slots only when they leave this many k-blocks in the ring
 // WIDE: rows of many k-blocks, whose query operands take most of the shared
-// memory: shorter row slices and candidate-test chunks make room for groups
-// of 64 where only 32 fit otherwise (an MMA of N = 32 costs 40 cycles, of 64
-// 48).
+// memory: shorter row slices and candidate-test chunks make room for a ring
+// (see group_plan).
 template <int QG, bool WIDE>
 struct Shape {
     static constexpr int CW = QG / 2;                                   // accumulator columns per epilogue warp
@@ -795,12 +795,13 @@ struct ItemSlot {
     alignas(16) float sc[QG];    // accumulator -> inner product scale (1, or list scale x query scale)
 };
 
-// Dynamic shared memory of the batched kernel for rows (and queries) of nkb
-// 128-byte k-blocks, `ring` k-blocks in the stage ring and nslot item slots.
+// Dynamic shared memory of the batched kernel for queries of nkb 128-byte
+// k-blocks in nbuf buffers, `ring` list k-blocks in the stage ring and nslot
+// item slots.
 template <int QG, bool WIDE>
-constexpr size_t batched_smem(int nkb, int ring, int nslot) {
+constexpr size_t batched_smem(int nkb, int ring, int nslot, int nbuf) {
     using S = Shape<QG, WIDE>;
-    return 1024 + nslot * static_cast<size_t>(nkb) * QG * 128 + static_cast<size_t>(ring) * KB_BYTES +
+    return 1024 + nbuf * static_cast<size_t>(nkb) * QG * 128 + static_cast<size_t>(ring) * KB_BYTES +
            nslot * sizeof(ItemSlot<QG, S::RS_MAX>) + N_EPI * CB * (sizeof(int) + sizeof(uint64_t)) + N_EPI * 32 * S::CC * sizeof(float);
 }
 // Dynamic shared memory per CTA: the 227 KiB opt-in limit less room for the
@@ -809,11 +810,38 @@ constexpr size_t BATCHED_SMEM_CAP = 227 * 1024 - 256;
 
 // Stages of the deepest ring that fits (0: fewer than RING_MIN k-blocks).
 template <int QG, bool WIDE>
-constexpr int batched_stages(int nkb, int nslot = 2) {
-    const int ks = stage_kblocks(nkb);
+constexpr int batched_stages(int nkb, int nslot, int nbuf, int ks) {
     for (int ns = NS_MAX; ns * ks >= RING_MIN; --ns)
-        if (batched_smem<QG, WIDE>(nkb, ns * ks, nslot) <= BATCHED_SMEM_CAP) return ns;
+        if (batched_smem<QG, WIDE>(nkb, ns * ks, nslot, nbuf) <= BATCHED_SMEM_CAP) return ns;
     return 0;
+}
+
+// How groups of QG queries of nkb k-blocks are laid out: one query buffer per
+// slot where that leaves a ring; else a single buffer, which the next item's
+// queries enter when the last tensor-core instruction of this one has read it
+// (its list tiles are by then on their way into the ring).  The ring's round
+// trip (about 2,500 cycles for two or three 32 KiB stages) sets a tile's time,
+// so twice the queries per tile nearly halve the kernel, and the wait for the
+// queries between items costs less: groups of 128 in one buffer against 64 in
+// two took 1,162 against 1,790 us (1M x 128 as TF32, 625 queries per list),
+// 1,393 against 2,190 (e4m3, 1M x 420) and 3,380 against 4,850 (bf16, 500k x
+// 500), and were level or ahead down to 12 queries per list.
+struct GroupPlan {
+    bool ok, wide;
+    int nbuf;
+};
+template <int QG>
+constexpr GroupPlan group_plan(int nkb) {
+    const int ks = stage_kblocks(nkb);
+    if (batched_stages<QG, false>(nkb, 2, 2, ks)) return {true, false, 2};
+    if (QG == 64 && batched_stages<QG, true>(nkb, 2, 2, ks)) return {true, true, 2};
+    const int narrow = batched_stages<QG, false>(nkb, 2, 1, ks), wide = batched_stages<QG, true>(nkb, 2, 1, ks);
+    if (narrow * ks >= 6 || (narrow && narrow >= wide)) return {true, false, 1};
+    if (wide && QG >= 64) return {true, true, 1};
+    return {narrow > 0, false, 1};
+}
+constexpr GroupPlan group_plan(int nkb, int qg) {
+    return qg == 128 ? group_plan<128>(nkb) : qg == 64 ? group_plan<64>(nkb) : group_plan<32>(nkb);
 }
 
 // Accumulator column of a group's i-th query (a bijection on [0, QG)).
@@ -854,10 +882,11 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
     const int nkb = p.nkb;                  // list (A) k-blocks per row
     const int nkbq = nkb >> p.ksplit;       // query (B) k-blocks per row
     const int nsl = p.nslot;                                         // item slots
-    unsigned char* sB = base;                                        // nsl slots x nkb x BKB (queries)
+    const int nbuf = p.nbuf;                                         // query operand buffers
+    unsigned char* sB = base;                                        // nbuf x nkbq x BKB (queries)
     const int ns = p.ns;                                             // stages in the ring
     const int ks = stage_kblocks(nkb);                               // list k-blocks per stage
-    unsigned char* sA = sB + static_cast<size_t>(nsl) * nkbq * BKB;  // ns x ks x 16 KiB (list k-blocks)
+    unsigned char* sA = sB + static_cast<size_t>(nbuf) * nkbq * BKB;  // ns x ks x 16 KiB (list k-blocks)
     Slot* slot = reinterpret_cast<Slot*>(sA + static_cast<size_t>(ns * ks) * KB_BYTES);  // [nsl], 1024-aligned
     static_assert(offsetof(Slot, xn) % 16 == 0 && offsetof(Slot, sc) % 16 == 0 && sizeof(Slot) % 16 == 0,
                   "ItemSlot alignment");
@@ -865,7 +894,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
     uint64_t* s_ck = reinterpret_cast<uint64_t*>(s_cq + N_EPI * CB);  // [N_EPI][CB]
     float* s_ip = reinterpret_cast<float*>(s_ck + N_EPI * CB);       // [N_EPI][32 lanes][CC] candidate chunks
 
-    __shared__ uint64_t full[NS_MAX], empty[NS_MAX], accf[2], acce[2], sfull[SLOT_MAX], sfree[SLOT_MAX];
+    __shared__ uint64_t full[NS_MAX], empty[NS_MAX], accf[2], acce[2], sfull[SLOT_MAX], sfree[SLOT_MAX],
+        smeta[SLOT_MAX], bfree[SLOT_MAX];
     __shared__ uint32_t tbase;
     __shared__ int s_abort;
     __shared__ long long s_g[SLOT_MAX];
@@ -886,6 +916,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
         for (int i = 0; i < nsl; ++i) {
             mbar_init(&sfull[i], 32 * N_GATHER);
             mbar_init(&sfree[i], 1 + N_EPI);  // MMA commit + every epilogue warp
+            mbar_init(&smeta[i], 32 * N_GATHER);
+            mbar_init(&bfree[i], 1);
         }
         s_abort = 0;
         fence_mbar_init();
@@ -911,6 +943,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             const long long g = s_g[b];
             if (g >= total_items || *vabort) {
                 if (gt == 0) S.ntiles = -1;
+                mbar_arrive_cta(&smeta[b]);
                 mbar_arrive_cta(&sfull[b]);
                 break;
             }
@@ -951,6 +984,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                 S.row0 = row0;
                 S.ntiles = (nrows + TM - 1) / TM;
             }
+            mbar_arrive_cta(&smeta[b]);  // the producer may start on the item's tiles
             // A dense item: the list's first slice records each query's
             // entry count (the list size).
             if (sz <= p.dense_max && rsl == 0)
@@ -991,24 +1025,24 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             }
             // The group's queries into the swizzled B operand (row = column
             // of the accumulator): every 16-byte chunk is its own
-            // asynchronous copy, all in flight at once; empty query slots are
-            // zero-filled.
-            unsigned char* dst = sB + static_cast<size_t>(b) * nkbq * BKB;
+            // asynchronous copy, eight lanes to a 128-byte row so that a
+            // warp reads whole rows, all in flight at once; empty query slots
+            // are zero-filled.
+            named_sync(1, 32 * N_GATHER);  // S.qid
+            const int bb = static_cast<int>(it % nbuf);
+            if (!wait_or_abort(&bfree[bb], ((it / nbuf) & 1u) ^ 1u, p.err, vabort)) break;
+            unsigned char* dst = sB + static_cast<size_t>(bb) * nkbq * BKB;
             const size_t qstride = static_cast<size_t>(nkbq) * 128;
-            for (int i = gt; i < QG; i += 32 * N_GATHER) {
-                const int col = group_col<QG>(i);
-                if (i < nqv) {
-                    const unsigned char* src = p.qb + static_cast<size_t>(grp[i]) * qstride;
-                    for (int kb = 0; kb < nkbq; ++kb)
-#pragma unroll
-                        for (int c = 0; c < 8; ++c)
-                            cp_async16(dst + kb * BKB + col * 128 + (((c ^ (col & 7)) & 7) << 4),
-                                       src + kb * 128 + c * 16);
+            const int c = gt & 7;
+            for (int col = gt >> 3; col < QG; col += 4 * N_GATHER) {
+                const int qid = S.qid[col];
+                unsigned char* dc = dst + col * 128 + ((c ^ (col & 7)) << 4);
+                if (qid >= 0) {
+                    const unsigned char* src = p.qb + static_cast<size_t>(qid) * qstride + c * 16;
+#pragma unroll 4
+                    for (int kb = 0; kb < nkbq; ++kb) cp_async16(dc + kb * BKB, src + kb * 128);
                 } else {
-                    for (int kb = 0; kb < nkbq; ++kb)
-#pragma unroll
-                        for (int c = 0; c < 8; ++c)
-                            *reinterpret_cast<uint4*>(dst + kb * BKB + col * 128 + (c << 4)) = make_uint4(0, 0, 0, 0);
+                    for (int kb = 0; kb < nkbq; ++kb) *reinterpret_cast<uint4*>(dc + kb * BKB) = make_uint4(0, 0, 0, 0);
                 }
             }
             cp_async_wait_all();
@@ -1023,7 +1057,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
         bool ok = true;
         for (uint32_t it = 0; ok; ++it) {
             const int b = static_cast<int>(it % nsl);
-            if (!__all_sync(FULL, wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort))) break;
+            if (!__all_sync(FULL, wait_or_abort(&smeta[b], (it / nsl) & 1u, p.err, vabort))) break;
             const int ntiles = slot[b].ntiles;
             if (ntiles < 0) break;
             const int64_t tile0 = slot[b].row0 / TM;
@@ -1064,7 +1098,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             if (!__all_sync(FULL, wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort))) break;
             const int ntiles = slot[b].ntiles;
             if (ntiles < 0) break;
-            const uint64_t b0 = bdesc + static_cast<uint32_t>(b * nkbq) * (BKB >> 4);
+            const int bb = static_cast<int>(it % nbuf);
+            const uint64_t b0 = bdesc + static_cast<uint32_t>(bb * nkbq) * (BKB >> 4);
             for (int t = 0; t < ntiles && ok; ++t, ++tile_it) {
                 const int buf = tile_it & 1;
                 ok = __all_sync(FULL, wait_or_abort(&acce[buf], ((tile_it >> 1) & 1u) ^ 1u, p.err, vabort));
@@ -1093,7 +1128,10 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                         tc::mma_commit(&empty[ms]);
                         if (last == nkb) {
                             tc::mma_commit(&accf[buf]);
-                            if (t == ntiles - 1) tc::mma_commit(&sfree[b]);  // the slot's queries are no longer read
+                            if (t == ntiles - 1) {
+                                tc::mma_commit(&bfree[bb]);  // the queries are no longer read
+                                tc::mma_commit(&sfree[b]);
+                            }
                         }
                     }
                     __syncwarp();
@@ -2855,38 +2893,32 @@ cudaError_t launch_invert_probes(const int64_t* probes, int nq, int nprobe, int 
     return cudaGetLastError();
 }
 
-// Whether groups of qg (64) take the WIDE shape at nkb k-blocks.
-static bool batched_wide(int nkb, int qg) { return qg == 64 && !batched_stages<64, false>(nkb); }
-
 int batched_group_size(int nkb) {
     if (nkb > NKB_MAX) return 0;
-    if (batched_stages<128, false>(nkb)) return 128;
-    if (batched_stages<64, false>(nkb) || batched_stages<64, true>(nkb)) return 64;
-    if (batched_stages<32, false>(nkb)) return 32;
+    for (int qg = 128; qg >= 32; qg /= 2)
+        if (group_plan(nkb, qg).ok) return qg;
     return 0;
 }
 
 int batched_row_slice(int nkb, int qg) {
-    return batched_wide(nkb, qg) ? Shape<64, true>::RS_MAX : Shape<64, false>::RS_MAX;
+    return group_plan(nkb, qg).wide ? Shape<64, true>::RS_MAX : Shape<64, false>::RS_MAX;
 }
 
 template <int QG, Operand OP, bool WIDE>
 static cudaError_t launch_batched_t(BatchedParams p, int nsm, cudaStream_t s) {
     const int nkbq = p.nkb >> p.ksplit;  // a split image has two list k-blocks per query k-block
     const int ks = stage_kblocks(p.nkb);
-    auto stages = [&](int nslot) {
-        for (int ns = NS_MAX; ns * ks >= RING_MIN; --ns)
-            if (batched_smem<QG, WIDE>(nkbq, ns * ks, nslot) <= BATCHED_SMEM_CAP) return ns;
-        return 0;
-    };
-    p.nslot = SLOT_MAX;
-    p.ns = stages(SLOT_MAX);
-    if (p.ns * ks < RING_SLOT3) {
+    p.nbuf = group_plan<QG>(nkbq).nbuf;
+    p.nslot = p.nbuf == 1 ? 2 : SLOT_MAX;
+    p.ns = batched_stages<QG, WIDE>(nkbq, p.nslot, p.nbuf == 1 ? 1 : SLOT_MAX, ks);
+    if (p.nbuf == 2 && p.ns * ks < RING_SLOT3) {
         p.nslot = 2;
-        p.ns = stages(2);
+        p.ns = batched_stages<QG, WIDE>(nkbq, 2, 2, ks);
+    } else if (p.nbuf == 2) {
+        p.nbuf = SLOT_MAX;
     }
     if (p.ns == 0 || p.rs > Shape<QG, WIDE>::RS_MAX) return cudaErrorInvalidValue;
-    const size_t smem = batched_smem<QG, WIDE>(nkbq, p.ns * ks, p.nslot);
+    const size_t smem = batched_smem<QG, WIDE>(nkbq, p.ns * ks, p.nslot, p.nbuf);
     auto kern = batched_scan_kernel<QG, OP, WIDE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
@@ -2936,11 +2968,13 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
         return cudaErrorInvalidValue;
     };
     constexpr std::false_type narrow;
+    constexpr std::true_type wide;
+    constexpr std::integral_constant<int, 128> g128;
+    constexpr std::integral_constant<int, 64> g64;
+    const GroupPlan plan = group_plan(b.nkb, b.qg);
     switch (b.qg) {
-        case 128: return run(std::integral_constant<int, 128>(), narrow);
-        case 64:
-            return batched_wide(b.nkb, 64) ? run(std::integral_constant<int, 64>(), std::true_type())
-                                           : run(std::integral_constant<int, 64>(), narrow);
+        case 128: return plan.wide ? run(g128, wide) : run(g128, narrow);
+        case 64: return plan.wide ? run(g64, wide) : run(g64, narrow);
         case 32: return run(std::integral_constant<int, 32>(), narrow);
         default: return cudaErrorInvalidValue;
     }
