@@ -1908,6 +1908,10 @@ __host__ __device__ inline size_t refine_warp_bytes(int d) {
 // dimension halves pipelined against the sums).  Up to 128 candidates the scored keys stay in
 // registers (lane i, round r: candidate 32 r + i); more are written back to
 // keys and merged through shared-memory-free warp sorts.
+// A coarse score in key order; what is not a number last, whatever its sign
+// (coarse_scores_kernel's arithmetic leaves it without one).
+__device__ inline uint32_t score_key(float score) { return score == score ? f2o(score) : 0xffffffffu; }
+
 template <int METRIC>
 __device__ inline float coarse_dot(const float* qs, const float* row, int j0, int j1, float acc) {
 #pragma unroll 4
@@ -2017,7 +2021,7 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
             if (!ok) break;
             if (lane < nr) {
                 const float score = METRIC == METRIC_L2 ? acc : -acc;
-                const uint64_t key = (static_cast<uint64_t>(f2o(score)) << 32) | static_cast<uint32_t>(cid);
+                const uint64_t key = (static_cast<uint64_t>(score_key(score)) << 32) | static_cast<uint32_t>(cid);
                 if (in_regs) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
@@ -2060,7 +2064,7 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
             }
             if (lane < nr) {
                 const float score = METRIC == METRIC_L2 ? acc : -acc;
-                const uint64_t key = (static_cast<uint64_t>(f2o(score)) << 32) | static_cast<uint32_t>(cidr);
+                const uint64_t key = (static_cast<uint64_t>(score_key(score)) << 32) | static_cast<uint32_t>(cidr);
                 if (in_regs) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
@@ -2120,6 +2124,19 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
     }
 }
 
+// The ordered value below which an upper bound places its centroid among the m
+// best of nlist: edge is at most the m-th smallest upper bound (ordered bits),
+// ebmax the lane's largest error bound.  0 (none) where a bound is no finite
+// number.
+__device__ inline uint32_t refine_definite_below(uint32_t edge, float ebmax, int m, int nlist) {
+    if (m >= nlist) return 0xffffffffu;
+    uint32_t b = __float_as_uint(ebmax);  // >= 0, or not a number (above every number's bits)
+    b = __reduce_max_sync(FULL, b & 0x7fffffffu);
+    const float h = o2f(edge), eb = __uint_as_float(b);
+    const float L = h - 2.0f * eb - 9.5367431640625e-7f * (fabsf(h) + eb);  // 2^-20
+    return fabsf(L) < INFINITY ? f2o(L) : 0u;
+}
+
 template <int METRIC, int PER>
 __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restrict__ cand, int nq, int nlist,
                                                             const float* __restrict__ q,
@@ -2127,7 +2144,8 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
                                                             const float* __restrict__ cxn,
                                                             const float2* __restrict__ caux,
                                                             const float4* __restrict__ qaux, float cK, float cN,
-                                                            int d, int m, int64_t* __restrict__ out_idx,
+                                                            int d, int m, int ordered,
+                                                            int64_t* __restrict__ out_idx,
                                                             float* __restrict__ out_score, int* err) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2153,12 +2171,13 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
     const bool vec = nlist == PER * 32;
     auto entry = [&](int r) { return vec ? 4 * ((r >> 2) * 32 + lane) + (r & 3) : r * 32 + lane; };
     uint32_t hi[PER];
-    float lo[PER];
+    float lo[PER], ebmax = 0.0f;
     auto bound = [&](int r, float sc, float ax, float ay, float xn) {
         const float eb = fmaf(ax, ec.aq, fmaf(ay, ec.bq, err_row_const(xn, l2, cN) + ec.cq));
         // What is not a finite number bounds nothing from above.
         hi[r] = fabsf(sc + eb) < INFINITY ? f2o(sc + eb) : 0xffffffffu;
         lo[r] = sc - eb;
+        ebmax = !(fabsf(sc) + eb < INFINITY) ? NAN : eb > ebmax ? eb : ebmax;  // (NaN stays)
     };
     if (vec) {
 #pragma unroll
@@ -2182,8 +2201,46 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
             if (e < nlist) bound(r, cs[e], caux[e].x, caux[e].y, cxn[e]);
         }
     }
-    const float U = o2f(warp_select_bound<PER>(hi, nlist, m, hist, lane));
+    uint32_t edge;
+    const float U = o2f(warp_select_bound<PER>(hi, nlist, m, hist, lane, &edge));
     __syncwarp();  // every pair has been read, and the histogram too
+    // Unordered: at most m centroids have a lower bound at or below L (the
+    // m-th smallest upper bound less twice the largest error bound, with room
+    // for the rounding of these sums), so one whose upper bound is below it is
+    // among the m best without its exact score; only the rest of the kept set
+    // is scored.  The (up to) three with the smallest bounds come first, for
+    // the first pass and the warm-up.
+    int nd = 0;
+    uint32_t L = 0u;  // below it: in the set
+    if (!ordered) {
+        L = refine_definite_below(edge, ebmax, m, nlist);
+        uint32_t prev = 0;
+        int top[3] = {-1, -1, -1};
+        int64_t* out = out_idx + static_cast<int64_t>(qi) * m;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            uint32_t best = 0xffffffffu;
+#pragma unroll
+            for (int r = 0; r < PER; ++r) best = min(best, hi[r] > prev ? hi[r] : 0xffffffffu);
+            prev = __reduce_min_sync(FULL, best);
+            if (prev >= L) break;
+            int at = 0;
+#pragma unroll
+            for (int r = 0; r < PER; ++r)
+                if (hi[r] == prev) at = entry(r);
+            top[i] = __shfl_sync(FULL, at, __ffs(__ballot_sync(FULL, best == prev)) - 1);
+            if (lane == 0) out[nd] = top[i];
+            ++nd;
+        }
+#pragma unroll
+        for (int r = 0; r < PER; ++r) {
+            const int e = entry(r);
+            const bool in = hi[r] < L && e != top[0] && e != top[1] && e != top[2];
+            const unsigned bal = __ballot_sync(FULL, in);
+            if (in) out[nd + __popc(bal & ((1u << lane) - 1u))] = e;
+            nd += __popc(bal);
+        }
+    }
     // Centroids that can be among the m best: the first 256 ids in the
     // histogram's space, the rest in keys (and there all of them when there
     // are more than 256).
@@ -2191,7 +2248,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
 #pragma unroll
     for (int r = 0; r < PER; ++r) {
         const int e = entry(r);
-        const bool keep = e < nlist && !(lo[r] > U);  // (what is not a number has no bound: kept)
+        const bool keep = e < nlist && hi[r] >= L && !(lo[r] > U);  // (what is not a number has no bound: kept)
         const unsigned bal = __ballot_sync(FULL, keep);
         if (keep) {
             const int at = c + __popc(bal & ((1u << lane) - 1u));
@@ -2206,8 +2263,9 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
     if (c > 256)
         for (int e = lane; e < 256; e += 32) keys[e] = static_cast<uint64_t>(hist[e]);
     __syncwarp();
-    coarse_exact_best<METRIC>(keys, hist, reinterpret_cast<uint64_t*>(hist), bars, c, qs, stage, pitch, cent, d, m,
-                              qi, out_idx, out_score, err, lane);
+    coarse_exact_best<METRIC>(keys, hist, reinterpret_cast<uint64_t*>(hist), bars, c, qs, stage, pitch, cent, d,
+                              m - nd, 0, out_idx + static_cast<int64_t>(qi) * m + nd,
+                              out_score ? out_score + static_cast<int64_t>(qi) * m : nullptr, err, lane);
 }
 
 // The coarse step for more than 2048 lists, in two tensor-core launches.
@@ -2729,7 +2787,7 @@ size_t coarse_refine_smem(int nlist, int d, int warps) {
 
 cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q, const float* cent,
                                  const float* cxn, const float2* caux, const float4* qaux, int d, int metric, int m,
-                                 int64_t* out_idx, float* out_score, int* err, cudaStream_t s) {
+                                 bool ordered, int64_t* out_idx, float* out_score, int* err, cudaStream_t s) {
     float cK, cN;
     err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
     int warps = 4;
@@ -2740,11 +2798,11 @@ cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q
     auto run = [&](auto kern) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
-        kern<<<grid, 32 * warps, smem, s>>>(cand, nq, nlist, q, cent, cxn, caux, qaux, cK, cN, d, m, out_idx,
-                                            out_score, err);
+        kern<<<grid, 32 * warps, smem, s>>>(cand, nq, nlist, q, cent, cxn, caux, qaux, cK, cN, d, m, ordered ? 1 : 0,
+                                            out_idx, out_score, err);
         return cudaGetLastError();
     };
-    if (nlist > 2048) return cudaErrorInvalidValue;
+    if (nlist > 2048 || (out_score && !ordered)) return cudaErrorInvalidValue;
     if (metric == METRIC_L2)
         return nlist <= 1024 ? run(coarse_refine_kernel<METRIC_L2, 32>) : run(coarse_refine_kernel<METRIC_L2, 64>);
     return nlist <= 1024 ? run(coarse_refine_kernel<METRIC_IP, 32>) : run(coarse_refine_kernel<METRIC_IP, 64>);

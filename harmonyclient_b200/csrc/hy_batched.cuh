@@ -146,13 +146,16 @@ cudaError_t launch_coarse_items(int nq, int nlist, int ngroups, int nslices, int
 // bytes, scores in each query's upper half) and the bounds recomputed from
 // cxn / caux (the centroid index's squared norms and {|c~|, |c - c~|}) and
 // qaux: the exact m best centroids per query and their exact coarse scores,
-// as launch_select gives them from coarse_scores (cand is overwritten).
+// as launch_select gives them from coarse_scores (cand is overwritten).  Not
+// ordered (and no out_score): the same m centroids in any order, one of the
+// nearest first; those that the bounds alone place among the m best are not
+// scored.
 // Needs m <= 256 and coarse_refine_smem(nlist, d, 1) <= 200 KiB.  A staging
 // copy that does not complete within the wait limit raises *err.
 size_t coarse_refine_smem(int nlist, int d, int warps);
 cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q, const float* cent,
                                  const float* cxn, const float2* caux, const float4* qaux, int d, int metric, int m,
-                                 int64_t* out_idx, float* out_score, int* err, cudaStream_t s);
+                                 bool ordered, int64_t* out_idx, float* out_score, int* err, cudaStream_t s);
 
 // More than 2048 centroids: thr[q] := a bound on the m-th smallest
 // score + bound among the S <= 1024 dense scores of query q (cand, nq x S

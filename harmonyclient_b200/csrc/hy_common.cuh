@@ -210,9 +210,10 @@ __device__ inline uint32_t warp_radix_select(const uint32_t (&v)[PER], int n, in
 // (found from the warp's minimum and maximum), so the passes split the values'
 // actual range; U is the upper edge of the bin that holds the k-th value,
 // within 2^(top - 15) of it in the ordered-bits order (top = the highest bit
-// in which the values differ).
+// in which the values differ).  *lower: that bin's lower edge.
 template <int PER>
-__device__ inline uint32_t warp_select_bound(const uint32_t (&v)[PER], int n, int k, int* hist, int lane) {
+__device__ inline uint32_t warp_select_bound(const uint32_t (&v)[PER], int n, int k, int* hist, int lane,
+                                             uint32_t* lower = nullptr) {
     uint32_t mn = 0xffffffffu, mx = 0u;
 #pragma unroll
     for (int r = 0; r < PER; ++r)
@@ -222,6 +223,7 @@ __device__ inline uint32_t warp_select_bound(const uint32_t (&v)[PER], int n, in
         }
     mn = __reduce_min_sync(FULL, mn);
     mx = __reduce_max_sync(FULL, mx);
+    if (lower) *lower = mn;
     if (mn == mx) return mn;
     int top = 31 - __clz(mn ^ mx);  // highest differing bit
     uint32_t mask = ~((2u << top) - 1u);
@@ -277,6 +279,7 @@ __device__ inline uint32_t warp_select_bound(const uint32_t (&v)[PER], int n, in
         top = shift - 1;
         __syncwarp();
     }
+    if (lower) *lower = prefix;
     return top >= 0 ? (prefix | ((2u << top) - 1u)) : prefix;
 }
 
