@@ -1468,9 +1468,10 @@ __device__ inline void tighten_warp_query(int qi, int cnt, const float* __restri
 // {score, bound} entries (get(e) gives entry e), with at least k entries at
 // or below it: two 8-bit radix passes below the bits all the entries'
 // ordered values share; U is the upper edge of the final bin that holds the
-// k-th value.  One warp; the entries are read on every pass.
+// k-th value (*lower: its lower edge).  One warp; the entries are read on
+// every pass.
 template <typename Get>
-__device__ inline float kth_bound_stream(Get get, int cnt, int k, int* hist, int lane) {
+__device__ inline float kth_bound_stream(Get get, int cnt, int k, int* hist, int lane, uint32_t* lower = nullptr) {
     uint32_t mn = 0xffffffffu, mx = 0u;
 #pragma unroll 8
     for (int e = lane; e < cnt; e += 32) {
@@ -1539,6 +1540,9 @@ __device__ inline float kth_bound_stream(Get get, int cnt, int k, int* hist, int
             __syncwarp();
         }
         ub = top >= 0 ? (prefix | ((2u << top) - 1u)) : prefix;
+        if (lower) *lower = prefix;
+    } else if (lower) {
+        *lower = mn;
     }
     return o2f(ub);
 }
@@ -2124,17 +2128,22 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
     }
 }
 
+// Query qi's own m (see launch_coarse_refine).
+__device__ inline int refine_count(int m, const int32_t* __restrict__ counts, int qi) {
+    return counts ? max(1, min(m, counts[qi])) : m;
+}
+
 // The ordered value below which an upper bound places its centroid among the m
 // best of nlist: edge is at most the m-th smallest upper bound (ordered bits),
-// ebmax the lane's largest error bound.  0 (none) where a bound is no finite
-// number.
-__device__ inline uint32_t refine_definite_below(uint32_t edge, float ebmax, int m, int nlist) {
+// ebmax and scmax the bits of the lane's largest error bound and |score|.  0
+// (none) where one of them is no finite number.
+__device__ inline uint32_t refine_definite_below(uint32_t edge, uint32_t ebmax, uint32_t scmax, int m, int nlist) {
     if (m >= nlist) return 0xffffffffu;
-    uint32_t b = __float_as_uint(ebmax);  // >= 0, or not a number (above every number's bits)
-    b = __reduce_max_sync(FULL, b & 0x7fffffffu);
-    const float h = o2f(edge), eb = __uint_as_float(b);
+    ebmax = __reduce_max_sync(FULL, ebmax);
+    scmax = __reduce_max_sync(FULL, scmax);
+    const float h = o2f(edge), eb = __uint_as_float(ebmax);
     const float L = h - 2.0f * eb - 9.5367431640625e-7f * (fabsf(h) + eb);  // 2^-20
-    return fabsf(L) < INFINITY ? f2o(L) : 0u;
+    return max(ebmax, scmax) < 0x7f800000u && fabsf(L) < INFINITY ? f2o(L) : 0u;
 }
 
 template <int METRIC, int PER>
@@ -2145,6 +2154,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
                                                             const float2* __restrict__ caux,
                                                             const float4* __restrict__ qaux, float cK, float cN,
                                                             int d, int m, int ordered,
+                                                            const int32_t* __restrict__ counts,
                                                             int64_t* __restrict__ out_idx,
                                                             float* __restrict__ out_score, int* err) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -2171,13 +2181,15 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
     const bool vec = nlist == PER * 32;
     auto entry = [&](int r) { return vec ? 4 * ((r >> 2) * 32 + lane) + (r & 3) : r * 32 + lane; };
     uint32_t hi[PER];
-    float lo[PER], ebmax = 0.0f;
+    float lo[PER];
+    uint32_t ebmax = 0u, scmax = 0u;
     auto bound = [&](int r, float sc, float ax, float ay, float xn) {
         const float eb = fmaf(ax, ec.aq, fmaf(ay, ec.bq, err_row_const(xn, l2, cN) + ec.cq));
         // What is not a finite number bounds nothing from above.
         hi[r] = fabsf(sc + eb) < INFINITY ? f2o(sc + eb) : 0xffffffffu;
         lo[r] = sc - eb;
-        ebmax = !(fabsf(sc) + eb < INFINITY) ? NAN : eb > ebmax ? eb : ebmax;  // (NaN stays)
+        ebmax = max(ebmax, __float_as_uint(eb));  // (what is not a number is above every number)
+        scmax = max(scmax, __float_as_uint(sc) & 0x7fffffffu);
     };
     if (vec) {
 #pragma unroll
@@ -2201,8 +2213,9 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
             if (e < nlist) bound(r, cs[e], caux[e].x, caux[e].y, cxn[e]);
         }
     }
+    const int mq = refine_count(m, counts, qi);
     uint32_t edge;
-    const float U = o2f(warp_select_bound<PER>(hi, nlist, m, hist, lane, &edge));
+    const float U = o2f(warp_select_bound<PER>(hi, nlist, mq, hist, lane, &edge));
     __syncwarp();  // every pair has been read, and the histogram too
     // Unordered: at most m centroids have a lower bound at or below L (the
     // m-th smallest upper bound less twice the largest error bound, with room
@@ -2213,7 +2226,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
     int nd = 0;
     uint32_t L = 0u;  // below it: in the set
     if (!ordered) {
-        L = refine_definite_below(edge, ebmax, m, nlist);
+        L = refine_definite_below(edge, ebmax, scmax, mq, nlist);
         uint32_t prev = 0;
         int top[3] = {-1, -1, -1};
         int64_t* out = out_idx + static_cast<int64_t>(qi) * m;
@@ -2264,7 +2277,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
         for (int e = lane; e < 256; e += 32) keys[e] = static_cast<uint64_t>(hist[e]);
     __syncwarp();
     coarse_exact_best<METRIC>(keys, hist, reinterpret_cast<uint64_t*>(hist), bars, c, qs, stage, pitch, cent, d,
-                              m - nd, 0, out_idx + static_cast<int64_t>(qi) * m + nd,
+                              mq - nd, 0, out_idx + static_cast<int64_t>(qi) * m + nd,
                               out_score ? out_score + static_cast<int64_t>(qi) * m : nullptr, err, lane);
 }
 
@@ -2279,7 +2292,8 @@ __global__ void __launch_bounds__(256) coarse_thr_kernel(const float2* __restric
                                                          const float* __restrict__ cxn,
                                                          const float2* __restrict__ caux,
                                                          const float4* __restrict__ qaux, int metric, float cK,
-                                                         float cN, float* __restrict__ thr) {
+                                                         float cN, const int32_t* __restrict__ counts,
+                                                         float* __restrict__ thr) {
     __shared__ int hist[8][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qi = blockIdx.x * 8 + warp;
@@ -2300,7 +2314,7 @@ __global__ void __launch_bounds__(256) coarse_thr_kernel(const float2* __restric
             hv[r] = f2o(cs[e] + eb);
         }
     }
-    const float U = o2f(warp_select_bound<32>(hv, S, m, hist[warp], lane));
+    const float U = o2f(warp_select_bound<32>(hv, S, refine_count(m, counts, qi), hist[warp], lane));
     if (lane == 0) thr[qi] = U;
 }
 
@@ -2317,6 +2331,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_keys_kernel(uint64_t* __
                                                                  const float* __restrict__ cxn,
                                                                  const float2* __restrict__ caux,
                                                                  const float4* __restrict__ qaux, int d, int m,
+                                                                 int ordered, const int32_t* __restrict__ counts,
                                                                  float cK, float cN, int64_t* __restrict__ out_idx,
                                                                  float* __restrict__ out_score, int* err) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -2342,27 +2357,65 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_keys_kernel(uint64_t* __
         const float eb = fmaf(xa.x, ec.aq, fmaf(xa.y, ec.bq, err_row_const(cxn[row], l2, cN) + ec.cq));
         return make_float2(o2f(static_cast<uint32_t>(kk >> 32)), eb);
     };
-    const float U = n >= m ? kth_bound_stream(get, n, m, hist, lane) : INFINITY;
-    // In place: the kept centroids' ids to the front (every element of a
-    // round is read before any of that round's writes).
+    const int mq = refine_count(m, counts, qi);
+    uint32_t edge = 0u;
+    const float U = n >= mq ? kth_bound_stream(get, n, mq, hist, lane, &edge) : INFINITY;
+    // Unordered: as in coarse_refine_kernel (a centroid that was not emitted
+    // has its lower bound above the emission's threshold, which is no less
+    // than the m-th smallest upper bound).  The first three come from the
+    // lanes' smallest.
+    int nd = 0;
+    uint32_t L = 0u;
+    uint32_t top[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
+    int64_t* out = out_idx + static_cast<int64_t>(qi) * m;
+    if (!ordered && n >= mq) {
+        uint32_t ebmax = 0u, scmax = 0u;
+        uint64_t best = KEY_MAX;
+#pragma unroll 4
+        for (int e = lane; e < n; e += 32) {
+            const float2 v = get(e);
+            ebmax = max(ebmax, __float_as_uint(v.y));
+            scmax = max(scmax, __float_as_uint(v.x) & 0x7fffffffu);
+            best = min(best, (static_cast<uint64_t>(f2o(v.x + v.y)) << 32) | (keys[e] & 0xffffffffu));
+        }
+        L = refine_definite_below(edge, ebmax, scmax, mq, stride);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint32_t h = __reduce_min_sync(FULL, static_cast<uint32_t>(best >> 32));
+            if (h >= L) break;
+            const int src = __ffs(__ballot_sync(FULL, static_cast<uint32_t>(best >> 32) == h)) - 1;
+            top[i] = __shfl_sync(FULL, static_cast<uint32_t>(best & 0xffffffffu), src);
+            if (lane == src) best = KEY_MAX;
+            if (lane == 0) out[nd] = top[i];
+            ++nd;
+        }
+    }
+    // In place: the ids of the kept centroids that need their exact score to
+    // the front (every element of a round is read before any of that round's
+    // writes).
     int c = 0;
     for (int b0 = 0; b0 < n; b0 += 32) {
         const int e = b0 + lane;
-        bool keep = false;
-        uint64_t id = 0;
+        bool keep = false, in = false;
+        uint32_t id = 0;
         if (e < n) {
             const float2 v = get(e);
-            keep = v.x - v.y <= U;
-            id = keys[e] & 0xffffffffu;
+            id = static_cast<uint32_t>(keys[e] & 0xffffffffu);
+            const bool sure = L != 0u && f2o(v.x + v.y) < L;
+            in = sure && id != top[0] && id != top[1] && id != top[2];
+            keep = !sure && v.x - v.y <= U;
         }
-        const unsigned bal = __ballot_sync(FULL, keep);
+        const unsigned bal = __ballot_sync(FULL, keep), bin = __ballot_sync(FULL, in);
         __syncwarp();
         if (keep) keys[c + __popc(bal & ((1u << lane) - 1u))] = id;
+        if (in) out[nd + __popc(bin & ((1u << lane) - 1u))] = id;
         c += __popc(bal);
+        nd += __popc(bin);
     }
     __syncwarp();
     coarse_exact_best<METRIC>(keys, nullptr, reinterpret_cast<uint64_t*>(hist), bars, c, qs, stage, pitch, cent, d,
-                              m, qi, out_idx, out_score, err, lane);
+                              mq - nd, 0, out + nd, out_score ? out_score + static_cast<int64_t>(qi) * m : nullptr,
+                              err, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -2787,7 +2840,8 @@ size_t coarse_refine_smem(int nlist, int d, int warps) {
 
 cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q, const float* cent,
                                  const float* cxn, const float2* caux, const float4* qaux, int d, int metric, int m,
-                                 bool ordered, int64_t* out_idx, float* out_score, int* err, cudaStream_t s) {
+                                 bool ordered, const int32_t* counts, int64_t* out_idx, float* out_score, int* err,
+                                 cudaStream_t s) {
     float cK, cN;
     err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
     int warps = 4;
@@ -2799,40 +2853,41 @@ cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
         kern<<<grid, 32 * warps, smem, s>>>(cand, nq, nlist, q, cent, cxn, caux, qaux, cK, cN, d, m, ordered ? 1 : 0,
-                                            out_idx, out_score, err);
+                                            counts, out_idx, out_score, err);
         return cudaGetLastError();
     };
-    if (nlist > 2048 || (out_score && !ordered)) return cudaErrorInvalidValue;
+    if (nlist > 2048 || (out_score && (!ordered || counts))) return cudaErrorInvalidValue;
     if (metric == METRIC_L2)
         return nlist <= 1024 ? run(coarse_refine_kernel<METRIC_L2, 32>) : run(coarse_refine_kernel<METRIC_L2, 64>);
     return nlist <= 1024 ? run(coarse_refine_kernel<METRIC_IP, 32>) : run(coarse_refine_kernel<METRIC_IP, 64>);
 }
 
 cudaError_t launch_coarse_thr(const float2* cand, int nq, int S, int m, const float* cxn, const float2* caux,
-                              const float4* qaux, int d, int metric, float* thr, cudaStream_t s) {
+                              const float4* qaux, int d, int metric, const int32_t* counts, float* thr,
+                              cudaStream_t s) {
     if (S > 1024 || m > S) return cudaErrorInvalidValue;
     float cK, cN;
     err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
-    coarse_thr_kernel<<<(nq + 7) / 8, 256, 0, s>>>(cand, nq, S, m, cxn, caux, qaux, metric, cK, cN, thr);
+    coarse_thr_kernel<<<(nq + 7) / 8, 256, 0, s>>>(cand, nq, S, m, cxn, caux, qaux, metric, cK, cN, counts, thr);
     return cudaGetLastError();
 }
 
 cudaError_t launch_coarse_refine_keys(uint64_t* cand, const int32_t* ccnt, int nq, int stride, const float* q,
                                       const float* cent, const float* cxn, const float2* caux, const float4* qaux,
-                                      int d, int metric, int m, int64_t* out_idx, float* out_score, int* err,
-                                      cudaStream_t s) {
+                                      int d, int metric, int m, bool ordered, const int32_t* counts,
+                                      int64_t* out_idx, float* out_score, int* err, cudaStream_t s) {
     int warps = 4;
     while (warps > 1 && coarse_refine_smem(0, d, warps) > 200 * 1024) warps >>= 1;
     const size_t smem = coarse_refine_smem(0, d, warps);
-    if (smem > 200 * 1024 || m > 256) return cudaErrorInvalidValue;
+    if (smem > 200 * 1024 || m > 256 || (out_score && (!ordered || counts))) return cudaErrorInvalidValue;
     float cK, cN;
     err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
     const dim3 grid((nq + warps - 1) / warps);
     auto run = [&](auto kern) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
-        kern<<<grid, 32 * warps, smem, s>>>(cand, ccnt, nq, stride, q, cent, cxn, caux, qaux, d, m, cK, cN, out_idx,
-                                            out_score, err);
+        kern<<<grid, 32 * warps, smem, s>>>(cand, ccnt, nq, stride, q, cent, cxn, caux, qaux, d, m, ordered ? 1 : 0, counts,
+                                            cK, cN, out_idx, out_score, err);
         return cudaGetLastError();
     };
     return metric == METRIC_L2 ? run(coarse_refine_keys_kernel<METRIC_L2>) : run(coarse_refine_keys_kernel<METRIC_IP>);

@@ -149,13 +149,15 @@ cudaError_t launch_coarse_items(int nq, int nlist, int ngroups, int nslices, int
 // as launch_select gives them from coarse_scores (cand is overwritten).  Not
 // ordered (and no out_score): the same m centroids in any order, one of the
 // nearest first; those that the bounds alone place among the m best are not
-// scored.
+// scored.  counts (or null; no out_score): query q's own m, counts[q] clamped
+// to [1, m]; its places past that are left as they are.
 // Needs m <= 256 and coarse_refine_smem(nlist, d, 1) <= 200 KiB.  A staging
 // copy that does not complete within the wait limit raises *err.
 size_t coarse_refine_smem(int nlist, int d, int warps);
 cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q, const float* cent,
                                  const float* cxn, const float2* caux, const float4* qaux, int d, int metric, int m,
-                                 bool ordered, int64_t* out_idx, float* out_score, int* err, cudaStream_t s);
+                                 bool ordered, const int32_t* counts, int64_t* out_idx, float* out_score, int* err,
+                                 cudaStream_t s);
 
 // More than 2048 centroids: thr[q] := a bound on the m-th smallest
 // score + bound among the S <= 1024 dense scores of query q (cand, nq x S
@@ -165,11 +167,12 @@ cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q
 // overwritten).  cxn / caux: the centroid index's squared norms and
 // {|c~|, |c - c~|}.
 cudaError_t launch_coarse_thr(const float2* cand, int nq, int S, int m, const float* cxn, const float2* caux,
-                              const float4* qaux, int d, int metric, float* thr, cudaStream_t s);
+                              const float4* qaux, int d, int metric, const int32_t* counts, float* thr,
+                              cudaStream_t s);
 cudaError_t launch_coarse_refine_keys(uint64_t* cand, const int32_t* ccnt, int nq, int stride, const float* q,
                                       const float* cent, const float* cxn, const float2* caux, const float4* qaux,
-                                      int d, int metric, int m, int64_t* out_idx, float* out_score, int* err,
-                                      cudaStream_t s);
+                                      int d, int metric, int m, bool ordered, const int32_t* counts, int64_t* out_idx,
+                                      float* out_score, int* err, cudaStream_t s);
 
 // Largest list the batched search's first pass scans densely (the candidate
 // buffer's size caps it further).

@@ -1044,7 +1044,7 @@ bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
 // over the centroid index, then the exact m best per query.  work: two
 // counters at zero.
 int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const float4* qn, size_t nprobe,
-                  bool ordered, int64_t* probes, float* pscore, unsigned int* work, cudaStream_t s) {
+                  bool ordered, const int32_t* counts, int64_t* probes, float* pscore, unsigned int* work, cudaStream_t s) {
     HY_RET(ensure_centroid_image(h, s));
     const int nlist = (int)h->nlist;
     const int nkb = (int)(h->d + 63) / 64;
@@ -1107,7 +1107,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
         HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
         HY_CUDA(hy::launch_coarse_refine(reinterpret_cast<float2*>(h->c_cand.p), (int)m, nlist, qq,
                                          h->cent.as<float>(), h->c_norm.as<float>(), h->c_aux.as<float2>(),
-                                         qn, (int)h->d, h->metric, (int)nprobe, ordered, probes, pscore,
+                                         qn, (int)h->d, h->metric, (int)nprobe, ordered, counts, probes, pscore,
                                          h->w_err.as<int>(), s));
         h->launches += 3;
         return HY_OK;
@@ -1127,7 +1127,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
     HY_CUDA(hy::launch_coarse_thr(reinterpret_cast<const float2*>(h->c_cand.p), (int)m, S, (int)nprobe,
                                   h->c_norm.as<float>(), h->c_aux.as<float2>(), qn, (int)h->d,
-                                  h->metric, h->b_thr.as<float>(), s));
+                                  h->metric, counts, h->b_thr.as<float>(), s));
     w.item_cap = (int64_t)ngroups * ns_full;
     HY_CUDA(hy::launch_coarse_items((int)m, nlist, ngroups, ns_full, h->c_off.as<int64_t>(), h->c_size.as<int32_t>(),
                                     w, s));
@@ -1139,7 +1139,8 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     HY_CUDA(hy::launch_batched_scan(b, w, h->w_err.as<int>(), s));
     HY_CUDA(hy::launch_coarse_refine_keys(h->c_cand.as<uint64_t>(), w.cand_cnt, (int)m, nlist, qq, h->cent.as<float>(),
                                           h->c_norm.as<float>(), h->c_aux.as<float2>(), qn,
-                                          (int)h->d, h->metric, (int)nprobe, probes, pscore, h->w_err.as<int>(), s));
+                                          (int)h->d, h->metric, (int)nprobe, ordered, counts, probes, pscore,
+                                          h->w_err.as<int>(), s));
     h->launches += 7;
     return HY_OK;
 }
@@ -1284,9 +1285,10 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
                 cqn = h->b_cqn.as<float4>();
                 h->launches += 1;
             }
-            // Probes are a set to the search, except where a query's own
-            // nprobe or the probe model cuts the list short.
-            HY_RET(coarse_tensor(h, m, qq, cqb, cqn, nprobe, learned_on(h) || h->q_nprobe, h->w_probes.as<int64_t>(),
+            // Probes are a set to the search, except where the probe model
+            // cuts the list short.
+            HY_RET(coarse_tensor(h, m, qq, cqb, cqn, nprobe, learned_on(h), h->q_nprobe && !learned_on(h) ? h->q_nprobe + q0 : nullptr,
+                                 h->w_probes.as<int64_t>(),
                                  learned_on(h) ? h->m_pscore.as<float>() : nullptr, work + 2, s));
         } else {
             HY_CUDA(hy::launch_coarse_scores(qq, (int)m, h->cent.as<float>(), (int)nlist, (int)h->d, h->metric,
@@ -2363,7 +2365,7 @@ int hy_index_probes(hy_index* h, size_t n, const float* q, int64_t* probes) {
         if (tensor) {
             HY_CUDA(hy::launch_prep_queries(qq, (int)m, (int)h->d, h->b_qb.p, h->b_qn.as<float4>(), nullptr, s));
             HY_CUDA(cudaMemsetAsync(h->b_zero.p, 0, 2 * sizeof(unsigned int), s));
-            HY_RET(coarse_tensor(h, m, qq, h->b_qb.p, h->b_qn.as<float4>(), nprobe, true,
+            HY_RET(coarse_tensor(h, m, qq, h->b_qb.p, h->b_qn.as<float4>(), nprobe, true, nullptr,
                                  h->w_probes.as<int64_t>() + q0 * nprobe,
                                  learned_on(h) ? h->m_pscore.as<float>() : nullptr, h->b_zero.as<unsigned int>(), s));
         } else {

@@ -58,3 +58,27 @@ def test_nonfinite_values(metric, what, bad):
         probes[mode] = np.sort(idx.probes(q), axis=1)
     np.testing.assert_array_equal(probes["tensor"], probes["exact"])
     _same(idx, np.delete(q, 3, 0) if what == "query" and not np.isfinite(bad) else q)
+
+
+@pytest.mark.parametrize("d,nlist,nprobe", [(24, 40, 40), (128, 1024, 64), (48, 2049, 128), (64, 4096, 200)])
+def test_each_query_its_own_nprobe(d, nlist, nprobe):
+    """From two launches above 2048 lists; counts of 1, nprobe and past it."""
+    rng = np.random.default_rng(nlist)
+    c = rng.uniform(-1, 1, (nlist, d)).astype(np.float32)
+    c[4::9] = c[4]
+    x = (c[rng.integers(0, nlist, 9_000)] + 0.3 * rng.standard_normal((9_000, d))).astype(np.float32)
+    q = (c[rng.integers(0, nlist, 700)] + 0.4 * rng.standard_normal((700, d))).astype(np.float32)
+    idx = hb.Index(d, nlist, nprobe)
+    idx.centroid_codes = c
+    idx.add(x)
+    idx.set_form("bf16")
+    npq = rng.integers(1, nprobe + 1, 700).astype(np.int32)
+    npq[:3] = 1, nprobe, nprobe
+    out = {}
+    for mode in ("exact", "tensor"):
+        idx.set_coarse(mode)
+        out[mode] = idx.search_nprobes(q, 10, npq)
+        if mode == "tensor":
+            _same(idx, q)
+    for a, b in zip(out["exact"], out["tensor"]):
+        np.testing.assert_array_equal(a, b)
