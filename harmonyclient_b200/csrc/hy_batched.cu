@@ -51,21 +51,7 @@ constexpr int NKB_MAX = 12;  // k-blocks of a row: at most (bf16 d <= 768, e4m3 
 __host__ __device__ constexpr int stage_kblocks(int nkb) { return nkb >= 2 ? 2 : 1; }
 
 // ---------------------------------------------------------------------------
-// Conversion of the FP32 arena into the bf16 tensor-core image.
-__global__ void to_bf16_arena_kernel(ArenaLayout L, const float* __restrict__ codes, int64_t rows, int nkb,
-                                     unsigned char* __restrict__ out) {
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i >= rows * L.d) return;
-    const int64_t r = i / L.d;
-    const int j = static_cast<int>(i % L.d);
-    int b = 0;
-    while (b + 1 < L.nb && j >= L.bstart[b + 1]) ++b;
-    const float v = codes[arena_offset(L, r, b, j - L.bstart[b])];
-    const int64_t tile = r >> 7;
-    const int kb = j >> 6;
-    unsigned char* dst = out + (tile * nkb + kb) * KB_BYTES + tc::kblock_offset(static_cast<uint32_t>(r & 127), j & 63);
-    *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(v);
-}
+// The FP32 arena's rows as tensor-core images.
 
 // e4m3 code of v / scale and its decoded value times scale (saturating at
 // the largest finite e4m3 magnitude, 448).
@@ -77,40 +63,100 @@ __device__ inline float e4m3_value(unsigned char c, float scale) {
     return __half2float(__half(h)) * scale;
 }
 
-// e4m3 image of the arena: per 128-row tile, ceil(d/128) k-blocks of 128 rows
-// x 128 bytes in the same swizzled K-major layout as the bf16 image; every
-// value is coded relative to its list's scale (tscale of its tile).
-__global__ void to_f8_arena_kernel(ArenaLayout L, const float* __restrict__ codes, int64_t rows, int nkb,
-                                   const float* __restrict__ tscale, unsigned char* __restrict__ out) {
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i >= rows * L.d) return;
-    const int64_t r = i / L.d;
-    const int j = static_cast<int>(i % L.d);
+// One pass over the FP32 arena: the bf16 or e4m3 image (per 128-row tile nkb
+// k-blocks of 128 rows x 128 bytes in the MMA's swizzled K-major layout, e4m3
+// values relative to their tile's tscale, zeros past d) and per row
+// {|x~|, |x - x~|} for the error bound (x~ the row as the tensor cores see it).
+// Bound by memory: 4 bytes read and 2 (or 1) written per value.  Eight lanes
+// take a row and write a 16-byte chunk each, so a row's 128 bytes of a k-block
+// leave in one store; a chunk inside one dimension block reads 16-byte chunks
+// of the arena, one across blocks (widths that are no multiple of 4) single
+// values.  A thread per value with 2- or 1-byte stores, a clear of the image
+// and a second pass for the bound terms took 2.6 ms for bf16 1M x 128, 5.2 ms for
+// bf16 500k x 500 and 8.1 ms for e4m3 1M x 420; this 0.125, 0.43 and 1.36 ms.
+template <bool F8>
+__global__ void __launch_bounds__(256) image_kernel(const __grid_constant__ ArenaLayout L,
+                                                    const float* __restrict__ codes, int64_t rows, int nkb,
+                                                    const float* __restrict__ tscale, unsigned char* __restrict__ out,
+                                                    float2* __restrict__ aux) {
+    constexpr int E = F8 ? 16 : 8;  // values per 16-byte chunk
+    const int lane = threadIdx.x & 31, c = lane & 7;
+    const int64_t r = (static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * 4 + (lane >> 3);
+    if (r >= rows) return;  // rows is a multiple of 128: whole warps
+    const uint32_t tr = static_cast<uint32_t>(r & (TM - 1));
+    unsigned char* dst = out + (r / TM) * nkb * KB_BYTES + tr * 128u + ((c ^ (tr & 7u)) << 4);
+    float ts = 1.0f;
+    if constexpr (F8) ts = tscale[r / TM];
+    float nn = 0.0f, ee = 0.0f;
     int b = 0;
-    while (b + 1 < L.nb && j >= L.bstart[b + 1]) ++b;
-    const float v = codes[arena_offset(L, r, b, j - L.bstart[b])];
-    const int64_t tile = r >> 7;
-    const uint32_t row = static_cast<uint32_t>(r & 127), by = static_cast<uint32_t>(j & 127);
-    out[(tile * nkb + (j >> 7)) * KB_BYTES + row * 128u + ((((by >> 4) ^ (row & 7u)) & 7u) << 4) + (by & 15u)] =
-        e4m3_code(v, tscale[tile]);
+#pragma unroll 2
+    for (int kb = 0; kb < nkb; ++kb) {
+        const int j = kb * 8 * E + c * E;
+        while (b + 1 < L.nb && j >= L.bstart[b + 1]) ++b;
+        float v[E];
+        if (j + E <= L.bstart[b + 1] && ((j - L.bstart[b]) & 3) == 0) {
+#pragma unroll
+            for (int i = 0; i < E; i += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(codes + arena_offset(L, r, b, j + i - L.bstart[b]));
+                v[i] = f.x;
+                v[i + 1] = f.y;
+                v[i + 2] = f.z;
+                v[i + 3] = f.w;
+            }
+        } else {
+            int bb = b;
+#pragma unroll
+            for (int i = 0; i < E; ++i) {
+                while (bb + 1 < L.nb && j + i >= L.bstart[bb + 1]) ++bb;
+                v[i] = j + i < L.d ? codes[arena_offset(L, r, bb, j + i - L.bstart[bb])] : 0.0f;
+            }
+        }
+        alignas(16) unsigned char o[16];
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            float vb;
+            if constexpr (F8) {
+                o[i] = e4m3_code(v[i], ts);
+                vb = e4m3_value(o[i], ts);
+            } else {
+                const __nv_bfloat16 h = __float2bfloat16_rn(v[i]);
+                reinterpret_cast<__nv_bfloat16*>(o)[i] = h;
+                vb = __bfloat162float(h);
+            }
+            nn = fmaf(vb, vb, nn);
+            ee = fmaf(v[i] - vb, v[i] - vb, ee);
+        }
+        *reinterpret_cast<uint4*>(dst + static_cast<size_t>(kb) * KB_BYTES) = *reinterpret_cast<const uint4*>(o);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        nn += __shfl_xor_sync(FULL, nn, o);
+        ee += __shfl_xor_sync(FULL, ee, o);
+    }
+    if (c == 0) aux[r] = make_float2(sqrtf(nn), sqrtf(ee));
 }
 
-// Largest |value| of each 128-row tile (one warp per tile).
-__global__ void tile_absmax_kernel(ArenaLayout L, const float* __restrict__ codes, int64_t tiles,
-                                   float* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (t >= tiles) return;
+// Largest |value| of each 128-row tile, a CTA per tile: the tile is one run of
+// the arena, zero where no value lies.  (A warp per tile that looked each value's
+// place up: 1.65 ms for 1M x 420; this 0.33, 5.4 TB/s.)
+__global__ void __launch_bounds__(256) tile_absmax_kernel(const float4* __restrict__ codes, int tile_vec,
+                                                          float* __restrict__ out) {
+    __shared__ float sh[8];
+    const float4* p = codes + static_cast<size_t>(blockIdx.x) * tile_vec;
     float m = 0.0f;
-    for (int r = 0; r < TM; ++r)
-        for (int j = lane; j < L.d; j += 32) {
-            int b = 0;
-            while (b + 1 < L.nb && j >= L.bstart[b + 1]) ++b;
-            m = fmaxf(m, fabsf(codes[arena_offset(L, t * TM + r, b, j - L.bstart[b])]));
-        }
+#pragma unroll 4
+    for (int i = threadIdx.x; i < tile_vec; i += 256) {
+        const float4 v = p[i];
+        m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
-    if (lane == 0) out[t] = m;
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i) m = fmaxf(m, sh[i]);
+        out[blockIdx.x] = m;
+    }
 }
 
 // Per list: scale = (largest |value| over its tiles) / 448, 1 for an all-zero
@@ -129,33 +175,7 @@ __global__ void list_scale_kernel(const int64_t* __restrict__ list_off, const in
     for (int t = 0; t < nt; ++t) tscale[t0 + t] = sc;
 }
 
-// Per-row quantities for the error bound: |x~| (norm of the row as the tensor
-// cores see it: bf16-rounded, or e4m3-coded times its tile's scale when
-// tscale is given) and |x - x~| (its rounding error), one warp per arena row.
-__global__ void row_aux_kernel(ArenaLayout L, const float* __restrict__ codes, int64_t rows,
-                               const float* __restrict__ tscale, float2* __restrict__ aux) {
-    const int lane = threadIdx.x & 31;
-    const int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (r >= rows) return;
-    float nn = 0.0f, ee = 0.0f;
-    const float ts = tscale ? tscale[r >> 7] : 1.0f;
-    for (int j = lane; j < L.d; j += 32) {
-        int b = 0;
-        while (b + 1 < L.nb && j >= L.bstart[b + 1]) ++b;
-        const float v = codes[arena_offset(L, r, b, j - L.bstart[b])];
-        const float vb = tscale ? e4m3_value(e4m3_code(v, ts), ts) : __bfloat162float(__float2bfloat16_rn(v));
-        nn = fmaf(vb, vb, nn);
-        ee = fmaf(v - vb, v - vb, ee);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        nn += __shfl_xor_sync(FULL, nn, o);
-        ee += __shfl_xor_sync(FULL, ee, o);
-    }
-    if (lane == 0) aux[r] = make_float2(sqrtf(nn), sqrtf(ee));
-}
-
-// The same for TF32 operands, read from the FP32 rows as they are: the tensor
+// The bound terms for TF32 operands, read from the FP32 rows as they are: the tensor
 // cores ignore a value's low 13 bits, so x~ is x with them cleared (an x~
 // rounded to nearest would be at least as near), and {norm of |x| + |x - x~|,
 // norm of x - x~} covers either.  Also, for the rule that sends a plain batch
@@ -2796,12 +2816,12 @@ inline int grid_for(int64_t n, int threads) {
 
 }  // namespace
 
-cudaError_t launch_to_bf16_arena(const ArenaLayout& L, const float* codes, int64_t rows, void* out, cudaStream_t s) {
-    const int nkb = (L.d + 63) / 64;
-    cudaError_t e = cudaMemsetAsync(out, 0, bf16_image_bytes(rows, L.d), s);
-    if (e != cudaSuccess) return e;
-    to_bf16_arena_kernel<<<grid_for(rows * L.d, 256), 256, 0, s>>>(L, codes, rows, nkb,
-                                                                    static_cast<unsigned char*>(out));
+cudaError_t launch_bf16_image(const ArenaLayout& L, const float* codes, int64_t rows, void* out, float2* aux,
+                              float2* tile_aux, cudaStream_t s) {
+    image_kernel<false><<<grid_for(rows, 32), 256, 0, s>>>(L, codes, rows, (L.d + 63) / 64, nullptr,
+                                                           static_cast<unsigned char*>(out), aux);
+    const int64_t tiles = rows / TM;
+    tile_aux_kernel<<<grid_for(tiles * 32, 256), 256, 0, s>>>(aux, tiles, tile_aux);
     return cudaGetLastError();
 }
 
@@ -2965,24 +2985,16 @@ cudaError_t launch_arena_integral(const float* codes, int64_t n, const float* xn
     return cudaGetLastError();
 }
 
-cudaError_t launch_to_f8_arena(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,
-                               const int32_t* list_size, int nlist, float* tile_max, float* lscale, float* tscale,
-                               void* out, cudaStream_t s) {
+cudaError_t launch_f8_image(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,
+                            const int32_t* list_size, int nlist, float* tile_max, float* lscale, float* tscale,
+                            void* out, float2* aux, float2* tile_aux, cudaStream_t s) {
     const int64_t tiles = rows / TM;
-    cudaError_t e = cudaMemsetAsync(out, 0, f8_image_bytes(rows, L.d), s);
-    if (e != cudaSuccess) return e;
     fill_f32_kernel<<<grid_for(tiles, 256), 256, 0, s>>>(tscale, tiles, 1.0f);
-    tile_absmax_kernel<<<grid_for(tiles * 32, 256), 256, 0, s>>>(L, codes, tiles, tile_max);
+    tile_absmax_kernel<<<grid_for(tiles, 1), 256, 0, s>>>(reinterpret_cast<const float4*>(codes), TM / 4 * L.row_pitch,
+                                                          tile_max);
     list_scale_kernel<<<grid_for(nlist, 128), 128, 0, s>>>(list_off, list_size, nlist, tile_max, lscale, tscale);
-    to_f8_arena_kernel<<<grid_for(rows * L.d, 256), 256, 0, s>>>(L, codes, rows, (L.d + 127) / 128, tscale,
-                                                                  static_cast<unsigned char*>(out));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_row_aux(const ArenaLayout& L, const float* codes, int64_t rows, const float* tscale, float2* aux,
-                           float2* tile_aux, cudaStream_t s) {
-    row_aux_kernel<<<grid_for(rows * 32, 256), 256, 0, s>>>(L, codes, rows, tscale, aux);
-    const int64_t tiles = rows / TM;
+    image_kernel<true><<<grid_for(rows, 32), 256, 0, s>>>(L, codes, rows, (L.d + 127) / 128, tscale,
+                                                          static_cast<unsigned char*>(out), aux);
     tile_aux_kernel<<<grid_for(tiles * 32, 256), 256, 0, s>>>(aux, tiles, tile_aux);
     return cudaGetLastError();
 }

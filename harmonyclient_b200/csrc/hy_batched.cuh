@@ -40,12 +40,15 @@ int batched_group_size(int nkb);
 // Largest rows per work item of groups of qg at nkb k-blocks.
 int batched_row_slice(int nkb, int qg);
 
-cudaError_t launch_to_bf16_arena(const ArenaLayout& L, const float* codes, int64_t rows, void* out, cudaStream_t s);
-// e4m3 image with per-list scales: tile_max [rows/128] scratch, lscale
+// bf16 image of the arena (rows a multiple of 128), per arena row {|x~|, |x - x~|}
+// for the error bound and per 128-row tile the maxima of both.
+cudaError_t launch_bf16_image(const ArenaLayout& L, const float* codes, int64_t rows, void* out, float2* aux,
+                              float2* tile_aux, cudaStream_t s);
+// The same as e4m3 with per-list scales: tile_max [rows/128] scratch, lscale
 // [nlist] and tscale [rows/128] outputs.
-cudaError_t launch_to_f8_arena(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,
-                               const int32_t* list_size, int nlist, float* tile_max, float* lscale, float* tscale,
-                               void* out, cudaStream_t s);
+cudaError_t launch_f8_image(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,
+                            const int32_t* list_size, int nlist, float* tile_max, float* lscale, float* tscale,
+                            void* out, float2* aux, float2* tile_aux, cudaStream_t s);
 // qscale == nullptr: bf16 queries; else e4m3 queries with per-query scales.
 // bf16 queries with qexact: qexact[i] = 1 when query i and the arena admit
 // exact tensor-core distances: cert (the arena's certificate on the device,
@@ -64,15 +67,9 @@ cudaError_t launch_prep_queries_tf32(const float* q, int nq, const ArenaLayout& 
 // largest of xn[0..rows).
 cudaError_t launch_arena_integral(const float* codes, int64_t n, const float* xn, int64_t rows, int* flag,
                                   unsigned int* maxxn, cudaStream_t s);
-// Per arena row {|x~|, |x - x~|} for the error bound (tscale == nullptr: the
-// bf16 image, else the e4m3 image with those tile scales), and per 128-row
-// tile the maxima of both.
 // tile_max[t] = the largest xn over rows [128 t, 128 t + 128) (rows a
 // multiple of 128).
 cudaError_t launch_tile_max(const float* xn, int64_t rows, float* tile_max, cudaStream_t s);
-cudaError_t launch_row_aux(const ArenaLayout& L, const float* codes, int64_t rows, const float* tscale, float2* aux,
-                           float2* tile_aux, cudaStream_t s);
-
 // The bound terms of the arena rows read as TF32, and two sums over a sample of
 // the rows (see row_aux_tf32_kernel).
 cudaError_t launch_row_aux_tf32(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,

@@ -963,11 +963,10 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
         HY_RET(h->lscale.ensure(h->nlist * sizeof(float)));
         HY_RET(h->tscale.ensure(tiles * sizeof(float)));
         HY_RET(h->tmax.ensure(tiles * sizeof(float)));
-        HY_CUDA(hy::launch_to_f8_arena(h->L, h->codes.as<float>(), (int64_t)rows, h->list_off.as<int64_t>(),
-                                       h->list_size.as<int32_t>(), (int)h->nlist, h->tmax.as<float>(),
-                                       h->lscale.as<float>(), h->tscale.as<float>(), h->a8.p, s));
-        HY_CUDA(hy::launch_row_aux(h->L, h->codes.as<float>(), (int64_t)rows, h->tscale.as<float>(),
-                                   h->x8aux.as<float2>(), h->t8aux.as<float2>(), s));
+        HY_CUDA(hy::launch_f8_image(h->L, h->codes.as<float>(), (int64_t)rows, h->list_off.as<int64_t>(),
+                                    h->list_size.as<int32_t>(), (int)h->nlist, h->tmax.as<float>(),
+                                    h->lscale.as<float>(), h->tscale.as<float>(), h->a8.p, h->x8aux.as<float2>(),
+                                    h->t8aux.as<float2>(), s));
         HY_RET(ensure_tile_norms(h, rows, s));
         h->a8_valid = true;
         return HY_OK;
@@ -1002,9 +1001,8 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
     HY_RET(h->abf.ensure(hy::bf16_image_bytes((int64_t)rows, (int)h->d)));
     HY_RET(h->xaux.ensure(rows * sizeof(float2)));
     HY_RET(h->taux.ensure(tiles * sizeof(float2)));
-    HY_CUDA(hy::launch_to_bf16_arena(h->L, h->codes.as<float>(), (int64_t)rows, h->abf.p, s));
-    HY_CUDA(hy::launch_row_aux(h->L, h->codes.as<float>(), (int64_t)rows, nullptr, h->xaux.as<float2>(), h->taux.as<float2>(),
-                               s));
+    HY_CUDA(hy::launch_bf16_image(h->L, h->codes.as<float>(), (int64_t)rows, h->abf.p, h->xaux.as<float2>(),
+                                  h->taux.as<float2>(), s));
     HY_RET(ensure_tile_norms(h, rows, s));
     HY_RET(ensure_certificate(h, rows, s));
     h->abf_valid = true;
