@@ -1209,9 +1209,13 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     // the first pass scans that list densely and the tightening step takes
     // the k-th smallest bound over all of its rows.
     const int dense_max = (int)std::min<size_t>(capq, hy::DENSE_MAX);
-    const size_t wl = h->warmup_list ? std::min<size_t>(h->warmup_list, 3) : 3;
-    const size_t wls = h->warmup_list_size ? h->warmup_list_size : k;
-    HY_CHECK(std::min(wl, nprobe) * wls <= 32768, HY_ERR_ARG, "presearch: warmup_list * warmup_list_size above 32768");
+    // A plain search takes the caller's warm-up sizes only where its other scans
+    // have a warm-up (L2, warmup_list > 0), and keeps their limit.
+    const bool own_wl = h->warmup_list > 0 && !(tf32 && h->metric != HY_METRIC_L2);
+    const size_t wl = own_wl ? std::min<size_t>(h->warmup_list, 3) : 3;
+    const size_t wls = h->warmup_list_size && (own_wl || !tf32) ? h->warmup_list_size : k;
+    HY_CHECK(std::min(tf32 && own_wl ? h->warmup_list : wl, nprobe) * wls <= 32768, HY_ERR_ARG,
+             "presearch: warmup_list * warmup_list_size above 32768");
     // Item descriptors: an upper bound on the item count from host-known
     // sizes (groups <= pairs/128 + lists, slices per list <= the largest
     // list's), capped at 4M; items beyond the cap are decoded by search.

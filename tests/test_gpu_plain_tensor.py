@@ -140,3 +140,22 @@ def test_first_search_under_capture_keeps_the_list_major_scan():
     torch.cuda.synchronize()
     np.testing.assert_array_equal(dI.cpu().numpy(), I)
     np.testing.assert_array_equal(dD.cpu().numpy(), D)
+
+
+@pytest.mark.parametrize("metric,lists,rows,taken", [
+    (hb.METRIC_L2, 0, 20_000, True),  # no warm-up: its size has no say
+    (hb.METRIC_IP, 10, 20_000, True),  # none for inner products
+    (hb.METRIC_L2, 8, 4_096, True), (hb.METRIC_L2, 8, 4_097, False),  # at and past the limit
+    (hb.METRIC_L2, 100, 2_049, False),  # lists count up to nprobe
+])
+def test_warmup_sizes_as_the_other_scans_take_them(metric, lists, rows, taken):
+    x, q = _data(128, 9_001, 1_025, "float", 3)
+    idx = _index(x, metric=metric)
+    idx.preSearch(warmUpSearchList=lists, warmUpSearchListSize=rows)
+    if taken:
+        _same(idx, q, 10)
+        return
+    for mode in ("query", "list", "auto"):
+        idx.set_plain_scan(mode)
+        with pytest.raises(hb.HyError):
+            idx.search(q, 10)
