@@ -626,6 +626,7 @@ def plain_roofline(st, scan_ms, launches, palg, clocks, args, hbm_peak, peak_kin
     `seg_sums`) against 148 SMs x 128 FP32 lanes x the SM clock measured
     during the run; the lists are read once per group of 32 queries, mostly
     from L2, so the pair bytes are reported beside it, not as a fraction.
+    Tensor (TF32): the pairs' flops against half the bf16 rate.
     Query-major: pair bytes (every probed row of every query, d x 4 bytes,
     plus queries and results) against the measured copy bandwidth."""
     if st.get("list_major"):
@@ -645,6 +646,17 @@ def plain_roofline(st, scan_ms, launches, palg, clocks, args, hbm_peak, peak_kin
                 "pair_bytes": palg, "pair_bytes_rate_gbs": round(palg / (scan_ms / 1e3) / 1e9, 1),
                 "traffic": KNOWN_TRAFFIC.get((args.workload, "plain-lm", args.nb, args.nq, args.nprobe)),
                 "traffic_source": TRAFFIC_SOURCE["plain-lm"]}
+    if st.get("kernel_launches", 1) > 1:
+        # The tensor cores with the FP32 arena as TF32 operands (two passes,
+        # exact re-rank): the pairs' flops at half the bf16 rate, no fraction of
+        # the pair bytes, which are read once per group of queries.
+        flops = palg / 2
+        ach = flops / (scan_ms / 1e3) / 1e12
+        peak = round((peaks()[1] or 0.0) / 2, 1)
+        return {"bound": "tensor", "achieved": round(ach, 1), "peak": peak, "unit": "TFLOP/s",
+                "frac": round(ach / peak, 4) if peak else None, "peak_kind": "half of measured bf16",
+                "kernel": "batched_scan_kernel (TF32)", "kernel_ms": round(scan_ms, 4),
+                "launches_per_search": launches, "pair_bytes": palg}
     pach = palg / (scan_ms / 1e3) / 1e9
     return {"bound": "hbm", "achieved": round(pach, 1), "peak": hbm_peak, "unit": "GB/s",
             "frac": round(pach / hbm_peak, 4), "peak_kind": peak_kind,
@@ -680,7 +692,7 @@ def _plain_work(st):
     """The list-major plain scan's executed share of its unpruned block sums."""
     if st.get("list_major") and st.get("seg_sums_max"):
         return {"scan": "list-major", "seg_sums_executed": round(st["seg_sums"] / st["seg_sums_max"], 4)}
-    return {"scan": "query-major"}
+    return {"scan": "tensor (TF32)" if st.get("kernel_launches", 1) > 1 else "query-major"}
 
 
 def extra_nprobe_sweep(idx, x, q, k, nprobes, steps, ts, dev, main_nprobe):
