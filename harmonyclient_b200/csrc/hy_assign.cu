@@ -388,7 +388,9 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
                     const float top = fmaf(2.0f * inflate, E, best.m1);
                     const bool sane = E > 1e-30f && smax < 1e37f && E < 1e37f;
                     const bool one = sane && best.m2 > top, two = sane && best.m3 > top;
-                    p.labels[row] = best.i1;
+                    // (A padding column wins where every real score overflows:
+                    // a listed row's label is still read as a centroid.)
+                    p.labels[row] = min(best.i1, p.nlist - 1);
                     p.second[row] = one || !two ? -1 : best.i2;
                     if (!two) p.hard[atomicAdd(p.hard_count, 1)] = static_cast<int32_t>(row);
                 }

@@ -114,3 +114,17 @@ def test_list_order_is_the_exact_scores():
             dlt = (x[ids, j] - c[l, j]).astype(np.float32)
             t = (t + (dlt * dlt).astype(np.float32)).astype(np.float32)
         assert np.all(np.diff(t) >= 0)
+
+
+@pytest.mark.parametrize("nlist,d", [(300, 33), (129, 64), (65, 200)])
+def test_scores_that_all_overflow(nlist, d):
+    """Finite rows whose score against every centroid overflows, beside list
+    counts that are no multiple of the tile: the exact kernel's labels."""
+    rng = np.random.default_rng(nlist)
+    c = rng.integers(1, 256, (nlist, d)).astype(np.float32)
+    x = np.clip(c[rng.integers(0, nlist, 5_000)] + rng.integers(-9, 10, (5_000, d)), 0, 255).astype(np.float32)
+    x[::7] = -1e37 * rng.uniform(0.9, 1.1, (len(x[::7]), d))
+    _check(x, c)
+    _check(x, c, hb.METRIC_IP)
+    # rows and centroids whose squared norms overflow
+    _check(rng.uniform(3e19, 6e19, (5_000, d)).astype(np.float32), c * np.float32(1e19))
