@@ -50,16 +50,6 @@ constexpr int NSTG = 2;       // stages of the centroid ring (a k-block of TN ce
 constexpr int W_MMA = 1, W_EPI0 = 4, N_EPI = 8, W_CONV0 = 12, N_CONV = 4;
 constexpr int ASSIGN_THREADS = 32 * (W_CONV0 + N_CONV);
 
-__device__ inline bool wait_abort(uint64_t* bar, uint32_t parity, int* err, volatile int* abort) {
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 1023u) == 1023u && *abort) return false;
-    }
-    if (err) atomicCAS(err, 0, DEV_ERR_TIMEOUT);
-    *abort = 1;
-    return false;
-}
-
 struct AssignParams {
     const float* x;
     const unsigned char* cimg;
@@ -70,8 +60,22 @@ struct AssignParams {
     int* err;
     int n, d, nlist, nkb, nbuf;  // nkb: 64-dimension blocks; nbuf: row tiles held
     int ntc, nit;                     // accumulators per row tile; 128-row tiles of the centroid image
+    uint32_t wait_limit;              // polls of a wait before it gives up
     float cK, cN;                     // (3K + 8) u, (3d + 16) u or (d + 4) u, inflated
 };
+
+// A bounded wait; one that gives up raises the status word and the abort flag,
+// on which every role leaves.  Roles run by a whole warp vote on the result,
+// so that no lane is left alone at a warp-wide step.
+__device__ inline bool wait_abort(uint64_t* bar, uint32_t parity, const AssignParams& p, volatile int* abort) {
+    for (uint32_t i = 0; i < p.wait_limit; ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((i & 1023u) == 1023u && *abort) return false;
+    }
+    if (p.err) atomicCAS(p.err, 0, DEV_ERR_TIMEOUT);
+    *abort = 1;
+    return false;
+}
 
 // The three smallest scores of a row and the first two's centroids.
 struct Best {
@@ -107,7 +111,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
     const int nkb = p.nkb, nbuf = p.nbuf;
     const size_t tileA = static_cast<size_t>(nkb) * 2 * KB;  // per 64 dimensions: hi k-block, lo k-block
     unsigned char* sB = sA + nbuf * tileA;                   // NSTG x 2 centroid k-blocks
-    __shared__ uint64_t afull[2], afree[2], full[NSTG], empty[NSTG], accf[2], acce[2], folded[2];
+    __shared__ uint64_t afull[2], afree[2], full[NSTG], empty[NSTG], accf[2], acce[2], folded[2], drain;
     __shared__ uint32_t tbase;
     __shared__ int s_abort;
     __shared__ float4 s_row[2][TM];          // per row {|x|, |x_lo|, |x_r|, A_x}
@@ -131,6 +135,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
         }
+        mbar_init(&drain, 1);
         s_abort = 0;
         s_lo[0] = s_lo[1] = 0;
         fence_mbar_init();
@@ -149,7 +154,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
         uint32_t it = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
             const int b = static_cast<int>(it % nbuf);
-            if (!wait_abort(&afree[b], ((it / nbuf) & 1u) ^ 1u, p.err, vabort)) break;
+            if (!__all_sync(FULL, wait_abort(&afree[b], ((it / nbuf) & 1u) ^ 1u, p, vabort))) break;
             unsigned char* A = sA + b * tileA;
             uint32_t lo_any = 0;
             for (int r0 = cw * 4; r0 < TM; r0 += N_CONV * 4) {
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
                     const uint32_t halves = min(2, p.nit - 2 * ct);
                     for (int k = 0; k < 2 * nkb; ++k, ++i) {
                         const uint32_t st = i % NSTG;
-                        if (!wait_abort(&empty[st], ((i / NSTG) & 1u) ^ 1u, p.err, vabort)) {
+                        if (!wait_abort(&empty[st], ((i / NSTG) & 1u) ^ 1u, p, vabort)) {
                             ok = false;
                             break;
                         }
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
             bool ok = true;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++it) {
                 const int b = static_cast<int>(it % nbuf);
-                if (!wait_abort(&afull[b], (it / nbuf) & 1u, p.err, vabort)) break;
+                if (!wait_abort(&afull[b], (it / nbuf) & 1u, p, vabort)) break;
                 tc::fence_after_sync();
                 const uint32_t a0 = smem_u32(sA + b * tileA);
                 // Rows without a lo part (integers to 256, bf16 values) need
@@ -252,7 +257,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
                     const int buf = acc & 1;
                     const uint32_t idesc = tc::idesc_bf16_f32(TM, 2 * tile + 1 < p.nit ? TN : TN / 2);
                     if (++tile == p.ntc) tile = 0;
-                    if (!wait_abort(&acce[buf], ((acc >> 1) & 1u) ^ 1u, p.err, vabort)) {
+                    if (!wait_abort(&acce[buf], ((acc >> 1) & 1u) ^ 1u, p, vabort)) {
                         ok = false;
                         break;
                     }
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
                     const uint32_t dcol = tmem + static_cast<uint32_t>(buf * TN);
                     for (int k = 0; k < 2 * nkb; ++k, ++i) {
                         const uint32_t st = i % NSTG;
-                        if (!wait_abort(&full[st], (i / NSTG) & 1u, p.err, vabort)) {
+                        if (!wait_abort(&full[st], (i / NSTG) & 1u, p, vabort)) {
                             ok = false;
                             break;
                         }
@@ -281,6 +286,10 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
                 }
                 if (ok) tc::mma_commit(&afree[b]);
             }
+            // No tensor-core instruction outlives the CTA either (one is
+            // still in flight here only after a wait gave up).
+            tc::mma_commit(&drain);
+            mbar_wait_bounded(&drain, 0, p.err);
         }
     } else if (warp >= W_EPI0 && warp < W_EPI0 + N_EPI) {
         // ---------------- epilogue: thread = row; each half scans 64 of a
@@ -308,7 +317,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
                     s_cn[e][lane + j] = c < p.nlist ? (l2 ? __ldg(p.cxn + c) : 0.0f) : FLT_MAX;
                 }
                 __syncwarp();
-                ok = __all_sync(FULL, wait_abort(&accf[buf], (acc >> 1) & 1u, p.err, vabort));
+                ok = __all_sync(FULL, wait_abort(&accf[buf], (acc >> 1) & 1u, p, vabort));
                 if (!ok) break;
                 tc::fence_after_sync();
 #pragma unroll 1
@@ -371,7 +380,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cta(&folded[xb]);
             } else {
-                ok = ok && __all_sync(FULL, wait_abort(&folded[xb], (it >> 1) & 1u, p.err, vabort));
+                ok = ok && __all_sync(FULL, wait_abort(&folded[xb], (it >> 1) & 1u, p, vabort));
             }
             if (half == 0 && ok) {
                 best.insert(s_m[xb][0][r], s_i[xb][0][r]);
@@ -475,6 +484,7 @@ cudaError_t launch_assign(const float* x, int n, int d, int nlist, int metric, c
     p.hard = w.hard;
     p.hard_count = w.hard_count;
     p.err = w.err;
+    p.wait_limit = w.wait_limit;
     p.n = n;
     p.d = d;
     p.nlist = nlist;

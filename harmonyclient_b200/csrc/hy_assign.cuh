@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "hy_device.cuh"
+
 namespace hy {
 
 // Largest d the kernel's resident row tile takes.
@@ -16,7 +18,8 @@ struct AssignWork {
     int32_t* second;       // [n] the other candidate of a row with two, else -1
     int32_t* hard;         // [n] rows whose candidates did not fit
     int32_t* hard_count;   // [1]
-    int* err;
+    int* err;              // DEV_ERR_TIMEOUT when a wait gave up: rows are then left unwritten
+    uint32_t wait_limit = WAIT_LIMIT;
 };
 
 // Tensor-core pass: per row its best centroid by score (labels), a second

@@ -129,10 +129,11 @@ ArenaLayout make_layout(int d, int nb) {
 
 }  // namespace
 
-// Device status of a call: one block on the device (w_err, w_counters, b_fbtot
-// and m_total point into it), read back in one copy.
+// Device status of a call: one block on the device (w_err, w_build_err,
+// w_counters, b_fbtot and m_total point into it), read back in one copy.
 struct HostStatus {
     int err = 0;
+    int build_err = 0;                        // the same of a train's or an add's assignment of rows
     unsigned long long counters[4] = {0, 0, 0, 0};  // scan counters (block copies, blocks unpruned, block sums, sums unpruned)
     unsigned long long fallback = 0;          // queries answered by the device fallback
     unsigned long long learned_total = 0;     // sum of the learned nprobes
@@ -157,9 +158,12 @@ struct hy_index {
     std::vector<int32_t> h_list_size;
 
     DevBuf cent, list_off, list_size, ids, codes, norms;
+    uint32_t wait_limit = hy::WAIT_LIMIT;  // polls of a bounded device-side wait (hy_selftest_wait_limit)
+
     // workspace
     DevBuf w_status;  // HostStatus on the device: w_err, w_counters, b_fbtot, m_total
     DevBuf w_q, w_scores, w_probes, w_thr, w_gthr, w_parts, w_D, w_I, w_f, w_counters, w_err;
+    DevBuf w_build_err;
     DevBuf w_undecided;  // tensor-core assignment: undecided rows (count, ids), second candidates
     DevBuf w_x, w_lab, w_dist, w_keys, w_keys2, w_vals, w_vals2, w_sort, w_start, w_sums, w_cnt, w_rows, w_xn;
 
@@ -340,6 +344,27 @@ bool assign_on_tensor(const hy_index* h, size_t n) {
     return h->d <= hy::ASSIGN_DMAX && n * h->nlist * h->d >= ASSIGN_TENSOR_MIN;
 }
 
+// Before the assignments of a train or an add of n rows: a tensor-core pass
+// whose wait gives up leaves rows unwritten, so every label (w_lab) and second
+// candidate starts as a valid one, and the status word clear.
+int begin_assign(hy_index* h, size_t n, cudaStream_t s) {
+    if (!assign_on_tensor(h, n)) return HY_OK;
+    HY_RET(h->w_undecided.ensure((2 * n + 1) * sizeof(int32_t)));
+    HY_CUDA(cudaMemsetAsync(h->w_lab.p, 0, n * sizeof(int64_t), s));
+    HY_CUDA(cudaMemsetAsync(h->w_undecided.p, 0xff, (2 * n + 1) * sizeof(int32_t), s));
+    HY_CUDA(cudaMemsetAsync(h->w_build_err.p, 0, sizeof(int), s));
+    return HY_OK;
+}
+
+// After them, with the stream's synchronisation: whether a wait gave up.
+int end_assign(hy_index* h, size_t n, cudaStream_t s) {
+    int e = 0;
+    if (assign_on_tensor(h, n)) HY_CUDA(cudaMemcpyAsync(&e, h->w_build_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    HY_CUDA(cudaStreamSynchronize(s));
+    if (e != 0) return fail(HY_ERR_TIMEOUT, "a device-side wait gave up in the assignment of rows to lists");
+    return HY_OK;
+}
+
 // Nearest centroid of each of n device rows (x): labels, scores (score may be
 // null).  On the tensor cores, rows the bound leaves undecided (usually none)
 // go through the exact scores of every centroid, in chunks up to their device
@@ -351,7 +376,6 @@ int assign_rows(hy_index* h, const float* x, size_t n, int64_t* labels, float* s
     if (assign_on_tensor(h, n)) {
         if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
         HY_RET(ensure_centroid_image(h, s));
-        HY_RET(h->w_undecided.ensure((2 * n + 1) * sizeof(int32_t)));
         hy::AssignWork w;
         w.cimg = h->c_img.p;
         w.cxn = h->c_norm.as<float>();
@@ -359,7 +383,8 @@ int assign_rows(hy_index* h, const float* x, size_t n, int64_t* labels, float* s
         w.hard_count = h->w_undecided.as<int32_t>();
         w.hard = w.hard_count + 1;
         w.second = w.hard + n;
-        w.err = h->w_err.as<int>();
+        w.err = h->w_build_err.as<int>();
+        w.wait_limit = h->wait_limit;
         HY_CUDA(hy::launch_assign(x, (int)n, (int)h->d, (int)h->nlist, h->metric, w, h->nsm, labels, s));
         HY_CUDA(hy::launch_assign_exact(x, (int)n, (int)h->d, h->cent.as<float>(), h->metric, w, labels, score, s));
         pick.rows = w.hard;
@@ -396,6 +421,7 @@ int kmeans_device(hy_index* h, const float* xs, size_t ns, const std::vector<int
     HY_RET(h->w_lab.ensure(ns * sizeof(int64_t)));
     HY_RET(h->w_sums.ensure(nlist * d * sizeof(double)));
     HY_RET(h->w_cnt.ensure(nlist * sizeof(unsigned long long)));
+    HY_RET(begin_assign(h, ns, s));
     for (int it = 0; it < niter; ++it) {
         h->cimg_valid = false;
         HY_RET(assign_rows(h, assign_src, ns, h->w_lab.as<int64_t>(), nullptr, s));
@@ -407,11 +433,18 @@ int kmeans_device(hy_index* h, const float* xs, size_t ns, const std::vector<int
                                          h->cent.as<float>(), s));
     }
     if (h->metric == HY_METRIC_IP) HY_CUDA(hy::launch_normalize_centroids(h->cent.as<float>(), (int)nlist, (int)d, s));
-    h->h_cent.resize(nlist * d);
-    HY_CUDA(cudaMemcpyAsync(h->h_cent.data(), h->cent.p, nlist * d * sizeof(float), cudaMemcpyDeviceToHost, s));
-    HY_CUDA(cudaStreamSynchronize(s));
-    h->trained = true;
     h->cimg_valid = false;
+    std::vector<float> cent(nlist * d);
+    HY_CUDA(cudaMemcpyAsync(cent.data(), h->cent.p, nlist * d * sizeof(float), cudaMemcpyDeviceToHost, s));
+    const int rc = end_assign(h, ns, s);
+    if (rc != HY_OK) {
+        // The centroids of before, if there were any.
+        if (h->trained)
+            HY_CUDA(cudaMemcpy(h->cent.p, h->h_cent.data(), nlist * d * sizeof(float), cudaMemcpyHostToDevice));
+        return rc;
+    }
+    h->h_cent.swap(cent);
+    h->trained = true;
     return HY_OK;
 }
 
@@ -558,6 +591,7 @@ int add_impl(hy_index* h, size_t n, const float* x, bool x_on_device, cudaStream
     }
     HY_RET(h->w_lab.ensure(n * sizeof(int64_t)));
     HY_RET(h->w_dist.ensure(n * sizeof(float)));
+    HY_RET(begin_assign(h, n, s));
     HY_RET(assign_rows(h, xd, n, h->w_lab.as<int64_t>(), h->w_dist.as<float>(), s));
     // list sizes
     HY_RET(h->w_cnt.ensure(nlist * sizeof(int32_t)));
@@ -581,7 +615,7 @@ int add_impl(hy_index* h, size_t n, const float* x, bool x_on_device, cudaStream
     tmp = h->w_sort.bytes;
     HY_CUDA(hy::radix_sort_pairs(h->w_sort.p, &tmp, h->w_keys.as<uint64_t>(), h->w_keys2.as<uint64_t>(),
                                  h->w_vals.as<int32_t>(), h->w_vals2.as<int32_t>(), (int64_t)n, 32 + lbits, s));
-    HY_CUDA(cudaStreamSynchronize(s));
+    HY_RET(end_assign(h, n, s));  // before the index changes
     return build_arena(h, xd, n, h->w_vals2.as<int32_t>(), h->w_lab.as<int64_t>(), sizes, s);
 }
 
@@ -841,6 +875,7 @@ int ensure_common(hy_index* h) {
     HY_CUDA(cudaMemset(h->w_status.p, 0, sizeof(HostStatus)));
     unsigned char* b = h->w_status.as<unsigned char>();
     h->w_err.alias(b + offsetof(HostStatus, err), sizeof(int));
+    h->w_build_err.alias(b + offsetof(HostStatus, build_err), sizeof(int));
     h->w_counters.alias(b + offsetof(HostStatus, counters), sizeof(HostStatus::counters));
     h->b_fbtot.alias(b + offsetof(HostStatus, fallback), sizeof(HostStatus::fallback));
     h->m_total.alias(b + offsetof(HostStatus, learned_total), sizeof(HostStatus::learned_total));
@@ -2438,6 +2473,14 @@ int hy_index_warmup_tops(hy_index* h, size_t n, const float* q, size_t k, size_t
                               h->w_err.as<int>(), s));
     HY_CUDA(cudaMemcpyAsync(tops, h->w_f.p, n * sizeof(float), cudaMemcpyDeviceToHost, s));
     HY_CUDA(cudaStreamSynchronize(s));
+    return HY_OK;
+}
+
+int hy_selftest_wait_limit(hy_index* h, unsigned int polls) {
+    HY_CHECK(h, HY_ERR_ARG, "wait_limit: NULL handle");
+    std::lock_guard<std::mutex> g(h->mu);
+    h->epoch++;  // a captured search graph no longer matches
+    h->wait_limit = std::min<uint32_t>(polls, hy::WAIT_LIMIT);
     return HY_OK;
 }
 

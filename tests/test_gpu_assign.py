@@ -7,6 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 import harmonyclient_b200 as hb  # noqa: E402
+from harmonyclient_b200 import _lib  # noqa: E402
 from oracle import port  # noqa: E402
 
 EXACT_MAX = (1 << 29) - 1  # rows x centroids x dimensions below the tensor-core rule
@@ -128,3 +129,51 @@ def test_scores_that_all_overflow(nlist, d):
     _check(x, c, hb.METRIC_IP)
     # rows and centroids whose squared norms overflow
     _check(rng.uniform(3e19, 6e19, (5_000, d)).astype(np.float32), c * np.float32(1e19))
+
+
+@pytest.mark.parametrize("metric", [hb.METRIC_L2, hb.METRIC_IP])
+def test_a_wait_that_gives_up(metric):
+    """Device-side waits that run out at their first poll: train and add
+    report it and leave the centroids and the lists as they were."""
+    L = _lib.load()
+    rng = np.random.default_rng(14)
+    x = rng.uniform(0, 50, (70_000, 70)).astype(np.float32)
+    q = x[:50] + np.float32(0.5)
+    idx = hb.Index(70, 130, 8, metric)
+    assert len(x) * 130 * 70 > EXACT_MAX and 130 * 256 * 130 * 70 < EXACT_MAX  # add runs there, train does not
+    idx.train(x)
+    idx.add(x)
+    cent = idx.centroid_codes.copy()
+    D, I = idx.search(q, 5)
+    fresh = hb.Index(70, 1_000, 8, metric)  # its train runs there too
+    _lib.check(L.hy_selftest_wait_limit(idx._h, 0))
+    _lib.check(L.hy_selftest_wait_limit(fresh._h, 0))
+    with pytest.raises(_lib.HyError) as e:
+        idx.add(x[::-1].copy())
+    assert e.value.code == _lib.HY_ERR_TIMEOUT
+    with pytest.raises(_lib.HyError) as e:
+        fresh.train(x)
+    assert e.value.code == _lib.HY_ERR_TIMEOUT
+    np.testing.assert_array_equal(idx.centroid_codes, cent)
+    for a, b in zip((D, I), idx.search(q, 5)):
+        np.testing.assert_array_equal(a, b)
+    with pytest.raises(_lib.HyError) as e:
+        fresh.add(x)
+    assert e.value.code == _lib.HY_ERR_STATE
+    # a trained index keeps its centroids
+    _lib.check(L.hy_selftest_wait_limit(fresh._h, 1 << 31))
+    fresh.train(x)
+    fresh.add(x)
+    cent = fresh.centroid_codes.copy()
+    D, I = fresh.search(q, 5)
+    _lib.check(L.hy_selftest_wait_limit(fresh._h, 0))
+    with pytest.raises(_lib.HyError):
+        fresh.train(x + np.float32(3))
+    np.testing.assert_array_equal(fresh.centroid_codes, cent)
+    for a, b in zip((D, I), fresh.search(q, 5)):
+        np.testing.assert_array_equal(a, b)
+    # and with the limit back, the same calls go through
+    _lib.check(L.hy_selftest_wait_limit(idx._h, 1 << 31))
+    _lib.check(L.hy_selftest_wait_limit(fresh._h, 1 << 31))
+    np.testing.assert_array_equal(_labels(idx, x), _exact_labels(idx, x))
+    np.testing.assert_array_equal(_labels(fresh, x), _exact_labels(fresh, x))
