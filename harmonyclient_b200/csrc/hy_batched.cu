@@ -811,6 +811,7 @@ struct BatchedParams {
     int nslot;                      // item slots (2 or SLOT_MAX)
     int nbuf;                       // query operand buffers: one per slot, or a single one
     int dense_max;                  // lists of at most this many rows: dense items (0 = none)
+    uint32_t wait_limit;            // polls of a wait before it gives up
     float cK, cN;                   // error-bound constants (see err_coef)
 };
 
@@ -866,7 +867,7 @@ constexpr size_t batched_smem(int nkb, int ring, int nslot, int nbuf) {
 }
 // Dynamic shared memory per CTA: the 227 KiB opt-in limit less room for the
 // kernel's static shared variables (barriers, TMEM base, flags).
-constexpr size_t BATCHED_SMEM_CAP = 227 * 1024 - 256;
+constexpr size_t BATCHED_SMEM_CAP = 227 * 1024 - 320;
 
 // Stages of the deepest ring that fits (0: fewer than RING_MIN k-blocks).
 template <int QG, bool WIDE>
@@ -910,8 +911,13 @@ __device__ __forceinline__ int group_col(int i) {
     return (i >> 1) + (i & 1) * (QG / 2);
 }
 
-__device__ inline bool wait_or_abort(uint64_t* bar, uint32_t parity, int* err, volatile int* abort) {
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
+// A bounded wait; one that gives up raises the status word and the abort flag,
+// on which every role leaves.  Roles of a warp or more vote on the result, so
+// that no thread is left alone at a warp-wide step or a barrier.  The polls
+// after the first are out of line (in line, the epilogue's code around its
+// waits took 2.5 % of the bf16 scan).
+__device__ __noinline__ bool wait_polls(uint64_t* bar, uint32_t parity, uint32_t limit, int* err, volatile int* abort) {
+    for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((i & 1023u) == 1023u && *abort) return false;
     }
@@ -919,10 +925,24 @@ __device__ inline bool wait_or_abort(uint64_t* bar, uint32_t parity, int* err, v
     *abort = 1;
     return false;
 }
+__device__ inline bool wait_or_abort(uint64_t* bar, uint32_t parity, const BatchedParams& p, volatile int* abort) {
+    return (p.wait_limit && mbar_try_wait(bar, parity)) || wait_polls(bar, parity, p.wait_limit, p.err, abort);
+}
 
-// Barrier over `nthreads` threads (a multiple of 32) on hardware barrier `id`.
-__device__ inline void named_sync(int id, int nthreads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+// Barrier over `nthreads` threads (a multiple of 32) on hardware barrier `id`:
+// whether any of them has `flag`.
+__device__ inline bool named_any(int id, int nthreads, bool flag) {
+    uint32_t any;
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(flag ? 1u : 0u), "r"(id), "r"(nthreads)
+        : "memory");
+    return any != 0;
 }
 
 // QG: queries per group (MMA N: 128, 64 or 32); OP: bf16 operands (kind::f16,
@@ -955,7 +975,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
     float* s_ip = reinterpret_cast<float*>(s_ck + N_EPI * CB);       // [N_EPI][32 lanes][CC] candidate chunks
 
     __shared__ uint64_t full[NS_MAX], empty[NS_MAX], accf[2], acce[2], sfull[SLOT_MAX], sfree[SLOT_MAX],
-        smeta[SLOT_MAX], bfree[SLOT_MAX];
+        smeta[SLOT_MAX], bfree[SLOT_MAX], drain;
     __shared__ uint32_t tbase;
     __shared__ int s_abort;
     __shared__ long long s_g[SLOT_MAX];
@@ -979,6 +999,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             mbar_init(&smeta[i], 32 * N_GATHER);
             mbar_init(&bfree[i], 1);
         }
+        mbar_init(&drain, 1);
         s_abort = 0;
         fence_mbar_init();
     }
@@ -994,14 +1015,14 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
         const int gt = threadIdx.x - 32 * W_GATHER0;  // 0..63
         for (uint32_t it = 0;; ++it) {
             const int b = static_cast<int>(it % nsl);
-            if (!wait_or_abort(&sfree[b], ((it / nsl) & 1u) ^ 1u, p.err, vabort)) break;
+            const bool free = wait_or_abort(&sfree[b], ((it / nsl) & 1u) ^ 1u, p, vabort);
             Slot& S = slot[b];
             // One index per slot: a gather thread may still be reading this
             // item's index while thread 0 already fetches the next one.
-            if (gt == 0) s_g[b] = atomicAdd(p.work, 1u);
-            named_sync(1, 32 * N_GATHER);
+            if (gt == 0 && free) s_g[b] = atomicAdd(p.work, 1u);
+            if (named_any(1, 32 * N_GATHER, !free || *vabort)) break;
             const long long g = s_g[b];
-            if (g >= total_items || *vabort) {
+            if (g >= total_items) {
                 if (gt == 0) S.ntiles = -1;
                 mbar_arrive_cta(&smeta[b]);
                 mbar_arrive_cta(&sfull[b]);
@@ -1088,9 +1109,12 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             // asynchronous copy, eight lanes to a 128-byte row so that a
             // warp reads whole rows, all in flight at once; empty query slots
             // are zero-filled.
-            named_sync(1, 32 * N_GATHER);  // S.qid
             const int bb = static_cast<int>(it % nbuf);
-            if (!wait_or_abort(&bfree[bb], ((it / nbuf) & 1u) ^ 1u, p.err, vabort)) break;
+            const bool bok = wait_or_abort(&bfree[bb], ((it / nbuf) & 1u) ^ 1u, p, vabort);
+            if (named_any(1, 32 * N_GATHER, !bok)) {  // (and S.qid is written)
+                cp_async_wait_all();
+                break;
+            }
             unsigned char* dst = sB + static_cast<size_t>(bb) * nkbq * BKB;
             const size_t qstride = static_cast<size_t>(nkbq) * 128;
             const int c = gt & 7;
@@ -1117,14 +1141,14 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
         bool ok = true;
         for (uint32_t it = 0; ok; ++it) {
             const int b = static_cast<int>(it % nsl);
-            if (!__all_sync(FULL, wait_or_abort(&smeta[b], (it / nsl) & 1u, p.err, vabort))) break;
+            if (!__all_sync(FULL, wait_or_abort(&smeta[b], (it / nsl) & 1u, p, vabort))) break;
             const int ntiles = slot[b].ntiles;
             if (ntiles < 0) break;
             const int64_t tile0 = slot[b].row0 / TM;
             const unsigned char* src = p.abf + tile0 * nkb * KB_BYTES;
             for (int t = 0; t < ntiles && ok; ++t) {
                 for (int kb = 0; kb < nkb; kb += ks) {
-                    ok = __all_sync(FULL, wait_or_abort(&empty[ls], lph ^ 1u, p.err, vabort));
+                    ok = __all_sync(FULL, wait_or_abort(&empty[ls], lph ^ 1u, p, vabort));
                     if (!ok) break;
                     const int n = min(ks, nkb - kb);
                     unsigned char* dst = sA + static_cast<size_t>(ls * ks) * KB_BYTES;
@@ -1141,6 +1165,9 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                 }
             }
         }
+        // After a wait that gave up: no copy outlives the CTA.
+        if (*vabort)
+            for (int s = 0; s < ns; ++s) mbar_wait_bounded(&full[s], s < ls ? lph : lph ^ 1u, p.err);
     } else if (warp == W_MMA) {
         // ---------------- MMA issuer (the whole warp keeps the loop, an
         // elected lane issues; descriptors are one base plus offsets in
@@ -1155,18 +1182,18 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
         bool ok = true;
         for (uint32_t it = 0; ok; ++it) {
             const int b = static_cast<int>(it % nsl);
-            if (!__all_sync(FULL, wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort))) break;
+            if (!__all_sync(FULL, wait_or_abort(&sfull[b], (it / nsl) & 1u, p, vabort))) break;
             const int ntiles = slot[b].ntiles;
             if (ntiles < 0) break;
             const int bb = static_cast<int>(it % nbuf);
             const uint64_t b0 = bdesc + static_cast<uint32_t>(bb * nkbq) * (BKB >> 4);
             for (int t = 0; t < ntiles && ok; ++t, ++tile_it) {
                 const int buf = tile_it & 1;
-                ok = __all_sync(FULL, wait_or_abort(&acce[buf], ((tile_it >> 1) & 1u) ^ 1u, p.err, vabort));
+                ok = __all_sync(FULL, wait_or_abort(&acce[buf], ((tile_it >> 1) & 1u) ^ 1u, p, vabort));
                 if (!ok) break;
                 const uint32_t dcol = tmem + static_cast<uint32_t>(buf * QG);
                 for (int kb0 = 0; kb0 < nkb; kb0 += ks) {
-                    ok = __all_sync(FULL, wait_or_abort(&full[ms], mph, p.err, vabort));
+                    ok = __all_sync(FULL, wait_or_abort(&full[ms], mph, p, vabort));
                     if (!ok) break;
                     tc::fence_after_sync();
                     const uint64_t a0 = adesc + static_cast<uint32_t>(ms * ks) * (KB_BYTES >> 4);
@@ -1202,6 +1229,10 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                 }
             }
         }
+        // No tensor-core instruction outlives the CTA either.
+        if (tc::elect_one()) tc::mma_commit(&drain);
+        __syncwarp();
+        mbar_wait_bounded(&drain, 0, p.err);
     } else if (warp >= W_EPI0) {
         // ---------------- epilogue: thread = row of the tile; each warp of a
         // TMEM lane quadrant handles half of the QG query columns.
@@ -1240,7 +1271,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
         uint32_t tile_it = 0;
         for (uint32_t it = 0;; ++it) {
             const int b = static_cast<int>(it % nsl);
-            if (!wait_or_abort(&sfull[b], (it / nsl) & 1u, p.err, vabort)) break;
+            if (!__all_sync(FULL, wait_or_abort(&sfull[b], (it / nsl) & 1u, p, vabort))) break;
             const Slot& S = slot[b];
             const int ntiles = S.ntiles;
             if (ntiles < 0) break;
@@ -1248,13 +1279,12 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             const int nact = (S.nqv + 1 - half) >> 1;
             const int nrows = S.nrows;
             const long long row0 = S.row0;
-            bool ok = true;
             for (int t = 0; t < ntiles; ++t, ++tile_it) {
                 const int buf = tile_it & 1;
-                if (!wait_or_abort(&accf[buf], (tile_it >> 1) & 1u, p.err, vabort)) {
-                    ok = false;
-                    break;
-                }
+                // (A tile whose wait gave up is scanned all the same, which
+                // keeps the warp whole: its rows and queries are valid ones,
+                // and the call reports the status.)
+                wait_or_abort(&accf[buf], (tile_it >> 1) & 1u, p, vabort);
                 tc::fence_after_sync();
                 const int rs_row = t * TM + quad * 32 + lane;
                 const bool rvalid = rs_row < nrows;
@@ -1396,7 +1426,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
                 }
             }
             if (lane == 0) mbar_arrive_cta(&sfree[b]);
-            if (!ok) break;
+            if (__any_sync(FULL, *vabort)) break;
         }
         // Drain: the reserved segments, then the partly filled one.
         const int last = (wc / SEG + NSEG - 1) % NSEG;  // newest reserved segment
@@ -2099,8 +2129,12 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
         if (!ok) {
             // A copy that did not complete in time: the status word is
             // raised; wait (bounded) for whatever is still in flight, and
-            // write nothing.
+            // leave no probe.
             while (used < issued && mbar_wait_bounded(bar, used & 1u, nullptr)) ++used;
+            for (int e = lane; e < m; e += 32) {
+                out_idx[static_cast<int64_t>(qi) * m + e] = -1;
+                if (out_score) out_score[static_cast<int64_t>(qi) * m + e] = FLT_MAX;
+            }
             return;
         }
         __syncwarp();
@@ -3113,6 +3147,7 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
     p.cand_cnt = w.cand_cnt;
     p.work = w.work;
     p.err = err;
+    p.wait_limit = b.wait_limit;
     p.nlist = b.nlist;
     p.ksplit = b.ksplit ? 1 : 0;
     p.nkb = b.nkb << p.ksplit;

@@ -191,6 +191,7 @@ struct BatchedLaunch {
     int qg = 128;     // queries per group (batched_group_size)
     Operand op = Operand::bf16;
     int nkb = 0;      // 128-byte k-blocks of a query (operand_kblocks)
+    uint32_t wait_limit = WAIT_LIMIT;  // polls of a bounded wait
     bool ksplit = false;  // abf is a split image (launch_centroid_image): two k-blocks per query k-block
     // Lists of at most dense_max rows (capped at capq) are scanned densely:
     // every row's f32 score lands at the row's offset in the list within the

@@ -1134,6 +1134,7 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     w.cand = h->c_cand.as<uint64_t>();
     w.cand_cnt = h->c_ccnt.as<int32_t>();
     hy::BatchedLaunch b;
+    b.wait_limit = h->wait_limit;
     b.abf = h->c_img.p;
     b.list_off = h->c_off.as<int64_t>();
     b.list_size = h->c_size.as<int32_t>();
@@ -1374,6 +1375,7 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
         if (timed && q0 == 0) HY_CUDA(ev_record(h->ev[1], s));
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[2], s));
         hy::BatchedLaunch b;
+        b.wait_limit = h->wait_limit;
         b.abf = f8 ? h->a8.p : tf32 ? h->codes.p : h->abf.p;
         b.list_off = h->list_off.as<int64_t>();
         b.list_size = h->list_size.as<int32_t>();

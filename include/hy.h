@@ -368,8 +368,9 @@ HY_API int hy_selftest_tcgen05_e4m3(const float* A, const float* B, float* D);
 
 /* Diagnostic with no counterpart in the reference: the polls after which a
  * bounded device-side wait of the handle's tensor-core row assignment gives up
- * (train and add then return HY_ERR_TIMEOUT and leave the index as it was);
- * values above the library's own limit set that limit. */
+ * (train and add then return HY_ERR_TIMEOUT and leave the index as it was), and
+ * one of its batched tensor-core scans (host-pointer searches then return
+ * HY_ERR_TIMEOUT); values above the library's own limit set that limit. */
 HY_API int hy_selftest_wait_limit(hy_index* h, unsigned int polls);
 
 #ifdef __cplusplus
