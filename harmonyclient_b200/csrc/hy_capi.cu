@@ -66,12 +66,17 @@ struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
     bool owned = true;
-    DevBuf() = default;
+    // Counts the moves of a handle's buffers: each member of a hy_index takes
+    // the counter that is being constructed around it.
+    uint64_t* const moves;
+    inline static thread_local uint64_t* owner = nullptr;
+    DevBuf() : moves(owner) {}
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     int ensure(size_t n) {
         if (n <= bytes) return HY_OK;
+        moved();
         release();
         owned = true;
         size_t want = std::max<size_t>(n, 256);
@@ -93,9 +98,13 @@ struct DevBuf {
     }
     // A piece of another buffer (not freed here).
     void alias(void* at, size_t n) {
+        if (at != p) moved();
         p = at;
         bytes = n;
         owned = false;
+    }
+    void moved() {
+        if (p && moves) ++*moves;
     }
     template <class T>
     T* as() const {
@@ -140,6 +149,11 @@ struct HostStatus {
 };
 
 struct hy_index {
+    hy_index() { DevBuf::owner = nullptr; }
+    uint64_t buffer_moves = 0;  // buffers below that were freed or replaced
+    struct OwnBuffers {
+        explicit OwnBuffers(uint64_t* moves) { DevBuf::owner = moves; }
+    } own_buffers{&buffer_moves};
     std::mutex mu;
     int device = 0;
     size_t d = 0, nlist = 0, nprobe = 0;
@@ -187,14 +201,14 @@ struct hy_index {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     struct GraphKey {
-        uint64_t epoch;
+        uint64_t epoch, moves;
         size_t n, k, nprobe;
         const void *dq, *dD, *dI, *np;
         cudaStream_t s;
         size_t learned_rows;
         int learned;
         bool operator==(const GraphKey& o) const {
-            return epoch == o.epoch && n == o.n && k == o.k && nprobe == o.nprobe && dq == o.dq && dD == o.dD &&
+            return epoch == o.epoch && moves == o.moves && n == o.n && k == o.k && nprobe == o.nprobe && dq == o.dq && dD == o.dD &&
                    dI == o.dI && np == o.np && s == o.s && learned_rows == o.learned_rows && learned == o.learned;
         }
     } gkey{};
@@ -1523,14 +1537,16 @@ void drop_graph(hy_index* h) {
 // The device-pointer search, through a CUDA graph in graph mode: the first
 // call with a new (buffers, sizes, stream, index state) runs normally (every
 // buffer reaches its size), then captures the same launch sequence; later
-// identical calls replay it with one cudaGraphLaunch.  The legacy default
+// identical calls replay it with one cudaGraphLaunch, as long as none of the
+// handle's own buffers has moved (other calls may grow the shared workspaces).  The legacy default
 // stream cannot be captured: such calls run the graph on the handle's stream,
 // ordered after and before the default stream's work by events.
 int run_device_search(hy_index* h, size_t n, const float* dq, size_t k, float* dD, int64_t* dI, cudaStream_t s) {
     h->stats.graph_replayed = 0;
     h->ev = h->ev_direct;
     if (!h->graph_on) return search_device_impl(h, n, dq, k, dD, dI, s, true);
-    const hy_index::GraphKey key{h->epoch, n, k, h->nprobe, dq, dD, dI, h->q_nprobe, s, h->learned_rows, h->learned};
+    hy_index::GraphKey key{h->epoch, h->buffer_moves, n,    k, h->nprobe,       dq,
+                           dD,       dI,              h->q_nprobe, s, h->learned_rows, h->learned};
     cudaStream_t run = s ? s : h->stream;
     if (h->gexec && key == h->gkey) {
         if (!s) {
@@ -1573,6 +1589,7 @@ int run_device_search(hy_index* h, size_t n, const float* dq, size_t k, float* d
         return fail(HY_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
     }
     h->graph = g;
+    key.moves = h->buffer_moves;  // (the direct run may have grown buffers)
     h->gkey = key;
     h->graph_kernels = h->launches;
     h->graph_kev = h->kev;
