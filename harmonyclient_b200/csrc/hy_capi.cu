@@ -76,13 +76,13 @@ struct DevBuf {
     ~DevBuf() { release(); }
     int ensure(size_t n) {
         if (n <= bytes) return HY_OK;
-        moved();
         release();
         owned = true;
         size_t want = std::max<size_t>(n, 256);
         cudaError_t e = cudaMalloc(&p, want);
         if (e != cudaSuccess) {
             p = nullptr;
+            cudaGetLastError();  // reported here, not by the next launch's check
             return fail(HY_ERR_OOM, std::string("cudaMalloc(") + std::to_string(want) + "): " + cudaGetErrorString(e));
         }
         bytes = want;
@@ -98,19 +98,17 @@ struct DevBuf {
     }
     // A piece of another buffer (not freed here).
     void alias(void* at, size_t n) {
-        if (at != p) moved();
+        if (at != p) release();
         p = at;
         bytes = n;
         owned = false;
-    }
-    void moved() {
-        if (p && moves) ++*moves;
     }
     template <class T>
     T* as() const {
         return static_cast<T*>(p);
     }
     void release() {
+        if (p && moves) ++*moves;
         if (p && owned) cudaFree(p);
         p = nullptr;
         bytes = 0;
@@ -243,6 +241,7 @@ struct hy_index {
     bool cert_valid = false;
     DevBuf x32aux, t32aux, a32stat;  // the arena read as TF32: bound terms, sums of launch_row_aux_tf32
     bool a32_valid = false, a32_fits = false;  // built; the plain form's batches may run on it
+    size_t a32_refused = SIZE_MAX;  // plain batches (per chunk) from here on found no memory for it
     DevBuf b_cqb, b_cqn;  // bf16 queries of the coarse step when the scan's operands are others
     DevBuf b_qx;              // per-query exact-distance flags
     DevBuf a8, x8aux, t8aux;  // the same for the e4m3 image
@@ -566,6 +565,7 @@ int build_arena(hy_index* h, const float* x, size_t n, const int32_t* order, con
     h->abf_valid = false;
     h->cert_valid = false;
     h->a32_valid = false;
+    h->a32_refused = SIZE_MAX;
     h->a8_valid = false;
     h->c2c_valid = false;
     HY_RET(h->codes.ensure(rows_alloc * h->L.row_pitch * sizeof(float)));
@@ -640,6 +640,13 @@ int check_search_args(hy_index* h, size_t n, size_t k) {
     return HY_OK;
 }
 
+// Bytes of the sorted lists of a scan of up to n counted queries (nq_dev below).
+size_t fallback_parts_bytes(const hy_index* h, size_t n, size_t k, size_t nprobe) {
+    const size_t kp = k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 256;
+    const size_t all = n * (size_t)hy::scan_probe_parts(h->L, (int)k, (int)nprobe);
+    return std::max(all, (size_t)h->nsm) * kp * sizeof(uint64_t);
+}
+
 // Search n device queries with device probe lists (nprobe per query) into
 // device D/I.  Runs on stream s; does not synchronise.
 // nq_dev (optional): a device count of the queries to search (the first
@@ -670,7 +677,7 @@ int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t npro
         }
     }
     const size_t all = n * (size_t)pparts;
-    HY_RET(h->w_parts.ensure((nq_dev ? std::max(all, nsm) : all * tsplit) * kp * sizeof(uint64_t)));
+    HY_RET(h->w_parts.ensure(nq_dev ? fallback_parts_bytes(h, n, k, nprobe) : all * tsplit * kp * sizeof(uint64_t)));
     uint32_t* gthr = nullptr;
     if (nq_dev) {
         gthr = h->w_gthr.as<uint32_t>();  // set by the gather of the counted queries
@@ -899,6 +906,8 @@ int ensure_common(hy_index* h) {
 int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, size_t k, float* dD, int64_t* dI,
                        cudaStream_t s, bool timed);
 bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s);
+bool capturing(cudaStream_t s);
+void release_batch_buffers(hy_index* h);
 
 // The scan counters and the fallback count (which follow one another) to zero.
 int clear_counters(hy_index* h, cudaStream_t s) {
@@ -942,9 +951,17 @@ int search_device_impl(hy_index* h, size_t n, const float* dq, size_t k, float* 
     HY_CHECK(h->nlist <= 40000, HY_ERR_ARG, "search: nlist above 40000 is not supported by the coarse selector");
     HY_RET(ensure_common(h));
     size_t qc = query_chunk(h->nlist, n);
-    h->fb_last = plain_on_tensor(h, std::min(qc, std::max<size_t>(1, (size_t(2) << 30) / (h->capq * 8))), nprobe, s);
-    if (h->fb_last)
-        return search_tensor_impl(h, hy::Operand::tf32, n, dq, k, dD, dI, s, timed);
+    const size_t tqc = std::min(qc, std::max<size_t>(1, (size_t(2) << 30) / (h->capq * 8)));
+    h->fb_last = plain_on_tensor(h, tqc, nprobe, s);
+    if (h->fb_last) {
+        // Its buffers (up to 2 GiB of candidates) are taken before its first
+        // launch; without the memory for them the other scans run, as for
+        // every such batch until the lists change.
+        const int rc = search_tensor_impl(h, hy::Operand::tf32, n, dq, k, dD, dI, s, timed);
+        if (rc != HY_ERR_OOM || capturing(s)) return rc;
+        release_batch_buffers(h);
+        h->a32_refused = tqc;
+    }
     // List-major scan: chunks sized so the candidate buffers stay within 2 GiB.
     const bool lm = use_list_major(h, qc, nprobe);
     if (lm) qc = std::min(qc, std::max<size_t>(1, (size_t(2) << 30) / (h->capq * 8)));
@@ -1019,6 +1036,11 @@ int ensure_certificate(hy_index* h, size_t rows, cudaStream_t s) {
     return HY_OK;
 }
 
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
 // What a batched search with these operands reads besides the arena, built on
 // first use after add/load: the bf16 or e4m3 image, the rows' bound terms, the
 // certificate.
@@ -1084,20 +1106,31 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
 // answer): from TF32_MIN_BYTES of pairs.  Not with the inner-product window of
 // OPT_TRIANGLE, whose answer off the unit sphere depends on the scan's own
 // thresholds.  The bound terms are built on first use; while the stream is
-// being captured, or without the memory for them, the other scans run.
+// being captured, or without the memory for them, the other scans run (a batch
+// for whose own buffers there is no memory: search_device_impl).
 bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s) {
     if (h->form != HY_FORM_PLAIN || h->plain_scan != HY_PLAIN_AUTO || h->arena_rows == 0 || ip_window(h)) return false;
     if (pair_bytes(h, m, nprobe) < TF32_MIN_BYTES) return false;
     if (hy::batched_group_size(hy::operand_kblocks(hy::Operand::tf32, h->L)) == 0) return false;
+    if (m >= h->a32_refused) return false;
     if (!h->a32_valid) {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return false;
+        if (capturing(s)) return false;
         if (ensure_operands(h, hy::Operand::tf32, s) != HY_OK) {
             cudaGetLastError();
+            h->a32_refused = 0;
             return false;
         }
     }
     return h->a32_fits;
+}
+
+// Gives back what only batched searches use (not the operands).
+void release_batch_buffers(hy_index* h) {
+    DevBuf* const bufs[] = {&h->b_cqb,   &h->b_cqn,  &h->b_qx,    &h->b_qs,   &h->b_qb,    &h->b_qn,   &h->b_thr,
+                            &h->b_pfill, &h->b_poff, &h->b_pairs, &h->b_icnt, &h->b_ioff,  &h->b_cand, &h->b_items,
+                            &h->b_zero,  &h->b_done, &h->b_fq,    &h->b_fpr,  &h->b_fD,    &h->b_fI,   &h->b_fcnt,
+                            &h->c_pcnt,  &h->c_poff, &h->c_pairs, &h->c_ioff, &h->c_items, &h->c_cand, &h->c_ccnt};
+    for (DevBuf* b : bufs) b->release();
 }
 
 // Whether a batched search's coarse step runs on the tensor cores (the
@@ -1107,6 +1140,24 @@ bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
            (h->form == HY_FORM_BF16 || h->nlist <= 2048) && hy::batched_group_size((int)(h->d + 63) / 64) > 0;
 }
 
+// The buffers of a tensor-core coarse step of up to m queries.
+int ensure_coarse(hy_index* h, size_t m) {
+    const int nkb = (int)(h->d + 63) / 64;
+    const int qg = hy::batched_group_size(nkb);
+    const size_t ngroups = (m + qg - 1) / qg, tiles = (h->nlist + 127) / 128;
+    const size_t most = (size_t)hy::batched_row_slice(nkb, qg) / 128;
+    HY_RET(h->c_pcnt.ensure(sizeof(int32_t)));
+    HY_RET(h->c_poff.ensure(2 * sizeof(int64_t)));
+    HY_RET(h->c_pairs.ensure(m * sizeof(int32_t)));
+    HY_RET(h->c_ioff.ensure(2 * sizeof(int64_t)));
+    // Items: groups x slices, of which there are at most nsm / groups + 1 or
+    // the tiles' / most + 1.
+    HY_RET(h->c_items.ensure(((size_t)h->nsm + ngroups * (tiles / most + 2)) * sizeof(int4)));
+    HY_RET(h->c_cand.ensure(m * h->nlist * sizeof(float2)));
+    HY_RET(h->c_ccnt.ensure(m * sizeof(int32_t)));
+    return HY_OK;
+}
+
 // Coarse step on the tensor cores for m queries whose bf16 image and
 // {|q|^2, |q|, |q~|, |q - q~|} are in qb / qn: one dense batched launch
 // over the centroid index, then the exact m best per query.  work: two
@@ -1114,6 +1165,7 @@ bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
 int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const float4* qn, size_t nprobe,
                   bool ordered, const int32_t* counts, int64_t* probes, float* pscore, unsigned int* work, cudaStream_t s) {
     HY_RET(ensure_centroid_image(h, s));
+    HY_RET(ensure_coarse(h, m));
     const int nlist = (int)h->nlist;
     const int nkb = (int)(h->d + 63) / 64;
     const int qg = hy::batched_group_size(nkb);
@@ -1131,13 +1183,6 @@ int coarse_tensor(hy_index* h, size_t m, const float* qq, const void* qb, const 
     };
     int rs_full;
     const int ns_full = slicing(nlist, &rs_full);
-    HY_RET(h->c_pcnt.ensure(sizeof(int32_t)));
-    HY_RET(h->c_poff.ensure(2 * sizeof(int64_t)));
-    HY_RET(h->c_pairs.ensure(m * sizeof(int32_t)));
-    HY_RET(h->c_ioff.ensure(2 * sizeof(int64_t)));
-    HY_RET(h->c_items.ensure((size_t)ngroups * ns_full * sizeof(int4)));
-    HY_RET(h->c_cand.ensure(m * nlist * sizeof(float2)));
-    HY_RET(h->c_ccnt.ensure(m * sizeof(int32_t)));
     hy::BatchWork w{};
     w.items = h->c_items.as<int4>();
     w.pair_cnt = h->c_pcnt.as<int32_t>();
@@ -1274,6 +1319,11 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     HY_RET(h->b_fD.ensure(fbcap * k * sizeof(float)));
     HY_RET(h->b_fI.ensure(fbcap * k * sizeof(int64_t)));
     HY_RET(h->b_fcnt.ensure(sizeof(int32_t)));
+    HY_RET(h->w_parts.ensure(fallback_parts_bytes(h, fbcap, k, nprobe)));
+    if (coarse_tc) {
+        HY_RET(ensure_centroid_image(h, s));
+        HY_RET(ensure_coarse(h, qc));
+    }
     // Warm-up for the bf16 form: its threshold only bounds the first pass
     // (each query's nearest list), so three lists suffice by default.  A
     // query whose nearest list has between k and dense_max rows needs none:
