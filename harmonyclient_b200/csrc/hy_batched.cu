@@ -12,7 +12,7 @@
 // tcgen05.mma (M = 128 rows, N = up to 128 queries) into one of two TMEM
 // accumulators; eight epilogue warps read the accumulator (thread = row) and
 // form dist = |x|^2 + |q|^2 - 2 q.x (or -q.x for inner product) with a
-// rigorous bound on its distance from the plain scan's exact FP32 value.
+// bound (err_coef) on its distance from the plain scan's exact FP32 value.
 //
 // First pass (each query's nearest list): dense items write the distance of
 // every row; the tightening step recomputes each row's bound, takes each
@@ -471,7 +471,7 @@ __global__ void arena_integral_kernel(const float* __restrict__ codes, int64_t n
 // Bound on |bf16 distance - exact FP32 distance| for one (query, row) pair,
 // the exact distance being the plain scan's sequential f32 sum.  With x~, q~
 // the bf16-rounded vectors: |x~.q~ - x.q| <= |x~||q - q~| + |q||x - x~|; the
-// f32 accumulation of K products adds at most cK |x~||q~| (cK = (K+8) 2^-24);
+// f32 accumulation of K products adds at most cK |x~||q~| (tc::accum_units);
 // the f32 norms, the final |x|^2 + |q|^2 - 2 x.q and the plain scan's own
 // d-term sum add at most cN (|x|^2 + |q|^2) (cN = (3d+16) 2^-24).  L2 doubles
 // the inner-product terms.  Both constants carry a 2^-7 inflation for the
@@ -2863,7 +2863,7 @@ cudaError_t launch_bf16_image(const ArenaLayout& L, const float* codes, int64_t 
 // err_coef).
 static void err_consts(int d, int K, float* cK, float* cN) {
     const double u = 1.0 / 16777216.0, inflate = 1.0 + 1.0 / 128.0;
-    *cK = static_cast<float>((K + 8) * u * inflate);
+    *cK = static_cast<float>(tc::accum_units(K) * u * inflate);
     *cN = static_cast<float>((3.0 * d + 16) * u * inflate);
 }
 

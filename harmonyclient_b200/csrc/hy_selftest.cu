@@ -13,8 +13,11 @@
 namespace hy {
 namespace {
 
-// F8: operands are e4m3 (K = 256 in two 128-byte k-blocks), else bf16 (K = 128).
-template <bool F8>
+// Operands: bf16 (K = 128 in two 128-byte k-blocks), e4m3 (K = 256) or tf32
+// (K = 64).
+enum class Op { bf16, e4m3, tf32 };
+constexpr int op_k(Op op) { return op == Op::bf16 ? 128 : op == Op::e4m3 ? 256 : 64; }
+template <Op OP>
 __global__ void __launch_bounds__(128) tc_selftest_kernel(const float* __restrict__ A, const float* __restrict__ B,
                                                           float* __restrict__ D, int* err) {
     extern __shared__ unsigned char sm_raw[];
@@ -25,13 +28,20 @@ __global__ void __launch_bounds__(128) tc_selftest_kernel(const float* __restric
     __shared__ uint32_t tbase;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    if constexpr (F8) {
+    if constexpr (OP == Op::e4m3) {
         for (int i = threadIdx.x; i < 128 * 256; i += blockDim.x) {
             const int r = i >> 8, k = i & 255;
             const int kb = k >> 7, by = k & 127;
             const uint32_t off = kb * 16384 + r * 128 + ((((by >> 4) ^ (r & 7)) & 7) << 4) + (by & 15);
             sA[off] = __nv_cvt_float_to_fp8(A[i], __NV_SATFINITE, __NV_E4M3);
             sB[off] = __nv_cvt_float_to_fp8(B[i], __NV_SATFINITE, __NV_E4M3);
+        }
+    } else if constexpr (OP == Op::tf32) {
+        for (int i = threadIdx.x; i < 128 * 64; i += blockDim.x) {
+            const int r = i >> 6, k = i & 63;
+            const uint32_t off = (k >> 5) * 16384 + r * 128 + (((((k & 31) >> 2) ^ (r & 7)) & 7) << 4) + (k & 3) * 4;
+            *reinterpret_cast<float*>(sA + off) = A[i];
+            *reinterpret_cast<float*>(sB + off) = B[i];
         }
     } else {
         for (int i = threadIdx.x; i < 128 * 128; i += blockDim.x) {
@@ -53,13 +63,17 @@ __global__ void __launch_bounds__(128) tc_selftest_kernel(const float* __restric
     tc::fence_after_sync();
     const uint32_t t = tbase;
     if (threadIdx.x == 0) {
-        const uint32_t idesc = F8 ? tc::idesc_e4m3_f32(128, 128) : tc::idesc_bf16_f32(128, 128);
+        const uint32_t idesc = OP == Op::e4m3   ? tc::idesc_e4m3_f32(128, 128)
+                               : OP == Op::tf32 ? tc::idesc_tf32_f32(128, 128)
+                                                : tc::idesc_bf16_f32(128, 128);
         for (int kb = 0; kb < 2; ++kb)
             for (int kk = 0; kk < 4; ++kk) {
                 const uint64_t a = tc::sdesc_sw128(smem_u32(sA + kb * 16384 + kk * 32));
                 const uint64_t b = tc::sdesc_sw128(smem_u32(sB + kb * 16384 + kk * 32));
-                if constexpr (F8)
+                if constexpr (OP == Op::e4m3)
                     tc::mma_e4m3(t, a, b, idesc, (kb | kk) != 0 ? 1u : 0u);
+                else if constexpr (OP == Op::tf32)
+                    tc::mma_tf32(t, a, b, idesc, (kb | kk) != 0 ? 1u : 0u);
                 else
                     tc::mma_bf16(t, a, b, idesc, (kb | kk) != 0 ? 1u : 0u);
             }
@@ -85,12 +99,12 @@ __global__ void __launch_bounds__(128) tc_selftest_kernel(const float* __restric
 
 namespace {
 
-template <bool F8>
+template <hy::Op OP>
 int run_selftest(const float* A, const float* B, float* D) {
     if (!A || !B || !D) return HY_ERR_ARG;
     float *dA = nullptr, *dB = nullptr, *dD = nullptr;
     int* derr = nullptr;
-    const size_t in_bytes = (F8 ? 128 * 256 : 128 * 128) * sizeof(float);
+    const size_t in_bytes = 128 * hy::op_k(OP) * sizeof(float);
     const size_t out_bytes = 128 * 128 * sizeof(float);
     int rc = HY_OK;
     if (cudaMalloc(&dA, in_bytes) != cudaSuccess || cudaMalloc(&dB, in_bytes) != cudaSuccess ||
@@ -103,8 +117,8 @@ int run_selftest(const float* A, const float* B, float* D) {
         cudaMemset(dD, 0, out_bytes);
         cudaMemset(derr, 0, sizeof(int));
         const int smem = 65536 + 1024;
-        cudaFuncSetAttribute(hy::tc_selftest_kernel<F8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        hy::tc_selftest_kernel<F8><<<1, 128, smem>>>(dA, dB, dD, derr);
+        cudaFuncSetAttribute(hy::tc_selftest_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        hy::tc_selftest_kernel<OP><<<1, 128, smem>>>(dA, dB, dD, derr);
         cudaError_t e = cudaDeviceSynchronize();
         int herr = 0;
         if (e == cudaSuccess) e = cudaMemcpy(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost);
@@ -121,6 +135,12 @@ int run_selftest(const float* A, const float* B, float* D) {
 
 }  // namespace
 
-extern "C" int hy_selftest_tcgen05(const float* A, const float* B, float* D) { return run_selftest<false>(A, B, D); }
+extern "C" int hy_selftest_tcgen05(const float* A, const float* B, float* D) { return run_selftest<hy::Op::bf16>(A, B, D); }
 
-extern "C" int hy_selftest_tcgen05_e4m3(const float* A, const float* B, float* D) { return run_selftest<true>(A, B, D); }
+extern "C" int hy_selftest_tcgen05_e4m3(const float* A, const float* B, float* D) { return run_selftest<hy::Op::e4m3>(A, B, D); }
+
+extern "C" int hy_selftest_tcgen05_tf32(const float* A, const float* B, float* D) {
+    return run_selftest<hy::Op::tf32>(A, B, D);
+}
+
+extern "C" double hy_selftest_accum_units(int K) { return hy::tc::accum_units(K); }

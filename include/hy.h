@@ -365,6 +365,12 @@ HY_API int hy_selftest_tcgen05(const float* A, const float* B, float* D);
 /* The same on e4m3 operands: A and B are 128 x 256 (values rounded to e4m3
  * with saturation), D = A B^T is 128 x 128, accumulated by kind::f8f6f4. */
 HY_API int hy_selftest_tcgen05_e4m3(const float* A, const float* B, float* D);
+/* The same on tf32 operands: A and B are 128 x 64 (the low 13 bits of a value
+ * do not take part), accumulated by kind::tf32. */
+HY_API int hy_selftest_tcgen05_tf32(const float* A, const float* B, float* D);
+/* The bound that the searches keep for the accumulation of K such products, in
+ * units of 2^-24 |a||b|. */
+HY_API double hy_selftest_accum_units(int K);
 
 /* Diagnostic with no counterpart in the reference: the polls after which a
  * bounded device-side wait of the handle's tensor-core row assignment gives up
