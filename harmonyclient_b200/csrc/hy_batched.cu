@@ -50,6 +50,12 @@ constexpr int NKB_MAX = 12;  // k-blocks of a row: at most (bf16 d <= 768, e4m3 
 // the copies (130 each) and MMAs, which one 16 KiB k-block does not cover.
 __host__ __device__ constexpr int stage_kblocks(int nkb) { return nkb >= 2 ? 2 : 1; }
 
+// Added to the norms that carry the accumulation's bound (cK, see err_coef): what
+// underflow takes from squares, products, sums and norms is below cK times
+// this floor (2^-126 a product, at most 2^-74 sqrt(d) a norm), also where row
+// and query are both tiny.  Norms above 1e-6 do not change by it.
+constexpr float NORM_FLOOR = 1e-14f;
+
 // ---------------------------------------------------------------------------
 // The FP32 arena's rows as tensor-core images.
 
@@ -133,7 +139,7 @@ __global__ void __launch_bounds__(256) image_kernel(const __grid_constant__ Aren
         nn += __shfl_xor_sync(FULL, nn, o);
         ee += __shfl_xor_sync(FULL, ee, o);
     }
-    if (c == 0) aux[r] = make_float2(sqrtf(nn), sqrtf(ee));
+    if (c == 0) aux[r] = make_float2(sqrtf(nn) + NORM_FLOOR, sqrtf(ee));
 }
 
 // Largest |value| of each 128-row tile, a CTA per tile: the tile is one run of
@@ -179,7 +185,8 @@ __global__ void list_scale_kernel(const int64_t* __restrict__ list_off, const in
 // cores ignore a value's low 13 bits, so x~ is x with them cleared (an x~
 // rounded to nearest would be at least as near), and {norm of |x| + |x - x~|,
 // norm of x - x~} covers either.  Also, for the rule that sends a plain batch
-// to the tensor cores: stat[0] sums |x - x~| + 2^-11 |x| over the rows and
+// to the tensor cores: stat[0] sums |x - x~| + 2^-11 |x| over the rows (and 3 %
+// of the norms' floor, so that rows spread no wider than that stay off) and
 // stat[1] the rows' distance to their list's centroid.
 // A warp takes 32 rows: four rows' 128-byte groups per step, a 16-byte chunk
 // per lane, the sums of a row's eight lanes added at its end; a CTA adds its
@@ -240,9 +247,9 @@ __global__ void __launch_bounds__(256) row_aux_tf32_kernel(const __grid_constant
             }
             if ((lane & 7) == 0) {
                 const int64_t r = tile * 32 + lr;
-                aux[r] = make_float2(sqrtf(nn), sqrtf(ee));
+                aux[r] = make_float2(sqrtf(nn) + NORM_FLOOR, sqrtf(ee));
                 if (r < end) {
-                    s0 += static_cast<double>(sqrtf(ee) + 0.00048828125f * sqrtf(vv));
+                    s0 += static_cast<double>(sqrtf(ee) + 0.00048828125f * sqrtf(vv) + 0.03f * NORM_FLOOR);
                     s1 += static_cast<double>(sqrtf(dd));
                 }
             }
@@ -483,12 +490,12 @@ __device__ inline ErrCoef err_coef(float4 qa, bool l2, float cK, float cN) {
     const float inflate = 1.0f + 0.0078125f;
     ErrCoef c;
     if (l2) {
-        c.aq = inflate * 2.0f * (qa.w + cK * qa.z);
-        c.bq = inflate * 2.0f * qa.y;
+        c.aq = inflate * 2.0f * (qa.w + cK * (qa.z + NORM_FLOOR));
+        c.bq = inflate * 2.0f * (qa.y + NORM_FLOOR);
         c.cq = cN * qa.x;
     } else {
-        c.aq = inflate * (qa.w + (cK + cN) * qa.z);
-        c.bq = inflate * qa.y;
+        c.aq = inflate * (qa.w + (cK + cN) * (qa.z + NORM_FLOOR));
+        c.bq = inflate * (qa.y + NORM_FLOOR);
         c.cq = 0.0f;
     }
     return c;
@@ -1931,7 +1938,7 @@ __global__ void __launch_bounds__(256) centroid_image_kernel(const float* __rest
         if (in)
 #pragma unroll 8
             for (int j = 0; j < d; ++j) sq = __fadd_rn(sq, __fmul_rn(x[r * d + j], x[r * d + j]));
-        const float2 a = make_float2(sqrtf(nn), sqrtf(ee));
+        const float2 a = make_float2(sqrtf(nn) + NORM_FLOOR, sqrtf(ee));
         aux[r] = a;
         xn[r] = sq;
         atomicMax(&taux[2 * (r >> 7)], __float_as_uint(fabsf(a.x)));
