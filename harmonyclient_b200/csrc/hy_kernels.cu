@@ -1239,9 +1239,11 @@ static size_t scan_smem(const ArenaLayout& L, int k, int nprobe, int pparts) {
 }
 
 int scan_probe_parts(const ArenaLayout& L, int k, int nprobe) {
+    // (Less the kernel's few static words, beside which exactly 227 KiB fails.)
+    constexpr size_t cap = 227 * 1024 - 128;
     int pp = (nprobe + 2047) / 2048;
     if (pp < 1) pp = 1;
-    while (pp < nprobe && scan_smem(L, k, nprobe, pp) > 227 * 1024) ++pp;
+    while (pp < nprobe && scan_smem(L, k, nprobe, pp) > cap) ++pp;
     return pp;
 }
 

@@ -76,3 +76,23 @@ def test_fallback_of_a_counted_few(noverflow):
     assert idx.last_stats()["fallback_queries"] == noverflow
     np.testing.assert_array_equal(Ib, I)
     np.testing.assert_array_equal(Db, D)
+
+
+@pytest.mark.parametrize("d,blocks,nlist,nprobes", [(768, 4, 900, range(880, 900, 2)), (192, 6, 2_100, (2_040, 2_048)),
+                                                     (384, 4, 3_000, (2_990,))])
+def test_probe_tables_that_fill_the_shared_memory(d, blocks, nlist, nprobes):
+    """Large k and probe counts about the largest table that fits beside the
+    kernel's staging: the answer of the smaller k, few queries and many."""
+    rng = np.random.default_rng(d)
+    x = rng.standard_normal((6_000, d)).astype(np.float32)
+    idx = hb.Index(d, nlist, nprobes[0], dim_blocks=blocks)
+    idx.centroid_codes = x[:nlist]
+    idx.add(x)
+    idx.set_plain_scan("query")
+    for nprobe in nprobes:
+        idx.nprobe = nprobe
+        for n in (8, 300):
+            D, I = idx.search(x[:n], 256)
+            D1, I1 = idx.search(x[:n], 64)
+            np.testing.assert_array_equal(D[:, :64], D1)
+            np.testing.assert_array_equal(I[:, :64], I1)
