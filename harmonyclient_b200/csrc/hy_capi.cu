@@ -321,6 +321,16 @@ size_t query_chunk(size_t nlist, size_t n) {
     return std::min(qc, n);
 }
 
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
+// Whether what was just launched on s to build data kept for later calls counts
+// as built: launches that a caller's capture records have not run, and do
+// so at each replay of that graph alone.
+bool built(cudaStream_t s) { return !capturing(s); }
+
 // The centroids' split tensor-core image and its bound terms, built on first
 // use of a centroid set.
 float* centroid_maxima(const hy_index* h) {
@@ -348,7 +358,7 @@ int ensure_centroid_image(hy_index* h, cudaStream_t s) {
     }
     HY_CUDA(hy::launch_centroid_image(h->cent.as<float>(), (int)h->nlist, (int)h->d, h->c_img.p, h->c_aux.as<float2>(),
                                       h->c_taux.as<float2>(), h->c_norm.as<float>(), centroid_maxima(h), s));
-    h->cimg_valid = true;
+    h->cimg_valid = built(s);
     return HY_OK;
 }
 
@@ -841,7 +851,7 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
                                             h->list_size.as<int32_t>(), (int)nlist, (int64_t)h->arena_rows,
                                             h->cent.as<float>(), h->metric, h->c2c.as<float>(),
                                             h->c2c_tile.as<float2>(), s));
-            h->c2c_valid = true;
+            h->c2c_valid = built(s);
         }
         p.triangle = 1;
         p.c2c = h->c2c.as<float>();
@@ -906,7 +916,6 @@ int ensure_common(hy_index* h) {
 int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, size_t k, float* dD, int64_t* dI,
                        cudaStream_t s, bool timed);
 bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s);
-bool capturing(cudaStream_t s);
 void release_batch_buffers(hy_index* h);
 
 // The scan counters and the fallback count (which follow one another) to zero.
@@ -1032,13 +1041,8 @@ int ensure_certificate(hy_index* h, size_t rows, cudaStream_t s) {
     HY_CUDA(hy::launch_arena_integral(h->codes.as<float>(), (int64_t)(rows * h->L.row_pitch), h->norms.as<float>(),
                                       (int64_t)rows, h->b_cert.as<int>(),
                                       reinterpret_cast<unsigned int*>(h->b_cert.as<int>() + 1), s));
-    h->cert_valid = true;
+    h->cert_valid = built(s);
     return HY_OK;
-}
-
-bool capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
 }
 
 // What a batched search with these operands reads besides the arena, built on
@@ -1060,7 +1064,7 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
                                     h->lscale.as<float>(), h->tscale.as<float>(), h->a8.p, h->x8aux.as<float2>(),
                                     h->t8aux.as<float2>(), s));
         HY_RET(ensure_tile_norms(h, rows, s));
-        h->a8_valid = true;
+        h->a8_valid = built(s);
         return HY_OK;
     }
     if (op == hy::Operand::tf32) {
@@ -1097,7 +1101,7 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
                                   h->taux.as<float2>(), s));
     HY_RET(ensure_tile_norms(h, rows, s));
     HY_RET(ensure_certificate(h, rows, s));
-    h->abf_valid = true;
+    h->abf_valid = built(s);
     return HY_OK;
 }
 
