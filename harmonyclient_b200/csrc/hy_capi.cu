@@ -657,22 +657,14 @@ size_t fallback_parts_bytes(const hy_index* h, size_t n, size_t k, size_t nprobe
     return std::max(all, (size_t)h->nsm) * kp * sizeof(uint64_t);
 }
 
-// Search n device queries with device probe lists (nprobe per query) into
-// device D/I.  Runs on stream s; does not synchronise.
-// nq_dev (optional): a device count of the queries to search (the first
-// *nq_dev of the n): one CTA per SM loops over their work units, whose
-// splits follow from the count, and the shared thresholds (w_gthr) hold each
-// query's starting bound (launch_fb_gather).
-int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t nprobe, const int64_t* dprobes,
-                   const uint32_t* init_thr, float* dD, int64_t* dI, cudaStream_t s, bool timed,
-                   int64_t* drows = nullptr, const int32_t* nq_dev = nullptr) {
-    const int kp = k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 256;
-    if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
-    const int pparts = hy::scan_probe_parts(h->L, (int)k, (int)nprobe);
-    // Tile splits: the fewest rounds of the chip (one CTA fills an SM) by what
-    // a unit takes: its set-up and folds, and its tiles 32 at a time (16 warps
-    // of two slots), at the average list size.  100 queries of 35 tiles: whole
-    // 22 us, 5 splits 37; 33 queries of 417 tiles: 4 splits as 18, 68 us.
+// Tile splits of a query-major scan of n queries of pparts probe parts: the
+// fewest rounds of the chip (one CTA fills an SM) by what a unit takes: its
+// set-up and folds, and its tiles 32 at a time (16 warps of two slots), at the
+// average list size.  100 queries of 35 tiles: whole 22 us, 5 splits 37; 33
+// queries of 417 tiles: 4 splits as 18, 68 us.  (Taken at d about 100.  Wider
+// rows have fewer warps and longer tiles, which the model does not know: not
+// measured there.)
+size_t scan_tsplit(const hy_index* h, size_t n, int pparts, size_t nprobe) {
     constexpr double UNIT_US = 6.0, ROUND_US = 4.0;
     const size_t nsm = (size_t)h->nsm;
     const size_t tiles = std::max<size_t>(1, h->arena_rows / 32 / std::max<size_t>(h->nlist, 1) * nprobe);
@@ -686,8 +678,24 @@ int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t npro
             tsplit = t;
         }
     }
-    const size_t all = n * (size_t)pparts;
-    HY_RET(h->w_parts.ensure(nq_dev ? fallback_parts_bytes(h, n, k, nprobe) : all * tsplit * kp * sizeof(uint64_t)));
+    return tsplit;
+}
+
+// Search n device queries with device probe lists (nprobe per query) into
+// device D/I.  Runs on stream s; does not synchronise.
+// nq_dev (optional): a device count of the queries to search (the first
+// *nq_dev of the n): one CTA per SM loops over their work units, whose
+// splits follow from the count, and the shared thresholds (w_gthr) hold each
+// query's starting bound (launch_fb_gather).
+int scan_and_merge(hy_index* h, size_t n, const float* dq, size_t k, size_t nprobe, const int64_t* dprobes,
+                   const uint32_t* init_thr, float* dD, int64_t* dI, cudaStream_t s, bool timed,
+                   int64_t* drows = nullptr, const int32_t* nq_dev = nullptr) {
+    const int kp = k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 256;
+    if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
+    const int pparts = hy::scan_probe_parts(h->L, (int)k, (int)nprobe);
+    const size_t tsplit = scan_tsplit(h, n, pparts, nprobe);
+    HY_RET(h->w_parts.ensure(nq_dev ? fallback_parts_bytes(h, n, k, nprobe)
+                                    : n * (size_t)pparts * tsplit * kp * sizeof(uint64_t)));
     uint32_t* gthr = nullptr;
     if (nq_dev) {
         gthr = h->w_gthr.as<uint32_t>();  // set by the gather of the counted queries
@@ -765,6 +773,23 @@ bool use_list_major(const hy_index* h, size_t m, size_t nprobe) {
     return m * nprobe >= 4 * h->nlist && (ip_window(h) || pair_bytes(h, m, nprobe) >= LIST_MAJOR_MIN_BYTES);
 }
 
+// Work items of the list-major scan of m queries: at most this many have a
+// descriptor.
+size_t list_item_cap(const hy_index* h, size_t m, size_t nprobe) {
+    int max_list = 1;
+    for (size_t l = 0; l < h->nlist; ++l) max_list = std::max(max_list, h->h_list_size[l]);
+    const size_t slices = ((size_t)max_list + LM_ROW_SLICE - 1) / LM_ROW_SLICE;
+    return std::min<size_t>((m * nprobe / hy::LM_GROUP + h->nlist) * slices, size_t(4) << 20);
+}
+
+// Each arena row's distance to its centroid and the tiles' extremes.
+int ensure_row_centroid_buffers(hy_index* h) {
+    const size_t rows = std::max<size_t>(h->arena_rows, hy::BATCH_ROW_ALIGN);
+    HY_RET(h->c2c.ensure(rows * sizeof(float)));
+    HY_RET(h->c2c_tile.ensure(rows / 32 * sizeof(float2)));
+    return HY_OK;
+}
+
 // The list-major plain scan of m device queries whose probe lists (m x
 // nprobe, -1 = skip) and ordered-key thresholds (thr: warm-up values or
 // 0xffffffff; lowered in place) are on the device, into D / I: first pass
@@ -791,10 +816,7 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
     HY_RET(h->b_zero.ensure(z.words * sizeof(int32_t)));
     int32_t* const zero = h->b_zero.as<int32_t>();
     HY_CUDA(cudaMemsetAsync(zero, 0, z.words * sizeof(int32_t), s));
-    size_t max_slices = 1;
-    for (size_t l = 0; l < nlist; ++l)
-        max_slices = std::max(max_slices, ((size_t)h->h_list_size[l] + rs - 1) / rs);
-    const size_t item_cap = std::min<size_t>((m * nprobe / hy::LM_GROUP + nlist) * max_slices, size_t(4) << 20);
+    const size_t item_cap = list_item_cap(h, m, nprobe);
     HY_RET(h->b_items.ensure(item_cap * sizeof(int4)));
     HY_RET(h->b_fq.ensure(m * h->d * sizeof(float)));
     HY_RET(h->b_fpr.ensure(m * nprobe * sizeof(int64_t)));
@@ -844,9 +866,7 @@ int scan_lists(hy_index* h, size_t m, const float* qq, size_t k, size_t nprobe, 
         // square root of its threshold cannot reach it, an exact prune that
         // pays when lists are tight balls around their centroids.
         if (!h->c2c_valid) {
-            const size_t rows = std::max<size_t>(h->arena_rows, hy::BATCH_ROW_ALIGN);
-            HY_RET(h->c2c.ensure(rows * sizeof(float)));
-            HY_RET(h->c2c_tile.ensure(rows / 32 * sizeof(float2)));
+            HY_RET(ensure_row_centroid_buffers(h));
             HY_CUDA(hy::launch_row_centroid(h->L, h->codes.as<float>(), h->list_off.as<int64_t>(),
                                             h->list_size.as<int32_t>(), (int)nlist, (int64_t)h->arena_rows,
                                             h->cent.as<float>(), h->metric, h->c2c.as<float>(),
@@ -1369,7 +1389,16 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     const size_t max_slices = std::max<size_t>(1, ((size_t)max_list + rs_min - 1) / rs_min);
     const size_t item_cap =
         std::min<size_t>((qc / qg1 + qc * nprobe / qg2 + 2 * nlist) * max_slices, size_t(4) << 20);
-    HY_RET(h->b_items.ensure(item_cap * sizeof(int4)));
+    HY_RET(h->b_items.ensure(std::max(item_cap, tf32 ? list_item_cap(h, qc, nprobe) : 0) * sizeof(int4)));
+    if (tf32) {
+        // A caller may capture its next search after another add, which then
+        // runs on the other plain scans: their buffers too, as every plain
+        // search of this size left them before.
+        const int pparts = hy::scan_probe_parts(h->L, (int)k, (int)nprobe);
+        const size_t kp = k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 256;
+        HY_RET(h->w_parts.ensure(qc * pparts * scan_tsplit(h, qc, pparts, nprobe) * kp * sizeof(uint64_t)));
+        if (h->opt_level & 1) HY_RET(ensure_row_centroid_buffers(h));
+    }
     hy::BatchWork w;
     w.items = h->b_items.as<int4>();
     w.item_cap = (int64_t)item_cap;

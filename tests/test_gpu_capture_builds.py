@@ -51,3 +51,42 @@ def test_search_after_a_capture(form):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(dI.cpu().numpy(), I)
     np.testing.assert_array_equal(dD.cpu().numpy(), D)
+
+
+@pytest.mark.parametrize("opt", [hb.OPT_NONE, hb.OPT_TRIANGLE])
+@pytest.mark.parametrize("nlist,n,m,nprobe", [(128, 40_000, 4_000, 32), (128, 40_000, 4_000, 128),
+                                              (64, 1_500_000, 15, 16)])
+def test_plain_batch_captured_after_an_add(opt, nlist, n, m, nprobe):
+    """Large plain batches: the capture runs the list-major or the query-major
+    scan, whose buffers the searches before have left large enough."""
+    rng = np.random.default_rng(9)
+    d, k = 64, 10
+    c = (20 * rng.standard_normal((nlist, d))).astype(np.float32)
+    lab = rng.integers(0, nlist, n)
+    x1, x2 = ((c[lab] + rng.standard_normal((n, d))).astype(np.float32) for _ in range(2))
+    q = (c[rng.integers(0, nlist, m)] + rng.standard_normal((m, d))).astype(np.float32)
+    idx = hb.Index(d, nlist, nprobe, opt_level=opt)
+    idx.centroid_codes = c
+    idx.add(x2)
+    assert m * nprobe * n / nlist * d * 4 > 1.2e9
+    D, I = idx.search(q, k)
+    idx = hb.Index(d, nlist, nprobe, opt_level=opt)
+    idx.centroid_codes = c
+    idx.add(x1)
+    dq = torch.from_numpy(q).cuda()
+    dD = torch.empty((m, k), device="cuda")
+    dI = torch.empty((m, k), dtype=torch.int64, device="cuda")
+
+    def search():
+        idx.search_device(m, dq.data_ptr(), k, dD.data_ptr(), dI.data_ptr(), torch.cuda.current_stream().cuda_stream)
+
+    search()
+    assert idx.last_stats()["list_major"] == 0
+    idx.add(x2)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        search()
+    g.replay()
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(dI.cpu().numpy(), I)
+    np.testing.assert_array_equal(dD.cpu().numpy(), D)
