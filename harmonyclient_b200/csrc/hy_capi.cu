@@ -9,6 +9,7 @@
 // data between host and device.  There is no CPU search path.
 #include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <fstream>
@@ -241,6 +242,7 @@ struct hy_index {
     bool cert_valid = false;
     DevBuf x32aux, t32aux, a32stat;  // the arena read as TF32: bound terms, sums of launch_row_aux_tf32
     bool a32_valid = false, a32_fits = false;  // built; the plain form's batches may run on it
+    double a32_spread = 0.0;  // the rows' TF32 error against their distance to their centroids
     size_t a32_refused = SIZE_MAX;  // plain batches (per chunk) from here on found no memory for it
     DevBuf b_cqb, b_cqn;  // bf16 queries of the coarse step when the scan's operands are others
     DevBuf b_qx;              // per-query exact-distance flags
@@ -295,12 +297,34 @@ int set_device(hy_index* h) {
 
 // FP32 bytes of (query, probed row) pairs from which a plain batch runs on the
 // tensor cores, and, where it cannot, from which the list-major scan serves
-// queries that share lists; below, the query-major scan's few launches win.
+// queries that share lists; below, the other scans' fewer launches win.
 // Measured (us, query-major / list-major / tensor): 1M x 128, nprobe 64: 512 MB
 // 187 / 344 / 283, 1 GB 412 / 383 / 289, 8 GB 1370 / 661 / 352; 200k x 200,
 // nprobe 16: 320 MB 249 / 456 / 253, 640 MB 352 / 525 / 265, 5 GB 1536 / 1241 /
 // 350; 10k x 128, nprobe 10: 524 MB 179 / 228 / 197.
 constexpr double TF32_MIN_BYTES = 600e6, LIST_MAJOR_MIN_BYTES = 1e9;
+// And the tensor cores only (us, tensor / the scan that then runs; shapes as
+// rows x dimensions, lists, nprobe, k, queries)
+//  - with 64 queries, 12 of them a list, 1.3 GB, or rows past 128 floats: a few
+//    queries leave the steps between the passes on a few warps (221,648 x 49,
+//    299, 139, 47, 12: 343 / 110; 278,816 x 82, 214, 64, 50, 18: 366 / 86; but
+//    138,475 x 166, 88, 78, 12, 9: 243 / 417);
+//  - where k is under a fifth of the rows a query scans, or k is small, many
+//    queries share lists, or the rows' TF32 error is small next to their spread:
+//    most candidates stay, and the re-rank takes them one by one (443,097 x 56,
+//    2435, 2, 176, 20,000: 3,326 / 1,827; 308,092 x 85, 2042, 2, 116, 4,207: 962 /
+//    530; but 39,178 x 44, 88, 2, 187, 8,774 with 199 queries a list 687 / 1,163,
+//    and 440,075 x 238, 2346, 5, 193, 4,164 of small error 1,028 / 1,511); for
+//    inner products, where the spread says little, under half of those rows
+//    (105,769 x 330, 758, 1, 242, 20,000: 2,316 / 1,632);
+//  - where two lists hold k rows, or the probed ones fit the candidate buffer:
+//    else the first pass bounds nothing, and the candidates overflow (86,227 x
+//    30, 1194, 123, 253, 175: 1,164 / 390);
+//  - for inner products, where lists fit the candidate buffer: nothing bounds
+//    the first pass over a larger list, and each query is scanned again
+//    (652,267 x 20, 29, 3, 31, 347: 7,279 / 1,229).
+constexpr size_t TF32_FEW_QUERIES = 64, TF32_FEW_SHARED = 12, TF32_LARGE_K = 64, TF32_MANY_SHARED = 30;
+constexpr double TF32_FEW_BYTES = 1.3e9, TF32_K_SHARE = 0.2, TF32_K_SHARE_IP = 0.5, TF32_SPREAD_LARGE_K = 0.005;
 // Largest mean TF32 error of a row against its distance to its centroid at
 // which a plain batch runs on the tensor cores (ensure_operands).
 constexpr double TF32_SPREAD_MAX = 0.03;
@@ -762,15 +786,53 @@ double pair_bytes(const hy_index* h, size_t m, size_t nprobe) {
     return (double)m * (double)nprobe * ((double)h->ntotal / (double)h->nlist) * (double)h->L.row_pitch * 4.0;
 }
 
+double mean_list(const hy_index* h) { return (double)h->ntotal / (double)h->nlist; }
+
+// Inner products over lists past the candidate buffer: the batched and the
+// list-major scan's first pass has no threshold there, and overflows.
+bool first_pass_overflows(const hy_index* h) {
+    return h->metric == HY_METRIC_IP && mean_list(h) > (double)std::min<size_t>(h->capq, hy::DENSE_MAX);
+}
+
+// A few queries: below these the query-major scan spreads each over the chip.
+bool few_queries(const hy_index* h, size_t m, size_t nprobe) {
+    return m < TF32_FEW_QUERIES && m * nprobe < TF32_FEW_SHARED * h->nlist && h->L.row_pitch <= 128 &&
+           pair_bytes(h, m, nprobe) < TF32_FEW_BYTES;
+}
+
+// What the query-major scan of m queries takes, and the list-major one, in us: fits
+// to 829 plain searches of 10 MB to 12 GB of pairs (16 to 384 dimensions, 16 to
+// 4096 lists, k to 256; half of them within a quarter).  A query's unit of
+// work folds its best k, whatever few rows it scans (20,000 queries of 55 rows,
+// k 89: 1,999 us, list-major 775); the list-major scan starts at its 17 launches.
+double query_major_us(const hy_index* h, size_t m, size_t nprobe, size_t k) {
+    const double kr = k <= 32 ? 1 : k <= 64 ? 2 : k <= 128 ? 4 : 8;
+    const double tiles = (double)nprobe * (mean_list(h) / 32.0 + 0.5);
+    const double units = std::max(1.0, (double)m / 148.0);             // per SM
+    const double t = tiles / std::max(1.0, 148.0 / (double)m);         // tiles of a unit
+    const double row = (double)h->L.row_pitch / 128.0 * 16.0 / hy::scan_warps(h->L);
+    return 60.0 + units * (7.0 + kr + 0.11 * kr * std::min(t, 32.0) + 0.026 * std::pow(kr, 1.5) * std::min(t, 400.0) +
+                           0.1 * row * t);
+}
+double list_major_us(const hy_index* h, size_t m, size_t nprobe, size_t k) {
+    const double kr = k <= 32 ? 1 : k <= 64 ? 2 : k <= 128 ? 4 : 8, n = (double)m / 1e6;
+    return 236.0 + 53e-9 * pair_bytes(h, m, nprobe) + 600.0 * kr * n + 65.0 * mean_list(h) * n +
+           62.0 * std::min((double)k, (double)nprobe * mean_list(h)) * n;
+}
+
 // Whether a plain search of m queries (per chunk) at nprobe runs the
 // list-major scan when it does not run on the tensor cores: when its queries
-// share lists (four per list) and their pairs are worth its 17 launches (with
-// the inner-product window, whose answer off the unit sphere is the list-major
-// scan's own, always when they share lists).
-bool use_list_major(const hy_index* h, size_t m, size_t nprobe) {
+// share lists (four per list) and their pairs are worth its 17 launches, by
+// their bytes or by those fits (with the inner-product window, whose answer off
+// the unit sphere is the list-major scan's own, always when they share lists).
+bool use_list_major(const hy_index* h, size_t m, size_t nprobe, size_t k) {
     if (h->plain_scan == HY_PLAIN_QUERY_MAJOR || h->arena_rows == 0 || !hy::list_scan_fits(h->L)) return false;
     if (h->plain_scan == HY_PLAIN_LIST_MAJOR) return true;
-    return m * nprobe >= 4 * h->nlist && (ip_window(h) || pair_bytes(h, m, nprobe) >= LIST_MAJOR_MIN_BYTES);
+    if (m * nprobe < 4 * h->nlist) return false;
+    if (ip_window(h)) return true;
+    if (first_pass_overflows(h) || few_queries(h, m, nprobe)) return false;
+    return pair_bytes(h, m, nprobe) >= LIST_MAJOR_MIN_BYTES ||
+           list_major_us(h, m, nprobe, k) < 0.8 * query_major_us(h, m, nprobe, k);
 }
 
 // Work items of the list-major scan of m queries: at most this many have a
@@ -935,7 +997,7 @@ int ensure_common(hy_index* h) {
 
 int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, size_t k, float* dD, int64_t* dI,
                        cudaStream_t s, bool timed);
-bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s);
+bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, size_t k, cudaStream_t s);
 void release_batch_buffers(hy_index* h);
 
 // The scan counters and the fallback count (which follow one another) to zero.
@@ -981,7 +1043,7 @@ int search_device_impl(hy_index* h, size_t n, const float* dq, size_t k, float* 
     HY_RET(ensure_common(h));
     size_t qc = query_chunk(h->nlist, n);
     const size_t tqc = std::min(qc, std::max<size_t>(1, (size_t(2) << 30) / (h->capq * 8)));
-    h->fb_last = plain_on_tensor(h, tqc, nprobe, s);
+    h->fb_last = plain_on_tensor(h, tqc, nprobe, k, s);
     if (h->fb_last) {
         // Its buffers (up to 2 GiB of candidates) are taken before its first
         // launch; without the memory for them the other scans run, as for
@@ -992,7 +1054,7 @@ int search_device_impl(hy_index* h, size_t n, const float* dq, size_t k, float* 
         h->a32_refused = tqc;
     }
     // List-major scan: chunks sized so the candidate buffers stay within 2 GiB.
-    const bool lm = use_list_major(h, qc, nprobe);
+    const bool lm = use_list_major(h, qc, nprobe, k);
     if (lm) qc = std::min(qc, std::max<size_t>(1, (size_t(2) << 30) / (h->capq * 8)));
     h->fb_last = lm;
     h->stats.list_major = lm ? 1 : 0;
@@ -1109,6 +1171,7 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
         // bound about 2 |q| (|x - x~| + 2^-11 |x|), so above a few percent
         // (values far from the origin next to their spread) the scores
         // separate too few rows.  Infinities, NaN and huge rows: never.
+        h->a32_spread = stat[0] / stat[1];
         h->a32_fits = maxxn < 1e37f && stat[0] < TF32_SPREAD_MAX * stat[1];
         h->a32_valid = true;
         return HY_OK;
@@ -1127,14 +1190,16 @@ int ensure_operands(hy_index* h, hy::Operand op, cudaStream_t s) {
 
 // Whether a plain search of m queries (per chunk) at nprobe runs on the tensor
 // cores (the FP32 arena as TF32 operands, exact FP32 re-rank: the other scans'
-// answer): from TF32_MIN_BYTES of pairs.  Not with the inner-product window of
+// answer): from TF32_MIN_BYTES of pairs, less the shapes named there.  Not with the inner-product window of
 // OPT_TRIANGLE, whose answer off the unit sphere depends on the scan's own
 // thresholds.  The bound terms are built on first use; while the stream is
 // being captured, or without the memory for them, the other scans run (a batch
 // for whose own buffers there is no memory: search_device_impl).
-bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s) {
+bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, size_t k, cudaStream_t s) {
     if (h->form != HY_FORM_PLAIN || h->plain_scan != HY_PLAIN_AUTO || h->arena_rows == 0 || ip_window(h)) return false;
-    if (pair_bytes(h, m, nprobe) < TF32_MIN_BYTES) return false;
+    if (pair_bytes(h, m, nprobe) < TF32_MIN_BYTES || first_pass_overflows(h) || few_queries(h, m, nprobe)) return false;
+    const double rows = (double)nprobe * mean_list(h);  // that a query scans
+    if ((double)k > 2.0 * mean_list(h) && rows > (double)h->capq) return false;
     if (hy::batched_group_size(hy::operand_kblocks(hy::Operand::tf32, h->L)) == 0) return false;
     if (m >= h->a32_refused) return false;
     if (!h->a32_valid) {
@@ -1145,6 +1210,11 @@ bool plain_on_tensor(hy_index* h, size_t m, size_t nprobe, cudaStream_t s) {
             return false;
         }
     }
+    const size_t pairs = m * nprobe;  // of a query and a list
+    const bool ip = h->metric == HY_METRIC_IP;
+    if (k >= TF32_LARGE_K && (double)k >= (ip ? TF32_K_SHARE_IP : TF32_K_SHARE) * rows && pairs >= 4 * h->nlist &&
+        pairs < TF32_MANY_SHARED * h->nlist && (ip || h->a32_spread >= TF32_SPREAD_LARGE_K))
+        return false;
     return h->a32_fits;
 }
 

@@ -1226,7 +1226,7 @@ cudaError_t launch_warmup(const ArenaLayout& L, const float* codes, const int64_
 // Warps, slots and K' are chosen so that one CTA's shared memory fits: 16
 // warps with 2 slots each for pitches up to 32 floats per block (d <= 128
 // with 4 blocks), 8 warps for wider blocks.  Slots are processed in pairs.
-static int scan_warps(const ArenaLayout& L) {
+int scan_warps(const ArenaLayout& L) {
     const int slot_kb = L.max_pitch / 8;  // 32 rows x pitch floats, in KiB
     return slot_kb * 2 * 16 <= 128 ? 16 : slot_kb * 2 * 8 <= 160 ? 8 : 4;
 }

@@ -69,6 +69,8 @@ __host__ __device__ inline int scan_tile_splits(int units, int nq, int pparts) {
     const int per = nq > 0 ? units / (nq * pparts) : 1;
     return per > 1 ? per : 1;
 }
+// Warps of a plain scan's CTA for layout L.
+int scan_warps(const ArenaLayout& L);
 // Probe parts of a plain scan: the fewest whose probe tables fit a CTA's
 // shared memory beside the staging for layout L and k.
 int scan_probe_parts(const ArenaLayout& L, int k, int nprobe);
