@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(ASSIGN_THREADS, 1) assign_kernel(const __grid_
             mbar_wait_bounded(&drain, 0, p.err);
         }
     } else if (warp >= W_EPI0 && warp < W_EPI0 + N_EPI) {
-        // ---------------- epilogue: thread = row; each half scans 64 of a
-        // centroid tile's 128 columns.
+        // ---------------- epilogue: thread = row; each half scans 128 of an
+        // accumulator's 256 columns, 64 at a time.
         const int e = warp - W_EPI0, quad = warp & 3, half = e >> 2;
         const int r = quad * 32 + lane;
         const float cf = l2 ? -2.0f : -1.0f;

@@ -1,14 +1,16 @@
-// Batched list-major scan on the tcgen05 tensor cores (the "bf16" and
-// "e4m3" forms) and the steps around it.
+// Batched list-major scan on the tcgen05 tensor cores (the bf16 and e4m3
+// forms, and large batches of the plain form on TF32 operands) and the steps
+// around it.
 //
 // Queries that probe the same list share one pass over it.  After coarse
 // quantisation, the (query, probed list) pairs are inverted into per-list
 // query groups; a persistent kernel (one CTA per SM) drains a work queue of
-// (list, group of <=128 queries, slice of <=2048 rows) items.  Per item the
+// (list, group of <=128 queries, slice of <=2048 rows, 512 for rows of many
+// k-blocks) items.  Per item the
 // CTA gathers the group's query vectors into shared memory (the MMA's B
 // operand), then streams the slice's 128-row tiles of the list image (already
 // in the tensor core's swizzled shared-memory layout, so each k-block of a
-// tile is one 16 KiB bulk copy) through a ring of stages.  One thread issues
+// tile is 16 KiB of a bulk copy) through a ring of stages.  One thread issues
 // tcgen05.mma (M = 128 rows, N = up to 128 queries) into one of two TMEM
 // accumulators; eight epilogue warps read the accumulator (thread = row) and
 // form dist = |x|^2 + |q|^2 - 2 q.x (or -q.x for inner product) with a
@@ -23,7 +25,7 @@
 // keeps the tensor-core distance when the exactness certificate shows it is
 // exact), so the answer is the plain scan's.  A query whose candidates
 // overflow its buffer is answered again by the plain scan.  The same kernel,
-// over the centroids as a one-list index, is the coarse step of the bf16 form.
+// over the centroids as a one-list index, is the coarse step of all of them.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
@@ -44,7 +46,10 @@ constexpr int TM = 128;      // rows per tile (MMA M)
 constexpr int NS_MAX = 8;    // stages of the list k-block ring: at most
 constexpr int RING_MIN = 4;  // k-blocks the ring holds: at least (64 KiB in flight)
 constexpr int KB_BYTES = 16384;
-constexpr int NKB_MAX = 12;  // k-blocks of a row: at most (bf16 d <= 768, e4m3 d <= 1536)
+// k-blocks of a row: at most (bf16 d <= 768, e4m3 d <= 1536, TF32 384 floats in
+// the arena's padded blocks).  By the kernel's shared memory groups of 64 queries
+// would fit to 16; more than 12 is not built or measured.
+constexpr int NKB_MAX = 12;
 // k-blocks per stage: two where rows have two or more.  A stage costs its
 // issuers a barrier wait, a commit and their loops (about 350 cycles) beside
 // the copies (130 each) and MMAs, which one 16 KiB k-block does not cover.
@@ -554,60 +559,7 @@ __global__ void probe_fill_kernel(const int64_t* __restrict__ probes, int nq, in
     }
 }
 
-// The same two steps with shared-memory counters (nlist <= INVERT_SMEM_LISTS):
-// each CTA takes a contiguous range of `per` pairs, counts them per list in
-// shared memory and adds each list's count to the global one once; the fill
-// reserves each list's share of the CTA with one global add and places the
-// pairs at shared-memory ranks.  Few global atomics per list instead of one
-// per pair.
 constexpr int INVERT_SMEM_LISTS = 6144;  // the fill's 8 bytes per list stay within 48 KiB
-__global__ void __launch_bounds__(512) probe_hist_smem_kernel(const int64_t* __restrict__ probes, int nq, int nprobe,
-                                                              int j0, int j1, int nlist, int64_t per,
-                                                              int32_t* __restrict__ cnt) {
-    extern __shared__ int h[];  // [nlist]
-    const int w = j1 - j0;
-    const int64_t n = static_cast<int64_t>(nq) * w;
-    const int64_t a = blockIdx.x * per, b = min(n, a + per);
-    for (int l = threadIdx.x; l < nlist; l += blockDim.x) h[l] = 0;
-    __syncthreads();
-    for (int64_t i = a + threadIdx.x; i < b; i += blockDim.x) {
-        const int64_t l = probes[(i / w) * nprobe + j0 + i % w];
-        if (l >= 0) atomicAdd(&h[l], 1);
-    }
-    __syncthreads();
-    for (int l = threadIdx.x; l < nlist; l += blockDim.x)
-        if (h[l]) atomicAdd(&cnt[l], h[l]);
-}
-
-__global__ void __launch_bounds__(512) probe_fill_smem_kernel(const int64_t* __restrict__ probes, int nq, int nprobe,
-                                                              int j0, int j1, int nlist, int64_t per,
-                                                              const int64_t* __restrict__ off,
-                                                              int32_t* __restrict__ fill,
-                                                              int32_t* __restrict__ pairs) {
-    extern __shared__ int h[];  // [nlist] counts, then ranks; [nlist] bases
-    int* base = h + nlist;
-    const int w = j1 - j0;
-    const int64_t n = static_cast<int64_t>(nq) * w;
-    const int64_t a = blockIdx.x * per, b = min(n, a + per);
-    for (int l = threadIdx.x; l < nlist; l += blockDim.x) h[l] = 0;
-    __syncthreads();
-    for (int64_t i = a + threadIdx.x; i < b; i += blockDim.x) {
-        const int64_t l = probes[(i / w) * nprobe + j0 + i % w];
-        if (l >= 0) atomicAdd(&h[l], 1);
-    }
-    __syncthreads();
-    for (int l = threadIdx.x; l < nlist; l += blockDim.x) {
-        base[l] = h[l] ? atomicAdd(&fill[l], h[l]) : 0;
-        h[l] = 0;
-    }
-    __syncthreads();
-    for (int64_t i = a + threadIdx.x; i < b; i += blockDim.x) {
-        const int64_t l = probes[(i / w) * nprobe + j0 + i % w];
-        if (l < 0) continue;
-        const int pos = base[l] + atomicAdd(&h[l], 1);
-        pairs[off[l] + pos] = static_cast<int32_t>(i / w);
-    }
-}
 
 // Items of a list = query groups x row slices (none for an empty list).
 __global__ void item_count_kernel(const int32_t* __restrict__ cnt, const int32_t* __restrict__ list_size, int nlist,
@@ -633,13 +585,15 @@ __global__ void item_fill_kernel(const int64_t* __restrict__ item_off, const int
     }
 }
 
-// The inversion in two launches (nlist <= INVERT_SMEM_LISTS).  The first
+// The inversion in two launches with shared-memory counters (nlist <=
+// INVERT_SMEM_LISTS: few global atomics per list instead of one per pair).  The first
 // counts pairs per list in shared memory (each CTA a contiguous range of
 // `per` pairs, loads in flight eight at a time) and adds the counts to
 // w.pair_cnt; the last CTA to finish (a ticket on w.done after a fence)
 // turns the counts into pair offsets and item offsets, zeroes the fill
-// counters and resets the ticket.  The second places the pairs (as
-// probe_fill_smem_kernel) and writes the item descriptors.
+// counters and resets the ticket.  The second reserves each list's share of a
+// CTA with one global add, places the pairs at shared-memory ranks and writes
+// the item descriptors.
 __device__ inline int64_t probe_list(const int64_t* __restrict__ probes, int64_t i, int wd, int nprobe, int j0) {
     return probes[(i / wd) * nprobe + j0 + i % wd];
 }
@@ -823,8 +777,8 @@ struct BatchedParams {
 };
 
 // Warp roles of the persistent batched kernel (12 warps).
-constexpr int W_PRODUCER = 0;   // lane 0: bulk copies of list k-blocks
-constexpr int W_MMA = 1;        // lane 0: tcgen05.mma issue; whole warp: TMEM alloc
+constexpr int W_PRODUCER = 0;   // bulk copies of list k-blocks (an elected lane issues)
+constexpr int W_MMA = 1;        // tcgen05.mma (an elected lane issues), TMEM allocation
 constexpr int W_GATHER0 = 2;    // warps 2-3: fetch items, gather their queries
 constexpr int N_GATHER = 2;
 constexpr int W_EPI0 = 4;       // warps 4-11: epilogue (two per TMEM lane quadrant)
@@ -2038,7 +1992,7 @@ __device__ inline float coarse_dot(const float* qs, const float* row, int j0, in
 // all c of them also in kbuf) among one another, and each of the m smallest
 // written at its rank.
 template <int R>
-__device__ inline void rank_write(const uint64_t (&kr)[4], const uint64_t* kbuf, int c, int m, int qi,
+__device__ inline void rank_write(const uint64_t (&kr)[4], const uint64_t* kbuf, int c, int m,
                                   int64_t* __restrict__ out_idx, float* __restrict__ out_score, int lane) {
     int rank[R];
 #pragma unroll
@@ -2057,8 +2011,8 @@ __device__ inline void rank_write(const uint64_t (&kr)[4], const uint64_t* kbuf,
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         if (i * 32 + lane < c && rank[i] < m) {
-            out_idx[static_cast<int64_t>(qi) * m + rank[i]] = static_cast<int64_t>(kr[i] & 0xffffffffu);
-            if (out_score) out_score[static_cast<int64_t>(qi) * m + rank[i]] = o2f(static_cast<uint32_t>(kr[i] >> 32));
+            out_idx[rank[i]] = static_cast<int64_t>(kr[i] & 0xffffffffu);
+            if (out_score) out_score[rank[i]] = o2f(static_cast<uint32_t>(kr[i] >> 32));
         }
     }
 }
@@ -2066,13 +2020,13 @@ __device__ inline void rank_write(const uint64_t (&kr)[4], const uint64_t* kbuf,
 template <int METRIC>
 __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64_t* kbuf, uint64_t* bars, int c,
                                          const float* qs, float* stage, int pitch, const float* __restrict__ cent,
-                                         int d, int m, int qi, int64_t* __restrict__ out_idx,
+                                         int d, int m, int64_t* __restrict__ out_idx,
                                          float* __restrict__ out_score, int* err, int lane) {
     // Fewer candidates than m (not reached when the bound holds m of them):
     // the missing probes are -1.
     for (int e = c + lane; e < m; e += 32) {
-        out_idx[static_cast<int64_t>(qi) * m + e] = -1;
-        if (out_score) out_score[static_cast<int64_t>(qi) * m + e] = FLT_MAX;
+        out_idx[e] = -1;
+        if (out_score) out_score[e] = FLT_MAX;
     }
     const bool v4 = (d & 3) == 0;
     const bool in_regs = c <= 128;
@@ -2139,8 +2093,8 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
             // leave no probe.
             while (used < issued && mbar_wait_bounded(bar, used & 1u, nullptr)) ++used;
             for (int e = lane; e < m; e += 32) {
-                out_idx[static_cast<int64_t>(qi) * m + e] = -1;
-                if (out_score) out_score[static_cast<int64_t>(qi) * m + e] = FLT_MAX;
+                out_idx[e] = -1;
+                if (out_score) out_score[e] = FLT_MAX;
             }
             return;
         }
@@ -2192,10 +2146,10 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
             if (r * 32 + lane < c) kbuf[r * 32 + lane] = kr[r];
         __syncwarp();
         switch ((c + 31) >> 5) {
-            case 1: rank_write<1>(kr, kbuf, c, m, qi, out_idx, out_score, lane); break;
-            case 2: rank_write<2>(kr, kbuf, c, m, qi, out_idx, out_score, lane); break;
-            case 3: rank_write<3>(kr, kbuf, c, m, qi, out_idx, out_score, lane); break;
-            case 4: rank_write<4>(kr, kbuf, c, m, qi, out_idx, out_score, lane); break;
+            case 1: rank_write<1>(kr, kbuf, c, m, out_idx, out_score, lane); break;
+            case 2: rank_write<2>(kr, kbuf, c, m, out_idx, out_score, lane); break;
+            case 3: rank_write<3>(kr, kbuf, c, m, out_idx, out_score, lane); break;
+            case 4: rank_write<4>(kr, kbuf, c, m, out_idx, out_score, lane); break;
             default: break;
         }
         return;
@@ -2223,8 +2177,8 @@ __device__ inline void coarse_exact_best(uint64_t* keys, const int* sids, uint64
     for (int r = 0; r < 8; ++r) {
         const int e = r * 32 + lane;
         if (e < m && e < c) {
-            out_idx[static_cast<int64_t>(qi) * m + e] = static_cast<int64_t>(t[r] & 0xffffffffu);
-            if (out_score) out_score[static_cast<int64_t>(qi) * m + e] = o2f(static_cast<uint32_t>(t[r] >> 32));
+            out_idx[e] = static_cast<int64_t>(t[r] & 0xffffffffu);
+            if (out_score) out_score[e] = o2f(static_cast<uint32_t>(t[r] >> 32));
         }
     }
 }
@@ -2378,7 +2332,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_kernel(float2* __restric
         for (int e = lane; e < 256; e += 32) keys[e] = static_cast<uint64_t>(hist[e]);
     __syncwarp();
     coarse_exact_best<METRIC>(keys, hist, reinterpret_cast<uint64_t*>(hist), bars, c, qs, stage, pitch, cent, d,
-                              mq - nd, 0, out_idx + static_cast<int64_t>(qi) * m + nd,
+                              mq - nd, out_idx + static_cast<int64_t>(qi) * m + nd,
                               out_score ? out_score + static_cast<int64_t>(qi) * m : nullptr, err, lane);
 }
 
@@ -2515,7 +2469,7 @@ __global__ void __launch_bounds__(128, 1) coarse_refine_keys_kernel(uint64_t* __
     }
     __syncwarp();
     coarse_exact_best<METRIC>(keys, nullptr, reinterpret_cast<uint64_t*>(hist), bars, c, qs, stage, pitch, cent, d,
-                              mq - nd, 0, out + nd, out_score ? out_score + static_cast<int64_t>(qi) * m : nullptr,
+                              mq - nd, out + nd, out_score ? out_score + static_cast<int64_t>(qi) * m : nullptr,
                               err, lane);
 }
 
@@ -3062,7 +3016,7 @@ cudaError_t launch_invert_probes(const int64_t* probes, int nq, int nprobe, int 
                                  const int32_t* list_size, int rs, int qg, const BatchWork& w, cudaStream_t s) {
     const int64_t n = static_cast<int64_t>(nq) * (j1 - j0);
     cudaError_t e;
-    if (nlist <= INVERT_SMEM_LISTS && w.done) {
+    if (nlist <= INVERT_SMEM_LISTS) {
         // Up to about one CTA of 512 threads per SM (at least 1024 pairs each).
         const int64_t per = std::max<int64_t>(1024, (n + 147) / 148);
         const int nblk = static_cast<int>(std::max<int64_t>(1, (n + per - 1) / per));
@@ -3077,21 +3031,9 @@ cudaError_t launch_invert_probes(const int64_t* probes, int nq, int nprobe, int 
         return cudaGetLastError();
     }
     if ((e = cudaMemsetAsync(w.pair_fill, 0, nlist * sizeof(int32_t), s)) != cudaSuccess) return e;
-    if (nlist <= INVERT_SMEM_LISTS) {
-        // About 160 CTAs of 512 threads (at least 512 pairs each).
-        const int64_t per = std::max<int64_t>(512, (n + 159) / 160);
-        const int nblk = static_cast<int>(std::max<int64_t>(1, (n + per - 1) / per));
-        probe_hist_smem_kernel<<<nblk, 512, static_cast<size_t>(nlist) * 4, s>>>(probes, nq, nprobe, j0, j1, nlist,
-                                                                                 per, w.pair_cnt);
-        scan_kernel<<<1, 1024, 0, s>>>(w.pair_cnt, nlist, w.pair_off);
-        probe_fill_smem_kernel<<<nblk, 512, static_cast<size_t>(nlist) * 8, s>>>(probes, nq, nprobe, j0, j1, nlist,
-                                                                                 per, w.pair_off, w.pair_fill, w.pairs);
-    } else {
-        probe_hist_kernel<<<grid_for(n, 256), 256, 0, s>>>(probes, nq, nprobe, j0, j1, w.pair_cnt);
-        scan_kernel<<<1, 1024, 0, s>>>(w.pair_cnt, nlist, w.pair_off);
-        probe_fill_kernel<<<grid_for(n, 256), 256, 0, s>>>(probes, nq, nprobe, j0, j1, w.pair_off, w.pair_fill,
-                                                           w.pairs);
-    }
+    probe_hist_kernel<<<grid_for(n, 256), 256, 0, s>>>(probes, nq, nprobe, j0, j1, w.pair_cnt);
+    scan_kernel<<<1, 1024, 0, s>>>(w.pair_cnt, nlist, w.pair_off);
+    probe_fill_kernel<<<grid_for(n, 256), 256, 0, s>>>(probes, nq, nprobe, j0, j1, w.pair_off, w.pair_fill, w.pairs);
     item_count_kernel<<<grid_for(nlist, 256), 256, 0, s>>>(w.pair_cnt, list_size, nlist, rs, qg, w.item_cnt);
     scan_kernel<<<1, 1024, 0, s>>>(w.item_cnt, nlist, w.item_off);
     item_fill_kernel<<<grid_for(static_cast<int64_t>(nlist) * 32, 256), 256, 0, s>>>(w.item_off, list_size, nlist, rs,

@@ -70,8 +70,8 @@ cudaError_t launch_arena_integral(const float* codes, int64_t n, const float* xn
 // tile_max[t] = the largest xn over rows [128 t, 128 t + 128) (rows a
 // multiple of 128).
 cudaError_t launch_tile_max(const float* xn, int64_t rows, float* tile_max, cudaStream_t s);
-// The bound terms of the arena rows read as TF32, and two sums over a sample of
-// the rows (see row_aux_tf32_kernel).
+// The bound terms of the arena rows read as TF32, and two sums over the rows
+// (see row_aux_tf32_kernel).
 cudaError_t launch_row_aux_tf32(const ArenaLayout& L, const float* codes, int64_t rows, const int64_t* list_off,
                                 const int32_t* list_size, int nlist, const float* cent, float2* aux, float2* tile_aux,
                                 double* stat, cudaStream_t s);
@@ -124,7 +124,7 @@ cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qa
                            int capq, int k, int metric, int d, int K, int nsm, float* thr, cudaStream_t s,
                            DenseFirst df);
 
-// The coarse quantiser on the tensor cores (bf16 form).  The centroids
+// The coarse quantiser on the tensor cores.  The centroids
 // (row-major, nlist x d) as a one-list index: split bf16 image (per 64
 // dimensions a hi k-block, bf16(c), then a lo k-block, bf16(c - hi); launched
 // with BatchedLaunch::ksplit), per-row {|(|hi| + |lo|)|, |c - hi - lo|},

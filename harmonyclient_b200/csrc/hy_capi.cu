@@ -238,7 +238,7 @@ struct hy_index {
     DevBuf taux;              // per 128-row tile, maxima of xaux
     DevBuf txn;               // per 128-row tile, the largest squared norm
     bool abf_valid = false;
-    DevBuf b_cert;            // the bf16 image's exactness certificate {integral, max row norm}
+    DevBuf b_cert;            // the arena's exactness certificate {integral, max row norm}
     bool cert_valid = false;
     DevBuf x32aux, t32aux, a32stat;  // the arena read as TF32: bound terms, sums of launch_row_aux_tf32
     bool a32_valid = false, a32_fits = false;  // built; the plain form's batches may run on it
@@ -254,7 +254,7 @@ struct hy_index {
     DevBuf b_zero;            // the counters of a search, cleared together
     DevBuf b_done;            // the probe inversion's ticket (zero between launches)
     DevBuf b_fq, b_fpr, b_fD, b_fI, b_fcnt, b_fbtot;  // device-side exact fallback
-    // coarse quantiser on the tensor cores (bf16 form): the centroids as a
+    // coarse quantiser on the tensor cores: the centroids as a
     // one-list index (image, row aux, tile aux, norms, list offsets/sizes)
     // and the work of one launch
     int coarse_mode = HY_COARSE_TENSOR;
@@ -1227,8 +1227,12 @@ void release_batch_buffers(hy_index* h) {
     for (DevBuf* b : bufs) b->release();
 }
 
-// Whether a batched search's coarse step runs on the tensor cores (the
-// conditions launch_coarse_refine's shared memory and select width need).
+// Whether a batched search's coarse step runs on the tensor cores: the
+// selection takes up to 256 probes, and the kernel rows up to its k-blocks.  Above
+// 2048 lists only the bf16 form to 256 dimensions does, as it did before the other
+// forms and wider rows were taken up to there; the two-launch step is not tested on
+// those, though it would be faster (10,000 queries, 4096 lists, nprobe 64, us: plain
+// 1M x 128 886 here, 705 there; e4m3 894 / 715; bf16 400k x 420 2,319 / 819).
 bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
     return h->coarse_mode == HY_COARSE_TENSOR && nprobe <= 256 && (h->d <= 256 || h->nlist <= 2048) &&
            (h->form == HY_FORM_BF16 || h->nlist <= 2048) && hy::batched_group_size((int)(h->d + 63) / 64) > 0;

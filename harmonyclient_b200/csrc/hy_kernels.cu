@@ -1257,7 +1257,7 @@ static cudaError_t launch_scan_t(const ScanParams& p, int W, int* smem_out, cuda
     if (e != cudaSuccess) return e;
     // With a device count, the CTAs loop over the work units.
     const int64_t all = static_cast<int64_t>(p.nq) * p.pparts;
-    const int64_t grid = p.nq_dev ? std::min<int64_t>(std::max<int64_t>(all, p.units), p.units) : all * p.tsplit;
+    const int64_t grid = p.nq_dev ? p.units : all * p.tsplit;
     if (p.nq < 1 || grid < 1) return cudaSuccess;
     scan_plain_kernel<KR, S><<<static_cast<unsigned>(grid), W * 32, smem, s>>>(p);
     return cudaGetLastError();

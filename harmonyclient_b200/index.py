@@ -137,16 +137,16 @@ class Index:
         check(self._L.hy_index_set_form(self._h, int(f)))
 
     def set_plain_scan(self, mode):
-        """The plain form's scan: 'auto' (default: list-major when the batch
-        has at least 4 queries per list on average), 'query' (one CTA per
-        query streams its probed lists) or 'list' (queries probing a list
+        """The plain form's scan: 'auto' (default: the fastest for the call's
+        sizes, large batches on the tensor cores), 'query' (each query's
+        probed lists are streamed by itself) or 'list' (queries probing a list
         share one pass over it).  All give the same answer."""
         m = {"auto": _lib.HY_PLAIN_AUTO, "query": _lib.HY_PLAIN_QUERY_MAJOR,
              "list": _lib.HY_PLAIN_LIST_MAJOR}.get(mode, mode)
         check(self._L.hy_index_set_plain_scan(self._h, int(m)))
 
     def set_coarse(self, mode):
-        """The bf16 form's coarse step: 'tensor' (default; bf16 tensor-core
+        """The tensor-core searches' coarse step: 'tensor' (default; bf16 tensor-core
         scores with error bounds, exact FP32 scores only for the centroids
         that can reach the nprobe best) or 'exact' (exact FP32 scores of every
         centroid).  Both give the same probe lists."""

@@ -50,15 +50,15 @@ enum { HY_METRIC_IP = 0, HY_METRIC_L2 = 1 };
 
 /* Scan forms selectable with hy_index_set_form. */
 enum {
-    HY_FORM_PLAIN = 0, /* exact FP32 query-major scan with dim-block pruning */
+    HY_FORM_PLAIN = 0, /* exact FP32 distances (hy_index_set_plain_scan says by which scan) */
     HY_FORM_BF16 = 1,  /* batched list-major bf16 tensor-core scan + exact FP32 re-rank */
     HY_FORM_FP8 = 2    /* the same on e4m3 codes with per-list / per-query scales, oversampled re-rank */
 };
 
-/* How the plain form scans (hy_index_set_plain_scan).  Both return the same
- * answer, bit for bit. */
+/* How the plain form scans (hy_index_set_plain_scan).  All return the same
+ * answer, bit for bit (but see OPT_TRIANGLE with inner product there). */
 enum {
-    HY_PLAIN_AUTO = 0,        /* list-major when the batch shares lists (>= 4 queries per list on average) */
+    HY_PLAIN_AUTO = 0,        /* by the work: query-major, list-major, or the tensor cores for large batches */
     HY_PLAIN_QUERY_MAJOR = 1, /* one CTA per (query, probe split) streams that query's probed lists */
     HY_PLAIN_LIST_MAJOR = 2   /* queries probing a list share one pass over it, 32 per group */
 };
@@ -170,13 +170,27 @@ HY_API int hy_index_set_opt_level(hy_index* h, int opt_level);
 /* Scan form (no counterpart in the reference, whose only scan is the exact
  * FP32 one): HY_FORM_PLAIN or HY_FORM_BF16 (d <= 128).  The bf16 form batches
  * queries per list on the tensor cores and re-ranks candidates with exact FP32
- * distances chosen by rigorous error bounds, so its results equal the plain
+ * distances chosen by error bounds, so its results equal the plain
  * form's.  Queries whose candidates overflow their buffers are answered again
  * by the plain scan on the device, however many overflow. */
 HY_API int hy_index_set_form(hy_index* h, int form);
 
 /* Plain form's scan (no counterpart in the reference): HY_PLAIN_AUTO (default),
- * HY_PLAIN_QUERY_MAJOR or HY_PLAIN_LIST_MAJOR.  The list-major scan inverts
+ * HY_PLAIN_QUERY_MAJOR or HY_PLAIN_LIST_MAJOR.
+ * HY_PLAIN_AUTO takes the scan that is fastest for the call's sizes: a batch
+ * of 600 MB or more of (query, probed row) pairs in FP32 runs on the tensor
+ * cores (the rows read as TF32, candidates kept by error bounds and re-ranked
+ * with exact FP32 distances) when its rows have up to 384 floats in the padded
+ * dimension blocks; smaller ones, and shapes that keep too many candidates,
+ * run query-major or, when their queries share lists, list-major.  Whether the
+ * rows suit TF32 is found out by the first such search after an add, load or
+ * train, which reads a few numbers back and so waits for its stream (also a
+ * device-pointer search); inside a caller's stream capture, where that cannot
+ * be, and where there is no device memory for the candidate buffers (up to 2
+ * GiB), the other scans run.  With inner product and OPT_TRIANGLE the
+ * answer depends on the scan where vectors lie off the unit sphere; there
+ * HY_PLAIN_AUTO is list-major whenever the queries share lists (four per list).
+ * The list-major scan inverts
  * the (query, probed list) pairs into per-list groups of 32 queries; each
  * group reads a list once, dimension block by dimension block, pruning each
  * (row, query) pair against the query's threshold between blocks, with the
@@ -203,17 +217,17 @@ HY_API int hy_index_set_batch_params(hy_index* h, size_t capq, size_t oversample
  * results do not depend on it. */
 HY_API int hy_index_set_group_size(hy_index* h, int qg);
 
-/* Coarse quantiser of the bf16 form (no counterpart in the reference, which
- * scores every centroid exactly, src/Index.cpp:985-990).  HY_COARSE_EXACT:
+/* Coarse quantiser of the tensor-core searches (no counterpart in the
+ * reference, which scores every centroid exactly, src/Index.cpp:985-990).  HY_COARSE_EXACT:
  * exact FP32 scores of every centroid, then the nprobe best.
  * HY_COARSE_TENSOR (default): bf16 tensor-core scores of every centroid with
- * rigorous error bounds, then exact FP32 scores only for the centroids whose
- * bound can reach the nprobe-th best; the probe lists (and the learned
- * predictor's coarse scores) are identical to HY_COARSE_EXACT's.  Used when
- * nprobe <= 256 and d <= 256 (above 2048 lists in two tensor-core launches:
- * a bound from the first 1024 centroids, then a thresholded pass over all);
- * otherwise the exact path runs.
- * The plain and e4m3 forms always use the exact path. */
+ * error bounds, then exact FP32 scores only for the centroids that the bounds
+ * leave open; the probed lists (and the learned predictor's coarse scores) are
+ * identical to HY_COARSE_EXACT's.  Used in every form when nprobe <= 256 and
+ * there are at most 2048 lists, and above that by the bf16 form when d <= 256
+ * (in two tensor-core launches: a bound from the first 1024 centroids, then a
+ * thresholded pass over all); otherwise, and by plain searches that do not run
+ * on the tensor cores, the exact path. */
 enum { HY_COARSE_EXACT = 0, HY_COARSE_TENSOR = 1 };
 HY_API int hy_index_set_coarse(hy_index* h, int mode);
 
