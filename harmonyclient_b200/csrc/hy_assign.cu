@@ -27,8 +27,8 @@
 // shared memory and streams every centroid tile once: 512 KB per 128 rows at
 // 1024 x 128.  MMAs of N = 256 read 12 KB of shared memory in 128 cycles of
 // math; N = 128 (8 KB in 64) ran at 40 % of the tensor rate.  Measured, 1M x
-// 128 to 1024 lists (20 steps on 262,144 rows, then add): 5.4 ms here and
-// 0.9 ms of exact scores, where scoring every centroid exactly and the argmin
+// 128 to 1024 lists (20 steps on 262,144 rows, then add): 5.5 ms here and
+// 1.0 ms of exact scores, where scoring every centroid exactly and the argmin
 // took 100.6 ms; the whole build and a first search 117 -> 21.7 ms.
 #include <cuda_bf16.h>
 
