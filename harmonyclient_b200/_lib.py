@@ -101,7 +101,7 @@ def load():
     L.hy_merge_topk.argtypes = [vp, vp, sz, sz, sz, i, vp, vp, vp]
     L.hy_selftest_tcgen05_e4m3.argtypes = [vp, vp, vp]
     L.hy_selftest_tcgen05_tf32.argtypes = [vp, vp, vp]
-    L.hy_selftest_accum_units.argtypes = [i]
+    L.hy_selftest_accum_units.argtypes = [i, i]
     L.hy_selftest_accum_units.restype = C.c_double
     L.hy_selftest_wait_limit.argtypes = [H, C.c_uint]
     L.hy_index_autotune.argtypes = [H, sz, vp, sz, i, vp]

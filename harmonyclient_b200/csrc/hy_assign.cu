@@ -15,7 +15,7 @@
 // E, with r = v - hi - lo the part of a value the split drops, A the norm of
 // |hi| + |lo|, u = 2^-24 and the centroid terms at their maxima over all
 // centroids: the dropped products |x_r||c| + |x||c_r| + |x_lo||c_lo|, the f32
-// accumulation tc::accum_units(3K) u A_x A_c, twice that for L2, plus the rounding of the
+// accumulation of 3d products (tc::accum_units), twice that for L2, plus the rounding of the
 // norms, of s_c and of the exact sums: (3d + 16) u (|x|^2 + |c|^2), or
 // (d + 4) u |x||c| for inner product; all inflated by 2^-7; and 2^-17 |s| for
 // the column index that a score carries in its low mantissa bits.  Rows whose E or
@@ -61,7 +61,7 @@ struct AssignParams {
     int n, d, nlist, nkb, nbuf;  // nkb: 64-dimension blocks; nbuf: row tiles held
     int ntc, nit;                     // accumulators per row tile; 128-row tiles of the centroid image
     uint32_t wait_limit;              // polls of a wait before it gives up
-    float cK, cN;                     // accum_units(3K) u, (3d + 16) u or (d + 4) u, inflated
+    float cK, cN;                     // accum_units u, (3d + 16) u or (d + 4) u, inflated
 };
 
 // A bounded wait; one that gives up raises the status word and the abort flag,
@@ -493,7 +493,7 @@ cudaError_t launch_assign(const float* x, int n, int d, int nlist, int metric, c
     p.nit = (nlist + TM - 1) / TM;
     p.ntc = (p.nit + 1) / 2;
     const double u = 1.0 / 16777216.0, inflate = 1.0 + 1.0 / 128.0;
-    p.cK = static_cast<float>(tc::accum_units(3 * p.nkb * 64) * u * inflate);
+    p.cK = static_cast<float>(tc::accum_units(3 * d, 16) * u * inflate);
     p.cN = static_cast<float>((metric == METRIC_L2 ? 3.0 * d + 16 : d + 4.0) * u * inflate);
     const size_t smem = 1024 + static_cast<size_t>(p.nbuf) * p.nkb * 2 * KB + NSTG * 2 * KB;
     cudaError_t e = cudaMemsetAsync(w.hard_count, 0, sizeof(int32_t), s);

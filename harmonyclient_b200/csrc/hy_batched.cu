@@ -483,7 +483,7 @@ __global__ void arena_integral_kernel(const float* __restrict__ codes, int64_t n
 // Bound on |bf16 distance - exact FP32 distance| for one (query, row) pair,
 // the exact distance being the plain scan's sequential f32 sum.  With x~, q~
 // the bf16-rounded vectors: |x~.q~ - x.q| <= |x~||q - q~| + |q||x - x~|; the
-// f32 accumulation of K products adds at most cK |x~||q~| (tc::accum_units);
+// f32 accumulation of d products adds at most cK |x~||q~| (tc::accum_units);
 // the f32 norms, the final |x|^2 + |q|^2 - 2 x.q and the plain scan's own
 // d-term sum add at most cN (|x|^2 + |q|^2) (cN = (3d+16) 2^-24).  L2 doubles
 // the inner-product terms.  Both constants carry a 2^-7 inflation for the
@@ -2820,20 +2820,20 @@ cudaError_t launch_bf16_image(const ArenaLayout& L, const float* codes, int64_t 
     return cudaGetLastError();
 }
 
-// Error-bound constants for dimension d and K accumulated products (see
-// err_coef).
-static void err_consts(int d, int K, float* cK, float* cN) {
+// Error-bound constants for dimension d and n accumulated products of type op
+// (see err_coef).
+static void err_consts(Operand op, int d, int n, float* cK, float* cN) {
     const double u = 1.0 / 16777216.0, inflate = 1.0 + 1.0 / 128.0;
-    *cK = static_cast<float>(tc::accum_units(K) * u * inflate);
+    *cK = static_cast<float>(tc::accum_units(n, operand_instr(op)) * u * inflate);
     *cN = static_cast<float>((3.0 * d + 16) * u * inflate);
 }
 
 cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qaux, int nq, const BatchWork& w,
-                           int capq, int k, int metric, int d, int K, int nsm, float* thr, cudaStream_t s,
+                           int capq, int k, int metric, int d, Operand op, int nsm, float* thr, cudaStream_t s,
                            DenseFirst df) {
     df.dense_max = std::min(df.dense_max, capq);
     float cK, cN;
-    err_consts(d, K, &cK, &cN);
+    err_consts(op, d, d, &cK, &cN);
     cudaError_t e;
     if (df.dense_max > 0) {
         tighten_dense_kernel<<<(nq + 7) / 8, 256, 0, s>>>(xn, xaux, qaux, nq, w, capq, k, metric, cK, cN, thr, df);
@@ -2898,7 +2898,7 @@ cudaError_t launch_coarse_refine(float2* cand, int nq, int nlist, const float* q
                                  bool ordered, const int32_t* counts, int64_t* out_idx, float* out_score, int* err,
                                  cudaStream_t s) {
     float cK, cN;
-    err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
+    err_consts(Operand::bf16, d, 2 * d, &cK, &cN);  // the split centroid image: hi and lo products
     int warps = 4;
     while (warps > 1 && coarse_refine_smem(nlist, d, warps) > 200 * 1024) warps >>= 1;
     const size_t smem = coarse_refine_smem(nlist, d, warps);
@@ -2922,7 +2922,7 @@ cudaError_t launch_coarse_thr(const float2* cand, int nq, int S, int m, const fl
                               cudaStream_t s) {
     if (S > 1024 || m > S) return cudaErrorInvalidValue;
     float cK, cN;
-    err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
+    err_consts(Operand::bf16, d, 2 * d, &cK, &cN);  // the split centroid image: hi and lo products
     coarse_thr_kernel<<<(nq + 7) / 8, 256, 0, s>>>(cand, nq, S, m, cxn, caux, qaux, metric, cK, cN, counts, thr);
     return cudaGetLastError();
 }
@@ -2936,7 +2936,7 @@ cudaError_t launch_coarse_refine_keys(uint64_t* cand, const int32_t* ccnt, int n
     const size_t smem = coarse_refine_smem(0, d, warps);
     if (smem > 200 * 1024 || m > 256 || (out_score && (!ordered || counts))) return cudaErrorInvalidValue;
     float cK, cN;
-    err_consts(d, (d + 63) / 64 * 128, &cK, &cN);  // the split centroid image: hi and lo products
+    err_consts(Operand::bf16, d, 2 * d, &cK, &cN);  // the split centroid image: hi and lo products
     const dim3 grid((nq + warps - 1) / warps);
     auto run = [&](auto kern) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -3105,7 +3105,7 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
     p.metric = b.metric;
     p.dense_max = std::min(b.dense_max, b.capq);
     p.xaux = b.xaux;
-    err_consts(b.d, operand_k(b.op, p.nkb), &p.cK, &p.cN);
+    err_consts(b.op, b.d, b.ksplit ? 2 * b.d : b.d, &p.cK, &p.cN);
     auto run = [&](auto qg, auto wide) -> cudaError_t {
         constexpr int QG = decltype(qg)::value;
         constexpr bool WIDE = decltype(wide)::value;
@@ -3131,10 +3131,10 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
 
 cudaError_t launch_rerank(const ArenaLayout& L, const float* codes, const int64_t* ids, const float* xn,
                           const float2* xaux, const float4* qaux, const float* q, int nq, const BatchWork& w, int qbase,
-                          int capq, int k, int rmax, int metric, int K, int nsm, float* D, int64_t* I,
+                          int capq, int k, int rmax, int metric, Operand op, int nsm, float* D, int64_t* I,
                           cudaStream_t s, const int32_t* qexact) {
     float cK, cN;
-    err_consts(L.d, K, &cK, &cN);
+    err_consts(op, L.d, L.d, &cK, &cN);
     cudaError_t e;
     const size_t wsmem = static_cast<size_t>(8) * (256 * sizeof(uint64_t) + L.row_pitch * sizeof(float));
     if ((e = cudaFuncSetAttribute(rerank_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -28,11 +28,11 @@ inline size_t f8_image_bytes(int64_t rows, int d) {
 // Operand type of a batched launch: the bf16 image, the e4m3 image or the FP32
 // arena itself read as TF32.
 enum class Operand { bf16, e4m3, tf32 };
-// 128-byte k-blocks of a row, and the products nkb of them accumulate.
+// 128-byte k-blocks of a row, and dimensions one MMA instruction takes.
 inline int operand_kblocks(Operand op, const ArenaLayout& L) {
     return op == Operand::bf16 ? (L.d + 63) / 64 : op == Operand::e4m3 ? (L.d + 127) / 128 : L.row_pitch / 32;
 }
-inline int operand_k(Operand op, int nkb) { return nkb * (op == Operand::bf16 ? 64 : op == Operand::e4m3 ? 128 : 32); }
+inline int operand_instr(Operand op) { return op == Operand::bf16 ? 16 : op == Operand::e4m3 ? 32 : 8; }
 
 // Queries per group of the batched kernel for rows of nkb k-blocks (128, 64 or
 // 32: the largest whose shared-memory footprint fits), 0 if none fits.
@@ -121,7 +121,7 @@ struct DenseFirst {
 // thr := min(thr, k-th smallest upper bound over each query's candidates),
 // and the candidates that can still reach the top-k are compacted as keys.
 cudaError_t launch_tighten(const float* xn, const float2* xaux, const float4* qaux, int nq, const BatchWork& w,
-                           int capq, int k, int metric, int d, int K, int nsm, float* thr, cudaStream_t s,
+                           int capq, int k, int metric, int d, Operand op, int nsm, float* thr, cudaStream_t s,
                            DenseFirst df);
 
 // The coarse quantiser on the tensor cores.  The centroids
@@ -211,7 +211,7 @@ cudaError_t launch_batched_scan(const BatchedLaunch& b, const BatchWork& w, int*
 // whose tensor-core distances are exact keep them instead of recomputing.
 cudaError_t launch_rerank(const ArenaLayout& L, const float* codes, const int64_t* ids, const float* xn,
                           const float2* xaux, const float4* qaux, const float* q, int nq, const BatchWork& w, int qbase,
-                          int capq, int k, int rmax, int metric, int K, int nsm, float* D, int64_t* I,
+                          int capq, int k, int rmax, int metric, Operand op, int nsm, float* D, int64_t* I,
                           cudaStream_t s, const int32_t* qexact = nullptr);
 cudaError_t launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s);
 

@@ -1374,7 +1374,6 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     qc = std::min(qc, n);
     const bool f8 = op == hy::Operand::e4m3, tf32 = op == hy::Operand::tf32;
     const size_t nkb = (size_t)hy::operand_kblocks(op, h->L);  // 128-byte k-blocks per row
-    const int K = hy::operand_k(op, (int)nkb);
     const float2* xaux = (f8 ? h->x8aux : tf32 ? h->x32aux : h->xaux).as<float2>();
     const float2* taux = (f8 ? h->t8aux : tf32 ? h->t32aux : h->taux).as<float2>();
     const int qg = hy::batched_group_size((int)nkb);
@@ -1595,7 +1594,7 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
         df.tile_aux = taux;
         df.tile_xn = h->txn.as<float>();
         HY_CUDA(hy::launch_tighten(h->norms.as<float>(), xaux, h->b_qn.as<float4>(), (int)m, w, (int)capq, (int)k,
-                                   h->metric, (int)h->d, K, h->nsm, h->b_thr.as<float>(), s, df));
+                                   h->metric, (int)h->d, op, h->nsm, h->b_thr.as<float>(), s, df));
         if (nprobe > 1) {
             w.pair_cnt = zero + z_pc2;
             w.work = work + 1;
@@ -1611,7 +1610,7 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[3], s));
         const int rmax = f8 ? (int)std::min<size_t>(h->oversample * k, 4096) : 0;
         HY_CUDA(hy::launch_rerank(h->L, h->codes.as<float>(), h->ids.as<int64_t>(), h->norms.as<float>(), xaux,
-                                  h->b_qn.as<float4>(), qq, (int)m, w, 0, (int)capq, (int)k, rmax, h->metric, K,
+                                  h->b_qn.as<float4>(), qq, (int)m, w, 0, (int)capq, (int)k, rmax, h->metric, op,
                                   h->nsm, dD + q0 * k, dI + q0 * k, s, f8 ? nullptr : h->b_qx.as<int32_t>()));
         if (timed && q0 + qc >= n) HY_CUDA(ev_record(h->ev[4], s));
         const int fb = (int)std::min<size_t>(m, fbcap);

@@ -143,4 +143,4 @@ extern "C" int hy_selftest_tcgen05_tf32(const float* A, const float* B, float* D
     return run_selftest<hy::Op::tf32>(A, B, D);
 }
 
-extern "C" double hy_selftest_accum_units(int K) { return hy::tc::accum_units(K); }
+extern "C" double hy_selftest_accum_units(int n, int G) { return hy::tc::accum_units(n, G); }

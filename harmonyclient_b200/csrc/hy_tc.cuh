@@ -35,16 +35,18 @@ __device__ inline uint64_t sdesc_sw128(uint32_t smem_addr) {
     return d;
 }
 
-// Bound on the error that the tensor cores' f32 accumulation of K products
-// adds to an inner product, in units of 2^-24 |x||q|.  How tcgen05.mma rounds is not
-// documented, so no rounding is assumed: an instruction of G products (G = 8
-// tf32, 16 bf16, 32 e4m3) takes them and the accumulator as terms aligned to
-// the largest, each cut off at 24 bits, and cuts the sum off again: G + 2
-// errors of at most 2^-23 of the largest term or the sum, neither above
-// |x||q|, for each of K / G instructions, at most 2.5 K 2^-24 in all.
-// (Measured where it should be worst, one large product and K - 1 that lie just
-// above the cut: bf16 50 at K 128, e4m3 100 at K 256.)
-__host__ __device__ constexpr double accum_units(int K) { return 2.5 * K + 16.0; }
+// Bound on the error that the tensor cores' f32 accumulation of n products
+// adds to an inner product, in units of 2^-24 |x||q|; G products an instruction
+// (8 tf32, 16 bf16, 32 e4m3).  How tcgen05.mma rounds is not documented, so no
+// rounding is assumed: an instruction takes its products and the accumulator as
+// terms aligned to the largest, each cut off at 24 bits, and cuts the sum off
+// again, errors of at most 2^-23 of the largest term or the sum, neither above
+// |x||q|: n for the products and two for each instruction with any, n / G and up
+// to eight more where blocks of dimensions end.  (Zeros that fill a k-block add
+// exactly.)
+// (Measured where it should be worst, one large product and n - 1 that lie just
+// above the cut: bf16 50 at n 128, e4m3 100 at n 256.)
+__host__ __device__ constexpr double accum_units(int n, int G) { return 2.0 * (n + 2.0 * (n / static_cast<double>(G) + 8.0)); }
 
 // True in one lane of a converged warp.  Instructions that one thread issues
 // (MMAs, bulk copies, commits) go under it, with the loop and the waits around

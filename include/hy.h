@@ -382,9 +382,9 @@ HY_API int hy_selftest_tcgen05_e4m3(const float* A, const float* B, float* D);
 /* The same on tf32 operands: A and B are 128 x 64 (the low 13 bits of a value
  * do not take part), accumulated by kind::tf32. */
 HY_API int hy_selftest_tcgen05_tf32(const float* A, const float* B, float* D);
-/* The bound that the searches keep for the accumulation of K such products, in
- * units of 2^-24 |a||b|. */
-HY_API double hy_selftest_accum_units(int K);
+/* The bound that the searches keep for the accumulation of n such products, G an
+ * instruction (8 tf32, 16 bf16, 32 e4m3), in units of 2^-24 |a||b|. */
+HY_API double hy_selftest_accum_units(int n, int G);
 
 /* Diagnostic with no counterpart in the reference: the polls after which a
  * bounded device-side wait of the handle's tensor-core row assignment gives up

@@ -48,7 +48,7 @@ def _cases(K, rng):
 
 @pytest.mark.parametrize("G,K", [(8, 64), (8, 384), (16, 64), (16, 768), (32, 128), (32, 1536)])
 def test_bound_holds_for_an_accumulator_that_cuts_off(G, K):
-    bound = _lib.load().hy_selftest_accum_units(K)
+    bound = _lib.load().hy_selftest_accum_units(K, G)
     worst = 0.0
     for a, b in _cases(K, np.random.default_rng(K)):
         a, b = a.astype(np.float16).astype(np.float64), b.astype(np.float16).astype(np.float64)  # exact products
@@ -58,9 +58,22 @@ def test_bound_holds_for_an_accumulator_that_cuts_off(G, K):
     assert worst > K + 8  # the bound of K rounded additions would not do
 
 
+@pytest.mark.parametrize("d", [5, 33, 100])
+def test_zeros_that_fill_a_block_add_exactly(d):
+    """Eight blocks of d dimensions, each filled up to whole instructions."""
+    G, w = 8, -(-d // 8) * 8
+    bound = _lib.load().hy_selftest_accum_units(8 * d, G)
+    for a, b in _cases(8 * d, np.random.default_rng(d)):
+        a, b = a.astype(np.float16).astype(np.float64), b.astype(np.float16).astype(np.float64)
+        p = np.zeros((8, w))
+        p[:, :d] = (a * b).reshape(8, d)
+        err = abs(_accumulate(list(p.reshape(-1)), G) - math.fsum(a * b))
+        assert err <= bound * U * np.linalg.norm(a) * np.linalg.norm(b)
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("op,K", [("", 128), ("_e4m3", 256), ("_tf32", 64)])
-def test_bound_holds_on_the_tensor_cores(op, K):
+@pytest.mark.parametrize("op,K,G", [("", 128, 16), ("_e4m3", 256, 32), ("_tf32", 64, 8)])
+def test_bound_holds_on_the_tensor_cores(op, K, G):
     L = _lib.load()
     rng = np.random.default_rng(1)
     scale = 2.0 ** 6 if op == "_e4m3" else 1.0
@@ -82,4 +95,4 @@ def test_bound_holds_on_the_tensor_cores(op, K):
     err = np.abs(D - A.astype(np.float64) @ B.astype(np.float64).T)
     norm = np.linalg.norm(A.astype(np.float64), axis=1)[:, None] * np.linalg.norm(B.astype(np.float64), axis=1)
     n = len(rows)
-    assert (err[:n, :n] / norm[:n, :n]).max() / U <= L.hy_selftest_accum_units(K)
+    assert (err[:n, :n] / norm[:n, :n]).max() / U <= L.hy_selftest_accum_units(K, G)
