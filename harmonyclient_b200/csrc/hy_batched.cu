@@ -890,8 +890,11 @@ __device__ inline bool wait_or_abort(uint64_t* bar, uint32_t parity, const Batch
     return (p.wait_limit && mbar_try_wait(bar, parity)) || wait_polls(bar, parity, p.wait_limit, p.err, abort);
 }
 
-// Barrier over `nthreads` threads (a multiple of 32) on hardware barrier `id`:
-// whether any of them has `flag`.
+// Barrier over `nthreads` threads (a multiple of 32) on hardware barrier `id`.
+__device__ inline void named_sync(int id, int nthreads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// The same, and whether any of them has `flag`.
 __device__ inline bool named_any(int id, int nthreads, bool flag) {
     uint32_t any;
     __syncwarp();
@@ -1070,12 +1073,11 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1) batched_scan_kernel(const __
             // asynchronous copy, eight lanes to a 128-byte row so that a
             // warp reads whole rows, all in flight at once; empty query slots
             // are zero-filled.
+            named_sync(1, 32 * N_GATHER);  // S.qid
             const int bb = static_cast<int>(it % nbuf);
-            const bool bok = wait_or_abort(&bfree[bb], ((it / nbuf) & 1u) ^ 1u, p, vabort);
-            if (named_any(1, 32 * N_GATHER, !bok)) {  // (and S.qid is written)
-                cp_async_wait_all();
-                break;
-            }
+            // (If the wait gives up, the queries are copied all the same and
+            // the gather leaves, together, at its next item.)
+            wait_or_abort(&bfree[bb], ((it / nbuf) & 1u) ^ 1u, p, vabort);
             unsigned char* dst = sB + static_cast<size_t>(bb) * nkbq * BKB;
             const size_t qstride = static_cast<size_t>(nkbq) * 128;
             const int c = gt & 7;
