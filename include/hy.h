@@ -241,7 +241,12 @@ HY_API int hy_index_presearch(hy_index* h, size_t warmup_list, size_t warmup_lis
 /* Search.  Replaces Index::search (src/Index.cpp:1638-1706): D and I are n x k
  * row-major; each row is sorted best first (ascending L2, descending IP);
  * unfilled entries hold FLT_MAX (L2) / -FLT_MAX (IP) and id -1
- * (src/heap.hpp:13-25). */
+ * (src/heap.hpp:13-25).
+ * A device-pointer search may be recorded by the caller's own stream capture
+ * once the same search has run outside it (nothing may be allocated in a
+ * capture).  That graph holds the handle's workspaces: a call that needs larger
+ * ones, or an add, load or train, may move them, and the search has to be
+ * captured again before the next replay (hy_index_set_graph does so itself). */
 HY_API int hy_index_search(hy_index* h, size_t n, const float* q, size_t k, float* D, int64_t* I);
 HY_API int hy_index_search_device(hy_index* h, size_t n, const float* dq, size_t k, float* dD, int64_t* dI,
                                   void* stream);
@@ -273,7 +278,8 @@ HY_API int hy_merge_topk(const float* dD, const int64_t* dI, size_t parts, size_
  * state runs normally and captures its launch sequence (coarse quantisation,
  * probe network, warm-up, the persistent batched scan, re-rank, fallback) in
  * a CUDA graph; identical later calls replay it with one launch.  Any call
- * that changes the index or its parameters retires the graph. */
+ * that changes the index or its parameters, or makes one of the handle's
+ * workspaces grow, retires the graph. */
 HY_API int hy_index_set_graph(hy_index* h, int enabled);
 
 /* Search with a per-query nprobe (no counterpart in the reference, whose
