@@ -1232,8 +1232,14 @@ void release_batch_buffers(hy_index* h) {
 // 2048 lists only the bf16 form to 256 dimensions does, as it did before the other
 // forms and wider rows were taken up to there; the two-launch step is not tested on
 // those, though it would be faster (10,000 queries, 4096 lists, nprobe 64, us: plain
-// 1M x 128 886 here, 705 there; e4m3 894 / 715; bf16 400k x 420 2,319 / 819).
-bool coarse_on_tensor(const hy_index* h, size_t nprobe) {
+// 1M x 128 886 here, 705 there; e4m3 894 / 715; bf16 400k x 420 2,319 / 819).  Below
+// COARSE_TENSOR_MIN queries x centroids x dimensions the others' FP32 step is ahead
+// of three more launches (whole search, us, tensor / FP32: e4m3 200k x 16, 512 lists,
+// 2,000 queries 353 / 319; x 64, 2048 lists, 2,000 queries even; plain 200k x 64, 512
+// lists, 2,000 queries 330 / 303).
+constexpr size_t COARSE_TENSOR_MIN = 250000000;
+bool coarse_on_tensor(const hy_index* h, size_t m, size_t nprobe) {
+    if (h->form != HY_FORM_BF16 && m * h->nlist * h->d < COARSE_TENSOR_MIN) return false;
     return h->coarse_mode == HY_COARSE_TENSOR && nprobe <= 256 && (h->d <= 256 || h->nlist <= 2048) &&
            (h->form == HY_FORM_BF16 || h->nlist <= 2048) && hy::batched_group_size((int)(h->d + 63) / 64) > 0;
 }
@@ -1377,7 +1383,7 @@ int search_tensor_impl(hy_index* h, hy::Operand op, size_t n, const float* dq, s
     const float2* xaux = (f8 ? h->x8aux : tf32 ? h->x32aux : h->xaux).as<float2>();
     const float2* taux = (f8 ? h->t8aux : tf32 ? h->t32aux : h->taux).as<float2>();
     const int qg = hy::batched_group_size((int)nkb);
-    const bool coarse_tc = coarse_on_tensor(h, nprobe);
+    const bool coarse_tc = coarse_on_tensor(h, qc, nprobe);
     HY_CHECK(qg > 0, HY_ERR_ARG, "search: d too large for the tensor-core form");
     const size_t nlist = h->nlist;
     HY_RET(h->w_scores.ensure(qc * nlist * sizeof(float)));
@@ -2588,7 +2594,7 @@ int hy_index_probes(hy_index* h, size_t n, const float* q, int64_t* probes) {
         HY_RET(h->m_total.ensure(sizeof(unsigned long long)));
     }
     HY_CUDA(cudaMemcpyAsync(h->w_q.p, q, n * h->d * sizeof(float), cudaMemcpyHostToDevice, s));
-    const bool tensor = coarse_on_tensor(h, nprobe);
+    const bool tensor = coarse_on_tensor(h, qc, nprobe);
     if (tensor) {
         HY_RET(ensure_common(h));
         if (h->nsm == 0) HY_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));

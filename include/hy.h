@@ -223,8 +223,9 @@ HY_API int hy_index_set_group_size(hy_index* h, int qg);
  * HY_COARSE_TENSOR (default): bf16 tensor-core scores of every centroid with
  * error bounds, then exact FP32 scores only for the centroids that the bounds
  * leave open; the probed lists (and the learned predictor's coarse scores) are
- * identical to HY_COARSE_EXACT's.  Used in every form when nprobe <= 256 and
- * there are at most 2048 lists, and above that by the bf16 form when d <= 256
+ * identical to HY_COARSE_EXACT's.  Used when nprobe <= 256 and there are at most
+ * 2048 lists (in the plain and e4m3 forms from 250 million queries x lists x
+ * dimensions), and above that by the bf16 form when d <= 256
  * (in two tensor-core launches: a bound from the first 1024 centroids, then a
  * thresholded pass over all); otherwise, and by plain searches that do not run
  * on the tensor cores, the exact path. */

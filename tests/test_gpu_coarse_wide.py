@@ -55,3 +55,26 @@ def test_search_in_every_form(form):
     Dt, It = idx.search(q, 10)
     np.testing.assert_array_equal(It, I)
     np.testing.assert_array_equal(Dt, D)
+
+
+@pytest.mark.parametrize("form", ["plain", "fp8", "bf16"])
+@pytest.mark.parametrize("nq,tensor", [(1_907, False), (1_908, True)])
+def test_small_batches_of_the_other_forms_keep_the_exact_step(form, nq, tensor):
+    """2048 lists x 64 dimensions: from 250 million products the plain and e4m3
+    forms score on the tensor cores too (the bf16 form always does)."""
+    rng = np.random.default_rng(9)
+    c = rng.uniform(-1, 1, (2048, 64)).astype(np.float32)
+    x = (c[rng.integers(0, 2048, 60_000)] + 0.3 * rng.standard_normal((60_000, 64))).astype(np.float32)
+    q = (c[rng.integers(0, 2048, nq)] + 0.3 * rng.standard_normal((nq, 64))).astype(np.float32)
+    idx = hb.Index(64, 2048, 128)
+    idx.centroid_codes = c
+    idx.add(x)
+    idx.set_form(form)
+    out, launches = {}, {}
+    for mode in ("exact", "tensor"):
+        idx.set_coarse(mode)
+        out[mode] = idx.search(q, 10)
+        launches[mode] = idx.last_stats()["launches"]
+    for a, b in zip(out["exact"], out["tensor"]):
+        np.testing.assert_array_equal(a, b)
+    assert (launches["exact"] != launches["tensor"]) == (tensor or form == "bf16")
